@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "../../include/b200_mixers.h"
+#include "b200_column_scan.cuh"
 #include "b200_common.cuh"
 
 namespace b200 {
@@ -1092,191 +1093,6 @@ causal_conv_silu_kernel(T* __restrict__ out, int64_t out_stride, const T* __rest
   }
 }
 
-// ---- gated delta rule --------------------------------------------------------------------------------------------
-// One CTA per (sequence, head, 32 value columns): a value column's part of the state never meets another column's, so
-// columns are independent.  Four adjacent lanes share a column; lane r keeps the state rows i = r, r + 4, ... of that
-// column in registers for the whole portion.  Eight tokens (fewer for the widest keys) are staged at a time, double buffered (the raw loads of
-// the next eight are issued before the current eight are computed): their activated q and k (unit length per head, q
-// also scaled), the decays g = exp(-exp(A_log) softplus(a + dt_bias)), the write strength sigmoid(b) and the CTA's
-// value columns (the decays as g - 1, so that one just below 1 is not rounded alike token after token).  Per token: S <- g S and d = S^T k in one pass, u = beta (v - d), then S <- S + k u and
-// o = S^T q in a second pass; the four lanes' partial sums meet in two shuffles.
-constexpr int kDeltaNT = 128;
-constexpr int kDeltaCols = kDeltaNT / 4;
-
-struct DeltaArgs {
-  float* o_raw;
-  const void* q; const void* k; const void* v; int64_t in_stride;
-  const void* beta; int64_t beta_stride;
-  const void* a; int64_t a_stride;
-  const void* dt_bias; const void* a_log;
-  float* state; const SeqSpan* seqs;
-  int H, G, dk, dv; float unit_eps, q_scale;
-  int per_channel;   // 1: a decay logit and a bias per key channel, 0: one of each per head
-};
-
-__host__ __device__ constexpr int delta_chunk(int dk_padded) { return dk_padded >= 256 ? 2 : (dk_padded >= 128 ? 4 : 8); }
-
-template <typename T, int DK>
-__global__ void __launch_bounds__(kDeltaNT)
-delta_scan_kernel(const DeltaArgs A) {
-  extern __shared__ __align__(16) float smem[];
-  constexpr int RW4 = DK / 4;
-  constexpr int kDeltaChunk = delta_chunk(DK);
-  constexpr int row_len = 3 * DK + kDeltaCols + 4;      // q | k | g (each grouped by r) | v[32] | beta, pad
-  constexpr int kPer = (kDeltaChunk * row_len + kDeltaNT - 1) / kDeltaNT;   // staged elements per thread and chunk
-  const SeqSpan sq = A.seqs[blockIdx.x];
-  const int h = blockIdx.y, H = A.H, dk = A.dk, dv = A.dv;
-  const int gq = h / (H / A.G);                          // the q / k head this value head reads
-  const int r = threadIdx.x & 3, cl = threadIdx.x >> 2;
-  const int col0 = blockIdx.z * kDeltaCols, col = col0 + cl;
-  const int ncol = min(kDeltaCols, dv - col0);
-  const bool has_col = col < dv;
-  float* st = A.state + (static_cast<int64_t>(sq.slot) * H + h) * dk * dv;
-  float S[RW4];
-#pragma unroll
-  for (int kk = 0; kk < RW4; ++kk) {
-    const int i = 4 * kk + r;
-    S[kk] = (!sq.fresh && i < dk && has_col) ? st[static_cast<int64_t>(i) * dv + col] : 0.f;
-  }
-  const T* qp = static_cast<const T*>(A.q);
-  const T* kp = static_cast<const T*>(A.k);
-  const T* vp = static_cast<const T*>(A.v);
-  const T* bp = static_cast<const T*>(A.beta);
-  const T* ap = static_cast<const T*>(A.a);
-  const T* dtb = static_cast<const T*>(A.dt_bias);
-  const float a_rate = expf(Cvt<T>::to_f32(static_cast<const T*>(A.a_log)[h]));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* buf0 = smem;
-  float* buf1 = smem + kDeltaChunk * row_len;
-  T rawv[kPer];
-  // staged element e of a chunk: token e / row_len, slot e % row_len; slot r * RW4 + kk of a section holds row 4 kk + r.
-  // `fetch` only issues the loads (nothing waits for them until `commit`), so they fly while a chunk is computed.
-  auto fetch = [&](int t0) {
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int e = threadIdx.x + u * kDeltaNT;
-      const int tt = e / row_len, sl = e - tt * row_len;
-      rawv[u] = Cvt<T>::from_f32(0.f);
-      if (tt < kDeltaChunk && t0 + tt < sq.count) {
-        const int64_t tok = sq.tok0 + t0 + tt;
-        if (sl < 3 * DK) {
-          const int which = sl / DK, s2 = sl - which * DK;
-          const int i = 4 * (s2 % RW4) + s2 / RW4;
-          if (i < dk) {
-            if (which == 0) rawv[u] = qp[tok * A.in_stride + gq * dk + i];
-            else if (which == 1) rawv[u] = kp[tok * A.in_stride + gq * dk + i];
-            else rawv[u] = ap[tok * A.a_stride + (A.per_channel ? h * dk + i : h)];
-          }
-        } else if (sl < 3 * DK + kDeltaCols) {
-          if (sl - 3 * DK < ncol) rawv[u] = vp[tok * A.in_stride + h * dv + col0 + sl - 3 * DK];
-        } else if (sl == 3 * DK + kDeltaCols) {
-          rawv[u] = bp[tok * A.beta_stride + h];
-        }
-      }
-    }
-  };
-  auto commit = [&](float* dst, int n_valid) {
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int e = threadIdx.x + u * kDeltaNT;
-      const int tt = e / row_len, sl = e - tt * row_len;
-      if (tt < n_valid) {
-        float val = Cvt<T>::to_f32(rawv[u]);
-        if (sl >= 2 * DK && sl < 3 * DK) {
-          const int s2 = sl - 2 * DK;
-          const int i = 4 * (s2 % RW4) + s2 / RW4;
-          val = i < dk ? expm1f(-a_rate * softplus_(val + Cvt<T>::to_f32(dtb[A.per_channel ? h * dk + i : h]))) : 0.f;
-        } else if (sl == 3 * DK + kDeltaCols) {
-          val = sigmoid_(val);
-        }
-        dst[e] = val;
-      }
-    }
-  };
-  auto unit = [&](float* dst, int n_valid) {   // warp w brings tokens w, w + 4, ... to unit length per head
-    for (int tt = warp; tt < n_valid; tt += kDeltaNT / 32) {
-      float* row = dst + tt * row_len;
-      float sq2 = 0.f, sk2 = 0.f;
-      for (int i = lane; i < DK; i += 32) {
-        sq2 = fmaf(row[i], row[i], sq2);
-        sk2 = fmaf(row[DK + i], row[DK + i], sk2);
-      }
-      const float iq = rsqrtf(warp_sum(sq2) + A.unit_eps) * A.q_scale;
-      const float ik = rsqrtf(warp_sum(sk2) + A.unit_eps);
-      for (int i = lane; i < DK; i += 32) {
-        row[i] *= iq;
-        row[DK + i] *= ik;
-      }
-    }
-  };
-  fetch(0);
-  commit(buf0, min(kDeltaChunk, sq.count));
-  __syncthreads();
-  unit(buf0, min(kDeltaChunk, sq.count));
-  __syncthreads();
-  for (int t0 = 0; t0 < sq.count; t0 += kDeltaChunk) {
-    const float* cur = ((t0 / kDeltaChunk) & 1) ? buf1 : buf0;
-    float* nxt = ((t0 / kDeltaChunk) & 1) ? buf0 : buf1;
-    const int n_here = min(kDeltaChunk, sq.count - t0);
-    const int n_next = min(kDeltaChunk, sq.count - t0 - kDeltaChunk);
-    if (n_next > 0) fetch(t0 + kDeltaChunk);
-    for (int tt = 0; tt < n_here; ++tt) {
-      const float* row = cur + tt * row_len;
-      const float* qr = row + r * RW4;
-      const float* kr = row + DK + r * RW4;
-      const float* gr = row + 2 * DK + r * RW4;
-      const float vc = row[3 * DK + cl], beta = row[3 * DK + kDeltaCols];
-      float d0 = 0.f, d1 = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < RW4; kk += 4) {
-        const float4 g4 = *reinterpret_cast<const float4*>(gr + kk);
-        const float4 k4 = *reinterpret_cast<const float4*>(kr + kk);
-        S[kk] = fmaf(g4.x, S[kk], S[kk]);
-        d0 = fmaf(S[kk], k4.x, d0);
-        S[kk + 1] = fmaf(g4.y, S[kk + 1], S[kk + 1]);
-        d1 = fmaf(S[kk + 1], k4.y, d1);
-        S[kk + 2] = fmaf(g4.z, S[kk + 2], S[kk + 2]);
-        d0 = fmaf(S[kk + 2], k4.z, d0);
-        S[kk + 3] = fmaf(g4.w, S[kk + 3], S[kk + 3]);
-        d1 = fmaf(S[kk + 3], k4.w, d1);
-      }
-      float d = d0 + d1;
-      d += __shfl_xor_sync(0xffffffffu, d, 1);
-      d += __shfl_xor_sync(0xffffffffu, d, 2);
-      const float u = beta * (vc - d);
-      float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < RW4; kk += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kr + kk);
-        const float4 q4 = *reinterpret_cast<const float4*>(qr + kk);
-        S[kk] = fmaf(k4.x, u, S[kk]);
-        o0 = fmaf(S[kk], q4.x, o0);
-        S[kk + 1] = fmaf(k4.y, u, S[kk + 1]);
-        o1 = fmaf(S[kk + 1], q4.y, o1);
-        S[kk + 2] = fmaf(k4.z, u, S[kk + 2]);
-        o0 = fmaf(S[kk + 2], q4.z, o0);
-        S[kk + 3] = fmaf(k4.w, u, S[kk + 3]);
-        o1 = fmaf(S[kk + 3], q4.w, o1);
-      }
-      float o = o0 + o1;
-      o += __shfl_xor_sync(0xffffffffu, o, 1);
-      o += __shfl_xor_sync(0xffffffffu, o, 2);
-      if (r == 0 && has_col) A.o_raw[(static_cast<int64_t>(sq.tok0 + t0 + tt) * H + h) * dv + col] = o;
-    }
-    if (n_next > 0) {
-      commit(nxt, n_next);       // `nxt` was last read two chunks ago, before the barrier that ended that chunk
-      __syncthreads();
-      unit(nxt, n_next);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int kk = 0; kk < RW4; ++kk) {
-    const int i = 4 * kk + r;
-    if (i < dk && has_col) st[static_cast<int64_t>(i) * dv + col] = S[kk];
-  }
-}
-
 // ---- o * rsqrt(mean(o^2) + eps) * w * sigmoid(gate); one warp per (token, head) ------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -1649,24 +1465,8 @@ int b200_delta_scan_ext(float* o_raw, const void* q, const void* k, const void* 
   if (n_seqs == 0) return 0;
   if (!o_raw || !q || !k || !v || !beta_logit || !a_logit || !dt_bias || !a_log || !state || !seqs)
     return fail(B200_EINVAL, "b200_delta_scan: null pointer");
-  const int dkt = dk <= 32 ? 32 : (dk <= 64 ? 64 : (dk <= 128 ? 128 : 256));
-  const size_t smem = sizeof(float) * 2 * delta_chunk(dkt) * (3 * static_cast<size_t>(dkt) + kDeltaCols + 4);
-  const dim3 grid(n_seqs, H, (dv + kDeltaCols - 1) / kDeltaCols);
-  DeltaArgs A{o_raw, q, k, v, in_stride, beta_logit, beta_stride, a_logit, a_stride, dt_bias, a_log, state,
-              reinterpret_cast<const SeqSpan*>(seqs), H, G, dk, dv, unit_eps, q_scale, per_channel};
-  return hybrid_by_dtype(dtype, "b200_delta_scan", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    auto s = static_cast<cudaStream_t>(stream);
-    auto launch = [&](auto kern) {
-      if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      kern<<<grid, kDeltaNT, smem, s>>>(A);
-    };
-    if (dkt == 32) launch(delta_scan_kernel<T, 32>);
-    else if (dkt == 64) launch(delta_scan_kernel<T, 64>);
-    else if (dkt == 128) launch(delta_scan_kernel<T, 128>);
-    else launch(delta_scan_kernel<T, 256>);
-    return check_launch("b200_delta_scan");
-  });
+  return delta_column_scan(o_raw, ScanRows{q, k, v, in_stride}, beta_logit, beta_stride, a_logit, a_stride, dt_bias, a_log, per_channel != 0,
+                           state, seqs, ScanShape{n_seqs, H, G, dk, dv}, unit_eps, q_scale, dtype, static_cast<cudaStream_t>(stream));
 }
 
 int b200_head_rmsnorm_gated(void* out, const float* x, const void* weight, const void* gate, int64_t gate_stride, float eps,

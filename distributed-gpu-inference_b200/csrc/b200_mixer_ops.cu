@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "../../include/b200_mixers.h"
+#include "b200_column_scan.cuh"
 #include "b200_common.cuh"
 
 namespace b200 {
@@ -751,248 +752,7 @@ grouped_linear_kernel(T* __restrict__ out, const T* __restrict__ xs, const T* __
   }
 }
 
-// ---- gated linear recurrence ------------------------------------------------------------------------------------
-// One CTA per (sequence, head).  The state [dk][dv] lives in shared memory for the whole portion; thread (rg, c)
-// owns column c and the rows i = rg, rg + RG, ...  Inputs of token t + 1 are fetched while token t is computed.
-struct ScanSeq {
-  int tok0;   // first packed row
-  int count;  // tokens of this sequence in the step
-  int slot;   // state slot
-  int fresh;  // 1: the sequence starts here, the state is zero
-};
-
-constexpr int kScanCols = 32;   // value columns per CTA (fixed, so the row-sum order never depends on the batch)
-constexpr int kScanRG = 256 / kScanCols;
-constexpr int kScanPF = 4;      // input elements per thread and token: 2 dk + 32 <= 1024
-
-template <typename T>
-__global__ void __launch_bounds__(256)
-gated_scan_kernel(float* __restrict__ o_raw, const T* __restrict__ zq, const T* __restrict__ zf, const T* __restrict__ v,
-                  int64_t in_stride, const T* __restrict__ f_bias, const T* __restrict__ lower, float* __restrict__ state,
-                  const ScanSeq* __restrict__ seqs, int H, int dk, int dv) {
-  extern __shared__ float smem[];
-  const ScanSeq sq = seqs[blockIdx.x];
-  const int h = blockIdx.y;
-  const int col0 = blockIdx.z * kScanCols;
-  const int ncol = min(kScanCols, dv - col0);
-  const int c = threadIdx.x % kScanCols, rg = threadIdx.x / kScanCols;
-  float* S = smem;                              // [dk][kScanCols]
-  float* in_s = S + dk * kScanCols;             // 2 x (q[dk], f[dk], v[kScanCols])
-  const int in_len = 2 * dk + kScanCols;
-  float* part = in_s + 2 * in_len;              // [kScanRG][kScanCols]
-  float* st = state + (static_cast<int64_t>(sq.slot) * H + h) * dk * dv;
-  for (int i = threadIdx.x; i < dk * kScanCols; i += blockDim.x) {
-    const int r = i / kScanCols, cc = i - r * kScanCols;
-    S[i] = (sq.fresh || cc >= ncol) ? 0.f : st[r * dv + col0 + cc];
-  }
-  // element i of a token's inputs is always handled by thread i % 256: its bias / bound are loaded once
-  float bias_r[kScanPF], low_r[kScanPF];
-#pragma unroll
-  for (int u = 0; u < kScanPF; ++u) {
-    const int i = threadIdx.x + u * 256;
-    bias_r[u] = low_r[u] = 0.f;
-    if (i >= dk && i < 2 * dk) {
-      bias_r[u] = Cvt<T>::to_f32(f_bias[h * dk + i - dk]);
-      low_r[u] = Cvt<T>::to_f32(lower[h * dk + i - dk]);
-    }
-  }
-  T raw[kScanPF];
-  auto fetch = [&](int t) {     // raw loads only: nothing waits for them until `commit`
-    const int64_t row = static_cast<int64_t>(sq.tok0 + t) * in_stride;
-#pragma unroll
-    for (int u = 0; u < kScanPF; ++u) {
-      const int i = threadIdx.x + u * 256;
-      raw[u] = Cvt<T>::from_f32(0.f);
-      if (i < dk) raw[u] = zq[row + h * dk + i];
-      else if (i < 2 * dk) raw[u] = zf[row + h * dk + i - dk];
-      else if (i < 2 * dk + ncol) raw[u] = v[row + h * dv + col0 + i - 2 * dk];
-    }
-  };
-  auto commit = [&](float* dst) {
-#pragma unroll
-    for (int u = 0; u < kScanPF; ++u) {
-      const int i = threadIdx.x + u * 256;
-      if (i < in_len) {
-        const float z = Cvt<T>::to_f32(raw[u]);
-        float r = z;                                              // value column
-        if (i < dk) r = z * sigmoidf_(z);                         // q = silu(zq)
-        else if (i < 2 * dk) r = low_r[u] + (1.0f - low_r[u]) * sigmoidf_(z + bias_r[u]);
-        dst[i] = r;
-      }
-    }
-  };
-  fetch(0);
-  commit(in_s);
-  __syncthreads();
-  for (int t = 0; t < sq.count; ++t) {
-    const float* cur = in_s + (t & 1) * in_len;
-    if (t + 1 < sq.count) fetch(t + 1);
-    {
-      const float vc = cur[2 * dk + c];
-      float sum = 0.f;
-      for (int i = rg; i < dk; i += kScanRG) {
-        const float f = cur[dk + i];
-        const float s_new = f * S[i * kScanCols + c] + (1.0f - f) * vc;
-        S[i * kScanCols + c] = s_new;
-        sum = fmaf(s_new, cur[i], sum);
-      }
-      part[rg * kScanCols + c] = sum;
-    }
-    if (t + 1 < sq.count) commit(in_s + ((t + 1) & 1) * in_len);
-    __syncthreads();
-    if (rg == 0 && c < ncol) {
-      float o = 0.f;
-#pragma unroll
-      for (int r = 0; r < kScanRG; ++r) o += part[r * kScanCols + c];
-      o_raw[(static_cast<int64_t>(sq.tok0 + t) * H + h) * dv + col0 + c] = o;
-    }
-    __syncthreads();
-  }
-  for (int i = threadIdx.x; i < dk * kScanCols; i += blockDim.x) {
-    const int r = i / kScanCols, cc = i - r * kScanCols;
-    if (cc < ncol) st[r * dv + col0 + cc] = S[i];
-  }
-}
-
-// Register form for key sizes up to 128: four adjacent lanes share a value column, lane r of the four keeps the state
-// rows i = r, r + 4, ... of that column in REGISTERS for the whole portion.  A token costs dk / 4 state updates per
-// thread, two shuffles to add the four partial read-outs, and no barrier; q and f of a token are broadcast reads
-// from shared memory, stored there grouped by r.  The CTA (128 threads = 32 columns) stages the activated inputs of
-// 4 tokens at a time, double buffered: raw loads of the next 4 tokens are issued before the current 4 are
-// computed and converted afterwards, one barrier per 4 tokens.  The summation order of a read-out is fixed by dk.
-constexpr int kScanChunk = 4;
-constexpr int kScanNT = 128;
-constexpr int kScanColsR = kScanNT / 4;   // value columns per CTA
-
-template <typename T, int DK>
-__global__ void __launch_bounds__(kScanNT)
-gated_scan_columns_kernel(float* __restrict__ o_raw, const T* __restrict__ zq, const T* __restrict__ zf,
-                          const T* __restrict__ v, int64_t in_stride, const T* __restrict__ f_bias,
-                          const T* __restrict__ lower, float* __restrict__ state, const ScanSeq* __restrict__ seqs, int H,
-                          int dk, int dv) {
-  extern __shared__ __align__(16) float smem[];
-  constexpr int RW4 = DK / 4;                           // state rows per thread
-  const ScanSeq sq = seqs[blockIdx.x];
-  const int h = blockIdx.y;
-  const int r = threadIdx.x & 3;
-  const int cl = threadIdx.x >> 2;                       // column within the CTA
-  const int col0 = blockIdx.z * kScanColsR;
-  const int col = col0 + cl;
-  const bool has_col = col < dv;
-  const int ncol = min(kScanColsR, dv - col0);
-  constexpr int row_len = 2 * DK + kScanColsR;           // q grouped by r [4][RW4] | f likewise | v[32]
-  float* buf0 = smem;
-  float* buf1 = smem + kScanChunk * row_len;
-  float* st = state + (static_cast<int64_t>(sq.slot) * H + h) * dk * dv;
-  float S[RW4];
-  // the CTA's slab of the state ([dk][32 columns]) moves through shared memory so that global rows are read and
-  // written as whole 128-byte segments; the staging buffers are free at both ends of the kernel
-  if (!sq.fresh) {
-    for (int idx = threadIdx.x; idx < dk * kScanColsR; idx += kScanNT) {
-      const int i = idx / kScanColsR, c = idx - i * kScanColsR;
-      smem[idx] = c < ncol ? st[i * dv + col0 + c] : 0.f;
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int k = 0; k < RW4; ++k) {
-    const int i = 4 * k + r;
-    S[k] = (!sq.fresh && i < dk) ? smem[i * kScanColsR + cl] : 0.f;
-  }
-  __syncthreads();
-  constexpr int kPer = (kScanChunk * row_len + kScanNT - 1) / kScanNT;   // staged elements per thread and chunk
-  T raw[kPer];
-  // staged element e of a chunk: token e / row_len, slot s = e % row_len; slots [0, DK) hold q with slot = r * RW4 + k
-  // for row i = 4 k + r, slots [DK, 2 DK) hold f the same way, the rest the CTA's value columns
-  auto fetch = [&](int t0) {
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int e = threadIdx.x + u * kScanNT;
-      const int tt = e / row_len, sl = e - tt * row_len;
-      raw[u] = Cvt<T>::from_f32(0.f);
-      if (tt < kScanChunk && t0 + tt < sq.count) {
-        const int64_t row = static_cast<int64_t>(sq.tok0 + t0 + tt) * in_stride;
-        if (sl < 2 * DK) {
-          const int s2 = sl < DK ? sl : sl - DK;
-          const int i = 4 * (s2 % RW4) + s2 / RW4;
-          if (i < dk) raw[u] = sl < DK ? zq[row + h * dk + i] : zf[row + h * dk + i];
-        } else if (sl - 2 * DK < ncol) {
-          raw[u] = v[row + h * dv + col0 + sl - 2 * DK];
-        }
-      }
-    }
-  };
-  auto commit = [&](float* dst, int n_valid) {   // tokens beyond the portion are not activated (nor read later)
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int e = threadIdx.x + u * kScanNT;
-      const int tt = e / row_len, sl = e - tt * row_len;
-      if (tt < n_valid) {
-        const float z = Cvt<T>::to_f32(raw[u]);
-        float val = z;
-        if (sl < DK) {
-          val = z * sigmoidf_(z);
-        } else if (sl < 2 * DK) {
-          const int s2 = sl - DK;
-          const int i = 4 * (s2 % RW4) + s2 / RW4;
-          val = 0.f;   // padded rows: f = 0 and q = 0, they never reach a read-out
-          if (i < dk) {
-            const float lo = Cvt<T>::to_f32(lower[h * dk + i]);
-            val = lo + (1.0f - lo) * sigmoidf_(z + Cvt<T>::to_f32(f_bias[h * dk + i]));
-          }
-        }
-        dst[e] = val;
-      }
-    }
-  };
-  fetch(0);
-  commit(buf0, min(kScanChunk, sq.count));
-  __syncthreads();
-  for (int t0 = 0; t0 < sq.count; t0 += kScanChunk) {
-    const float* cur = ((t0 / kScanChunk) & 1) ? buf1 : buf0;
-    float* nxt = ((t0 / kScanChunk) & 1) ? buf0 : buf1;
-    const bool more = t0 + kScanChunk < sq.count;
-    if (more) fetch(t0 + kScanChunk);
-    const int n_here = min(kScanChunk, sq.count - t0);
-    for (int tt = 0; tt < n_here; ++tt) {
-      const float* row = cur + tt * row_len;
-      const float vc = row[2 * DK + cl];
-      const float* qr = row + r * RW4;
-      const float* fr = row + DK + r * RW4;
-      float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-      for (int k = 0; k < RW4; k += 4) {
-        const float4 q4 = *reinterpret_cast<const float4*>(qr + k);
-        const float4 f4 = *reinterpret_cast<const float4*>(fr + k);
-        S[k] = f4.x * S[k] + (1.0f - f4.x) * vc;
-        o0 = fmaf(S[k], q4.x, o0);
-        S[k + 1] = f4.y * S[k + 1] + (1.0f - f4.y) * vc;
-        o1 = fmaf(S[k + 1], q4.y, o1);
-        S[k + 2] = f4.z * S[k + 2] + (1.0f - f4.z) * vc;
-        o0 = fmaf(S[k + 2], q4.z, o0);
-        S[k + 3] = f4.w * S[k + 3] + (1.0f - f4.w) * vc;
-        o1 = fmaf(S[k + 3], q4.w, o1);
-      }
-      float o = o0 + o1;
-      o += __shfl_xor_sync(0xffffffffu, o, 1);
-      o += __shfl_xor_sync(0xffffffffu, o, 2);
-      if (r == 0 && has_col) o_raw[(static_cast<int64_t>(sq.tok0 + t0 + tt) * H + h) * dv + col] = o;
-    }
-    if (more) commit(nxt, min(kScanChunk, sq.count - t0 - kScanChunk));
-    __syncthreads();
-  }
-#pragma unroll
-  for (int k = 0; k < RW4; ++k) {
-    const int i = 4 * k + r;
-    if (i < dk) smem[i * kScanColsR + cl] = S[k];
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < dk * kScanColsR; idx += kScanNT) {
-    const int i = idx / kScanColsR, c = idx - i * kScanColsR;
-    if (c < ncol) st[i * dv + col0 + c] = smem[idx];
-  }
-}
-
+// ---- per-head norm of the recurrence's read-outs ------------------------------------------------------------------
 // per-head weighted RMS norm of fp32 rows [rows, dv] -> T; one warp per row
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -1335,42 +1095,10 @@ int b200_gated_scan(float* o_raw, const void* zq, const void* zf, const void* v,
   if (n_seqs < 0 || H <= 0 || dk <= 0 || dv <= 0) return fail(B200_EINVAL, "b200_gated_scan: bad sizes");
   if (n_seqs == 0) return 0;
   if (!o_raw || !zq || !zf || !v || !f_bias || !lower || !state || !seqs) return fail(B200_EINVAL, "b200_gated_scan: null pointer");
-  if (dk <= 128 && max_count >= 8) {
-    // register kernel: 32 value columns per CTA, four lanes per column
-    const int dkt = dk <= 16 ? 16 : (dk <= 32 ? 32 : (dk <= 64 ? 64 : 128));
-    // the staging buffers double as the [dk][32] slab the state moves through at both ends of the kernel
-    const size_t smem_c = sizeof(float) * std::max<size_t>(2 * kScanChunk * (2 * static_cast<size_t>(dkt) + kScanColsR),
-                                                           static_cast<size_t>(dkt) * kScanColsR);
-    const dim3 grid_c(n_seqs, H, (dv + kScanColsR - 1) / kScanColsR);
-    return mixer_by_dtype(dtype, "b200_gated_scan", [&](auto* tag) {
-      using T = std::remove_pointer_t<decltype(tag)>;
-      auto launch = [&](auto kern) {
-        kern<<<grid_c, kScanNT, smem_c, static_cast<cudaStream_t>(stream)>>>(
-            o_raw, static_cast<const T*>(zq), static_cast<const T*>(zf), static_cast<const T*>(v), in_stride,
-            static_cast<const T*>(f_bias), static_cast<const T*>(lower), state, reinterpret_cast<const ScanSeq*>(seqs), H,
-            dk, dv);
-      };
-      if (dkt == 16) launch(gated_scan_columns_kernel<T, 16>);
-      else if (dkt == 32) launch(gated_scan_columns_kernel<T, 32>);
-      else if (dkt == 64) launch(gated_scan_columns_kernel<T, 64>);
-      else launch(gated_scan_columns_kernel<T, 128>);
-      return check_launch("b200_gated_scan");
-    });
-  }
-  if (2 * dk + kScanCols > kScanPF * 256) return fail(B200_ESHAPE, "b200_gated_scan: key size %d beyond %d", dk, (kScanPF * 256 - kScanCols) / 2);
-  const size_t smem = sizeof(float) * (static_cast<size_t>(dk) * kScanCols + 2 * (2 * static_cast<size_t>(dk) + kScanCols) +
-                                       static_cast<size_t>(kScanRG) * kScanCols);
-  const dim3 grid(n_seqs, H, (dv + kScanCols - 1) / kScanCols);
-  return mixer_by_dtype(dtype, "b200_gated_scan", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    auto kern = gated_scan_kernel<T>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    kern<<<grid, 256, smem, static_cast<cudaStream_t>(stream)>>>(
-        o_raw, static_cast<const T*>(zq), static_cast<const T*>(zf), static_cast<const T*>(v), in_stride,
-        static_cast<const T*>(f_bias), static_cast<const T*>(lower), state, reinterpret_cast<const ScanSeq*>(seqs), H, dk,
-        dv);
-    return check_launch("b200_gated_scan");
-  });
+  (void)max_count;   // one kernel for portions of any length
+  if (2 * dk + 32 > 1024) return fail(B200_ESHAPE, "b200_gated_scan: key size %d beyond 496", dk);
+  return gated_column_scan(o_raw, ScanRows{zq, zf, v, in_stride}, f_bias, lower, state, seqs, ScanShape{n_seqs, H, H, dk, dv}, dtype,
+                           static_cast<cudaStream_t>(stream));
 }
 
 int b200_head_rmsnorm(void* out, const float* x, const void* weight, float eps, int64_t rows, int dv, int dtype,

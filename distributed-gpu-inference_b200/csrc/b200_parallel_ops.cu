@@ -20,6 +20,7 @@
 #include <type_traits>
 
 #include "../../include/b200_mixers.h"
+#include "b200_column_scan.cuh"
 #include "b200_common.cuh"
 
 namespace b200 {
@@ -115,165 +116,9 @@ qknorm_rotary_append_kernel(T* __restrict__ q, int64_t q_stride, const T* __rest
   }
 }
 
-// ---- retention scan -------------------------------------------------------------------------------------------------
-// One CTA (128 threads) per (sequence, head, 32 value columns).  Four adjacent lanes share a value column; lane r of the
-// four keeps the state rows i = r, r + 4, ... of that column in registers for the whole portion.  The inputs of 4 tokens
-// are staged in shared memory at a time, double buffered (q and k grouped by r so a thread's rows are contiguous); a
-// token costs DK / 4 updates per thread and two shuffles, and a barrier falls once per 4 tokens.
 struct RetSeq {
   int tok0, count, slot, fresh;
 };
-constexpr int kRetChunk = 4;
-constexpr int kRetNT = 128;
-constexpr int kRetCols = kRetNT / 4;
-
-template <typename T, int DK>
-__global__ void __launch_bounds__(kRetNT)
-retention_scan_kernel(float* __restrict__ o_raw, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-                      int64_t in_stride, const float* __restrict__ decay, float k_scale, float* __restrict__ state,
-                      const RetSeq* __restrict__ seqs, int H, int dk, int dv) {
-  extern __shared__ __align__(16) float ret_sm[];
-  constexpr int RW4 = DK / 4;
-  const RetSeq sq = seqs[blockIdx.x];
-  const int h = blockIdx.y;
-  const int r = threadIdx.x & 3, cl = threadIdx.x >> 2;
-  const int col0 = blockIdx.z * kRetCols, col = col0 + cl;
-  const bool has_col = col < dv;
-  const int ncol = min(kRetCols, dv - col0);
-  constexpr int row_len = 2 * DK + kRetCols;
-  float* buf0 = ret_sm;
-  float* buf1 = ret_sm + kRetChunk * row_len;
-  float* st = state + (static_cast<int64_t>(sq.slot) * H + h) * dk * dv;
-  const float d = decay[h];
-  float S[RW4];
-  if (!sq.fresh) {   // the CTA's slab of the state passes shared memory so that global rows move as whole segments
-    for (int idx = threadIdx.x; idx < dk * kRetCols; idx += kRetNT) {
-      const int i = idx / kRetCols, c = idx - i * kRetCols;
-      ret_sm[idx] = c < ncol ? st[i * dv + col0 + c] : 0.f;
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int j = 0; j < RW4; ++j) {
-    const int i = 4 * j + r;
-    S[j] = (!sq.fresh && i < dk) ? ret_sm[i * kRetCols + cl] : 0.f;
-  }
-  __syncthreads();
-  constexpr int kPer = (kRetChunk * row_len + kRetNT - 1) / kRetNT;
-  // staged element e = thread + u * 128 of a chunk is (token e / row_len, slot e % row_len); where it comes from does
-  // not change from chunk to chunk, so for key sizes whose tables fit in registers the source pointer, the token and
-  // the factor (k_scale on key slots) of every element are worked out once
-  constexpr bool kTabled = DK <= 128;
-  constexpr int kTab = kTabled ? kPer : 1;
-  T raw[kPer];
-  const T* src[kTab];
-  int tok_of[kTab];
-  float mul[kTab];
-  if constexpr (kTabled) {
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int e = threadIdx.x + u * kRetNT;
-      const int tt = e / row_len, sl = e - tt * row_len;
-      src[u] = nullptr;
-      tok_of[u] = tt;
-      mul[u] = (sl >= DK && sl < 2 * DK) ? k_scale : 1.0f;
-      if (tt < kRetChunk) {
-        const int64_t row = static_cast<int64_t>(sq.tok0 + tt) * in_stride;
-        if (sl < 2 * DK) {
-          const int s2 = sl < DK ? sl : sl - DK;
-          const int i = 4 * (s2 % RW4) + s2 / RW4;
-          if (i < dk) src[u] = (sl < DK ? q : k) + row + h * dk + i;
-        } else if (sl - 2 * DK < ncol) {
-          src[u] = v + row + h * dv + col0 + sl - 2 * DK;
-        }
-      }
-    }
-  }
-  auto fetch = [&](int t0) {
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      raw[u] = Cvt<T>::from_f32(0.f);
-      if constexpr (kTabled) {
-        if (src[u] != nullptr && t0 + tok_of[u] < sq.count) raw[u] = src[u][static_cast<int64_t>(t0) * in_stride];
-      } else {
-        const int e = threadIdx.x + u * kRetNT;
-        const int tt = e / row_len, sl = e - tt * row_len;
-        if (tt < kRetChunk && t0 + tt < sq.count) {
-          const int64_t row = static_cast<int64_t>(sq.tok0 + t0 + tt) * in_stride;
-          if (sl < 2 * DK) {
-            const int s2 = sl < DK ? sl : sl - DK;
-            const int i = 4 * (s2 % RW4) + s2 / RW4;
-            if (i < dk) raw[u] = sl < DK ? q[row + h * dk + i] : k[row + h * dk + i];
-          } else if (sl - 2 * DK < ncol) {
-            raw[u] = v[row + h * dv + col0 + sl - 2 * DK];
-          }
-        }
-      }
-    }
-  };
-  auto commit = [&](float* dst, int n_valid) {
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int e = threadIdx.x + u * kRetNT;
-      if constexpr (kTabled) {
-        if (tok_of[u] < n_valid) dst[e] = Cvt<T>::to_f32(raw[u]) * mul[u];
-      } else {
-        const int tt = e / row_len, sl = e - tt * row_len;
-        if (tt < n_valid) {
-          float val = Cvt<T>::to_f32(raw[u]);
-          if (sl >= DK && sl < 2 * DK) val *= k_scale;
-          dst[e] = val;
-        }
-      }
-    }
-  };
-  fetch(0);
-  commit(buf0, min(kRetChunk, sq.count));
-  __syncthreads();
-  for (int t0 = 0; t0 < sq.count; t0 += kRetChunk) {
-    const float* cur = ((t0 / kRetChunk) & 1) ? buf1 : buf0;
-    float* nxt = ((t0 / kRetChunk) & 1) ? buf0 : buf1;
-    const bool more = t0 + kRetChunk < sq.count;
-    if (more) fetch(t0 + kRetChunk);
-    const int n_here = min(kRetChunk, sq.count - t0);
-    for (int tt = 0; tt < n_here; ++tt) {
-      const float* row = cur + tt * row_len;
-      const float vc = row[2 * DK + cl];
-      const float* qr = row + r * RW4;
-      const float* kr = row + DK + r * RW4;
-      float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-      for (int j = 0; j < RW4; j += 4) {
-        const float4 q4 = *reinterpret_cast<const float4*>(qr + j);
-        const float4 k4 = *reinterpret_cast<const float4*>(kr + j);
-        S[j] = fmaf(d, S[j], k4.x * vc);
-        o0 = fmaf(S[j], q4.x, o0);
-        S[j + 1] = fmaf(d, S[j + 1], k4.y * vc);
-        o1 = fmaf(S[j + 1], q4.y, o1);
-        S[j + 2] = fmaf(d, S[j + 2], k4.z * vc);
-        o0 = fmaf(S[j + 2], q4.z, o0);
-        S[j + 3] = fmaf(d, S[j + 3], k4.w * vc);
-        o1 = fmaf(S[j + 3], q4.w, o1);
-      }
-      float o = o0 + o1;
-      o += __shfl_xor_sync(0xffffffffu, o, 1);
-      o += __shfl_xor_sync(0xffffffffu, o, 2);
-      if (r == 0 && has_col) o_raw[(static_cast<int64_t>(sq.tok0 + t0 + tt) * H + h) * dv + col] = o;
-    }
-    if (more) commit(nxt, min(kRetChunk, sq.count - t0 - kRetChunk));
-    __syncthreads();
-  }
-#pragma unroll
-  for (int j = 0; j < RW4; ++j) {
-    const int i = 4 * j + r;
-    if (i < dk) ret_sm[i * kRetCols + cl] = S[j];
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < dk * kRetCols; idx += kRetNT) {
-    const int i = idx / kRetCols, c = idx - i * kRetCols;
-    if (c < ncol) st[i * dv + col0 + c] = ret_sm[idx];
-  }
-}
 
 // ---- retention over long portions: segments in parallel, then the carry ---------------------------------------------
 // A long portion is cut into segments that the scan above runs as independent fresh sequences (their end states go to a
@@ -633,25 +478,8 @@ int b200_retention_scan(float* o_raw, const void* q, const void* k, const void* 
   if (dk > 512) return fail(B200_ESHAPE, "b200_retention_scan: key size %d beyond 512", dk);
   if (n_seqs == 0) return 0;
   if (!o_raw || !q || !k || !v || !decay || !state || !seqs) return fail(B200_EINVAL, "b200_retention_scan: null pointer");
-  const int dkt = dk <= 32 ? 32 : (dk <= 64 ? 64 : (dk <= 128 ? 128 : (dk <= 256 ? 256 : 512)));
-  const size_t smem = sizeof(float) * std::max<size_t>(2 * kRetChunk * (2 * static_cast<size_t>(dkt) + kRetCols),
-                                                       static_cast<size_t>(dk) * kRetCols);
-  const dim3 grid(n_seqs, H, (dv + kRetCols - 1) / kRetCols);
-  return parallel_by_dtype(dtype, "b200_retention_scan", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    auto s = static_cast<cudaStream_t>(stream);
-    auto launch = [&](auto kern) {
-      if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      kern<<<grid, kRetNT, smem, s>>>(o_raw, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v),
-                                      in_stride, decay, k_scale, state, reinterpret_cast<const RetSeq*>(seqs), H, dk, dv);
-    };
-    if (dkt == 32) launch(retention_scan_kernel<T, 32>);
-    else if (dkt == 64) launch(retention_scan_kernel<T, 64>);
-    else if (dkt == 128) launch(retention_scan_kernel<T, 128>);
-    else if (dkt == 256) launch(retention_scan_kernel<T, 256>);
-    else launch(retention_scan_kernel<T, 512>);
-    return check_launch("b200_retention_scan");
-  });
+  return retention_column_scan(o_raw, ScanRows{q, k, v, in_stride}, decay, k_scale, state, seqs, ScanShape{n_seqs, H, H, dk, dv}, dtype,
+                               static_cast<cudaStream_t>(stream));
 }
 
 int b200_retention_carry(float* state, float* seg_state, const int32_t* parents, int n_parents, const int32_t* seg_spans,
