@@ -28,6 +28,7 @@
 #include "../../include/b200_mixers.h"
 #include "b200_column_scan.cuh"
 #include "b200_common.cuh"
+#include "b200_tile_attn.cuh"
 
 namespace b200 {
 namespace {
@@ -897,14 +898,15 @@ mixed_prompt_attn_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, co
   }
 }
 
-// Merge of the key splits: one CTA per token.  out(h) = sum_s O_s e^(m_s - M) / (sum_s l_s e^(m_s - M) + e^(sink - M)),
+// Merge of the key splits: one CTA per token of a tile (tile blockIdx.x, its token blockIdx.y).  out(h) = sum_s O_s e^(m_s - M) / (sum_s l_s e^(m_s - M) + e^(sink - M)),
 // then the turn back and the gate, as in the single-CTA epilogue.
 template <typename T>
 __global__ void __launch_bounds__(256)
-attn_split_combine_kernel(const AttnArgs A, const float* __restrict__ ws, int n_splits, int n_tok, int dvp,
-                          const float* __restrict__ rot_tab) {
+attn_split_combine_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, const float* __restrict__ ws, int n_splits, int n_tok,
+                          int dvp, const float* __restrict__ rot_tab) {
   extern __shared__ float res[];   // [H][dv]
-  const int n = blockIdx.x, H = A.H, dv = A.dv, stride = dvp + 2;
+  if (static_cast<int>(blockIdx.y) >= tiles[3 * blockIdx.x + 1]) return;
+  const int n = tiles[3 * blockIdx.x] + blockIdx.y, H = A.H, dv = A.dv, stride = dvp + 2;
   for (int e = threadIdx.x; e < H * dv; e += blockDim.x) {
     const int h = e / dv, c = e - h * dv;
     float M = A.sink ? A.sink[h] : -INFINITY;
@@ -1296,6 +1298,58 @@ int b200_mixed_prompt_attn_splits(int n_tiles, int key_tiles, int H, int G, int 
   return std::max(1, std::min({8, (2 * kNumSMs + ctas - 1) / ctas, key_tiles / 4}));
 }
 
+int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bias, int dtype) {
+  return tile_attn_supported(H, G, dk, dv, same_pool != 0, bias != 0, dtype) ? 1 : 0;
+}
+
+int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk) { return tile_attn_splits(n_tiles, key_tiles, G, dk); }
+
+int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
+                   const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,
+                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, const int32_t* tok_pos, int n_tok,
+                   const float* sink, const float* bias_lut, int lut_len, float scale, float softcap, float temp_coef, int temp_every,
+                   int window, int keep_first, int chunk, int H, int G, int dk, int dv, int v_row, int v_div, int out_f32, int block_size,
+                   int n_splits, float* workspace, int dtype, void* stream) {
+  const bool alias = k_pool == v_pool;
+  if (n_tiles < 0 || n_tok < 0 || H <= 0 || G <= 0 || H % G || block_size <= 0 || n_splits < 1 || n_splits > 64 || chunk < 0 ||
+      v_div < 1 || G % v_div || v_row < dv || v_row % 8 || (bias_lut && (lut_len <= 0 || softcap > 0.f)))
+    return fail(B200_EINVAL, "b200_tile_attn: bad sizes");
+  if (!tile_attn_supported(H, G, dk, dv, alias, bias_lut != nullptr, dtype) || (alias && (v_div != 1 || v_row != dk)))
+    return fail(B200_ESHAPE, "b200_tile_attn: head layout (%d over %d, %d / %d) is not served", H, G, dk, dv);
+  if (n_tiles == 0) return 0;
+  if (!out || !q || !k_pool || !v_pool || !block_tables || !tiles || !tok_pos || (n_splits > 1 && !workspace))
+    return fail(B200_EINVAL, "b200_tile_attn: null pointer");
+  if (!aligned16(q) || ((q_tok_stride | q_head_stride) & 7) || !aligned16(k_pool) || !aligned16(v_pool))
+    return fail(B200_ESHAPE, "b200_tile_attn: queries and pools need 16-byte aligned rows");
+  if (((out_tok_stride | out_head_stride) & 1) || reinterpret_cast<uintptr_t>(out) % (out_f32 ? 8 : 4))
+    return fail(B200_ESHAPE, "b200_tile_attn: odd output strides");
+  TileAttn A{};
+  A.out = out, A.out_tok_stride = out_tok_stride, A.out_head_stride = out_head_stride;
+  A.q = q, A.q_tok_stride = q_tok_stride, A.q_head_stride = q_head_stride;
+  A.gate = gate, A.gate_stride = gate_stride, A.gate_dim = gate_per_channel ? dv : 0;
+  A.k_pool = k_pool, A.v_pool = v_pool, A.block_tables = block_tables, A.table_stride = table_stride;
+  A.tiles = tiles, A.tok_pos = tok_pos, A.sink = sink, A.bias_lut = bias_lut, A.lut_len = lut_len, A.ws = workspace;
+  A.n_tok = n_tok, A.H = H, A.G = G, A.block_size = block_size, A.v_row = v_row, A.v_div = v_div;
+  A.window = window, A.keep_first = keep_first, A.chunk = chunk;
+  A.out_f32 = out_f32, A.out_vec = aligned16(out) && ((out_tok_stride | out_head_stride) & 7) == 0;
+  A.scale = scale, A.softcap = softcap, A.temp_coef = temp_coef, A.temp_every = temp_every;
+  const auto s = static_cast<cudaStream_t>(stream);
+  const int rc = tile_attn_launch(A, dk, dv, alias, n_tiles, n_splits, dtype, s);
+  if (rc != 0 || n_splits == 1) return rc;
+  AttnArgs M{out, out_tok_stride, out_head_stride, q, q_tok_stride, q_head_stride, gate, gate_stride, k_pool, v_pool,
+             block_tables, table_stride, nullptr, tok_pos, nullptr, sink, scale, window, keep_first, 0,
+             0, 0.0, H, G, dk, dv, block_size, softcap, chunk, v_row, v_div, 0, out_f32, 0, gate_per_channel ? dv : 0};
+  const size_t smem = sizeof(float) * static_cast<size_t>(H) * dv;
+  if (smem > 200 * 1024) return fail(B200_ESHAPE, "b200_tile_attn: %d heads of %d are too many to merge", H, dv);
+  return hybrid_by_dtype(dtype, "b200_tile_attn", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    auto merge = attn_split_combine_kernel<T>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    merge<<<dim3(n_tiles, kTileRows / (H / G)), 256, smem, s>>>(M, tiles, workspace, n_splits, n_tok, dv, nullptr);
+    return check_launch("b200_tile_attn (merge)");
+  });
+}
+
 size_t b200_mixed_prompt_attn_workspace(int n_splits, int n_tok, int H, int dv) {
   if (n_splits <= 1 || n_tok <= 0 || H <= 0 || dv <= 0) return 0;
   const int dvp = (dv <= 64 ? 8 : (dv <= 128 ? 16 : 32)) * 8;
@@ -1395,12 +1449,13 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
       else pick(std::integral_constant<int, kTcPlain>{});
       int rc = check_launch("b200_mixed_prompt_attn");
       if (rc != 0 || n_splits == 1) return rc;
-      // every packed row belongs to exactly one tile, so the merge runs over all rows
+      // the merge runs over the tiles' rows only: others of the step belong to another launch (as many tiles as rows: one each)
       A.H = H_real;
+      const dim3 rows(n_tiles, n_tiles == n_tok ? 1 : kTcRows);
       const size_t smem_c = sizeof(float) * static_cast<size_t>(H_real) * dv;
       auto comb = attn_split_combine_kernel<T>;
       if (smem_c > 48 * 1024) cudaFuncSetAttribute(comb, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_c));
-      comb<<<n_tok, 256, smem_c, s>>>(A, workspace, n_splits, n_tok, plan.dv8 * 8, value_rot);
+      comb<<<rows, 256, smem_c, s>>>(A, tiles, workspace, n_splits, n_tok, plan.dv8 * 8, value_rot);
       return check_launch("b200_mixed_prompt_attn (merge)");
     }
   });

@@ -1,0 +1,33 @@
+// Launchers of b200_tile_attn.cu (the C entry point b200_tile_attn checks the arguments and runs the merge of key splits).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+namespace b200 {
+
+constexpr int kTileRows = 128;   // query rows of a tile: up to 128 / (H / G) tokens
+
+struct TileAttn {
+  void* out; int64_t out_tok_stride, out_head_stride;
+  const void* q; int64_t q_tok_stride, q_head_stride;
+  const void* gate; int64_t gate_stride;
+  const void* k_pool; const void* v_pool;
+  const int32_t* block_tables; int table_stride;
+  const int32_t* tiles; const int32_t* tok_pos;
+  const float* sink;
+  const float* bias_lut; int lut_len;        // distance biases [H][lut_len], or null
+  float* ws;                                 // key splits: [split][n_tok][H][dv + 2]
+  int n_tok, H, G, block_size, v_row, v_div;
+  int window, keep_first, chunk;
+  int gate_dim, out_f32, out_vec;            // gates per channel: the value size; 16-byte stores possible
+  float scale, softcap, temp_coef;
+  int temp_every;
+};
+
+bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, int dtype);
+int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk);
+int tile_attn_launch(const TileAttn& A, int dk, int dv, bool alias, int n_tiles, int n_splits, int dtype, cudaStream_t stream);
+
+}  // namespace b200

@@ -163,6 +163,7 @@ class ParallelMixer(nn.Module):
         self.w_out = _param(w_out, device, dtype)
         self.tensor_cores = mixer_ops.mixed_prompt_attention_supported(self.H, self.G, self.dk, self.dv, False, False, False,
                                                                        self.w_in.dtype) and self.Kl % 2 == 0
+        self.in_tiles = mixer_ops.tile_attention_supported(self.H, self.G, self.dk, self.dv, False, False, self.w_in.dtype)
 
     def forward(self, h: torch.Tensor, cache: RaggedLayerCache) -> torch.Tensor:
         st, n, c = cache.state, h.shape[0], self.cuts
@@ -177,10 +178,13 @@ class ParallelMixer(nn.Module):
                                        st.slot_mapping, st.tok_pos, H, interleaved=True)
         attn = buf[:, :self.Kl].unflatten(1, (H, dv))
         if self.tensor_cores:
-            tiles, _ = st.prompt_tiles(1, mixer_ops.PROMPT_TILE_TOKENS)
-            mixer_ops.mixed_prompt_attention(attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
-                                             tiles, st.tok_pos, self.scale, sink=self.sink, window=self.window,
-                                             max_context=st.max_context(), softcap=self.softcap)
+            tiles, rest = st.attention_tiles(H, G, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            args = (attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables)
+            kw = dict(sink=self.sink, window=self.window, max_context=st.max_context(), softcap=self.softcap)
+            if tiles is not None:
+                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+            if rest is not None:
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
         else:
             mixer_ops.mixed_paged_attention(attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
                                             st.tok_row, st.tok_pos, self.scale, sink=self.sink, window=self.window,

@@ -525,6 +525,61 @@ def mixed_prompt_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Ten
     _lib.check_mixers(rc, "b200_mixed_prompt_attn")
 
 
+TILE_ROWS = 128             # query rows (tokens x heads of a kv group) a CTA of ``tile_attention`` serves
+
+
+def tile_attention_supported(H: int, G: int, dk: int, dv: int, same_pool: bool, bias: bool, dtype: torch.dtype) -> bool:
+    """Whether ``tile_attention`` serves this head layout (aligned query rows are checked per call)."""
+    return bool(_lib_().b200_tile_attn_supported(int(H), int(G), int(dk), int(dv), int(same_pool), int(bias), DTYPE_ID[dtype]))
+
+
+def tile_attention_from(H: int, G: int) -> int:
+    """Tokens from which a portion goes to ``tile_attention``: from half a tile's rows on.  Below, most of the 128 rows of a product
+    would be padding."""
+    return max(2, TILE_ROWS // 2 // (H // G))
+
+
+@_timed
+def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_tables: torch.Tensor,
+                   tiles: torch.Tensor, tok_pos: torch.Tensor, scale: float, sink: Optional[torch.Tensor] = None, window: int = 0,
+                   keep_first: int = 0, gate: Optional[torch.Tensor] = None, max_context: int = 0, softcap: float = 0.0, chunk: int = 0,
+                   value_width: Optional[int] = None, value_div: int = 1, bias_lut: Optional[torch.Tensor] = None,
+                   temp_coef: float = 0.0, temp_every: int = 1) -> None:
+    """``mixed_prompt_attention`` (or, with ``bias_lut``, ``biased_prompt_attention``) for prompt portions in tiles of up to
+    ``TILE_ROWS`` rows: ``tiles`` int32 ``[n_tiles, 3]`` with up to ``TILE_ROWS // (H // G)`` consecutive tokens of one sequence each.
+    Only the tiles' rows of ``out`` are written, so the other portions of a step may go through another kernel."""
+    _need_cuda(out, q, k_pool, v_pool, block_tables, tiles, tok_pos)
+    nb, G, bs, dk = k_pool.shape
+    dv, v_row = _value_layout(k_pool, v_pool, value_width, value_div)
+    n, H = q.shape[0], q.shape[1]
+    if q.dim() != 3 or q.shape[2] != dk or tuple(out.shape) != (n, H, dv) or q.stride(2) != 1 or out.stride(2) != 1:
+        raise ValueError("q must be [n, H, dk] and out [n, H, dv] with contiguous last dimensions")
+    if out.dtype not in (q.dtype, torch.float32) or k_pool.dtype != q.dtype or v_pool.dtype != q.dtype:
+        raise TypeError("q and the pools share one dtype; out has it too, or is fp32")
+    if tiles.dtype != torch.int32 or tiles.dim() != 2 or tiles.shape[1] != 3 or not tiles.is_contiguous():
+        raise ValueError("tiles must be contiguous int32 [n_tiles, 3]")
+    if block_tables.dtype != torch.int32 or tok_pos.dtype != torch.int32:
+        raise TypeError("block tables and positions are int32")
+    if sink is not None and (sink.dtype != torch.float32 or tuple(sink.shape) != (H,) or not sink.is_contiguous()):
+        raise ValueError("sink is contiguous fp32 [H]")
+    if bias_lut is not None and (bias_lut.dtype != torch.float32 or bias_lut.shape[0] != H or not bias_lut.is_contiguous()):
+        raise ValueError("bias_lut must be contiguous fp32 [H, L]")
+    per_channel = _gate_kind(gate, n, H, dv, q.dtype)
+    lib = _lib_()
+    seen = min(max_context, window + keep_first + TILE_ROWS) if window > 0 else max_context
+    if chunk > 0:
+        seen = min(seen, chunk + TILE_ROWS)
+    splits = lib.b200_tile_attn_splits(tiles.shape[0], (seen + 63) // 64, G, dk) if max_context > 0 else 1
+    ws = torch.empty((splits, n, H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+    rc = lib.b200_tile_attn(out.data_ptr(), out.stride(0), out.stride(1), q.data_ptr(), q.stride(0), q.stride(1), _ptr(gate),
+                            _rows2(gate) if gate is not None else 0, per_channel, k_pool.data_ptr(), v_pool.data_ptr(),
+                            block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), tiles.shape[0], tok_pos.data_ptr(), n,
+                            _ptr(sink), _ptr(bias_lut), bias_lut.shape[1] if bias_lut is not None else 0, float(scale), float(softcap),
+                            float(temp_coef), int(temp_every), int(window), int(keep_first), int(chunk), H, G, dk, dv, v_row,
+                            int(value_div), int(out.dtype == torch.float32), bs, int(splits), _ptr(ws), DTYPE_ID[q.dtype], _stream())
+    _lib.check_mixers(rc, "b200_tile_attn")
+
+
 @_timed
 def causal_conv_silu(x: torch.Tensor, weight: torch.Tensor, tail: torch.Tensor, seqs: torch.Tensor,
                      max_count: int, bias: Optional[torch.Tensor] = None) -> torch.Tensor:

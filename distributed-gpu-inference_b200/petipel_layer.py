@@ -146,6 +146,7 @@ class BiasedPagedAttention(nn.Module):
         self.w_in = _param(torch.cat([w_in, w_in.new_zeros(pad, w_in.shape[1])], dim=0), device, dtype)
         self.w_o = _param(t["o"], device, dtype)
         self.tensor_core_prompt = mixer_ops.prompt_attention_supported(self.dk, self.dv, self.w_in.dtype)
+        self.in_tiles = mixer_ops.tile_attention_supported(self.H, self.G, self.dk, self.dv, False, True, self.w_in.dtype)
         self.register_buffer("bias_lut", distance_bias_table(t["rel"], float(spec["bias_max"])).to(device), persistent=False)
         self.lam = float(t["vmix"].to(torch.float32)) if "vmix" in t else 0.0
 
@@ -167,10 +168,15 @@ class BiasedPagedAttention(nn.Module):
         q, gate = proj[:, :a], proj[:, c:c + H]
         attn = torch.empty((h.shape[0], H * dv), dtype=h.dtype, device=h.device)
         if self.tensor_core_prompt:   # 16-bit storage and sizes the tensor-core kernel takes: portions and single tokens
-            tiles, most = st.prompt_tiles(1, mixer_ops.prompt_tile_tokens(H, G))
-            mixer_ops.biased_prompt_attention(attn, q, gate, cache.k_pool, cache.v_pool, st.block_tables, tiles,
-                                              st.tok_pos, self.bias_lut, self.scale, self.temp_coef, self.temp_every, H,
-                                              max_tile_tokens=most)
+            tiles, rest = st.attention_tiles(H, G, mixer_ops.prompt_tile_tokens(H, G), self.in_tiles)
+            if tiles is not None:
+                mixer_ops.tile_attention(attn.view(-1, H, dv), q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
+                                         tiles, st.tok_pos, self.scale, gate=gate, max_context=st.max_context(),
+                                         bias_lut=self.bias_lut, temp_coef=self.temp_coef, temp_every=self.temp_every)
+            if rest is not None:
+                mixer_ops.biased_prompt_attention(attn, q, gate, cache.k_pool, cache.v_pool, st.block_tables, rest[0], st.tok_pos,
+                                                  self.bias_lut, self.scale, self.temp_coef, self.temp_every, H,
+                                                  max_tile_tokens=rest[1])
         else:                         # fp32, or head sizes off the tensor-core grid: the row kernel
             tiles, most = st.tiles_for(H, G)
             mixer_ops.biased_paged_attention(q, gate, cache.k_pool, cache.v_pool, st.block_tables, tiles, most,

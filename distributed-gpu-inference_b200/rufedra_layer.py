@@ -184,6 +184,7 @@ class KeyValueSelectiveMixer(nn.Module):
         self.w_out = _param(w_out, device, dtype)
         self.tensor_cores = mixer_ops.mixed_prompt_attention_supported(self.H, self.G, self.dk, self.dk, False, False, False,
                                                                        self.w_in.dtype)
+        self.in_tiles = mixer_ops.tile_attention_supported(self.H, self.G, self.dk, self.dk, False, False, self.w_in.dtype)
         self.rows = (self.tensor_cores and self.G == 1 and self.H >= LatentRotaryAttention.HEADS_AS_ROWS_FROM and
                      mixer_ops.heads_as_rows_supported(self.H, self.dk, self.dk, self.w_in.dtype))
 
@@ -202,10 +203,14 @@ class KeyValueSelectiveMixer(nn.Module):
                                        st.tok_pos, H, interleaved=False, unit_norm=True)
         attn = buf[:, :self.Kl].unflatten(1, (H, dk))
         if self.tensor_cores:
-            tiles, _ = st.prompt_tiles(1, mixer_ops.PROMPT_TILE_TOKENS)
-            mixer_ops.mixed_prompt_attention(attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables, tiles,
-                                             st.tok_pos, self.scale, window=self.window, gate=gate,
-                                             max_context=st.max_context(), heads_as_rows=self.rows and st.max_count() == 1)
+            tiles, rest = st.attention_tiles(H, G, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            args = (attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables)
+            kw = dict(window=self.window, gate=gate, max_context=st.max_context())
+            if tiles is not None:
+                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+            if rest is not None:
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale,
+                                                 heads_as_rows=self.rows and st.max_count() == 1, **kw)
         else:
             mixer_ops.mixed_paged_attention(attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
                                             st.tok_row, st.tok_pos, self.scale, window=self.window, gate=gate)

@@ -202,6 +202,7 @@ class LatentAttention(nn.Module):
         self.w_o = _param(t["o"], device, dtype)
         self.tensor_cores = mixer_ops.mixed_prompt_attention_supported(self.H, 1, self.rank, self.rank, False, True,
                                                                        False, self.w_in.dtype)
+        self.in_tiles = mixer_ops.tile_attention_supported(self.H, 1, self.rank, self.rank, True, False, self.w_in.dtype)
 
     def forward(self, h: torch.Tensor, cache: RaggedLayerCache) -> torch.Tensor:
         st, n = cache.state, h.shape[0]
@@ -213,10 +214,13 @@ class LatentAttention(nn.Module):
         q_lat = torch.bmm(q.transpose(0, 1), self.w_uk)                          # [H, n, r]
         o_lat = torch.empty((H, n, r), dtype=h.dtype, device=h.device)
         if self.tensor_cores:
-            tiles, _ = st.prompt_tiles(1, mixer_ops.PROMPT_TILE_TOKENS)
-            mixer_ops.mixed_prompt_attention(o_lat.transpose(0, 1), q_lat.transpose(0, 1), cache.k_pool, cache.k_pool,
-                                             st.block_tables, tiles, st.tok_pos, self.scale, gate=proj[:, c[2]:c[2] + H],
-                                             max_context=st.max_context())
+            tiles, rest = st.attention_tiles(H, 1, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            args = (o_lat.transpose(0, 1), q_lat.transpose(0, 1), cache.k_pool, cache.k_pool, st.block_tables)
+            kw = dict(gate=proj[:, c[2]:c[2] + H], max_context=st.max_context())
+            if tiles is not None:
+                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+            if rest is not None:
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
         else:
             mixer_ops.mixed_paged_attention(o_lat.transpose(0, 1), q_lat.transpose(0, 1), cache.k_pool, cache.k_pool,
                                             st.block_tables, st.tok_row, st.tok_pos, self.scale,

@@ -159,6 +159,7 @@ class LatentRotaryAttention(nn.Module):
         D = self.rank + self.dr
         self.tensor_cores = D % 8 == 0 and mixer_ops.mixed_prompt_attention_supported(
             self.H, 1, D, self.rank, False, True, False, self.w_in.dtype)
+        self.in_tiles = mixer_ops.tile_attention_supported(self.H, 1, D, self.rank, True, False, self.w_in.dtype)
 
     def forward(self, h: torch.Tensor, cache: RaggedLayerCache) -> torch.Tensor:
         st, n = cache.state, h.shape[0]
@@ -171,12 +172,14 @@ class LatentRotaryAttention(nn.Module):
         torch.bmm(q[:, :, :dn].transpose(0, 1), self.w_uk, out=q_lat[:, :, :r].transpose(0, 1))
         o_lat = torch.empty((H, n, r), dtype=h.dtype, device=h.device)
         if self.tensor_cores:
-            tiles, _ = st.prompt_tiles(1, mixer_ops.PROMPT_TILE_TOKENS)
-            # steps of single tokens: all heads read the same rows, so 16 heads share a tensor-core tile
-            mixer_ops.mixed_prompt_attention(o_lat.transpose(0, 1), q_lat, cache.k_pool, cache.k_pool, st.block_tables,
-                                             tiles, st.tok_pos, self.scale, sink=self.sink, window=self.window,
-                                             max_context=st.max_context(), value_width=r,
-                                             heads_as_rows=H >= self.HEADS_AS_ROWS_FROM and st.max_count() == 1)
+            tiles, rest = st.attention_tiles(H, 1, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            args = (o_lat.transpose(0, 1), q_lat, cache.k_pool, cache.k_pool, st.block_tables)
+            kw = dict(sink=self.sink, window=self.window, max_context=st.max_context(), value_width=r)
+            if tiles is not None:
+                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+            if rest is not None:    # single tokens: all heads read the same rows, so 16 heads share a tensor-core tile
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale,
+                                                 heads_as_rows=H >= self.HEADS_AS_ROWS_FROM and st.max_count() == 1, **kw)
         else:
             mixer_ops.mixed_paged_attention(o_lat.transpose(0, 1), q_lat, cache.k_pool, cache.k_pool, st.block_tables,
                                             st.tok_row, st.tok_pos, self.scale, sink=self.sink, window=self.window,
@@ -221,6 +224,7 @@ class DifferentialAttention(nn.Module):
         self.b_o = _param(t["o.b"], device, dtype) if "o.b" in t else None
         self.tensor_cores = self.dv % 8 == 0 and mixer_ops.mixed_prompt_attention_supported(
             2 * H, 2 * G, dk, self.dv, False, False, False, self.w_in.dtype)
+        self.in_tiles = mixer_ops.tile_attention_supported(2 * H, 2 * G, dk, self.dv, False, False, self.w_in.dtype)
 
     def forward(self, h: torch.Tensor, cache: RaggedLayerCache) -> torch.Tensor:
         st, n, c = cache.state, h.shape[0], self.cuts
@@ -233,10 +237,13 @@ class DifferentialAttention(nn.Module):
                                        st.slot_mapping, st.tok_pos, 2 * H)
         maps = torch.empty((n, 2 * H, dv), dtype=torch.float32, device=h.device)    # rounded only after their difference
         if self.tensor_cores:
-            tiles, _ = st.prompt_tiles(1, mixer_ops.PROMPT_TILE_TOKENS)
-            mixer_ops.mixed_prompt_attention(maps, q.unflatten(1, (2 * H, dk)), k_pool, cache.v_pool, st.block_tables, tiles,
-                                             st.tok_pos, self.scale, chunk=self.chunk, max_context=st.max_context(),
-                                             value_div=2)
+            tiles, rest = st.attention_tiles(2 * H, 2 * G, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            args = (maps, q.unflatten(1, (2 * H, dk)), k_pool, cache.v_pool, st.block_tables)
+            kw = dict(chunk=self.chunk, max_context=st.max_context(), value_div=2)
+            if tiles is not None:
+                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+            if rest is not None:
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
         else:
             mixer_ops.mixed_paged_attention(maps, q.unflatten(1, (2 * H, dk)), k_pool, cache.v_pool, st.block_tables,
                                             st.tok_row, st.tok_pos, self.scale, chunk=self.chunk, value_div=2)

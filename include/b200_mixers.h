@@ -463,6 +463,20 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
                                 int dv, int v_row, int v_div, int heads_as_rows, int out_f32, int block_size, int n_splits,
                                 float* workspace, int dtype, void* stream);
 
+/* b200_mixed_prompt_attn_ext2 and b200_biased_prompt_attn for prompt portions on the fifth-generation tensor cores: tiles of up to
+ * 128 / (H / G) tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
+ * touched.  bias_lut fp32 [H][lut_len] with temp_coef / temp_every as in b200_biased_prompt_attn, or NULL.  The values are v_pool's
+ * rows, or the first dv columns of the key rows when v_pool == k_pool.  n_splits > 1 divides the keys over as many CTAs and needs a
+ * workspace fp32 [n_splits][n_tok][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte aligned query rows. */
+int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bias, int dtype);
+int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk);
+int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
+                   const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,
+                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, const int32_t* tok_pos, int n_tok,
+                   const float* sink, const float* bias_lut, int lut_len, float scale, float softcap, float temp_coef, int temp_every,
+                   int window, int keep_first, int chunk, int H, int G, int dk, int dv, int v_row, int v_div, int out_f32, int block_size,
+                   int n_splits, float* workspace, int dtype, void* stream);
+
 /* Whether b200_mixed_prompt_attn_ext2 takes H heads over one kv head with heads_as_rows (separate key and value pools). */
 int b200_mixed_prompt_attn_rows_supported(int H, int dk, int dv, int dtype);
 

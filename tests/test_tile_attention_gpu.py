@@ -1,0 +1,130 @@
+"""Prompt attention in tiles of 128 rows against float64: portions around the tiles' edges, contexts around the key tiles', every mask
+and option the layers use, head layouts of each instantiation, page sizes that are no power of two, keys divided over CTAs."""
+import pytest
+import torch
+
+from dgi_b200 import mixer_ops
+from dgi_b200.paged_layer import RaggedBatchState
+
+pytestmark = pytest.mark.gpu
+
+F64 = torch.float64
+#           H, G, key size, value size (0: the key rows' first 256 columns), value heads per key head
+GROUPED, WIDE, NARROW, ONE, LATENT, LATENT_ROT, PAIRED = ((8, 2, 128, 128, 1), (16, 1, 128, 128, 1), (6, 2, 64, 64, 1), (3, 3, 128, 128, 1),
+                                                          (8, 1, 256, 0, 1), (16, 1, 320, 0, 1), (8, 4, 128, 128, 2))
+# portions as (new tokens, tokens before)
+EDGES = [(32, 0), (33, 31), (31, 64), (64, 1), (65, 200), (128, 0), (1, 5)]
+
+
+def _case(layout, portions, page, dtype):
+    H, G, dk, dv, div = layout
+    gen = torch.Generator(device="cuda").manual_seed(H * dk + len(portions))
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    need = [(n + past + page - 1) // page for n, past in portions]
+    order = torch.randperm(sum(need) + 3, generator=gen, device="cuda").to(torch.int32)
+    tables = torch.zeros(len(portions), max(need) + 1, dtype=torch.int32, device="cuda")
+    lo, spans, pos, first = 0, [], [], 0
+    for b, (n, past) in enumerate(portions):
+        tables[b, :need[b]] = order[lo:lo + need[b]]
+        lo += need[b]
+        spans.append((first, n, b, past))
+        pos += range(past, past + n)
+        first += n
+    k_pool = rnd(sum(need) + 3, G, page, dk).to(dtype)
+    v_pool = k_pool if dv == 0 else rnd(sum(need) + 3, G // div, page, dv).to(dtype)
+    q = (rnd(first, H * dk + 16) * 1.5).to(dtype)[:, 8:8 + H * dk].unflatten(1, (H, dk))    # rows of a wider projection
+    st = RaggedBatchState(tok_pos=torch.tensor(pos, dtype=torch.int32, device="cuda"), slot_mapping=None, block_tables=tables,
+                          scan_seqs=None, spans=spans)
+    return q, k_pool, v_pool, st, rnd
+
+
+def _reference(q, k_pool, v_pool, st, dv, div, scale, sink=None, window=0, keep_first=0, softcap=0.0, chunk=0, gate=None, bias=None, temp=None):
+    n_all, H, dk = q.shape
+    G, page = k_pool.shape[1], k_pool.shape[2]
+    out = torch.empty(n_all, H, dv, dtype=F64, device=q.device)
+    for first, n, b, past in st.spans:
+        T = past + n
+        j, i = torch.arange(T, device=q.device), torch.arange(past, T, device=q.device)[:, None]
+        rows = lambda pool: pool[st.block_tables[b, j // page].long(), :, j % page].to(F64)  # noqa: E731
+        K, V = rows(k_pool), rows(v_pool)[..., :dv]
+        seen = j[None] <= i
+        if window:
+            seen &= (i - j[None] < window) | (j[None] < keep_first)
+        if chunk:
+            seen &= i // chunk == j[None] // chunk
+        for h in range(H):
+            g = h // (H // G)
+            s = q[first:first + n, h].to(F64) @ K[:, g].T * scale
+            if temp:
+                s = s * (1 + temp[0] * torch.log(((i + 1) // temp[1] + 1).to(F64)))
+            if softcap:
+                s = softcap * torch.tanh(s / softcap)
+            if bias is not None:
+                s = s + bias[h].to(F64)[(i - j[None]).clamp(0, bias.shape[1] - 1)]
+            s = s.masked_fill(~seen, float("-inf"))
+            m = s.amax(1, keepdim=True) if sink is None else torch.maximum(s.amax(1, keepdim=True), sink[h].to(F64))
+            e = torch.exp(s - m)
+            out[first:first + n, h] = e @ V[:, g // div] / (e.sum(1, keepdim=True) + (0 if sink is None else torch.exp(sink[h].to(F64) - m)))
+    if gate is not None:
+        out = out * torch.sigmoid(gate.to(F64)).view(n_all, H, -1)
+    return out
+
+
+OPTIONS = {
+    "plain": (GROUPED, {}),
+    "window": (GROUPED, dict(window=40)),
+    "kept": (GROUPED, dict(window=33, keep_first=5)),
+    "cap_sink": (WIDE, dict(window=100, softcap=5.0, sink=True)),
+    "gate": (LATENT, dict(gate="head")),
+    "gates": (ONE, dict(window=70, gate="channel")),
+    "narrow": (NARROW, dict(sink=True)),
+    "rotated": (LATENT_ROT, dict(window=64, sink=True)),
+    "blocks": (PAIRED, dict(chunk=50, fp32=True)),
+    "bias": (GROUPED, dict(bias=90, temp=(0.3, 16), gate="head")),
+    "bias_wide": (WIDE, dict(bias=3000, temp=(0.1, 8))),
+    "bias_narrow": (NARROW, dict(bias=1)),
+}
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("portions,page", [(EDGES, 16), (EDGES, 7), ([(40, 900)], 16), ([(300, 0), (17, 300)], 32)], ids=["edges", "page7", "split", "long"])
+@pytest.mark.parametrize("name", OPTIONS)
+def test_tile_attention(name, portions, page, dtype):
+    layout, opt = OPTIONS[name]
+    H, G, dk, dv, div = layout
+    opt = dict(opt)
+    q, k_pool, v_pool, st, rnd = _case(layout, portions, page, dtype)
+    n, D, scale = q.shape[0], dv or 256, dk ** -0.5
+    kw = {k: opt[k] for k in ("window", "keep_first", "softcap", "chunk") if k in opt}
+    if opt.get("sink"):
+        kw["sink"] = rnd(H)
+    if "gate" in opt:
+        kw["gate"] = rnd(n, H if opt["gate"] == "head" else H * D).to(dtype)
+    bias = rnd(H, opt["bias"]) if "bias" in opt else None
+    extra = dict(bias_lut=bias, temp_coef=opt["temp"][0], temp_every=opt["temp"][1]) if "temp" in opt else dict(bias_lut=bias)
+    out = torch.full((n, H, D), 7.0, dtype=torch.float32 if opt.get("fp32") else dtype, device="cuda")
+    tiles = st.prompt_tiles(2, mixer_ops.TILE_ROWS // (H // G))[0]
+    mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, scale, max_context=st.max_context(),
+                             value_width=D, value_div=div, **kw, **extra)
+    want = _reference(q, k_pool, v_pool, st, D, div, scale, bias=bias, temp=opt.get("temp"), **kw)
+    ours = torch.cat([torch.arange(f, f + c) for f, c, _b, _p in st.spans if c > 1]).cuda()
+    # weights rounded to 8 (bf16) or 11 bits, summed with random signs: one rounding of the result and a share of one per weight
+    tol = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.5
+    err = (out[ours].to(F64) - want[ours]).norm() / want[ours].norm()
+    assert err <= tol, float(err)
+    assert (out[ours].to(F64) - want[ours]).abs().max() <= 16 * tol * want[ours].square().mean().sqrt() + 8 * tol * want[ours].abs().max()
+    left = [f for f, c, _b, _p in st.spans if c == 1]
+    assert all((out[f] == 7.0).all() for f in left)       # rows outside the tiles are another launch's
+
+
+def test_steep_scores_and_rescaling():
+    """Maxima that grow by hundreds from key tile to key tile, and rows whose first visible key tile comes late."""
+    q, k_pool, v_pool, st, rnd = _case((8, 2, 128, 128, 1), [(64, 500)], 16, torch.bfloat16)
+    st.block_tables[0, :36] = torch.arange(36, dtype=torch.int32, device="cuda")
+    k_pool[:36] *= torch.linspace(0.01, 12, 36, device="cuda").to(k_pool.dtype)[:, None, None, None]
+    out = torch.empty(64, 8, 128, dtype=torch.bfloat16, device="cuda")
+    tiles = st.prompt_tiles(2, 32)[0]
+    for window in (0, 60):
+        mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, 0.5, window=window)
+        want = _reference(q, k_pool, v_pool, st, 128, 1, 0.5, window=window)
+        assert (out.to(F64) - want).norm() / want.norm() <= 1.5 * 2.0 ** -8
