@@ -1302,6 +1302,8 @@ int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bi
   return tile_attn_supported(H, G, dk, dv, same_pool != 0, bias != 0, dtype) ? 1 : 0;
 }
 
+int b200_tile_attn_rows(int dk) { return tile_attn_rows(dk); }
+
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk) { return tile_attn_splits(n_tiles, key_tiles, G, dk); }
 
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
@@ -1345,7 +1347,7 @@ int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, c
     using T = std::remove_pointer_t<decltype(tag)>;
     auto merge = attn_split_combine_kernel<T>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    merge<<<dim3(n_tiles, kTileRows / (H / G)), 256, smem, s>>>(M, tiles, workspace, n_splits, n_tok, dv, nullptr);
+    merge<<<dim3(n_tiles, tile_attn_rows(dk) / (H / G)), 256, smem, s>>>(M, tiles, workspace, n_splits, n_tok, dv, nullptr);
     return check_launch("b200_tile_attn (merge)");
   });
 }

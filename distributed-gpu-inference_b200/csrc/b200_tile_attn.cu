@@ -1,20 +1,30 @@
 // Attention of prompt portions over the paged cache on the fifth-generation tensor cores (16-bit storage types).
 //
-// A CTA serves 128 query rows of one sequence and one kv head: up to 128 / rep consecutive tokens x the rep = H / G query heads that
-// read this kv head, so a key tile is fetched once for all of them.  Keys are walked in tiles of 64.
+// A CTA serves 256 query rows of one sequence and one kv head (128 where the head sizes leave no room for more): up to 256 / rep
+// consecutive tokens x the rep = H / G query heads that read this kv head, so a key tile is fetched once for all of them.  Keys are
+// walked in tiles of 64.
 //
-//   S = Q K^T   tcgen05.mma, 128 x 64, both operands in shared memory (128-byte swizzled lines), S in tensor memory, two of them
-//   P           256 threads, two per row: 32 scores each -> scale, query temperature, distance bias or soft cap, mask, running
-//               maximum, exp2 in fp32; rounded to the storage type into the tensor memory S was in
+//   S = Q K^T   tcgen05.mma, 128 x 64 per half of the rows, both operands in shared memory (128-byte swizzled lines), S in tensor
+//               memory, two of them per half
+//   P           four warps per half, one thread per row: scale, query temperature, distance bias or soft cap, mask, running maximum, exp2 in
+//               fp32; rounded to the storage type into the tensor memory S was in
 //   O += P V    tcgen05.mma with P from tensor memory; V lies in shared memory as the pool holds it (one line per key), read with the
 //               transposed descriptor; O stays in tensor memory in fp32 for the whole walk
 //
+// Four more warps copy pages (cp.async a tile or two ahead; any page size; rows past the sequence are zero-filled), one thread of a
+// another one issues the products; they meet at mbarriers only.  While the softmax works on tile i the tensor cores run S of tile i + 1 and
+// P V of tile i - 1.  256 rows per fetched tile halve what two CTAs of 128 rows per SM ask of L2 (32 KB per 64 keys and 4.2 MFLOP).
+//
+// Measured on B200 (bf16, 8 x 2048 tokens, 16 heads over 4 kv heads of 128): 212 us plain, 261 us with distance biases (the mma.sync
+// kernel: 1419), 141 us with a window of 512; latent 320 / 256, 4 x 1500 tokens of 16 heads behind 700, window 512: 142 us (417).
+// A tile of 64 keys x 256 rows takes about 2200 clocks: 1280 of the tensor cores (S with 64 columns is bound by reading Q from shared
+// memory), 1000 of exponentials (two warps per scheduler at four per clock), the copies 2000 (64 threads per pool); about a third of
+// the launch is the CTAs' beginnings and ends, which nothing covers with one CTA per SM.  128 rows and two CTAs: 242 and 321 us.
+//
 // O is scaled down only when a row's maximum has grown by more than 2^8 since the reference its weights use (the weights then reach
 // 256 at most, far inside both storage types, and the quotient O / l does not change): reading and writing O for every tile would
-// cost as many tensor-memory accesses as the scores.  While the threads work on tile i the tensor cores run P V of tile i - 1; two
-// CTAs share an SM where shared memory allows it (head sizes up to 128), so the products of one run under the softmax of the other.
-// Pages arrive by cp.async a tile ahead (any page size; rows past the sequence are zero-filled).  A latent cache (values = the first
-// DV columns of the key rows) is fetched once and read through both descriptors.
+// cost as many tensor-memory accesses as the scores.  A latent cache (values = the first DV columns of the key rows) is fetched once
+// and read through both descriptors.
 //
 // Steps that give fewer CTAs than the chip has room for divide the keys over several CTAs (gridDim.z), which leave (maximum, sum,
 // output) per row for the merge kernel of the older path.
@@ -31,14 +41,16 @@
 namespace b200 {
 namespace {
 
-constexpr int kRows = kTileRows, kKeys = 64, kNT = 256;
+constexpr int kRows = kTileRows, kKeys = 64;
+constexpr int kLoad = 128;                // threads that copy pages; kRows more per half do the softmax, one warp issues products
 constexpr int kBlk = kKeys * 128;        // bytes of 64 keys x 64 columns
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 constexpr float kSlack = 8.0f;           // growth of a row's maximum (in powers of two) that O is not rescaled for
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+  // no memory clobber: the rows of the next copies may be looked up in between (the group's commit and wait carry it)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0));
 }
 __device__ __forceinline__ void cp4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
@@ -62,16 +74,19 @@ __device__ __forceinline__ bool bar_done(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 // false when the barrier did not complete within about a second (or an earlier wait of the CTA already failed)
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
-  bool ok = bar_done(bar, parity);
+__device__ __forceinline__ bool bar_wait1(uint32_t bar, uint32_t parity, volatile int* dead) {
+  if (bar_done(bar, parity)) return true;
   const long long t0 = clock64();
-  while (!ok) {
-    ok = bar_done(bar, parity);
-    if (!ok && (*dead || clock64() - t0 > 2000000000ll)) {
+  while (!bar_done(bar, parity)) {
+    if (*dead || clock64() - t0 > 2000000000ll) {
       *dead = 1;
-      break;
+      return false;
     }
   }
+  return true;
+}
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {   // by a whole warp
+  const bool ok = bar_wait1(bar, parity, dead);
   __syncwarp();
   return ok;
 }
@@ -88,18 +103,25 @@ __device__ __forceinline__ constexpr uint32_t instr(int n, bool b_transposed) {
   return (1u << 4) | (type << 7) | (type << 10) | (b_transposed ? 1u << 16 : 0u) | (static_cast<uint32_t>(n / 8) << 17) |
          (static_cast<uint32_t>(kRows / 16) << 24);
 }
+// Executed by a whole warp: one elected lane issues.  Operands that are the same in all lanes stay in uniform registers that way; a
+// branch on the lane makes every operand of every product pass through a register move, which was most of the walk's time.
 __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool add) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a),
-               "l"(b), "r"(idesc), "r"(add ? 1u : 0u)
-               : "memory");
+  asm volatile(
+      "{\n.reg .pred p, q;\nelect.sync _|q, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(add ? 1u : 0u)
+      : "memory");
 }
 __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool add) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d), "r"(a),
-               "l"(b), "r"(idesc), "r"(add ? 1u : 0u)
-               : "memory");
+  asm volatile(
+      "{\n.reg .pred p, q;\nelect.sync _|q, 0xffffffff;\nsetp.ne.b32 p, %4, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(add ? 1u : 0u)
+      : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar)
+      : "memory");
 }
 
 __device__ __forceinline__ void tm_ld32(float (&r)[32], uint32_t addr) {
@@ -113,15 +135,12 @@ __device__ __forceinline__ void tm_ld32(float (&r)[32], uint32_t addr) {
         "=r"(u[30]), "=r"(u[31])
       : "r"(addr));
 }
-__device__ __forceinline__ void tm_st32(uint32_t addr, const float (&r)[32]) {
-  const uint32_t* u = reinterpret_cast<const uint32_t*>(r);
+__device__ __forceinline__ void tm_ld16(uint32_t (&u)[16], uint32_t addr) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,"
-      "%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(addr),
-      "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]), "r"(u[10]), "r"(u[11]),
-      "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15]), "r"(u[16]), "r"(u[17]), "r"(u[18]), "r"(u[19]), "r"(u[20]), "r"(u[21]), "r"(u[22]),
-      "r"(u[23]), "r"(u[24]), "r"(u[25]), "r"(u[26]), "r"(u[27]), "r"(u[28]), "r"(u[29]), "r"(u[30]), "r"(u[31])
-      : "memory");
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]),
+        "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+      : "r"(addr));
 }
 __device__ __forceinline__ void tm_st16(uint32_t addr, const uint32_t (&u)[16]) {
   asm volatile(
@@ -135,6 +154,16 @@ __device__ __forceinline__ float exp2_fast(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
+}
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 both(float x) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+// (a, b) <- (a, b) * k + m
+__device__ __forceinline__ void scale_shift(float& a, float& b, f32x2 k, f32x2 m) {
+  asm("{\n.reg .b64 t;\nmov.b64 t, {%0, %1};\nfma.rn.f32x2 t, t, %2, %3;\nmov.b64 {%0, %1}, t;\n}\n" : "+f"(a), "+f"(b) : "l"(k), "l"(m));
 }
 template <typename T>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
@@ -150,41 +179,43 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // shared memory of one CTA, from a 1024-byte boundary
 template <int DK, int DV, bool ALIAS>
 struct Plan {
-  static constexpr int kKBufs = ALIAS ? 3 : 2;
+  static constexpr int kHalves = DK <= 128 ? 2 : 1;     // sets of 128 rows
+  static constexpr int kSoft = kHalves * kRows, kNT = kSoft + kLoad + 32;
+  static constexpr int kBufs = 3;                       // of keys, and of values
   static constexpr int kQ = 0;
-  static constexpr int kK = kQ + DK / 64 * kRows * 128;
-  static constexpr int kV = kK + kKBufs * (DK / 64) * kBlk;
-  static constexpr int kEnd = kV + (ALIAS ? 0 : 2 * (DV / 64) * kBlk);
-  static constexpr int kMax = kEnd;                    // float [2][2][128]: row maxima of the two halves, by tile parity
-  static constexpr int kBar = kMax + 2 * 2 * kRows * 4;  // two barriers, the tensor memory's address, the failure flag
-  static constexpr int kLut = kBar + 64;               // float [3][rep][pitch]: biases of the tiles' distances
-  static constexpr int kO = 2 * kKeys;                 // columns of tensor memory: S0 | S1 | O
-  static constexpr int kTm = kO + DV <= 256 ? 256 : 512;
+  static constexpr int kK = kQ + kHalves * (DK / 64) * kRows * 128;
+  static constexpr int kV = kK + kBufs * (DK / 64) * kBlk;
+  static constexpr int kEnd = kV + (ALIAS ? 0 : kBufs * (DV / 64) * kBlk);
+  static constexpr int kBar = kEnd;                    // barriers, the tensor memory's address, the failure flag
+  static constexpr int kPage = kBar + 256;             // int [2][2][64]: rows of the pools that a tile's keys / values are in (-1: none)
+  static constexpr int kLut = kPage + 2 * 2 * kKeys * 4;  // float [4][rep][pitch]: biases of the tiles' distances
+  static constexpr int kO = 2 * kKeys;                 // columns of tensor memory per half: S0 | S1 | O
+  static constexpr int kHalfTm = kHalves == 2 ? 256 : 512;
+  static constexpr int kTm = 512;
+  static_assert(kO + DV <= kHalfTm, "tensor memory");
 };
 
 template <typename T, int DK, int DV, bool ALIAS, bool BIAS>
-__global__ void __launch_bounds__(kNT, DK <= 128 ? 2 : 1)
+__global__ void __launch_bounds__(Plan<DK, DV, ALIAS>::kNT, 1)
 tile_attn_kernel(const TileAttn A) {
   using P = Plan<DK, DV, ALIAS>;
+  constexpr int NB = P::kBufs, kSoft = P::kSoft;
   extern __shared__ unsigned char raw_smem[];
   unsigned char* sm = raw_smem + ((1024 - (smem_u32(raw_smem) & 1023)) & 1023);
   const uint32_t sm0 = smem_u32(sm);
-  float* mx_s = reinterpret_cast<float*>(sm + P::kMax);
-  const uint32_t bar_s = sm0 + P::kBar, bar_o = bar_s + 8;
-  volatile uint32_t* tm_slot = reinterpret_cast<volatile uint32_t*>(sm + P::kBar + 16);
-  volatile int* dead = reinterpret_cast<volatile int*>(sm + P::kBar + 20);
+  // barriers: queries in; keys of a buffer in, and read; values of a buffer in; P V of a value buffer done; per half: S of a buffer
+  // done, P of a buffer written.  All readers of one wait for a tile before the tile that completes it again can get that far.
+  const uint32_t bar_q = sm0 + P::kBar, bar_k = bar_q + 8, bar_ke = bar_k + 24, bar_v = bar_ke + 24, bar_o = bar_v + 24,
+                 bar_s = bar_o + 24, bar_p = bar_s + 32;
+  volatile uint32_t* tm_slot = reinterpret_cast<volatile uint32_t*>(sm + P::kBar + 192);
+  volatile int* dead = reinterpret_cast<volatile int*>(sm + P::kBar + 196);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row = 32 * (warp & 3) + lane, half = warp >> 2;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int g = blockIdx.y, rep = A.H / A.G, bs = A.block_size;
   const int tok0 = A.tiles[3 * blockIdx.x], trow = A.tiles[3 * blockIdx.x + 2];
-  const int cnt = min(A.tiles[3 * blockIdx.x + 1], kRows / rep), n_rows = cnt * rep;
+  const int cnt = min(A.tiles[3 * blockIdx.x + 1], kSoft / rep), n_rows = cnt * rep;
+  const int halves = P::kHalves == 2 && n_rows > kRows ? 2 : 1;       // in use
   const int p0 = A.tok_pos[tok0], p_last = p0 + cnt - 1;
-  const int32_t* table = A.block_tables + static_cast<int64_t>(trow) * A.table_stride;
-  const T* kp = static_cast<const T*>(A.k_pool);
-  const T* vp = static_cast<const T*>(A.v_pool);
-  const int Gv = A.G / A.v_div, gv = g / A.v_div;
-  const int bs_shift = (bs & (bs - 1)) == 0 ? __ffs(bs) - 1 : -1;
   auto first_seen = [&](int p) {
     int lo = A.window > 0 ? max(0, p - A.window + 1) : 0;
     if (A.chunk > 0) lo = max(lo, (p / A.chunk) * A.chunk);
@@ -202,273 +233,334 @@ tile_attn_kernel(const TileAttn A) {
     const int it = it0 + i;
     return (it < nA ? it : cB0 + it - nA) * kKeys;
   };
+  const int pitch = ((cnt + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep);
+  float* lut_s = reinterpret_cast<float*>(sm + P::kLut);
 
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_s));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_o));
+    auto init = [](uint32_t bar, int count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); };
+    init(bar_q, kSoft);
+    for (int b = 0; b < NB; ++b) {
+      init(bar_k + 8 * b, ALIAS ? kLoad : kLoad / 2);
+      init(bar_ke + 8 * b, 1);
+      init(bar_v + 8 * b, kLoad / 2);
+      init(bar_o + 8 * b, 1);
+    }
+    for (int b = 0; b < 4; ++b) {
+      init(bar_s + 8 * b, 1);
+      init(bar_p + 8 * b, kRows);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *dead = 0;
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sm0 + P::kBar + 16), "n"(P::kTm) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sm0 + P::kBar + 192), "n"(P::kTm) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-
-  // ---- loads --------------------------------------------------------------------------------------------------------------
-  auto page_row = [&](int j, int heads, int head) -> int64_t {
-    const int b = bs_shift >= 0 ? j >> bs_shift : j / bs;
-    return (static_cast<int64_t>(table[b]) * heads + head) * bs + (j - b * bs);
-  };
-  auto line = [](uint32_t base, int r, int ch, int rows) {     // 16-byte piece ch of row r: blocks of 64 columns, swizzled lines
-    return base + (ch >> 3) * (rows * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4);
-  };
-  {
-    constexpr int kCh = DK / 8;
-    const T* qp = static_cast<const T*>(A.q);
-    for (int c = tid; c < kRows * kCh; c += kNT) {
-      const int r = c / kCh, ch = c - r * kCh;
-      const int t = r / rep, hh = g * rep + r - t * rep;
-      const bool ok = r < n_rows;
-      cp16(line(sm0 + P::kQ, r, ch, kRows), ok ? qp + (tok0 + t) * A.q_tok_stride + hh * A.q_head_stride + ch * 8 : qp, ok);
-    }
-  }
-  auto load_rows = [&](uint32_t base, const T* pool, int heads, int head, int width, auto cols, int j0) {
-    constexpr int kCh = decltype(cols)::value / 8;
-#pragma unroll
-    for (int u = 0; u < kKeys * kCh / kNT; ++u) {
-      const int c = tid + u * kNT, key = c / kCh, ch = c - key * kCh, j = j0 + key;
-      const bool ok = j <= p_last;
-      cp16(line(base, key, ch, kKeys), ok ? pool + page_row(j, heads, head) * width + ch * 8 : pool, ok);
-    }
-  };
-  const int pitch = ((cnt + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep);
-  float* lut_s = reinterpret_cast<float*>(sm + P::kLut);
-  auto load_bias = [&](int i) {       // entry [hh][x]: the bias of distance p0 - key0 - 63 + x
-    if constexpr (BIAS) {
-      const int d0 = p0 - key0(i) - (kKeys - 1), span = cnt + kKeys - 1;
-      const uint32_t dst = smem_u32(lut_s + (i % 3) * rep * pitch);
-      for (int e = tid; e < rep * span; e += kNT) {
-        const int hh = e / span, x = e - hh * span;
-        cp4(dst + 4 * (hh * pitch + x), A.bias_lut + static_cast<int64_t>(g * rep + hh) * A.lut_len + min(max(d0 + x, 0), A.lut_len - 1));
-      }
-    }
-  };
-  auto load_k = [&](int i) {
-    if (i < n_it) {
-      load_rows(sm0 + P::kK + (i % P::kKBufs) * (DK / 64) * kBlk, kp, A.G, g, DK, std::integral_constant<int, DK>{}, key0(i));
-      if constexpr (BIAS) load_bias(i);
-    }
-    cp_commit();
-  };
-  auto load_v = [&](int i) {
-    if constexpr (!ALIAS) {
-      if (i < n_it) load_rows(sm0 + P::kV + (i & 1) * (DV / 64) * kBlk, vp, Gv, gv, A.v_row, std::integral_constant<int, DV>{}, key0(i));
-      cp_commit();
-    }
-  };
-
-  // ---- products, issued by one thread ---------------------------------------------------------------------------------------
-  auto issue_scores = [&](int i, uint32_t tm) {
-    const uint32_t k = sm0 + P::kK + (i % P::kKBufs) * (DK / 64) * kBlk;
-#pragma unroll
-    for (int kk = 0; kk < DK / 16; ++kk)
-      mma_ss(tm + (i & 1) * kKeys, operand(sm0 + P::kQ + (kk >> 2) * (kRows * 128) + (kk & 3) * 32, 16, 1024),
-             operand(k + (kk >> 2) * kBlk + (kk & 3) * 32, 16, 1024), instr<T>(kKeys, false), kk > 0);
-    mma_commit(bar_s);
-  };
-  auto issue_values = [&](int i, uint32_t tm) {
-    const uint32_t v = ALIAS ? sm0 + P::kK + (i % P::kKBufs) * (DK / 64) * kBlk : sm0 + P::kV + (i & 1) * (DV / 64) * kBlk;
-#pragma unroll
-    for (int kk = 0; kk < kKeys / 16; ++kk)
-      mma_ts(tm + P::kO, tm + (i & 1) * kKeys + 8 * kk, operand(v + kk * 2048, kBlk, 1024), instr<T>(DV, true), i > 0 || kk > 0);
-    mma_commit(bar_o);
-  };
-
-  // this thread's row
-  const int t_row = row / rep, h_row = g * rep + row - t_row * rep;
-  const bool live = row < n_rows;
-  const int p = live ? p0 + t_row : -1;
-  const int lo_p = live ? first_seen(p) : 0;
-  float mult = A.scale;
-  if (BIAS) mult *= 1.0f + A.temp_coef * logf(static_cast<float>((p + 1) / max(A.temp_every, 1)) + 1.0f);
-  const float c2 = mult * kLog2e, two_over_cap = A.softcap > 0.f ? 2.0f / A.softcap : 0.f;
-  float m_ref = -INFINITY, l = 0.f;
-
-  load_k(0);
-  load_k(1);
-  load_v(0);
-  cp_wait<ALIAS ? 1 : 2>();          // the queries and the first keys
-  fence_smem_to_mma();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tm = *tm_slot;
-  const uint32_t tm_row = tm + (static_cast<uint32_t>(32 * (warp & 3)) << 16);
-  bool ok = true;
-  if (n_it > 0 && tid == 0) issue_scores(0, tm);
-  __syncwarp();
+  const uint32_t tm = __shfl_sync(0xffffffffu, *tm_slot, 0);
 
-  for (int i = 0; i < n_it; ++i) {
-    ok = bar_wait(bar_s, i & 1, dead) && ok;
-    tc_fence_after();
-    if constexpr (!ALIAS) load_k(i + 2);        // the product that just completed was the last reader of that buffer
-    const int j0 = key0(i);
-    float s[32];
-    tm_ld32(s, tm_row + (i & 1) * kKeys + half * 32);
-    tc_wait_ld();
-    // scores in powers of two
-    if constexpr (BIAS) {
-      const float* b = lut_s + (i % 3) * rep * pitch + (row - t_row * rep) * pitch + t_row + (kKeys - 1) - half * 32;
-#pragma unroll
-      for (int c = 0; c < 32; ++c) s[c] = fmaf(live ? b[-c] : 0.f, kLog2e, s[c] * c2);
-    } else if (A.softcap > 0.f) {
-#pragma unroll
-      for (int c = 0; c < 32; ++c)
-        s[c] = kLog2e * A.softcap * (1.0f - __fdividef(2.0f, __expf(s[c] * mult * two_over_cap) + 1.0f));
-    } else {
-#pragma unroll
-      for (int c = 0; c < 32; ++c) s[c] *= c2;
-    }
-    // keys in sight of every token of the tile need no mask
-    if (j0 + kKeys - 1 > p0 || j0 < first_seen(p_last) || cnt * rep < kRows) {
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const int j = j0 + half * 32 + c;
-        if (!(j <= p && (j >= lo_p || (A.window > 0 && j < A.keep_first)))) s[c] = -INFINITY;
+  auto line = [](uint32_t base, int r, int ch, int rows) {     // 16-byte piece ch of row r: blocks of 64 columns, swizzled lines
+    return base + (ch >> 3) * (rows * 128) + r * 128 + (((ch & 7) ^ (r & 7)) << 4);
+  };
+  // P V of tile i is done, for all rows
+  auto values_done = [&](int i) { return bar_wait(bar_o + 8 * (i % NB), (i / NB) & 1, dead); };
+
+  if (warp >= kSoft / 32 && warp < (kSoft + kLoad) / 32) {
+    // ---- the warps that copy pages: half of them keys, half values; a latent cache: all of them its rows ------------------------
+    const bool values = !ALIAS && warp >= kSoft / 32 + kLoad / 64;
+    constexpr int kTeam = ALIAS ? kLoad : kLoad / 2;
+    const int me = (tid - kSoft) % kTeam;
+    const T* pool = static_cast<const T*>(values ? A.v_pool : A.k_pool);
+    const int heads = values ? A.G / A.v_div : A.G, head = values ? g / A.v_div : g, width = values ? A.v_row : DK;
+    const int32_t* table = A.block_tables + static_cast<int64_t>(trow) * A.table_stride;
+    const int shift = (bs & (bs - 1)) == 0 ? __ffs(bs) - 1 : -1;
+    int* rows_s = reinterpret_cast<int*>(sm + P::kPage) + (values ? 2 * kKeys : 0);
+    // the page of one key of a tile, looked up by the team's first 64 threads a tile ahead of its copies
+    auto look_up = [&](int i) {
+      const int j = key0(i) + me;
+      return me < kKeys && i < n_it && j <= p_last ? table[shift >= 0 ? j >> shift : j / bs] : -1;
+    };
+    auto copy = [&](int i, int page) {
+      if (me < kKeys) {
+        const int j = key0(i) + me, off = shift >= 0 ? j & (bs - 1) : j % bs;
+        rows_s[(i & 1) * kKeys + me] = page < 0 ? -1 : (page * heads + head) * bs + off;
       }
-    }
-    float mx = s[0];
-#pragma unroll
-    for (int c = 1; c < 32; ++c) mx = fmaxf(mx, s[c]);
-    float* ex = mx_s + (i & 1) * 2 * kRows;
-    ex[half * kRows + row] = mx;
-    asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");    // the two warps of these 32 rows
-    mx = fmaxf(mx, ex[(half ^ 1) * kRows + row]);
-    if (i > 0) {
-      ok = bar_wait(bar_o, (i - 1) & 1, dead) && ok;
-      tc_fence_after();
-      load_v(i + 1);
-    } else {
-      load_v(1);
-    }
-    if constexpr (ALIAS) load_k(i + 2);
-    const bool grow = mx > m_ref + kSlack || (m_ref == -INFINITY && mx > -INFINITY);
-    if (__any_sync(0xffffffffu, grow)) {
-      const float corr = grow ? exp2_fast(m_ref - mx) : 1.0f;      // 0 where nothing was seen before
-      if (grow) m_ref = mx;
-      l *= corr;
-      if (i > 0) {
+      asm volatile("bar.sync %0, %1;" ::"r"(values ? 2 : 1), "n"(kTeam) : "memory");
+      const uint32_t base = values ? sm0 + P::kV + (i % NB) * (DV / 64) * kBlk : sm0 + P::kK + (i % NB) * (DK / 64) * kBlk;
+      auto move = [&](auto cols) {
+        constexpr int kCh = decltype(cols)::value / 8;
+        constexpr int kPer = kKeys * kCh / kTeam, kBatch = kPer % 8 == 0 ? 8 : (kPer % 10 == 0 ? 10 : 4);
+        static_assert(kPer % kBatch == 0, "copies per thread");
 #pragma unroll 1
-        for (int c = 0; c < DV / 2; c += 32) {
-          float o[32];
-          tm_ld32(o, tm_row + P::kO + half * (DV / 2) + c);
-          tc_wait_ld();
+        for (int u0 = 0; u0 < kPer; u0 += kBatch) {
+          int r[kBatch];
 #pragma unroll
-          for (int x = 0; x < 32; ++x) o[x] *= corr;
-          tm_st32(tm_row + P::kO + half * (DV / 2) + c, o);
+          for (int u = 0; u < kBatch; ++u) r[u] = rows_s[(i & 1) * kKeys + (me + (u0 + u) * kTeam) / kCh];
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) {
+            const int c = me + (u0 + u) * kTeam, key = c / kCh, ch = c - key * kCh;
+            cp16(line(base, key, ch, kKeys), r[u] >= 0 ? pool + static_cast<int64_t>(r[u]) * width + ch * 8 : pool, r[u] >= 0);
+          }
+        }
+      };
+      if (DK == DV || !values) move(std::integral_constant<int, DK>{});
+      else move(std::integral_constant<int, DV>{});
+      if (BIAS && !values) {      // entry [hh][x]: the bias of distance p0 - key0 - 63 + x
+        const int d0 = p0 - key0(i) - (kKeys - 1), span = cnt + kKeys - 1;
+        const uint32_t dst = smem_u32(lut_s + (i & 3) * rep * pitch);
+        for (int hh = 0; hh < rep; ++hh) {
+          const float* src = A.bias_lut + static_cast<int64_t>(g * rep + hh) * A.lut_len;
+          for (int x = me; x < span; x += kTeam) cp4(dst + 4 * (hh * pitch + x), src + min(max(d0 + x, 0), A.lut_len - 1));
         }
       }
+      cp_commit();
+    };
+    auto arrived = [&](int i) {     // this thread's copies of the tile are in shared memory, for the tensor cores too
+      fence_smem_to_mma();
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((values ? bar_v : bar_k) + 8 * (i % NB)) : "memory");
+    };
+    int page = look_up(0);
+    const int ahead = min(n_it, NB);
+    for (int i = 0; i < ahead; ++i) {      // a tile is handed over while the next one is under way
+      const int next = look_up(i + 1);
+      copy(i, page);
+      page = next;
+      if (i > 0) {
+        cp_wait<1>();
+        arrived(i - 1);
+      }
     }
-    const float m_safe = m_ref == -INFINITY ? 0.f : m_ref;          // a row that sees no key yet keeps weights 0
-    uint32_t w[16];
-    float sum0 = 0.f, sum1 = 0.f;
+    cp_wait<0>();
+    if (ahead > 0) arrived(ahead - 1);
+    for (int i = ahead; i < n_it; ++i) {
+      const int next = look_up(i + 1);
+      if (values || ALIAS) values_done(i - NB);
+      else bar_wait(bar_ke + 8 * (i % NB), (i / NB - 1) & 1, dead);
+      copy(i, page);
+      page = next;
+      cp_wait<0>();
+      arrived(i);
+    }
+  } else if (warp == (kSoft + kLoad) / 32) {
+    // ---- products -----------------------------------------------------------------------------------------------------------------
+    {
+      auto scores = [&](int i) {
+        const uint32_t k = sm0 + P::kK + (i % NB) * (DK / 64) * kBlk;
+        bar_wait(bar_k + 8 * (i % NB), (i / NB) & 1, dead);
+        tc_fence_after();
+        for (int hf = 0; hf < halves; ++hf) {
 #pragma unroll
-    for (int c = 0; c < 32; c += 2) {
-      const float a = exp2_fast(s[c] - m_safe), b = exp2_fast(s[c + 1] - m_safe);
-      sum0 += a;
-      sum1 += b;
-      w[c >> 1] = pack2<T>(a, b);
+          for (int kk = 0; kk < DK / 16; ++kk)
+            mma_ss(tm + hf * P::kHalfTm + (i & 1) * kKeys,
+                   operand(sm0 + P::kQ + (hf * (DK / 64) + (kk >> 2)) * (kRows * 128) + (kk & 3) * 32, 16, 1024),
+                   operand(k + (kk >> 2) * kBlk + (kk & 3) * 32, 16, 1024), instr<T>(kKeys, false), kk > 0);
+          mma_commit(bar_s + 16 * hf + 8 * (i & 1));
+        }
+        if (!ALIAS) mma_commit(bar_ke + 8 * (i % NB));
+      };
+      bar_wait(bar_q, 0, dead);
+      if (n_it > 0) scores(0);
+      for (int i = 0; i < n_it; ++i) {
+        if (i + 1 < n_it) {
+          // S of tile i + 1 goes where P of tile i - 1 is being read
+          if (i > 0) bar_wait(bar_o + 8 * ((i - 1) % NB), ((i - 1) / NB) & 1, dead);
+          scores(i + 1);
+        }
+        if (!ALIAS) bar_wait(bar_v + 8 * (i % NB), (i / NB) & 1, dead);
+        const uint32_t v = ALIAS ? sm0 + P::kK + (i % NB) * (DK / 64) * kBlk : sm0 + P::kV + (i % NB) * (DV / 64) * kBlk;
+        for (int hf = 0; hf < halves; ++hf) {
+          bar_wait(bar_p + 16 * hf + 8 * (i & 1), (i >> 1) & 1, dead);
+          tc_fence_after();
+          const uint32_t t = tm + hf * P::kHalfTm;
+#pragma unroll
+          for (int kk = 0; kk < kKeys / 16; ++kk)
+            mma_ts(t + P::kO, t + (i & 1) * kKeys + 8 * kk, operand(v + kk * 2048, kBlk, 1024), instr<T>(DV, true), i > 0 || kk > 0);
+        }
+        mma_commit(bar_o + 8 * (i % NB));
+      }
     }
-    l += sum0 + sum1;
-    tm_st16(tm_row + (i & 1) * kKeys + half * 16, w);
-    tc_wait_st();
-    cp_wait<ALIAS ? 1 : 2>();        // the next keys and (own pool) this tile's values are in
-    fence_smem_to_mma();
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
+    __syncwarp();
+  } else {
+    // ---- softmax: thread = row -------------------------------------------------------------------------------------------------------
+    {
+      constexpr int kCh = DK / 8;
+      const T* qp = static_cast<const T*>(A.q);
+#pragma unroll 8
+      for (int u = 0; u < kCh; ++u) {
+        const int c = tid + u * kSoft, r = c / kCh, ch = c - r * kCh;
+        const int t = r / rep, hh = g * rep + r - t * rep;
+        const bool in = r < n_rows;
+        cp16(line(sm0 + P::kQ + (r / kRows) * (DK / 64) * (kRows * 128), r % kRows, ch, kRows), in ? qp + (tok0 + t) * A.q_tok_stride + hh * A.q_head_stride + ch * 8 : qp, in);
+      }
+      cp_commit();
+      cp_wait<0>();
+      fence_smem_to_mma();
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_q) : "memory");
+    }
+    const int hf = tid / kRows;
+    const uint32_t tm_row = tm + hf * P::kHalfTm + (static_cast<uint32_t>(32 * (warp & 3)) << 16);
+    const uint32_t my_s = bar_s + 16 * hf, my_p = bar_p + 16 * hf;
+    const int mine = hf < halves ? n_it : 0;
+    const int row = tid, t_row = row / rep, hh = row - t_row * rep, h_row = g * rep + hh;
+    const bool live = row < n_rows;
+    const int p = live ? p0 + t_row : -1;
+    const int lo_p = live ? first_seen(p) : 0, lo_last = first_seen(p_last);
+    float mult = A.scale;
+    if (BIAS) mult *= 1.0f + A.temp_coef * logf(static_cast<float>((p + 1) / max(A.temp_every, 1)) + 1.0f);
+    const float two_over_cap = A.softcap > 0.f ? 2.0f / A.softcap : 0.f;
+    // plain scores are compared before they are scaled: weight = 2^(s * k2 - m), in one multiply-add
+    const bool plain = !BIAS && A.softcap <= 0.f && mult > 0.f;
+    const float k2 = plain ? mult * kLog2e : kLog2e;
+    float m_ref = -INFINITY, l = 0.f;       // in powers of two; -inf until the row sees a key
+    bool ok = true;
+
+    for (int i = 0; i < mine; ++i) {
+      const int j0 = key0(i);
+      ok = bar_wait(my_s + 8 * (i & 1), (i >> 1) & 1, dead) && ok;
       tc_fence_after();
-      if (i + 1 < n_it) issue_scores(i + 1, tm);
-      issue_values(i, tm);
+      float s[2][32];
+      tm_ld32(s[0], tm_row + (i & 1) * kKeys);
+      tm_ld32(s[1], tm_row + (i & 1) * kKeys + 32);
+      tc_wait_ld();
+      if constexpr (BIAS) {
+        const float* b = lut_s + ((i & 3) * rep + (live ? hh : 0)) * pitch + (live ? t_row : 0) + kKeys - 1;
+#pragma unroll
+        for (int c = 0; c < kKeys; ++c) s[c >> 5][c & 31] = fmaf(s[c >> 5][c & 31], mult, b[-c]);
+      } else if (!plain) {
+#pragma unroll
+        for (int c = 0; c < kKeys; ++c) {
+          float x = s[c >> 5][c & 31] * mult;
+          if (A.softcap > 0.f) x = A.softcap * (1.0f - __fdividef(2.0f, __expf(x * two_over_cap) + 1.0f));
+          s[c >> 5][c & 31] = x;
+        }
+      }
+      // keys in sight of every token of the tile need no mask
+      if (j0 + kKeys - 1 > p0 || j0 < lo_last || n_rows < halves * kRows) {
+#pragma unroll
+        for (int c = 0; c < kKeys; ++c) {
+          const int j = j0 + c;
+          if (!(j <= p && (j >= lo_p || (A.window > 0 && j < A.keep_first)))) s[c >> 5][c & 31] = -INFINITY;
+        }
+      }
+      float mx[4] = {s[0][0], s[0][1], s[0][2], s[0][3]};
+#pragma unroll
+      for (int c = 4; c < kKeys; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c >> 5][c & 31]);
+      const float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * k2;
+      const bool grow = m_new > m_ref + kSlack || (m_ref == -INFINITY && m_new > -INFINITY);
+      if (__any_sync(0xffffffffu, grow)) {
+        const float corr = grow ? exp2_fast(m_ref - m_new) : 1.0f;      // 0 where nothing was seen before
+        if (grow) m_ref = m_new;
+        l *= corr;
+        if (i > 0) {
+          ok = values_done(i - 1) && ok;
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < DV; c += 16) {
+            uint32_t o[16];
+            tm_ld16(o, tm_row + P::kO + c);
+            tc_wait_ld();
+#pragma unroll
+            for (int x = 0; x < 16; ++x) o[x] = __float_as_uint(__uint_as_float(o[x]) * corr);
+            tm_st16(tm_row + P::kO + c, o);
+          }
+        }
+      }
+      const f32x2 kk = both(k2), mm = both(m_ref == -INFINITY ? 0.f : -m_ref);     // a row that sees no key yet keeps weights 0
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        uint32_t w[16];
+#pragma unroll
+        for (int c = 0; c < 32; c += 2) {
+          float a = s[x][c], b = s[x][c + 1];
+          scale_shift(a, b, kk, mm);
+          a = exp2_fast(a);
+          b = exp2_fast(b);
+          sum[c & 2] += a;
+          sum[(c & 2) + 1] += b;
+          w[c >> 1] = pack2<T>(a, b);
+        }
+        tm_st16(tm_row + (i & 1) * kKeys + x * 16, w);
+      }
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      tc_wait_st();
+      tc_fence_before();
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(my_p + 8 * (i & 1)) : "memory");
+    }
+    if (mine > 0) {
+      ok = values_done(n_it - 1) && ok;
+      tc_fence_after();
+    }
+
+    // ---- sink, gate, output --------------------------------------------------------------------------------------------------------
+    ok = ok && !*dead;
+    const float m_nat = m_ref * kLn2;
+    const int64_t n = tok0 + t_row;
+    if (gridDim.z > 1) {
+      float* dst = A.ws + ((static_cast<int64_t>(blockIdx.z) * A.n_tok + n) * A.H + h_row) * (DV + 2);
+      if (live) {
+        dst[0] = ok ? m_nat : NAN;
+        dst[1] = l;
+      }
+#pragma unroll 1
+      for (int c = 0; c < DV; c += 32) {
+        float o[32];
+        __syncwarp();
+        if (n_it > 0) {
+          tm_ld32(o, tm_row + P::kO + c);
+          tc_wait_ld();
+        }
+        if (live) {
+#pragma unroll
+          for (int x = 0; x < 32; x += 2)
+            *reinterpret_cast<float2*>(dst + 2 + c + x) = n_it > 0 ? make_float2(o[x], o[x + 1]) : make_float2(0.f, 0.f);
+        }
+      }
+    } else {
+      float f = 1.0f / l;
+      if (A.sink && live) {
+        const float sk = A.sink[h_row], M = fmaxf(m_nat, sk);
+        const float e = expf(m_nat - M);
+        f = e / (l * e + expf(sk - M));
+      }
+      if (!ok) f = NAN;
+      const T* gate = static_cast<const T*>(A.gate);
+      if (gate && live && !A.gate_dim) f *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row])));
+#pragma unroll 1
+      for (int c = 0; c < DV; c += 32) {
+        float o[32];
+        __syncwarp();
+        tm_ld32(o, tm_row + P::kO + c);
+        tc_wait_ld();
+        if (!live) continue;       // reconverges at the loop's head
+#pragma unroll
+        for (int x = 0; x < 32; ++x) {
+          o[x] *= f;
+          if (gate && A.gate_dim) o[x] *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row * A.gate_dim + c + x])));
+        }
+        const int64_t at = n * A.out_tok_stride + h_row * A.out_head_stride + c;
+        if (A.out_f32) {
+          float* dst = static_cast<float*>(A.out) + at;
+#pragma unroll
+          for (int x = 0; x < 32; x += 2) *reinterpret_cast<float2*>(dst + x) = make_float2(o[x], o[x + 1]);
+        } else {
+          T* dst = static_cast<T*>(A.out) + at;
+          if (A.out_vec) {
+#pragma unroll
+            for (int x = 0; x < 32; x += 8)
+              *reinterpret_cast<uint4*>(dst + x) = make_uint4(pack2<T>(o[x], o[x + 1]), pack2<T>(o[x + 2], o[x + 3]),
+                                                              pack2<T>(o[x + 4], o[x + 5]), pack2<T>(o[x + 6], o[x + 7]));
+          } else {
+#pragma unroll
+            for (int x = 0; x < 32; x += 2) *reinterpret_cast<uint32_t*>(dst + x) = pack2<T>(o[x], o[x + 1]);
+          }
+        }
+      }
     }
     __syncwarp();
   }
-  if (n_it > 0) {
-    ok = bar_wait(bar_o, (n_it - 1) & 1, dead) && ok;
-    tc_fence_after();
-  }
-  cp_wait<0>();
-
-  // ---- the rows' sums, sink, gate, output --------------------------------------------------------------------------------------
-  mx_s[half * kRows + row] = l;
-  __syncthreads();
-  l += mx_s[(half ^ 1) * kRows + row];
-  ok = ok && !*dead;
-  const float m_nat = m_ref * kLn2;
-  const int64_t n = tok0 + t_row;
-  if (gridDim.z > 1) {
-    float* dst = A.ws + ((static_cast<int64_t>(blockIdx.z) * A.n_tok + n) * A.H + h_row) * (DV + 2);
-    if (live && half == 0) {
-      dst[0] = ok ? m_nat : NAN;
-      dst[1] = l;
-    }
-#pragma unroll 1
-    for (int c = 0; c < DV / 2; c += 32) {
-      float o[32];
-      __syncwarp();
-      if (n_it > 0) {
-        tm_ld32(o, tm_row + P::kO + half * (DV / 2) + c);
-        tc_wait_ld();
-      }
-      if (live) {
-#pragma unroll
-        for (int x = 0; x < 32; x += 2)
-          *reinterpret_cast<float2*>(dst + 2 + half * (DV / 2) + c + x) = n_it > 0 ? make_float2(o[x], o[x + 1]) : make_float2(0.f, 0.f);
-      }
-    }
-  } else {
-    float f = 1.0f / l;
-    if (A.sink && live) {
-      const float sk = A.sink[h_row], M = fmaxf(m_nat, sk);
-      const float e = expf(m_nat - M);
-      f = e / (l * e + expf(sk - M));
-    }
-    if (!ok) f = NAN;
-    const T* gate = static_cast<const T*>(A.gate);
-    if (gate && live && !A.gate_dim) f *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row])));
-#pragma unroll 1
-    for (int c = 0; c < DV / 2; c += 32) {
-      float o[32];
-      __syncwarp();
-      tm_ld32(o, tm_row + P::kO + half * (DV / 2) + c);
-      tc_wait_ld();
-      if (!live) continue;       // reconverges at the loop's head
-      const int col = half * (DV / 2) + c;
-#pragma unroll
-      for (int x = 0; x < 32; ++x) {
-        o[x] *= f;
-        if (gate && A.gate_dim) o[x] *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row * A.gate_dim + col + x])));
-      }
-      const int64_t at = n * A.out_tok_stride + h_row * A.out_head_stride + col;
-      if (A.out_f32) {
-        float* dst = static_cast<float*>(A.out) + at;
-#pragma unroll
-        for (int x = 0; x < 32; x += 2) *reinterpret_cast<float2*>(dst + x) = make_float2(o[x], o[x + 1]);
-      } else {
-        T* dst = static_cast<T*>(A.out) + at;
-        if (A.out_vec) {
-#pragma unroll
-          for (int x = 0; x < 32; x += 8)
-            *reinterpret_cast<uint4*>(dst + x) = make_uint4(pack2<T>(o[x], o[x + 1]), pack2<T>(o[x + 2], o[x + 3]),
-                                                            pack2<T>(o[x + 4], o[x + 5]), pack2<T>(o[x + 6], o[x + 7]));
-        } else {
-#pragma unroll
-          for (int x = 0; x < 32; x += 2) *reinterpret_cast<uint32_t*>(dst + x) = pack2<T>(o[x], o[x + 1]);
-        }
-      }
-    }
-  }
-  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "n"(P::kTm));
@@ -479,13 +571,12 @@ int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stre
   using P = Plan<DK, DV, ALIAS>;
   const int rep = A.H / A.G;
   size_t smem = 1024 + P::kLut;
-  if (BIAS) smem += sizeof(float) * 3 * rep * (((kRows / rep + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep));
-  // tensor memory (512 columns per SM) has room for two CTAs of 256 columns: shared memory admits no third one
-  smem = std::max<size_t>(smem, P::kTm == 256 ? 80 * 1024 : 120 * 1024);
+  if (BIAS) smem += sizeof(float) * 4 * rep * (((P::kSoft / rep + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep));
+  smem = std::max<size_t>(smem, 120 * 1024);      // a CTA takes all of an SM's tensor memory: one per SM
   if (smem > 227 * 1024) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
   auto kern = tile_attn_kernel<T, DK, DV, ALIAS, BIAS>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  kern<<<dim3(n_tiles, A.G, n_splits), kNT, smem, stream>>>(A);
+  kern<<<dim3(n_tiles, A.G, n_splits), P::kNT, smem, stream>>>(A);
   return check_launch("b200_tile_attn");
 }
 
@@ -507,15 +598,18 @@ int launch_shape(const TileAttn& A, int dk, int dv, bool alias, int n_tiles, int
 
 bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, int dtype) {
   if (dtype != B200_DTYPE_BF16 && dtype != B200_DTYPE_F16) return false;
-  if (H <= 0 || G <= 0 || H % G || H / G > (bias ? 16 : kRows)) return false;
+  if (H <= 0 || G <= 0 || H % G || H / G > (bias ? 16 : kTileRows)) return false;
   if (alias) return !bias && dv == 256 && (dk == 256 || dk == 320);
   return dk == dv && (dk == 64 || dk == 128);
 }
 
+int tile_attn_rows(int dk) { return dk <= 128 ? 2 * kTileRows : kTileRows; }
+
 int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk) {
-  const int64_t ctas = static_cast<int64_t>(n_tiles) * G, room = (dk <= 128 ? 2 : 1) * kNumSMs;
-  if (ctas <= 0 || ctas * 2 > room) return 1;
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({16, room / ctas, key_tiles / 3})));
+  (void)dk;
+  const int64_t ctas = static_cast<int64_t>(n_tiles) * G;
+  if (ctas <= 0 || ctas * 2 > kNumSMs) return 1;
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({16, kNumSMs / ctas, key_tiles / 3})));
 }
 
 int tile_attn_launch(const TileAttn& A, int dk, int dv, bool alias, int n_tiles, int n_splits, int dtype, cudaStream_t stream) {

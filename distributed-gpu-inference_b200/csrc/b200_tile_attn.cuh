@@ -7,7 +7,7 @@
 
 namespace b200 {
 
-constexpr int kTileRows = 128;   // query rows of a tile: up to 128 / (H / G) tokens
+constexpr int kTileRows = 128;   // rows of a product; a tile has one or two times as many (tile_attn_rows)
 
 struct TileAttn {
   void* out; int64_t out_tok_stride, out_head_stride;
@@ -27,6 +27,7 @@ struct TileAttn {
 };
 
 bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, int dtype);
+int tile_attn_rows(int dk);
 int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk);
 int tile_attn_launch(const TileAttn& A, int dk, int dv, bool alias, int n_tiles, int n_splits, int dtype, cudaStream_t stream);
 

@@ -525,7 +525,9 @@ def mixed_prompt_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Ten
     _lib.check_mixers(rc, "b200_mixed_prompt_attn")
 
 
-TILE_ROWS = 128             # query rows (tokens x heads of a kv group) a CTA of ``tile_attention`` serves
+def tile_tokens(H: int, G: int, dk: int) -> int:
+    """Tokens of one sequence a CTA of ``tile_attention`` serves: 256 rows over the heads of a kv group, 128 for the widest heads."""
+    return max(1, int(_lib_().b200_tile_attn_rows(int(dk))) // (H // G))
 
 
 def tile_attention_supported(H: int, G: int, dk: int, dv: int, same_pool: bool, bias: bool, dtype: torch.dtype) -> bool:
@@ -534,9 +536,12 @@ def tile_attention_supported(H: int, G: int, dk: int, dv: int, same_pool: bool, 
 
 
 def tile_attention_from(H: int, G: int) -> int:
-    """Tokens from which a portion goes to ``tile_attention``: from half a tile's rows on.  Below, most of the 128 rows of a product
-    would be padding."""
-    return max(2, TILE_ROWS // 2 // (H // G))
+    """Tokens from which a portion goes to ``tile_attention``: from two tokens and 8 rows (tokens x heads of a kv group) on.  Most of
+    the 128 rows of a product are padding then, but the walk is as long as one of the 16-row kernels and divides the keys over as
+    many CTAs (B200, 16 heads over 4: two tokens per sequence, 8 sequences at 4000: 44 us, 50 with biases, against 96 / 183 us in 16-row
+    tiles; 48 sequences: 197 / 255 against 346 / 225; nothing cached: level at launch latency; 32 tokens, 48 sequences at 1000: 61 / 75
+    against 262 / 207)."""
+    return max(2, 8 // (H // G))
 
 
 @_timed
@@ -546,7 +551,7 @@ def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_p
                    value_width: Optional[int] = None, value_div: int = 1, bias_lut: Optional[torch.Tensor] = None,
                    temp_coef: float = 0.0, temp_every: int = 1) -> None:
     """``mixed_prompt_attention`` (or, with ``bias_lut``, ``biased_prompt_attention``) for prompt portions in tiles of up to
-    ``TILE_ROWS`` rows: ``tiles`` int32 ``[n_tiles, 3]`` with up to ``TILE_ROWS // (H // G)`` consecutive tokens of one sequence each.
+    128 or 256 rows: ``tiles`` int32 ``[n_tiles, 3]`` with up to ``tile_tokens(H, G, dk)`` consecutive tokens of one sequence each.
     Only the tiles' rows of ``out`` are written, so the other portions of a step may go through another kernel."""
     _need_cuda(out, q, k_pool, v_pool, block_tables, tiles, tok_pos)
     nb, G, bs, dk = k_pool.shape
@@ -566,9 +571,9 @@ def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_p
         raise ValueError("bias_lut must be contiguous fp32 [H, L]")
     per_channel = _gate_kind(gate, n, H, dv, q.dtype)
     lib = _lib_()
-    seen = min(max_context, window + keep_first + TILE_ROWS) if window > 0 else max_context
+    seen = min(max_context, window + keep_first + 128) if window > 0 else max_context
     if chunk > 0:
-        seen = min(seen, chunk + TILE_ROWS)
+        seen = min(seen, chunk + 128)
     splits = lib.b200_tile_attn_splits(tiles.shape[0], (seen + 63) // 64, G, dk) if max_context > 0 else 1
     ws = torch.empty((splits, n, H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
     rc = lib.b200_tile_attn(out.data_ptr(), out.stride(0), out.stride(1), q.data_ptr(), q.stride(0), q.stride(1), _ptr(gate),

@@ -464,11 +464,12 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
                                 float* workspace, int dtype, void* stream);
 
 /* b200_mixed_prompt_attn_ext2 and b200_biased_prompt_attn for prompt portions on the fifth-generation tensor cores: tiles of up to
- * 128 / (H / G) tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
+ * b200_tile_attn_rows(dk) / (H / G) tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
  * touched.  bias_lut fp32 [H][lut_len] with temp_coef / temp_every as in b200_biased_prompt_attn, or NULL.  The values are v_pool's
  * rows, or the first dv columns of the key rows when v_pool == k_pool.  n_splits > 1 divides the keys over as many CTAs and needs a
  * workspace fp32 [n_splits][n_tok][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte aligned query rows. */
 int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bias, int dtype);
+int b200_tile_attn_rows(int dk);
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk);
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,

@@ -1,4 +1,4 @@
-"""Prompt attention in tiles of 128 rows against float64: portions around the tiles' edges, contexts around the key tiles', every mask
+"""Prompt attention in tiles of 128 or 256 rows against float64: portions around the tiles' edges, contexts around the key tiles', every mask
 and option the layers use, head layouts of each instantiation, page sizes that are no power of two, keys divided over CTAs."""
 import pytest
 import torch
@@ -13,7 +13,7 @@ F64 = torch.float64
 GROUPED, WIDE, NARROW, ONE, LATENT, LATENT_ROT, PAIRED = ((8, 2, 128, 128, 1), (16, 1, 128, 128, 1), (6, 2, 64, 64, 1), (3, 3, 128, 128, 1),
                                                           (8, 1, 256, 0, 1), (16, 1, 320, 0, 1), (8, 4, 128, 128, 2))
 # portions as (new tokens, tokens before)
-EDGES = [(32, 0), (33, 31), (31, 64), (64, 1), (65, 200), (128, 0), (1, 5)]
+EDGES = [(32, 0), (33, 31), (31, 64), (64, 1), (65, 200), (130, 0), (1, 5)]
 
 
 def _case(layout, portions, page, dtype):
@@ -103,7 +103,7 @@ def test_tile_attention(name, portions, page, dtype):
     bias = rnd(H, opt["bias"]) if "bias" in opt else None
     extra = dict(bias_lut=bias, temp_coef=opt["temp"][0], temp_every=opt["temp"][1]) if "temp" in opt else dict(bias_lut=bias)
     out = torch.full((n, H, D), 7.0, dtype=torch.float32 if opt.get("fp32") else dtype, device="cuda")
-    tiles = st.prompt_tiles(2, mixer_ops.TILE_ROWS // (H // G))[0]
+    tiles = st.prompt_tiles(2, mixer_ops.tile_tokens(H, G, dk))[0]
     mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, scale, max_context=st.max_context(),
                              value_width=D, value_div=div, **kw, **extra)
     want = _reference(q, k_pool, v_pool, st, D, div, scale, bias=bias, temp=opt.get("temp"), **kw)
@@ -123,7 +123,7 @@ def test_steep_scores_and_rescaling():
     st.block_tables[0, :36] = torch.arange(36, dtype=torch.int32, device="cuda")
     k_pool[:36] *= torch.linspace(0.01, 12, 36, device="cuda").to(k_pool.dtype)[:, None, None, None]
     out = torch.empty(64, 8, 128, dtype=torch.bfloat16, device="cuda")
-    tiles = st.prompt_tiles(2, 32)[0]
+    tiles = st.prompt_tiles(2, mixer_ops.tile_tokens(8, 2, 128))[0]
     for window in (0, 60):
         mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, 0.5, window=window)
         want = _reference(q, k_pool, v_pool, st, 128, 1, 0.5, window=window)
