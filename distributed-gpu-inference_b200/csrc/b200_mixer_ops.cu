@@ -399,7 +399,8 @@ struct Mma16<__half> {
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src, bool valid) {
   const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
   const int bytes = valid ? 16 : 0;  // fewer source bytes than 16: the rest is zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem_src), "r"(bytes) : "memory");
+  // no memory clobber: what the next copies need may be looked up in between (commit and wait carry it)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem_src), "r"(bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -409,7 +410,11 @@ constexpr int kMmaRows = 64;   // query rows per CTA
 constexpr int kMmaKeys = 64;   // keys per tile
 
 // KSPLIT (tiles of at most 16 rows, i.e. decoded tokens): all four warps work on the SAME 16 rows and each takes 16
-// of a tile's 64 keys; their running (max, sum, output) are merged through shared memory at the end.
+// of a tile's 64 keys; their running (max, sum, output) are merged through shared memory at the end.  With a workspace the keys are
+// divided over CTAs as well, kSplitKeys at absolute multiples each (so a token's sums do not depend on its neighbours): one CTA per
+// sequence and kv head left the chip to the longest sequences, 163 us for 48 sequences of up to 3000 tokens over 4 kv heads.
+constexpr int kSplitKeys = 256;
+constexpr int kMmaRowsSplit = 16;
 template <typename T, int DV8, bool KSPLIT>
 __global__ void __launch_bounds__(128)
 biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int64_t q_stride, const T* __restrict__ gate,
@@ -417,13 +422,15 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
                               const int32_t* __restrict__ block_tables, int table_stride,
                               const AttnTile* __restrict__ tiles, const int32_t* __restrict__ tok_pos,
                               const float* __restrict__ bias_lut, int lut_len, int lut_in_smem, int q_vec, float scale,
-                              float temp_coef, int temp_every, int H, int G, int dk, int dv, int block_size) {
+                              float temp_coef, int temp_every, int H, int G, int dk, int dv, int block_size, float* __restrict__ ws,
+                              int n_tok) {
   // Row r of the CTA's 64 is (token r / rep, head g * rep + r % rep): the heads of a kv group share the K / V tiles.
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int dvp = DV8 * 8;
   const int ldq = dk + 8, ldv = dvp + 8;       // element strides: 16-byte multiples, conflict-free fragment reads
-  T* q_s = reinterpret_cast<T*>(smem_raw);     // [64][ldq]
-  T* k_s = q_s + kMmaRows * ldq;               // 2 x [64][ldq]
+  T* q_s = reinterpret_cast<T*>(smem_raw);     // [64 or 16][ldq]
+  constexpr int kQRows = KSPLIT ? kMmaRowsSplit : kMmaRows;
+  T* k_s = q_s + kQRows * ldq;                 // 2 x [64][ldq]
   T* v_s = k_s + 2 * kMmaKeys * ldq;           // 2 x [64][ldv]
   float* lut_s = reinterpret_cast<float*>(v_s + 2 * kMmaKeys * ldv);
   const AttnTile tile = tiles[blockIdx.x];
@@ -433,6 +440,11 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
   const int gq = lane >> 2, tq = lane & 3;
   const int pos0 = tok_pos[tile.tok0];
   const int pos_last = pos0 + tile.count - 1;
+  // key tiles of this CTA: all, or its kSplitKeys
+  const bool split = KSPLIT && ws != nullptr;
+  const int kt0 = split ? blockIdx.z * (kSplitKeys / kMmaKeys) : 0;
+  const int kt1 = split ? min(pos_last / kMmaKeys + 1, kt0 + kSplitKeys / kMmaKeys) : pos_last / kMmaKeys + 1;
+  if (kt0 >= kt1) return;
   const int32_t* table = block_tables + static_cast<int64_t>(tile.seq) * table_stride;
   if (lut_in_smem) {   // the group's heads, one after the other
     for (int i = threadIdx.x; i < rep * lut_len; i += blockDim.x) lut_s[i] = bias_lut[static_cast<int64_t>(g) * rep * lut_len + i];
@@ -441,14 +453,14 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
 
   // Q tile (rows beyond the tile's are zero); element-wise when the rows are not 16-byte aligned
   if (q_vec) {
-    for (int c = threadIdx.x; c < kMmaRows * qc; c += blockDim.x) {
+    for (int c = threadIdx.x; c < kQRows * qc; c += blockDim.x) {
       const int r = c / qc, e = (c - r * qc) * 8;
       const bool ok = r < n_rows;
       const int t = r / rep, hh = g * rep + (r - t * rep);
       cp_async16(q_s + r * ldq + e, ok ? q + (tile.tok0 + t) * q_stride + hh * dk + e : q, ok);
     }
   } else {
-    for (int i = threadIdx.x; i < kMmaRows * dk; i += blockDim.x) {
+    for (int i = threadIdx.x; i < kQRows * dk; i += blockDim.x) {
       const int r = i / dk, d = i - r * dk;
       const int t = r / rep, hh = g * rep + (r - t * rep);
       q_s[r * ldq + d] = r < n_rows ? q[(tile.tok0 + t) * q_stride + hh * dk + d] : Cvt<T>::from_f32(0.f);
@@ -465,23 +477,27 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
   auto load_kv = [&](int j0, int stage) {
     T* kd = k_s + stage * kMmaKeys * ldq;
     T* vd = v_s + stage * kMmaKeys * ldv;
-    if (k_row0 < k_step) {
-      for (int j = k_row0; j < kMmaKeys; j += k_step) {
-        const int key = j0 + j;
-        const bool ok = key <= pos_last;
-        cp_async16(kd + j * ldq + k_e, k_pool + (ok ? pool_row(key) * dk + k_e : 0), ok);
+    // four rows at a time: their look-ups overlap, and none waits between two copies
+    auto rows = [&](T* dst, const T* pool, int ld, int width, int row0, int step, int e, bool col_ok) {
+      if (row0 >= step) return;
+      for (int j = row0; j < kMmaKeys; j += 4 * step) {
+        int64_t r[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int key = j0 + j + u * step;
+          r[u] = col_ok && j + u * step < kMmaKeys && key <= pos_last ? pool_row(key) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const bool ok = r[u] >= 0;
+          if (j + u * step < kMmaKeys) cp_async16(dst + (j + u * step) * ld + e, pool + (ok ? r[u] * width + e : 0), ok);
+        }
       }
-    }
-    if (v_row0 < v_step) {
-      const bool col_ok = v_e < dv;
-      for (int j = v_row0; j < kMmaKeys; j += v_step) {
-        const int key = j0 + j;
-        const bool ok = col_ok && key <= pos_last;
-        cp_async16(vd + j * ldv + v_e, v_pool + (ok ? pool_row(key) * dv + v_e : 0), ok);
-      }
-    }
+    };
+    rows(kd, k_pool, ldq, dk, k_row0, k_step, k_e, true);
+    rows(vd, v_pool, ldv, dv, v_row0, v_step, v_e, v_e < dv);
   };
-  load_kv(0, 0);
+  load_kv(kt0 * kMmaKeys, 0);
   cp_async_commit();
 
   const int row_a = (KSPLIT ? 0 : warp * 16) + gq;       // this thread's rows: row_a and row_a + 8
@@ -506,10 +522,10 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
 #pragma unroll
   for (int n = 0; n < DV8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
 
-  const int n_kt = pos_last / kMmaKeys + 1;
-  for (int it = 0; it < n_kt; ++it) {
-    if (it + 1 < n_kt) {
-      load_kv((it + 1) * kMmaKeys, (it + 1) & 1);
+  for (int it = kt0; it < kt1; ++it) {
+    const int stage = (it - kt0) & 1;
+    if (it + 1 < kt1) {
+      load_kv((it + 1) * kMmaKeys, stage ^ 1);
       cp_async_commit();
       cp_async_wait<1>();
     } else {
@@ -518,8 +534,8 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
     __syncthreads();
     const int j0 = it * kMmaKeys;
     if (warp_live && j0 <= warp_pos_max) {
-      const T* kt = k_s + (it & 1) * kMmaKeys * ldq;
-      const T* vt = v_s + (it & 1) * kMmaKeys * ldv;
+      const T* kt = k_s + stage * kMmaKeys * ldq;
+      const T* vt = v_s + stage * kMmaKeys * ldv;
       float s[NT][4];
 #pragma unroll
       for (int n = 0; n < NT; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
@@ -630,6 +646,7 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
 #pragma unroll
       for (int w2 = 0; w2 < 4; ++w2) lsum += mg[64 + w2 * 16 + r] * expf(mg[w2 * 16 + r] - mall);
       l[i] = lsum;
+      m[i] = mall;
 #pragma unroll
       for (int n = 0; n < DV8; ++n) {
         og[(warp * 16 + r) * dvp + n * 8 + 2 * tq] = o[n][2 * i] * w;
@@ -637,7 +654,24 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
       }
     }
     __syncthreads();
-    if (warp != 0) return;
+    if (!split && warp != 0) return;
+    if (split) {     // (maximum, sum, output) of these keys, all warps: the merge kernel below reads them
+      for (int e = threadIdx.x; e < n_rows * dv; e += blockDim.x) {
+        const int r = e / dv, c = e - r * dv, t = r / rep;
+        float* dst = ws + ((static_cast<int64_t>(blockIdx.z) * n_tok + tile.tok0 + t) * H + g * rep + r - t * rep) * (dv + 2);
+        dst[2 + c] = (og[r * dvp + c] + og[(16 + r) * dvp + c]) + (og[(32 + r) * dvp + c] + og[(48 + r) * dvp + c]);
+      }
+      if (warp == 0 && tq == 0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          if (gq + 8 * i >= n_rows) continue;
+          float* dst = ws + ((static_cast<int64_t>(blockIdx.z) * n_tok + tile.tok0 + tokr[i]) * H + headr[i]) * (dv + 2);
+          dst[0] = m[i];
+          dst[1] = l[i];
+        }
+      }
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int r = gq + 8 * i;
@@ -667,6 +701,32 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
       }
     }
   }
+}
+
+// The key splits of a token and head brought together: one CTA per (tile, token of it, head), a thread per value column.
+template <typename T>
+__global__ void __launch_bounds__(128)
+biased_split_merge_kernel(T* __restrict__ out, const float* __restrict__ ws, const T* __restrict__ gate, int64_t gate_stride,
+                          const AttnTile* __restrict__ tiles, const int32_t* __restrict__ tok_pos, int n_tok, int H, int dv) {
+  const AttnTile tile = tiles[blockIdx.x];
+  if (static_cast<int>(blockIdx.y) >= tile.count) return;
+  const int64_t n = tile.tok0 + blockIdx.y;
+  const int h = blockIdx.z, c = threadIdx.x;
+  const int splits = (tok_pos[tile.tok0] + tile.count - 1) / kSplitKeys + 1;     // as the tile's CTAs cut its keys
+  const int64_t step = static_cast<int64_t>(n_tok) * H * (dv + 2);
+  const float* src = ws + (n * H + h) * (dv + 2);
+  float M = -INFINITY;
+  for (int sp = 0; sp < splits; ++sp) M = fmaxf(M, src[sp * step]);
+  float L = 0.f, O = 0.f;
+#pragma unroll 4
+  for (int sp = 0; sp < splits; ++sp) {
+    const float f = expf(src[sp * step] - M);        // a row that saw none of a split's keys left sum 0 and output 0
+    L = fmaf(src[sp * step + 1], f, L);
+    if (c < dv) O = fmaf(src[sp * step + 2 + c], f, O);
+  }
+  if (c >= dv) return;
+  const float gt = gate ? sigmoidf_(Cvt<T>::to_f32(gate[n * gate_stride + h])) : 1.0f;
+  out[(n * H + h) * dv + c] = Cvt<T>::from_f32(O * gt / L);
 }
 
 // ---- grouped linear for expert-sorted rows (16-bit storage) ---------------------------------------------------------
@@ -1011,6 +1071,18 @@ int b200_biased_prompt_attn(void* out, const void* q, int64_t q_stride, const vo
                             const int32_t* tiles, int n_tiles, int max_tile_tokens, const int32_t* tok_pos, const float* bias_lut,
                             int lut_len, float scale, float temp_coef, int temp_every, int H, int G, int dk, int dv,
                             int block_size, int dtype, void* stream) {
+  return b200_biased_prompt_attn_ext(out, q, q_stride, gate, gate_stride, k_pool, v_pool, block_tables, table_stride, tiles, n_tiles,
+                                     max_tile_tokens, tok_pos, bias_lut, lut_len, scale, temp_coef, temp_every, H, G, dk, dv, block_size,
+                                     0, nullptr, 0, dtype, stream);
+}
+
+int b200_biased_attn_split_keys(void) { return kSplitKeys; }
+
+int b200_biased_prompt_attn_ext(void* out, const void* q, int64_t q_stride, const void* gate, int64_t gate_stride,
+                            const void* k_pool, const void* v_pool, const int32_t* block_tables, int table_stride,
+                            const int32_t* tiles, int n_tiles, int max_tile_tokens, const int32_t* tok_pos, const float* bias_lut,
+                            int lut_len, float scale, float temp_coef, int temp_every, int H, int G, int dk, int dv,
+                            int block_size, int max_context, float* workspace, int n_tok, int dtype, void* stream) {
   if (n_tiles < 0 || H <= 0 || G <= 0 || H % G || block_size <= 0 || lut_len <= 0)
     return fail(B200_EINVAL, "b200_biased_prompt_attn: bad sizes");
   if (!b200_biased_prompt_attn_supported(dk, dv, dtype))
@@ -1022,14 +1094,18 @@ int b200_biased_prompt_attn(void* out, const void* q, int64_t q_stride, const vo
     return fail(B200_ESHAPE, "b200_biased_prompt_attn: pools must be 16-byte aligned");
   const int q_vec = aligned16(q) && (q_stride * 2) % 16 == 0;
   const int dv8 = dv <= 32 ? 4 : (dv <= 64 ? 8 : 16);
-  const size_t tiles_bytes = 2u * (static_cast<size_t>(kMmaRows) * (dk + 8) * 3 + 2u * kMmaKeys * (dv8 * 8 + 8));
   const int rep = H / G;
   if (rep > kMmaRows) return fail(B200_ESHAPE, "b200_biased_prompt_attn: %d heads per kv head > %d", rep, kMmaRows);
+  // tiles of at most 16 rows (decoded tokens): the four warps split the keys instead of the rows, and with a workspace CTAs do too
+  const bool ksplit = max_tile_tokens > 0 && max_tile_tokens * rep <= kMmaRowsSplit;
+  const int n_splits = ksplit && workspace && max_context > kSplitKeys ? (max_context + kSplitKeys - 1) / kSplitKeys : 1;
+  const size_t tiles_bytes = 2u * (static_cast<size_t>(dk + 8) * ((ksplit ? kMmaRowsSplit : kMmaRows) + 2u * kMmaKeys) + 2u * kMmaKeys * (dv8 * 8 + 8));
   // the group's bias tables go to shared memory when they are small enough to leave room for two CTAs per SM
   const size_t lut_bytes = static_cast<size_t>(rep) * lut_len * 4;
   const int lut_in_smem = lut_bytes <= 20 * 1024;
   const size_t smem = tiles_bytes + (lut_in_smem ? lut_bytes : 0);
-  const dim3 grid(n_tiles, G);
+  const dim3 grid(n_tiles, G, n_splits);
+  float* ws = n_splits > 1 ? workspace : nullptr;
   return mixer_by_dtype(dtype, "b200_biased_prompt_attn", [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
     if constexpr (std::is_same_v<T, float>) {
@@ -1041,10 +1117,8 @@ int b200_biased_prompt_attn(void* out, const void* q, int64_t q_stride, const vo
             static_cast<T*>(out), static_cast<const T*>(q), q_stride, static_cast<const T*>(gate), gate_stride,
             static_cast<const T*>(k_pool), static_cast<const T*>(v_pool), block_tables, table_stride,
             reinterpret_cast<const AttnTile*>(tiles), tok_pos, bias_lut, lut_len, lut_in_smem, q_vec, scale, temp_coef,
-            temp_every, H, G, dk, dv, block_size);
+            temp_every, H, G, dk, dv, block_size, ws, n_tok);
       };
-      // tiles of at most 16 rows (decoded tokens): the four warps split the keys instead of the rows
-      const bool ksplit = max_tile_tokens > 0 && max_tile_tokens * rep <= 16;
       if (ksplit) {
         if (dv8 == 4) launch(biased_prompt_attn_mma_kernel<T, 4, true>);
         else if (dv8 == 8) launch(biased_prompt_attn_mma_kernel<T, 8, true>);
@@ -1054,7 +1128,11 @@ int b200_biased_prompt_attn(void* out, const void* q, int64_t q_stride, const vo
         else if (dv8 == 8) launch(biased_prompt_attn_mma_kernel<T, 8, false>);
         else launch(biased_prompt_attn_mma_kernel<T, 16, false>);
       }
-      return check_launch("b200_biased_prompt_attn");
+      const int rc = check_launch("b200_biased_prompt_attn");
+      if (rc != 0 || !ws) return rc;
+      biased_split_merge_kernel<T><<<dim3(n_tiles, max_tile_tokens, H), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+          static_cast<T*>(out), ws, static_cast<const T*>(gate), gate_stride, reinterpret_cast<const AttnTile*>(tiles), tok_pos, n_tok, H, dv);
+      return check_launch("b200_biased_prompt_attn (merge)");
     }
   });
 }

@@ -153,11 +153,11 @@ def prompt_attention_supported(dk: int, dv: int, dtype: torch.dtype) -> bool:
 def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[torch.Tensor], k_pool: torch.Tensor,
                             v_pool: torch.Tensor, block_tables: torch.Tensor, tiles: torch.Tensor, tok_pos: torch.Tensor,
                             bias_lut: torch.Tensor, scale: float, temp_coef: float, temp_every: int, H: int,
-                            max_tile_tokens: int = 0) -> None:
+                            max_tile_tokens: int = 0, max_context: int = 0) -> None:
     """``biased_paged_attention`` on the tensor cores, for prompt portions and decoded tokens alike; writes the tiles'
     rows of ``out`` ``[n, H*dv]`` (16-bit dtypes, see ``prompt_attention_supported``).  ``tiles``: up to
     ``prompt_tile_tokens(H, G)`` tokens each; ``max_tile_tokens``: the largest tile (0 = unknown) — steps of decoded
-    tokens only take the variant whose warps split the keys."""
+    tokens only take the variant whose warps split the keys; with ``max_context`` (a bound on the step's contexts) its CTAs do too."""
     _need_cuda(out, q, k_pool, v_pool, block_tables, tiles, tok_pos, bias_lut)
     nb, G, bs, dk = k_pool.shape
     dv = v_pool.shape[3]
@@ -170,11 +170,16 @@ def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[t
         raise ValueError("tiles must be contiguous int32 [n_tiles, 3]")
     if bias_lut.dtype != torch.float32 or bias_lut.shape[0] != H or not bias_lut.is_contiguous():
         raise ValueError("bias_lut must be contiguous fp32 [H, L]")
-    rc = _lib_().b200_biased_prompt_attn(out.data_ptr(), q.data_ptr(), _rows2(q), _ptr(gate),
+    lib = _lib_()
+    ws = None
+    if 0 < max_tile_tokens * (H // G) <= 16 and max_context > lib.b200_biased_attn_split_keys():
+        splits = -(-max_context // lib.b200_biased_attn_split_keys())
+        ws = torch.empty((splits, n, H, dv + 2), dtype=torch.float32, device=q.device)
+    rc = lib.b200_biased_prompt_attn_ext(out.data_ptr(), q.data_ptr(), _rows2(q), _ptr(gate),
                                          _rows2(gate) if gate is not None else 0, k_pool.data_ptr(), v_pool.data_ptr(),
                                          block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), tiles.shape[0],
                                          int(max_tile_tokens), tok_pos.data_ptr(), bias_lut.data_ptr(), bias_lut.shape[1], float(scale),
-                                         float(temp_coef), int(temp_every), H, G, dk, dv, bs, DTYPE_ID[q.dtype], _stream())
+                                         float(temp_coef), int(temp_every), H, G, dk, dv, bs, int(max_context), _ptr(ws), n, DTYPE_ID[q.dtype], _stream())
     _lib.check_mixers(rc, "b200_biased_prompt_attn")
 
 

@@ -176,7 +176,7 @@ class BiasedPagedAttention(nn.Module):
             if rest is not None:
                 mixer_ops.biased_prompt_attention(attn, q, gate, cache.k_pool, cache.v_pool, st.block_tables, rest[0], st.tok_pos,
                                                   self.bias_lut, self.scale, self.temp_coef, self.temp_every, H,
-                                                  max_tile_tokens=rest[1])
+                                                  max_tile_tokens=rest[1], max_context=st.max_context())
         else:                         # fp32, or head sizes off the tensor-core grid: the row kernel
             tiles, most = st.tiles_for(H, G)
             mixer_ops.biased_paged_attention(q, gate, cache.k_pool, cache.v_pool, st.block_tables, tiles, most,

@@ -71,6 +71,14 @@ int b200_biased_prompt_attn(void* out, const void* q, int64_t q_stride, const vo
                             const int32_t* tiles, int n_tiles, int max_tile_tokens, const int32_t* tok_pos,
                             const float* bias_lut, int lut_len, float scale, float temp_coef, int temp_every, int H, int G,
                             int dk, int dv, int block_size, int dtype, void* stream);
+/* The same; tiles of at most 16 rows (decoded tokens) whose longest context (max_context, a bound) exceeds b200_biased_attn_split_keys()
+ * divide their keys over CTAs when workspace is given: fp32 [ceil(max_context / split keys)][n_tok][H][dv + 2], n_tok the packed rows. */
+int b200_biased_attn_split_keys(void);
+int b200_biased_prompt_attn_ext(void* out, const void* q, int64_t q_stride, const void* gate, int64_t gate_stride,
+                            const void* k_pool, const void* v_pool, const int32_t* block_tables, int table_stride,
+                            const int32_t* tiles, int n_tiles, int max_tile_tokens, const int32_t* tok_pos,
+                            const float* bias_lut, int lut_len, float scale, float temp_coef, int temp_every, int H, int G,
+                            int dk, int dv, int block_size, int max_context, float* workspace, int n_tok, int dtype, void* stream);
 
 /* Gated linear recurrence per (sequence, head) over the sequence's tokens of this step, in order:
  *   q = silu(zq), f = lower + (1 - lower) * sigmoid(zf + f_bias), S <- diag(f) S + (1 - f) v^T, o = S^T q.
