@@ -128,6 +128,8 @@ MIXER_SIGNATURES = {
     "b200_head_rmsnorm": (c_int, [c_void_p, c_void_p, c_void_p, c_float, c_int64, c_int, c_int, c_void_p]),
     "b200_polynorm": (c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_float, c_int, c_int, c_int, c_void_p]),
     "b200_sigmoid_topk": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
+    "b200_expert_order_supported": (c_int, [c_int64, c_int]),
+    "b200_expert_order": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p]),
     "b200_scaled_gather": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
     "b200_grouped_linear_supported": (c_int, [c_int, c_int]),
     "b200_grouped_linear": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p]),
@@ -277,11 +279,11 @@ MIXER_SIGNATURES = {
                 c_int, c_void_p]),
     # prompt portions on the fifth-generation tensor cores (csrc/b200_tile_attn.cu)
     "b200_tile_attn_supported": (c_int, [c_int] * 7),
-    "b200_tile_attn_rows": (c_int, [c_int]),
-    "b200_tile_attn_splits": (c_int, [c_int] * 4),
+    "b200_tile_attn_rows": (c_int, [c_int] * 4),
+    "b200_tile_attn_splits": (c_int, [c_int] * 5),
     "b200_tile_attn": (
         c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p,
-                c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_float, c_float, c_int,
+                c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_float, c_float, c_int,
                 c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]),
     "b200_mixed_prompt_attn_rows_supported": (c_int, [c_int, c_int, c_int, c_int]),
     "b200_qknorm_rotary_append_ext2": (
@@ -368,7 +370,7 @@ def _build_mixers() -> None:
         fcntl.flock(lock, fcntl.LOCK_EX)
         if os.path.exists(MIXER_LIB_PATH):
             return
-        proc = subprocess.run(["make", "-j10", "-C", csrc, "mixers"], stdout=subprocess.PIPE, stderr=subprocess.STDOUT)
+        proc = subprocess.run(["make", "-j11", "-C", csrc, "mixers"], stdout=subprocess.PIPE, stderr=subprocess.STDOUT)
         if proc.returncode != 0 or not os.path.exists(MIXER_LIB_PATH):
             raise B200LibraryError("building libb200_mixers.so failed:\n" + proc.stdout.decode(errors="replace")[-4000:])
 

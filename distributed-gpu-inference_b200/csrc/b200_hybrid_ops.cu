@@ -1302,13 +1302,15 @@ int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bi
   return tile_attn_supported(H, G, dk, dv, same_pool != 0, bias != 0, dtype) ? 1 : 0;
 }
 
-int b200_tile_attn_rows(int dk) { return tile_attn_rows(dk); }
+int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens) { return tile_attn_rows(rep, G, dk, n_tokens); }
 
-int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk) { return tile_attn_splits(n_tiles, key_tiles, G, dk); }
+int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows) {
+  return tile_attn_splits(n_tiles, key_tiles, G, dk, tile_rows);
+}
 
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,
-                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, const int32_t* tok_pos, int n_tok,
+                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, int tile_rows, const int32_t* tok_pos, int n_tok,
                    const float* sink, const float* bias_lut, int lut_len, float scale, float softcap, float temp_coef, int temp_every,
                    int window, int keep_first, int chunk, int H, int G, int dk, int dv, int v_row, int v_div, int out_f32, int block_size,
                    int n_splits, float* workspace, int dtype, void* stream) {
@@ -1318,6 +1320,8 @@ int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, c
     return fail(B200_EINVAL, "b200_tile_attn: bad sizes");
   if (!tile_attn_supported(H, G, dk, dv, alias, bias_lut != nullptr, dtype) || (alias && (v_div != 1 || v_row != dk)))
     return fail(B200_ESHAPE, "b200_tile_attn: head layout (%d over %d, %d / %d) is not served", H, G, dk, dv);
+  if (tile_rows != kTileRows && (tile_rows != 2 * kTileRows || dk > 128))
+    return fail(B200_EINVAL, "b200_tile_attn: tiles have %d rows", kTileRows);
   if (n_tiles == 0) return 0;
   if (!out || !q || !k_pool || !v_pool || !block_tables || !tiles || !tok_pos || (n_splits > 1 && !workspace))
     return fail(B200_EINVAL, "b200_tile_attn: null pointer");
@@ -1336,7 +1340,7 @@ int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, c
   A.out_f32 = out_f32, A.out_vec = aligned16(out) && ((out_tok_stride | out_head_stride) & 7) == 0;
   A.scale = scale, A.softcap = softcap, A.temp_coef = temp_coef, A.temp_every = temp_every;
   const auto s = static_cast<cudaStream_t>(stream);
-  const int rc = tile_attn_launch(A, dk, dv, alias, n_tiles, n_splits, dtype, s);
+  const int rc = tile_attn_launch(A, dk, dv, alias, tile_rows, n_tiles, n_splits, dtype, s);
   if (rc != 0 || n_splits == 1) return rc;
   AttnArgs M{out, out_tok_stride, out_head_stride, q, q_tok_stride, q_head_stride, gate, gate_stride, k_pool, v_pool,
              block_tables, table_stride, nullptr, tok_pos, nullptr, sink, scale, window, keep_first, 0,
@@ -1347,7 +1351,7 @@ int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, c
     using T = std::remove_pointer_t<decltype(tag)>;
     auto merge = attn_split_combine_kernel<T>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    merge<<<dim3(n_tiles, tile_attn_rows(dk) / (H / G)), 256, smem, s>>>(M, tiles, workspace, n_splits, n_tok, dv, nullptr);
+    merge<<<dim3(n_tiles, tile_rows / (H / G)), 256, smem, s>>>(M, tiles, workspace, n_splits, n_tok, dv, nullptr);
     return check_launch("b200_tile_attn (merge)");
   });
 }

@@ -1,17 +1,13 @@
 // Sequence mixers and feed-forward pieces for decoder designs that keep an fp32 residual stream and run ragged
 // batches (prompt portions beside single decoded tokens, packed token-major):
 //
-//   offset RMS norm            y = x * rsqrt(mean(x^2) + eps) * (1 + w)            fp32 in, storage dtype out
-//   post-norm residual update  x += m * norm(y; w_post), optionally followed by the next sublayer's input norm
-//   value prep + paged append  per-head unit-RMS values, optional mix with an earlier layer's values, K/V scatter
-//                              into pools whose K and V rows have different widths
 //   biased paged attention     causal softmax attention of packed query rows over the paged cache with a learned
 //                              bias per (distance bucket, head), a per-position query temperature and a per-head
 //                              sigmoid output gate
 //   gated linear recurrence    S_t = diag(f_t) S_(t-1) + (1 - f_t) v_t^T, o_t = S_t^T q_t with the state in fp32,
-//                              carried per sequence in a slot pool; then a per-head weighted RMS norm
-//   PolyNorm activation        a N(z) + b N(z^2) + c N(z^3) + e over a token's feed-forward row
-//   sigmoid top-k routing, input-scaled expert rows, clamped GLU, combine
+//                              carried per sequence in a slot pool (kernel: b200_column_scan.cu)
+//   sigmoid top-k routing, grouped linear for expert-sorted rows
+// (norms, residual updates, activations and what moves rows to experts and back: b200_row_ops.cu)
 //
 // Every constant of a design (eps, multipliers, temperatures, limits, table sizes) is a parameter.  Scores, softmax,
 // norms, gates of the recurrence, the state and the residual are fp32 whatever the storage dtype T is.  Summation
@@ -48,103 +44,7 @@ int mixer_by_dtype(int dtype, const char* name, F&& f) {
   }
 }
 
-__device__ __forceinline__ float block_sum_256(float v, float* red) {
-  // every thread returns the total; `red` holds 32 floats and may be reused after the call's second barrier
-  v = warp_sum(v);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  float t = (lane < nw) ? red[lane] : 0.f;
-  return warp_sum(t);
-}
-
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.0f / (1.0f + expf(-z)); }
-
-// ---- offset RMS norm ------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256)
-offset_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ x, const T* __restrict__ w, float eps, int width) {
-  __shared__ float red[32];
-  const float* xr = x + static_cast<int64_t>(blockIdx.x) * width;
-  float ss = 0.f;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) ss = fmaf(xr[i], xr[i], ss);
-  const float inv = rsqrtf(block_sum_256(ss, red) / static_cast<float>(width) + eps);
-  T* orow = out + static_cast<int64_t>(blockIdx.x) * width;
-  for (int i = threadIdx.x; i < width; i += blockDim.x)
-    orow[i] = Cvt<T>::from_f32(xr[i] * inv * (1.0f + Cvt<T>::to_f32(w[i])));
-}
-
-// ---- x += mult * norm(y; w_post); optionally out_next = norm(x; w_next) ------------------------------------------
-// One CTA per token.  The updated row is kept in shared memory between the update and the second norm.
-template <typename T, typename Y>
-__global__ void __launch_bounds__(256)
-postnorm_residual_kernel(float* __restrict__ x, const Y* __restrict__ y, int64_t y_stride, const T* __restrict__ w_post,
-                         float mult, const T* __restrict__ w_next, T* __restrict__ out_next, float eps, int width) {
-  extern __shared__ float row_s[];
-  __shared__ float red[32];
-  const Y* yr = y + static_cast<int64_t>(blockIdx.x) * y_stride;
-  float* xr = x + static_cast<int64_t>(blockIdx.x) * width;
-  float ss = 0.f;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) {
-    const float v = Cvt<Y>::to_f32(yr[i]);
-    ss = fmaf(v, v, ss);
-  }
-  const float inv = rsqrtf(block_sum_256(ss, red) / static_cast<float>(width) + eps);
-  float sx = 0.f;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) {
-    const float n = Cvt<Y>::to_f32(yr[i]) * inv * (1.0f + Cvt<T>::to_f32(w_post[i]));
-    const float v = xr[i] + mult * n;
-    xr[i] = v;
-    row_s[i] = v;
-    sx = fmaf(v, v, sx);
-  }
-  if (w_next == nullptr) return;
-  const float inv2 = rsqrtf(block_sum_256(sx, red) / static_cast<float>(width) + eps);
-  T* orow = out_next + static_cast<int64_t>(blockIdx.x) * width;
-  for (int i = threadIdx.x; i < width; i += blockDim.x)
-    orow[i] = Cvt<T>::from_f32(row_s[i] * inv2 * (1.0f + Cvt<T>::to_f32(w_next[i])));
-}
-
-// ---- value prep + K/V append ------------------------------------------------------------------------------------
-// One CTA per token, one warp per kv head (looping).  v <- v / rms(v) per head; with `v_prev` the stored value is
-// (1 - lam) v + lam v_prev.  The stored value also goes to `v_keep` (for later layers of the same step) when given.
-template <typename T>
-__global__ void __launch_bounds__(128)
-value_prep_append_kernel(const T* __restrict__ k, int64_t k_stride, const T* __restrict__ v, int64_t v_stride,
-                         const T* __restrict__ v_prev, T* __restrict__ v_keep, float lam, float eps,
-                         T* __restrict__ k_pool, T* __restrict__ v_pool, const int64_t* __restrict__ slot_mapping,
-                         int G, int dk, int dv, int block_size, int64_t max_blocks) {
-  const int tok = blockIdx.x;
-  const int64_t slot = slot_mapping[tok];
-  const int64_t blk = slot >= 0 ? slot / block_size : -1;
-  const bool store = blk >= 0 && blk < max_blocks;
-  const int off = store ? static_cast<int>(slot - blk * block_size) : 0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int g = warp; g < G; g += nw) {
-    const T* vr = v + tok * v_stride + g * dv;
-    float ss = 0.f;
-    for (int c = lane; c < dv; c += 32) {
-      const float f = Cvt<T>::to_f32(vr[c]);
-      ss = fmaf(f, f, ss);
-    }
-    const float inv = rsqrtf(warp_sum(ss) / static_cast<float>(dv) + eps);
-    T* dst = store ? v_pool + ((blk * G + g) * block_size + off) * dv : nullptr;
-    for (int c = lane; c < dv; c += 32) {
-      float f = Cvt<T>::to_f32(vr[c]) * inv;
-      if (v_prev) f = (1.0f - lam) * f + lam * Cvt<T>::to_f32(v_prev[static_cast<int64_t>(tok) * G * dv + g * dv + c]);
-      const T r = Cvt<T>::from_f32(f);
-      if (dst) dst[c] = r;
-      if (v_keep) v_keep[static_cast<int64_t>(tok) * G * dv + g * dv + c] = r;
-    }
-  }
-  if (store) {
-    for (int i = threadIdx.x; i < G * dk; i += blockDim.x) {
-      const int g = i / dk, d = i - g * dk;
-      k_pool[((blk * G + g) * block_size + off) * dk + d] = k[tok * k_stride + i];
-    }
-  }
-}
 
 // ---- biased paged attention over packed query rows ----------------------------------------------------------------
 // A CTA serves up to QT consecutive tokens of ONE sequence and one kv head: QT * (H / G) query rows.  Keys are
@@ -812,51 +712,6 @@ grouped_linear_kernel(T* __restrict__ out, const T* __restrict__ xs, const T* __
   }
 }
 
-// ---- per-head norm of the recurrence's read-outs ------------------------------------------------------------------
-// per-head weighted RMS norm of fp32 rows [rows, dv] -> T; one warp per row
-template <typename T>
-__global__ void __launch_bounds__(256)
-head_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ x, const T* __restrict__ w, float eps, int64_t rows,
-                    int dv) {
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const float* xr = x + row * dv;
-  float ss = 0.f;
-  for (int c = lane; c < dv; c += 32) ss = fmaf(xr[c], xr[c], ss);
-  const float inv = rsqrtf(warp_sum(ss) / static_cast<float>(dv) + eps);
-  for (int c = lane; c < dv; c += 32) out[row * dv + c] = Cvt<T>::from_f32(xr[c] * inv * Cvt<T>::to_f32(w[c]));
-}
-
-// ---- PolyNorm ---------------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256)
-polynorm_kernel(T* __restrict__ out, const T* __restrict__ z, int64_t z_stride, const T* __restrict__ coef, float eps,
-                int ff) {
-  __shared__ float red[32];
-  const T* zr = z + static_cast<int64_t>(blockIdx.x) * z_stride;
-  float s1 = 0.f, s2 = 0.f, s3 = 0.f;
-  for (int i = threadIdx.x; i < ff; i += blockDim.x) {
-    const float a = Cvt<T>::to_f32(zr[i]);
-    const float a2 = a * a, a3 = a2 * a;
-    s1 = fmaf(a, a, s1);
-    s2 = fmaf(a2, a2, s2);
-    s3 = fmaf(a3, a3, s3);
-  }
-  const float n = static_cast<float>(ff);
-  const float i1 = rsqrtf(block_sum_256(s1, red) / n + eps);
-  const float i2 = rsqrtf(block_sum_256(s2, red) / n + eps);
-  const float i3 = rsqrtf(block_sum_256(s3, red) / n + eps);
-  const float ca = Cvt<T>::to_f32(coef[0]), cb = Cvt<T>::to_f32(coef[1]), cc = Cvt<T>::to_f32(coef[2]),
-              ce = Cvt<T>::to_f32(coef[3]);
-  T* orow = out + static_cast<int64_t>(blockIdx.x) * ff;
-  for (int i = threadIdx.x; i < ff; i += blockDim.x) {
-    const float a = Cvt<T>::to_f32(zr[i]);
-    const float a2 = a * a;
-    orow[i] = Cvt<T>::from_f32(ca * a * i1 + cb * a2 * i2 + cc * a2 * a * i3 + ce);
-  }
-}
-
 // ---- routing ----------------------------------------------------------------------------------------------------
 // One warp per token: the `top` largest logits (ties: lowest index), weight = sigmoid(logit).
 __global__ void __launch_bounds__(128)
@@ -895,46 +750,6 @@ sigmoid_topk_kernel(int32_t* __restrict__ ids, float* __restrict__ weights, cons
   }
 }
 
-// rows of the expert-sorted input: xs[r] = T(w[src[r]] * h[src[r] / top])
-template <typename T>
-__global__ void __launch_bounds__(256)
-scaled_gather_kernel(T* __restrict__ xs, const T* __restrict__ h, const float* __restrict__ weights,
-                     const int64_t* __restrict__ src, int top, int width) {
-  const int64_t pair = src[blockIdx.x];
-  const float w = weights[pair];
-  const T* hr = h + (pair / top) * width;
-  T* o = xs + static_cast<int64_t>(blockIdx.x) * width;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) o[i] = Cvt<T>::from_f32(w * Cvt<T>::to_f32(hr[i]));
-}
-
-// y = g' * sigmoid(alpha g') * (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit); gu rows hold g | u
-template <typename T>
-__global__ void __launch_bounds__(256)
-clamped_glu_kernel(T* __restrict__ y, const T* __restrict__ gu, int64_t rows, int ff, float limit, float alpha) {
-  const int64_t n = rows * ff;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t r = i / ff;
-    const int c = static_cast<int>(i - r * ff);
-    const float g = fminf(Cvt<T>::to_f32(gu[r * 2 * ff + c]), limit);
-    const float u = fminf(fmaxf(Cvt<T>::to_f32(gu[r * 2 * ff + ff + c]), -limit), limit);
-    y[i] = Cvt<T>::from_f32(g * sigmoidf_(alpha * g) * (u + 1.0f));
-  }
-}
-
-// out[n] = sum_k ys[where[n * top + k]] in fp32, k ascending
-template <typename T>
-__global__ void __launch_bounds__(256)
-expert_combine_kernel(float* __restrict__ out, const T* __restrict__ ys, const int64_t* __restrict__ where, int top,
-                      int width) {
-  const int64_t n = blockIdx.x;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) {
-    float a = 0.f;
-    for (int k = 0; k < top; ++k) a += Cvt<T>::to_f32(ys[where[n * top + k] * width + i]);
-    out[n * width + i] = a;
-  }
-}
-
 }  // namespace
 }  // namespace b200
 
@@ -945,57 +760,6 @@ extern "C" {
 int b200_mixers_abi_version(void) { return B200_MIXERS_ABI_VERSION; }
 
 const char* b200_mixers_last_error(void) { return last_error_buf(); }
-
-int b200_offset_rmsnorm(void* out, const float* x, const void* weight, float eps, int rows, int width, int dtype,
-                        void* stream) {
-  if (rows < 0 || width <= 0) return fail(B200_EINVAL, "b200_offset_rmsnorm: bad sizes");
-  if (rows == 0) return 0;
-  if (!out || !x || !weight) return fail(B200_EINVAL, "b200_offset_rmsnorm: null pointer");
-  return mixer_by_dtype(dtype, "b200_offset_rmsnorm", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    offset_rmsnorm_kernel<T><<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<T*>(out), x, static_cast<const T*>(weight), eps, width);
-    return check_launch("b200_offset_rmsnorm");
-  });
-}
-
-int b200_postnorm_residual(float* x, const void* y, int64_t y_stride, int y_is_f32, const void* w_post, float mult,
-                           const void* w_next, void* out_next, float eps, int rows, int width, int dtype, void* stream) {
-  if (rows < 0 || width <= 0 || width > 40000) return fail(B200_EINVAL, "b200_postnorm_residual: bad sizes");
-  if (rows == 0) return 0;
-  if (!x || !y || !w_post || (w_next && !out_next)) return fail(B200_EINVAL, "b200_postnorm_residual: null pointer");
-  const size_t smem = static_cast<size_t>(width) * sizeof(float);
-  return mixer_by_dtype(dtype, "b200_postnorm_residual", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    auto launch = [&](auto kern, auto* ytag) {
-      using Y = std::remove_pointer_t<decltype(ytag)>;
-      if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      kern<<<rows, 256, smem, static_cast<cudaStream_t>(stream)>>>(x, static_cast<const Y*>(y), y_stride,
-                                                                  static_cast<const T*>(w_post), mult,
-                                                                  static_cast<const T*>(w_next), static_cast<T*>(out_next),
-                                                                  eps, width);
-    };
-    if (y_is_f32) launch(postnorm_residual_kernel<T, float>, static_cast<float*>(nullptr));
-    else launch(postnorm_residual_kernel<T, T>, static_cast<T*>(nullptr));
-    return check_launch("b200_postnorm_residual");
-  });
-}
-
-int b200_value_prep_append(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const void* v_prev,
-                           void* v_keep, float lam, float eps, void* k_pool, void* v_pool, const int64_t* slot_mapping,
-                           int n_tok, int G, int dk, int dv, int block_size, int64_t max_blocks, int dtype, void* stream) {
-  if (n_tok < 0 || G <= 0 || dk <= 0 || dv <= 0 || block_size <= 0) return fail(B200_EINVAL, "b200_value_prep_append: bad sizes");
-  if (n_tok == 0) return 0;
-  if (!k || !v || !k_pool || !v_pool || !slot_mapping) return fail(B200_EINVAL, "b200_value_prep_append: null pointer");
-  return mixer_by_dtype(dtype, "b200_value_prep_append", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    value_prep_append_kernel<T><<<n_tok, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const T*>(k), k_stride, static_cast<const T*>(v), v_stride, static_cast<const T*>(v_prev),
-        static_cast<T*>(v_keep), lam, eps, static_cast<T*>(k_pool), static_cast<T*>(v_pool), slot_mapping, G, dk, dv,
-        block_size, max_blocks);
-    return check_launch("b200_value_prep_append");
-  });
-}
 
 int b200_biased_attn_tile_tokens(int n_tokens_in_portion, int H, int G) {
   // tokens per CTA: prompt portions fill 8 warps x 4 rows, a decoded token takes what its head group needs
@@ -1179,78 +943,12 @@ int b200_gated_scan(float* o_raw, const void* zq, const void* zf, const void* v,
                            static_cast<cudaStream_t>(stream));
 }
 
-int b200_head_rmsnorm(void* out, const float* x, const void* weight, float eps, int64_t rows, int dv, int dtype,
-                      void* stream) {
-  if (rows < 0 || dv <= 0) return fail(B200_EINVAL, "b200_head_rmsnorm: bad sizes");
-  if (rows == 0) return 0;
-  if (!out || !x || !weight) return fail(B200_EINVAL, "b200_head_rmsnorm: null pointer");
-  return mixer_by_dtype(dtype, "b200_head_rmsnorm", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    head_rmsnorm_kernel<T><<<static_cast<unsigned>((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<T*>(out), x, static_cast<const T*>(weight), eps, rows, dv);
-    return check_launch("b200_head_rmsnorm");
-  });
-}
-
-int b200_polynorm(void* out, const void* z, int64_t z_stride, const void* coef, float eps, int rows, int ff, int dtype,
-                  void* stream) {
-  if (rows < 0 || ff <= 0) return fail(B200_EINVAL, "b200_polynorm: bad sizes");
-  if (rows == 0) return 0;
-  if (!out || !z || !coef) return fail(B200_EINVAL, "b200_polynorm: null pointer");
-  return mixer_by_dtype(dtype, "b200_polynorm", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    polynorm_kernel<T><<<rows, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<T*>(out), static_cast<const T*>(z), z_stride, static_cast<const T*>(coef), eps, ff);
-    return check_launch("b200_polynorm");
-  });
-}
-
 int b200_sigmoid_topk(int32_t* ids, float* weights, const float* logits, int n_tok, int E, int top, void* stream) {
   if (n_tok < 0 || E <= 0 || top <= 0 || top > E) return fail(B200_EINVAL, "b200_sigmoid_topk: bad sizes");
   if (n_tok == 0) return 0;
   if (!ids || !weights || !logits) return fail(B200_EINVAL, "b200_sigmoid_topk: null pointer");
   sigmoid_topk_kernel<<<(n_tok + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(ids, weights, logits, n_tok, E, top);
   return check_launch("b200_sigmoid_topk");
-}
-
-int b200_scaled_gather(void* xs, const void* h, const float* weights, const int64_t* src, int64_t n_rows, int top,
-                       int width, int dtype, void* stream) {
-  if (n_rows < 0 || top <= 0 || width <= 0) return fail(B200_EINVAL, "b200_scaled_gather: bad sizes");
-  if (n_rows == 0) return 0;
-  if (!xs || !h || !weights || !src) return fail(B200_EINVAL, "b200_scaled_gather: null pointer");
-  return mixer_by_dtype(dtype, "b200_scaled_gather", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    scaled_gather_kernel<T><<<static_cast<unsigned>(n_rows), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<T*>(xs), static_cast<const T*>(h), weights, src, top, width);
-    return check_launch("b200_scaled_gather");
-  });
-}
-
-int b200_clamped_glu(void* y, const void* gu, int64_t rows, int ff, float limit, float alpha, int dtype, void* stream) {
-  if (rows < 0 || ff <= 0) return fail(B200_EINVAL, "b200_clamped_glu: bad sizes");
-  if (rows == 0) return 0;
-  if (!y || !gu) return fail(B200_EINVAL, "b200_clamped_glu: null pointer");
-  const int64_t n = rows * ff;
-  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, 148 * 16));
-  return mixer_by_dtype(dtype, "b200_clamped_glu", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    clamped_glu_kernel<T><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<T*>(y), static_cast<const T*>(gu),
-                                                                               rows, ff, limit, alpha);
-    return check_launch("b200_clamped_glu");
-  });
-}
-
-int b200_expert_combine(float* out, const void* ys, const int64_t* where, int64_t n_tok, int top, int width, int dtype,
-                        void* stream) {
-  if (n_tok < 0 || top <= 0 || width <= 0) return fail(B200_EINVAL, "b200_expert_combine: bad sizes");
-  if (n_tok == 0) return 0;
-  if (!out || !ys || !where) return fail(B200_EINVAL, "b200_expert_combine: null pointer");
-  return mixer_by_dtype(dtype, "b200_expert_combine", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    expert_combine_kernel<T><<<static_cast<unsigned>(n_tok), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        out, static_cast<const T*>(ys), where, top, width);
-    return check_launch("b200_expert_combine");
-  });
 }
 
 }  // extern "C"

@@ -1,0 +1,747 @@
+// Row-wise pieces of the ragged-batch mixers: norms, residual updates, value preparation, activations, and what moves rows to experts
+// and back.  All are bound by the bytes of their rows, so a row is read once, in 16-byte pieces, and stays in registers between the
+// passes over it; rows that cannot be read that way (sizes or addresses off the 16-byte grid) take the element-wise form.
+//
+//   offset RMS norm            y = x * rsqrt(mean(x^2) + eps) * (1 + w)            fp32 in, storage dtype out
+//   post-norm residual update  x += m * norm(y; w_post), optionally followed by the next sublayer's input norm
+//   value prep + paged append  per-head unit-RMS values, optional mix with an earlier layer's values, K/V scatter
+//   per-head RMS norm          of a recurrence's fp32 read-outs
+//   PolyNorm activation        a N(z) + b N(z^2) + c N(z^3) + e over a token's feed-forward row
+//   expert order               a stable sort of (token, choice) pairs by expert in one CTA, with the experts' row offsets
+//   input-scaled expert rows, clamped GLU, combine
+//
+// Measured on B200 (bf16), element-wise -> this: post-norm residual with the next norm, 2600 rows of 1024: 15.1 -> 7.7 us; PolyNorm, 2600 x
+// 4096: 26.4 -> 11.5; value prep, 16384 tokens of 4 heads of 128 + 128: 52 -> 34; clamped GLU, 8198 x 1024: 28.5 -> 12.6; expert rows in
+// 14.5 -> 6.6, out 12.1 -> 7.2; expert order of 8198 pairs: 12.6 (sort, count and inverse by library calls: 75 and a wait on the host).
+#include <algorithm>
+#include <type_traits>
+
+#include "../../include/b200_mixers.h"
+#include "b200_common.cuh"
+
+namespace b200 {
+namespace {
+
+template <typename F>
+int rows_by_dtype(int dtype, const char* name, F&& f) {
+  switch (dtype) {
+    case B200_DTYPE_F16:
+      return f(static_cast<__half*>(nullptr));
+    case B200_DTYPE_BF16:
+      return f(static_cast<__nv_bfloat16*>(nullptr));
+    case B200_DTYPE_F32:
+      return f(static_cast<float*>(nullptr));
+    default:
+      return fail(B200_EINVAL, "%s: unsupported dtype %d", name, dtype);
+  }
+}
+
+__device__ __forceinline__ float logistic(float z) { return 1.0f / (1.0f + expf(-z)); }
+
+// N consecutive elements as fp32 (N * sizeof(T) a multiple of 8: 8- or 16-byte accesses)
+template <int N, typename T>
+__device__ __forceinline__ void get(float (&d)[N], const T* p) {
+  if constexpr (N * sizeof(T) == 8) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+    for (int i = 0; i < N; ++i) d[i] = Cvt<T>::to_f32(e[i]);
+  } else {
+    constexpr int E = 16 / sizeof(T);
+#pragma unroll
+    for (int j = 0; j < N / E; ++j) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(p + j * E);
+      const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+      for (int i = 0; i < E; ++i) d[j * E + i] = Cvt<T>::to_f32(e[i]);
+    }
+  }
+}
+template <int N, typename T>
+__device__ __forceinline__ void put(T* p, const float (&d)[N]) {
+  if constexpr (N * sizeof(T) == 8) {
+    uint2 raw;
+    T* e = reinterpret_cast<T*>(&raw);
+#pragma unroll
+    for (int i = 0; i < N; ++i) e[i] = Cvt<T>::from_f32(d[i]);
+    *reinterpret_cast<uint2*>(p) = raw;
+  } else {
+    constexpr int E = 16 / sizeof(T);
+#pragma unroll
+    for (int j = 0; j < N / E; ++j) {
+      uint4 raw;
+      T* e = reinterpret_cast<T*>(&raw);
+#pragma unroll
+      for (int i = 0; i < E; ++i) e[i] = Cvt<T>::from_f32(d[j * E + i]);
+      *reinterpret_cast<uint4*>(p + j * E) = raw;
+    }
+  }
+}
+
+// Sum over the WPR warps that share a row (one row per warp, or one per CTA); `red` holds WPR floats per call.
+template <int WPR>
+__device__ __forceinline__ float row_sum(float v, float* red) {
+  v = warp_sum(v);
+  if constexpr (WPR == 1) return v;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.f;
+#pragma unroll
+  for (int w = 0; w < WPR; ++w) t += red[w];
+  return t;
+}
+
+// squares of a piece, added pairwise (three roundings deep instead of eight)
+__device__ __forceinline__ float squares(const float (&d)[8]) {
+  const float a = fmaf(d[0], d[0], d[1] * d[1]), b = fmaf(d[2], d[2], d[3] * d[3]);
+  const float c = fmaf(d[4], d[4], d[5] * d[5]), e = fmaf(d[6], d[6], d[7] * d[7]);
+  return (a + b) + (c + e);
+}
+
+__device__ __forceinline__ float block_sum(float v, float* red) {
+  v = warp_sum(v);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  __syncthreads();
+  if (lane == 0) red[warp] = v;
+  __syncthreads();
+  return warp_sum(lane < nw ? red[lane] : 0.f);
+}
+
+// A row over WPR warps, NCH pieces of eight elements per lane: by its width alone, so that a row's sums do not depend on the step.
+// Rows of up to 1024 elements go to one warp each (no barrier).
+template <typename F>
+bool by_row_shape(int width, F&& f) {
+  auto go = [&](auto wpr, auto nch) { f(wpr, nch); };
+  using std::integral_constant;
+  if (width <= 512) go(integral_constant<int, 1>{}, integral_constant<int, 2>{});
+  else if (width <= 1024) go(integral_constant<int, 1>{}, integral_constant<int, 4>{});
+  else if (width <= 2048) go(integral_constant<int, 4>{}, integral_constant<int, 2>{});
+  else if (width <= 4096) go(integral_constant<int, 4>{}, integral_constant<int, 4>{});
+  else if (width <= 8192) go(integral_constant<int, 8>{}, integral_constant<int, 4>{});
+  else if (width <= 16384) go(integral_constant<int, 8>{}, integral_constant<int, 8>{});
+  else return false;
+  return true;
+}
+template <int WPR>
+struct RowCta {
+  static constexpr int kWarps = WPR == 1 ? 4 : WPR;      // per CTA
+  static constexpr int kNT = 32 * kWarps;
+  static unsigned grid(int64_t rows) { return static_cast<unsigned>(WPR == 1 ? (rows + 3) / 4 : rows); }
+};
+template <int WPR>
+__device__ __forceinline__ int64_t my_row() {
+  return WPR == 1 ? static_cast<int64_t>(blockIdx.x) * 4 + (threadIdx.x >> 5) : blockIdx.x;
+}
+template <int WPR>
+__device__ __forceinline__ int my_piece(int c) {       // first element of the lane's piece c
+  return ((WPR == 1 ? threadIdx.x & 31 : threadIdx.x) + c * 32 * WPR) * 8;
+}
+
+// ---- offset RMS norm ------------------------------------------------------------------------------------------
+template <typename T, int WPR, int NCH>
+__global__ void __launch_bounds__(RowCta<WPR>::kNT)
+offset_rmsnorm_rows(T* __restrict__ out, const float* __restrict__ x, const T* __restrict__ w, float eps, int64_t rows, int width) {
+  __shared__ float red[8];
+  const int64_t row = my_row<WPR>();
+  if (row >= rows) return;
+  float v[NCH][8], ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int i = my_piece<WPR>(c);
+    if (i < width) {
+      get(v[c], x + row * width + i);
+      ss += squares(v[c]);
+    }
+  }
+  const float inv = rsqrtf(row_sum<WPR>(ss, red) / static_cast<float>(width) + eps);
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int i = my_piece<WPR>(c);
+    if (i < width) {
+      float g[8];
+      get(g, w + i);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[c][u] = v[c][u] * inv * (1.0f + g[u]);
+      put(out + row * width + i, v[c]);
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(256)
+offset_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ x, const T* __restrict__ w, float eps, int width) {
+  __shared__ float red[32];
+  const float* xr = x + static_cast<int64_t>(blockIdx.x) * width;
+  float ss = 0.f;
+  for (int i = threadIdx.x; i < width; i += blockDim.x) ss = fmaf(xr[i], xr[i], ss);
+  const float inv = rsqrtf(block_sum(ss, red) / static_cast<float>(width) + eps);
+  T* orow = out + static_cast<int64_t>(blockIdx.x) * width;
+  for (int i = threadIdx.x; i < width; i += blockDim.x)
+    orow[i] = Cvt<T>::from_f32(xr[i] * inv * (1.0f + Cvt<T>::to_f32(w[i])));
+}
+
+// ---- x += mult * norm(y; w_post); optionally out_next = norm(x; w_next) ------------------------------------------
+template <typename T, typename Y, int WPR, int NCH>
+__global__ void __launch_bounds__(RowCta<WPR>::kNT)
+postnorm_residual_rows(float* __restrict__ x, const Y* __restrict__ y, int64_t y_stride, const T* __restrict__ w_post, float mult,
+                       const T* __restrict__ w_next, T* __restrict__ out_next, float eps, int64_t rows, int width) {
+  __shared__ float red[16];
+  const int64_t row = my_row<WPR>();
+  if (row >= rows) return;
+  float v[NCH][8], r[NCH][8], ss = 0.f;
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int i = my_piece<WPR>(c);
+    if (i < width) {
+      get(v[c], y + row * y_stride + i);
+      get(r[c], x + row * width + i);
+      ss += squares(v[c]);
+    }
+  }
+  const float inv = rsqrtf(row_sum<WPR>(ss, red) / static_cast<float>(width) + eps);
+  float sx = 0.f;
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int i = my_piece<WPR>(c);
+    if (i < width) {
+      float g[8];
+      get(g, w_post + i);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float n = v[c][u] * inv * (1.0f + g[u]);
+        r[c][u] += mult * n;
+      }
+      sx += squares(r[c]);
+      put(x + row * width + i, r[c]);
+    }
+  }
+  if (w_next == nullptr) return;
+  const float inv2 = rsqrtf(row_sum<WPR>(sx, red + 8) / static_cast<float>(width) + eps);
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int i = my_piece<WPR>(c);
+    if (i < width) {
+      float g[8];
+      get(g, w_next + i);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) r[c][u] = r[c][u] * inv2 * (1.0f + g[u]);
+      put(out_next + row * width + i, r[c]);
+    }
+  }
+}
+// element-wise form: the updated row is kept in shared memory between the update and the second norm
+template <typename T, typename Y>
+__global__ void __launch_bounds__(256)
+postnorm_residual_kernel(float* __restrict__ x, const Y* __restrict__ y, int64_t y_stride, const T* __restrict__ w_post,
+                         float mult, const T* __restrict__ w_next, T* __restrict__ out_next, float eps, int width) {
+  extern __shared__ float row_s[];
+  __shared__ float red[32];
+  const Y* yr = y + static_cast<int64_t>(blockIdx.x) * y_stride;
+  float* xr = x + static_cast<int64_t>(blockIdx.x) * width;
+  float ss = 0.f;
+  for (int i = threadIdx.x; i < width; i += blockDim.x) {
+    const float v = Cvt<Y>::to_f32(yr[i]);
+    ss = fmaf(v, v, ss);
+  }
+  const float inv = rsqrtf(block_sum(ss, red) / static_cast<float>(width) + eps);
+  float sx = 0.f;
+  for (int i = threadIdx.x; i < width; i += blockDim.x) {
+    const float n = Cvt<Y>::to_f32(yr[i]) * inv * (1.0f + Cvt<T>::to_f32(w_post[i]));
+    const float v = xr[i] + mult * n;
+    xr[i] = v;
+    row_s[i] = v;
+    sx = fmaf(v, v, sx);
+  }
+  if (w_next == nullptr) return;
+  const float inv2 = rsqrtf(block_sum(sx, red) / static_cast<float>(width) + eps);
+  T* orow = out_next + static_cast<int64_t>(blockIdx.x) * width;
+  for (int i = threadIdx.x; i < width; i += blockDim.x)
+    orow[i] = Cvt<T>::from_f32(row_s[i] * inv2 * (1.0f + Cvt<T>::to_f32(w_next[i])));
+}
+
+// ---- value prep + K/V append ------------------------------------------------------------------------------------
+// One warp per (token, kv head).  v <- v / rms(v); with `v_prev` the stored value is (1 - lam) v + lam v_prev.  The stored value also
+// goes to `v_keep` (for later layers of the same step) when given.  N elements per access (four, or one where rows are not aligned).
+template <typename T, int N>
+__global__ void __launch_bounds__(256)
+value_prep_append_kernel(const T* __restrict__ k, int64_t k_stride, const T* __restrict__ v, int64_t v_stride,
+                         const T* __restrict__ v_prev, T* __restrict__ v_keep, float lam, float eps,
+                         T* __restrict__ k_pool, T* __restrict__ v_pool, const int64_t* __restrict__ slot_mapping,
+                         int64_t n_tok, int G, int dk, int dv, int block_size, int64_t max_blocks) {
+  const int64_t pair = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const int64_t tok = pair / G;
+  const int g = static_cast<int>(pair - tok * G), lane = threadIdx.x & 31;
+  if (tok >= n_tok) return;
+  const int64_t slot = slot_mapping[tok];
+  const int64_t blk = slot >= 0 ? slot / block_size : -1;
+  const bool store = blk >= 0 && blk < max_blocks;
+  const int64_t at = store ? (blk * G + g) * block_size + (slot - blk * block_size) : 0;
+  auto load = [](float (&d)[N], const T* p) {
+    if constexpr (N == 1) d[0] = Cvt<T>::to_f32(p[0]);
+    else get(d, p);
+  };
+  auto save = [](T* p, const float (&d)[N]) {
+    if constexpr (N == 1) p[0] = Cvt<T>::from_f32(d[0]);
+    else put(p, d);
+  };
+  const T* vr = v + tok * v_stride + g * dv;
+  float ss = 0.f;
+  for (int c = lane * N; c < dv; c += 32 * N) {
+    float f[N];
+    load(f, vr + c);
+#pragma unroll
+    for (int u = 0; u < N; ++u) ss = fmaf(f[u], f[u], ss);
+  }
+  const float inv = rsqrtf(warp_sum(ss) / static_cast<float>(dv) + eps);
+  for (int c = lane * N; c < dv; c += 32 * N) {
+    float f[N];
+    load(f, vr + c);
+#pragma unroll
+    for (int u = 0; u < N; ++u) f[u] *= inv;
+    if (v_prev) {
+      float o[N];
+      load(o, v_prev + (tok * G + g) * dv + c);
+#pragma unroll
+      for (int u = 0; u < N; ++u) f[u] = (1.0f - lam) * f[u] + lam * o[u];
+    }
+    if (store) save(v_pool + at * dv + c, f);
+    if (v_keep) save(v_keep + (tok * G + g) * dv + c, f);
+  }
+  if (store) {
+    for (int c = lane * N; c < dk; c += 32 * N) {
+      const T* src = k + tok * k_stride + g * dk + c;
+      T* dst = k_pool + at * dk + c;
+      if constexpr (N == 1) {
+        dst[0] = src[0];
+      } else if constexpr (N * sizeof(T) == 8) {
+        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
+      } else {
+        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+      }
+    }
+  }
+}
+
+// ---- per-head weighted RMS norm of fp32 rows [rows, dv] -> T; one warp per row -------------------------------------
+template <typename T, int NCH>
+__global__ void __launch_bounds__(256)
+head_rmsnorm_rows(T* __restrict__ out, const float* __restrict__ x, const T* __restrict__ w, float eps, int64_t rows, int dv) {
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int c0 = (threadIdx.x & 31) * 4;
+  float v[NCH][4], ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NCH; ++j) {
+    if (c0 + 128 * j < dv) {
+      get(v[j], x + row * dv + c0 + 128 * j);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) ss = fmaf(v[j][u], v[j][u], ss);
+    }
+  }
+  const float inv = rsqrtf(warp_sum(ss) / static_cast<float>(dv) + eps);
+#pragma unroll
+  for (int j = 0; j < NCH; ++j) {
+    if (c0 + 128 * j < dv) {
+      float g[4];
+      get(g, w + c0 + 128 * j);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[j][u] = v[j][u] * inv * g[u];
+      put(out + row * dv + c0 + 128 * j, v[j]);
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(256)
+head_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ x, const T* __restrict__ w, float eps, int64_t rows,
+                    int dv) {
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
+  const float* xr = x + row * dv;
+  float ss = 0.f;
+  for (int c = lane; c < dv; c += 32) ss = fmaf(xr[c], xr[c], ss);
+  const float inv = rsqrtf(warp_sum(ss) / static_cast<float>(dv) + eps);
+  for (int c = lane; c < dv; c += 32) out[row * dv + c] = Cvt<T>::from_f32(xr[c] * inv * Cvt<T>::to_f32(w[c]));
+}
+
+// ---- PolyNorm ---------------------------------------------------------------------------------------------------
+template <typename T, int WPR, int NCH>
+__global__ void __launch_bounds__(RowCta<WPR>::kNT)
+polynorm_rows(T* __restrict__ out, const T* __restrict__ z, int64_t z_stride, const T* __restrict__ coef, float eps, int64_t rows, int ff) {
+  __shared__ float red[24];
+  const int64_t row = my_row<WPR>();
+  if (row >= rows) return;
+  float a[NCH][8], s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int i = my_piece<WPR>(c);
+    if (i < ff) {
+      get(a[c], z + row * z_stride + i);
+      float a2[8], a3[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        a2[u] = a[c][u] * a[c][u];
+        a3[u] = a2[u] * a[c][u];
+      }
+      s1 += squares(a[c]);
+      s2 += squares(a2);
+      s3 += squares(a3);
+    }
+  }
+  const float n = static_cast<float>(ff);
+  const float i1 = rsqrtf(row_sum<WPR>(s1, red) / n + eps);
+  const float i2 = rsqrtf(row_sum<WPR>(s2, red + 8) / n + eps);
+  const float i3 = rsqrtf(row_sum<WPR>(s3, red + 16) / n + eps);
+  const float ca = Cvt<T>::to_f32(coef[0]), cb = Cvt<T>::to_f32(coef[1]), cc = Cvt<T>::to_f32(coef[2]), ce = Cvt<T>::to_f32(coef[3]);
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    const int i = my_piece<WPR>(c);
+    if (i < ff) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float a1 = a[c][u], a2 = a1 * a1;
+        a[c][u] = ca * a1 * i1 + cb * a2 * i2 + cc * a2 * a1 * i3 + ce;
+      }
+      put(out + row * ff + i, a[c]);
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(256)
+polynorm_kernel(T* __restrict__ out, const T* __restrict__ z, int64_t z_stride, const T* __restrict__ coef, float eps,
+                int ff) {
+  __shared__ float red[32];
+  const T* zr = z + static_cast<int64_t>(blockIdx.x) * z_stride;
+  float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  for (int i = threadIdx.x; i < ff; i += blockDim.x) {
+    const float a = Cvt<T>::to_f32(zr[i]);
+    const float a2 = a * a, a3 = a2 * a;
+    s1 = fmaf(a, a, s1);
+    s2 = fmaf(a2, a2, s2);
+    s3 = fmaf(a3, a3, s3);
+  }
+  const float n = static_cast<float>(ff);
+  const float i1 = rsqrtf(block_sum(s1, red) / n + eps);
+  const float i2 = rsqrtf(block_sum(s2, red) / n + eps);
+  const float i3 = rsqrtf(block_sum(s3, red) / n + eps);
+  const float ca = Cvt<T>::to_f32(coef[0]), cb = Cvt<T>::to_f32(coef[1]), cc = Cvt<T>::to_f32(coef[2]),
+              ce = Cvt<T>::to_f32(coef[3]);
+  T* orow = out + static_cast<int64_t>(blockIdx.x) * ff;
+  for (int i = threadIdx.x; i < ff; i += blockDim.x) {
+    const float a = Cvt<T>::to_f32(zr[i]);
+    const float a2 = a * a;
+    orow[i] = Cvt<T>::from_f32(ca * a * i1 + cb * a2 * i2 + cc * a2 * a * i3 + ce);
+  }
+}
+
+// ---- expert order -------------------------------------------------------------------------------------------------
+// One CTA of 1024 threads; thread t owns the pairs of a contiguous chunk.  count[e][t] pairs of expert e in chunk t -> their running
+// sums over the chunks (a warp per expert) -> where every chunk's pairs of every expert start: a stable counting sort.  The ids are
+// read twice and every output is written once; a radix sort of the same pairs is eight launches.
+constexpr int kOrderNT = 1024;
+constexpr int kOrderExperts = 48;
+__global__ void __launch_bounds__(kOrderNT)
+expert_order_kernel(int64_t* __restrict__ order, int64_t* __restrict__ where, int32_t* __restrict__ offsets, const int32_t* __restrict__ ids,
+                    int n_pairs, int E) {
+  extern __shared__ int count[];          // [E][1024], then [E + 1]
+  int* start = count + E * kOrderNT;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int per = (n_pairs + kOrderNT - 1) / kOrderNT, lo = min(t * per, n_pairs), hi = min(lo + per, n_pairs);
+  for (int e = 0; e < E; ++e) count[e * kOrderNT + t] = 0;
+  for (int i = lo; i < hi; ++i) {
+    const int e = ids[i];
+    if (e >= 0 && e < E) ++count[e * kOrderNT + t];
+  }
+  __syncthreads();
+  for (int e = warp; e < E; e += kOrderNT / 32) {
+    int run = 0;
+    for (int c = lane; c < kOrderNT; c += 32) {
+      const int v = count[e * kOrderNT + c];
+      int s = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += u;
+      }
+      count[e * kOrderNT + c] = run + s - v;
+      run += __shfl_sync(0xffffffffu, s, 31);
+    }
+    if (lane == 0) start[e + 1] = run;
+  }
+  __syncthreads();
+  if (t == 0) {
+    start[0] = 0;
+    for (int e = 0; e < E; ++e) start[e + 1] += start[e];
+  }
+  __syncthreads();
+  if (t <= E) offsets[t] = start[t];
+  for (int i = lo; i < hi; ++i) {
+    const int e = ids[i];
+    if (e < 0 || e >= E) continue;
+    const int at = start[e] + count[e * kOrderNT + t]++;
+    order[at] = i;
+    where[i] = at;
+  }
+}
+
+// ---- rows of the expert-sorted input: xs[r] = T(w[src[r]] * h[src[r] / top]) ------------------------------------------
+template <typename T, int N>
+__global__ void __launch_bounds__(128)
+scaled_gather_kernel(T* __restrict__ xs, const T* __restrict__ h, const float* __restrict__ weights,
+                     const int64_t* __restrict__ src, int top, int width) {
+  const int64_t pair = src[blockIdx.x];
+  const float w = weights[pair];
+  const T* hr = h + (pair / top) * width;
+  T* o = xs + static_cast<int64_t>(blockIdx.x) * width;
+  for (int i = threadIdx.x * N; i < width; i += 128 * N) {
+    if constexpr (N == 1) {
+      o[i] = Cvt<T>::from_f32(w * Cvt<T>::to_f32(hr[i]));
+    } else {
+      float f[N];
+      get(f, hr + i);
+#pragma unroll
+      for (int u = 0; u < N; ++u) f[u] *= w;
+      put(o + i, f);
+    }
+  }
+}
+
+// ---- y = g' * sigmoid(alpha g') * (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit); gu rows hold g | u ---------
+template <typename T, int N>
+__global__ void __launch_bounds__(256)
+clamped_glu_kernel(T* __restrict__ y, const T* __restrict__ gu, int64_t rows, int ff, float limit, float alpha) {
+  const int64_t n = rows * (ff / N);
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t r = i / (ff / N);
+    const int c = static_cast<int>(i - r * (ff / N)) * N;
+    float a[N], b[N];
+    if constexpr (N == 1) {
+      a[0] = Cvt<T>::to_f32(gu[r * 2 * ff + c]);
+      b[0] = Cvt<T>::to_f32(gu[r * 2 * ff + ff + c]);
+    } else {
+      get(a, gu + r * 2 * ff + c);
+      get(b, gu + r * 2 * ff + ff + c);
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const float g = fminf(a[u], limit);
+      const float up = fminf(fmaxf(b[u], -limit), limit);
+      a[u] = g * logistic(alpha * g) * (up + 1.0f);
+    }
+    if constexpr (N == 1) y[i] = Cvt<T>::from_f32(a[0]);
+    else put(y + r * ff + c, a);
+  }
+}
+
+// ---- out[n] = sum_k ys[where[n * top + k]] in fp32, k ascending ---------------------------------------------------------
+template <typename T, int N>
+__global__ void __launch_bounds__(128)
+expert_combine_kernel(float* __restrict__ out, const T* __restrict__ ys, const int64_t* __restrict__ where, int top,
+                      int width) {
+  const int64_t n = blockIdx.x;
+  for (int i = threadIdx.x * N; i < width; i += 128 * N) {
+    float a[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) a[u] = 0.f;
+    for (int k = 0; k < top; ++k) {
+      const T* src = ys + where[n * top + k] * width + i;
+      if constexpr (N == 1) {
+        a[0] += Cvt<T>::to_f32(src[0]);
+      } else {
+        float f[N];
+        get(f, src);
+#pragma unroll
+        for (int u = 0; u < N; ++u) a[u] += f[u];
+      }
+    }
+    if constexpr (N == 1) out[n * width + i] = a[0];
+    else put(out + n * width + i, a);
+  }
+}
+
+template <typename... P>
+bool all16(const P*... p) {
+  return (... && (p == nullptr || aligned16(p)));
+}
+
+}  // namespace
+}  // namespace b200
+
+using namespace b200;
+
+extern "C" {
+
+int b200_offset_rmsnorm(void* out, const float* x, const void* weight, float eps, int rows, int width, int dtype,
+                        void* stream) {
+  if (rows < 0 || width <= 0) return fail(B200_EINVAL, "b200_offset_rmsnorm: bad sizes");
+  if (rows == 0) return 0;
+  if (!out || !x || !weight) return fail(B200_EINVAL, "b200_offset_rmsnorm: null pointer");
+  const auto s = static_cast<cudaStream_t>(stream);
+  return rows_by_dtype(dtype, "b200_offset_rmsnorm", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    const bool whole = width % 8 == 0 && all16(out, x, weight) && by_row_shape(width, [&](auto wpr, auto nch) {
+      constexpr int W = decltype(wpr)::value;
+      offset_rmsnorm_rows<T, W, decltype(nch)::value><<<RowCta<W>::grid(rows), RowCta<W>::kNT, 0, s>>>(
+          static_cast<T*>(out), x, static_cast<const T*>(weight), eps, rows, width);
+    });
+    if (!whole)
+      offset_rmsnorm_kernel<T><<<rows, 256, 0, s>>>(static_cast<T*>(out), x, static_cast<const T*>(weight), eps, width);
+    return check_launch("b200_offset_rmsnorm");
+  });
+}
+
+int b200_postnorm_residual(float* x, const void* y, int64_t y_stride, int y_is_f32, const void* w_post, float mult,
+                           const void* w_next, void* out_next, float eps, int rows, int width, int dtype, void* stream) {
+  if (rows < 0 || width <= 0 || width > 40000) return fail(B200_EINVAL, "b200_postnorm_residual: bad sizes");
+  if (rows == 0) return 0;
+  if (!x || !y || !w_post || (w_next && !out_next)) return fail(B200_EINVAL, "b200_postnorm_residual: null pointer");
+  const size_t smem = static_cast<size_t>(width) * sizeof(float);
+  const auto s = static_cast<cudaStream_t>(stream);
+  return rows_by_dtype(dtype, "b200_postnorm_residual", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    auto launch = [&](auto* ytag) {
+      using Y = std::remove_pointer_t<decltype(ytag)>;
+      const bool whole = width % 8 == 0 && y_stride % 8 == 0 && all16(x, y, w_post, w_next, out_next) &&
+                         by_row_shape(width, [&](auto wpr, auto nch) {
+        constexpr int W = decltype(wpr)::value;
+        postnorm_residual_rows<T, Y, W, decltype(nch)::value><<<RowCta<W>::grid(rows), RowCta<W>::kNT, 0, s>>>(
+            x, static_cast<const Y*>(y), y_stride, static_cast<const T*>(w_post), mult, static_cast<const T*>(w_next),
+            static_cast<T*>(out_next), eps, rows, width);
+      });
+      if (whole) return;
+      auto kern = postnorm_residual_kernel<T, Y>;
+      if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+      kern<<<rows, 256, smem, s>>>(x, static_cast<const Y*>(y), y_stride, static_cast<const T*>(w_post), mult,
+                                   static_cast<const T*>(w_next), static_cast<T*>(out_next), eps, width);
+    };
+    if (y_is_f32) launch(static_cast<float*>(nullptr));
+    else launch(static_cast<T*>(nullptr));
+    return check_launch("b200_postnorm_residual");
+  });
+}
+
+int b200_value_prep_append(const void* k, int64_t k_stride, const void* v, int64_t v_stride, const void* v_prev,
+                           void* v_keep, float lam, float eps, void* k_pool, void* v_pool, const int64_t* slot_mapping,
+                           int n_tok, int G, int dk, int dv, int block_size, int64_t max_blocks, int dtype, void* stream) {
+  if (n_tok < 0 || G <= 0 || dk <= 0 || dv <= 0 || block_size <= 0) return fail(B200_EINVAL, "b200_value_prep_append: bad sizes");
+  if (n_tok == 0) return 0;
+  if (!k || !v || !k_pool || !v_pool || !slot_mapping) return fail(B200_EINVAL, "b200_value_prep_append: null pointer");
+  const bool four = dk % 4 == 0 && dv % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 && all16(v_prev, v_keep, k_pool, v_pool) &&
+                    reinterpret_cast<uintptr_t>(k) % (4 * dtype_size(dtype)) == 0 && reinterpret_cast<uintptr_t>(v) % (4 * dtype_size(dtype)) == 0;
+  const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(n_tok) * G + 7) / 8);
+  return rows_by_dtype(dtype, "b200_value_prep_append", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    auto launch = [&](auto kern) {
+      kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+          static_cast<const T*>(k), k_stride, static_cast<const T*>(v), v_stride, static_cast<const T*>(v_prev),
+          static_cast<T*>(v_keep), lam, eps, static_cast<T*>(k_pool), static_cast<T*>(v_pool), slot_mapping, n_tok, G, dk, dv,
+          block_size, max_blocks);
+    };
+    if (four) launch(value_prep_append_kernel<T, 4>);
+    else launch(value_prep_append_kernel<T, 1>);
+    return check_launch("b200_value_prep_append");
+  });
+}
+
+int b200_head_rmsnorm(void* out, const float* x, const void* weight, float eps, int64_t rows, int dv, int dtype,
+                      void* stream) {
+  if (rows < 0 || dv <= 0) return fail(B200_EINVAL, "b200_head_rmsnorm: bad sizes");
+  if (rows == 0) return 0;
+  if (!out || !x || !weight) return fail(B200_EINVAL, "b200_head_rmsnorm: null pointer");
+  return rows_by_dtype(dtype, "b200_head_rmsnorm", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    auto launch = [&](auto kern) {
+      kern<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+          static_cast<T*>(out), x, static_cast<const T*>(weight), eps, rows, dv);
+    };
+    if (dv % 4 == 0 && dv <= 128 && all16(out, x, weight)) launch(head_rmsnorm_rows<T, 1>);
+    else if (dv % 4 == 0 && dv <= 512 && all16(out, x, weight)) launch(head_rmsnorm_rows<T, 4>);
+    else launch(head_rmsnorm_kernel<T>);
+    return check_launch("b200_head_rmsnorm");
+  });
+}
+
+int b200_polynorm(void* out, const void* z, int64_t z_stride, const void* coef, float eps, int rows, int ff, int dtype,
+                  void* stream) {
+  if (rows < 0 || ff <= 0) return fail(B200_EINVAL, "b200_polynorm: bad sizes");
+  if (rows == 0) return 0;
+  if (!out || !z || !coef) return fail(B200_EINVAL, "b200_polynorm: null pointer");
+  const auto s = static_cast<cudaStream_t>(stream);
+  return rows_by_dtype(dtype, "b200_polynorm", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    const bool whole = ff % 8 == 0 && z_stride % 8 == 0 && all16(out, z) && by_row_shape(ff, [&](auto wpr, auto nch) {
+      constexpr int W = decltype(wpr)::value;
+      polynorm_rows<T, W, decltype(nch)::value><<<RowCta<W>::grid(rows), RowCta<W>::kNT, 0, s>>>(
+          static_cast<T*>(out), static_cast<const T*>(z), z_stride, static_cast<const T*>(coef), eps, rows, ff);
+    });
+    if (!whole)
+      polynorm_kernel<T><<<rows, 256, 0, s>>>(static_cast<T*>(out), static_cast<const T*>(z), z_stride, static_cast<const T*>(coef), eps, ff);
+    return check_launch("b200_polynorm");
+  });
+}
+
+int b200_expert_order_supported(int64_t n_pairs, int n_experts) {
+  return n_pairs >= 0 && n_pairs <= (1 << 17) && n_experts > 0 && n_experts <= kOrderExperts;
+}
+
+int b200_expert_order(int64_t* order, int64_t* where, int32_t* offsets, const int32_t* ids, int64_t n_pairs, int n_experts, void* stream) {
+  if (!b200_expert_order_supported(n_pairs, n_experts)) return fail(B200_ESHAPE, "b200_expert_order: up to %d pairs and %d experts", 1 << 17, kOrderExperts);
+  if (!offsets || (n_pairs > 0 && (!order || !where || !ids))) return fail(B200_EINVAL, "b200_expert_order: null pointer");
+  const size_t smem = sizeof(int) * (static_cast<size_t>(n_experts) * kOrderNT + n_experts + 1);
+  if (smem > 48 * 1024) cudaFuncSetAttribute(expert_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  expert_order_kernel<<<1, kOrderNT, smem, static_cast<cudaStream_t>(stream)>>>(order, where, offsets, ids, static_cast<int>(n_pairs), n_experts);
+  return check_launch("b200_expert_order");
+}
+
+int b200_scaled_gather(void* xs, const void* h, const float* weights, const int64_t* src, int64_t n_rows, int top,
+                       int width, int dtype, void* stream) {
+  if (n_rows < 0 || top <= 0 || width <= 0) return fail(B200_EINVAL, "b200_scaled_gather: bad sizes");
+  if (n_rows == 0) return 0;
+  if (!xs || !h || !weights || !src) return fail(B200_EINVAL, "b200_scaled_gather: null pointer");
+  return rows_by_dtype(dtype, "b200_scaled_gather", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    auto launch = [&](auto kern) {
+      kern<<<static_cast<unsigned>(n_rows), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+          static_cast<T*>(xs), static_cast<const T*>(h), weights, src, top, width);
+    };
+    if (width % 8 == 0 && all16(xs, h)) launch(scaled_gather_kernel<T, 8>);
+    else launch(scaled_gather_kernel<T, 1>);
+    return check_launch("b200_scaled_gather");
+  });
+}
+
+int b200_clamped_glu(void* y, const void* gu, int64_t rows, int ff, float limit, float alpha, int dtype, void* stream) {
+  if (rows < 0 || ff <= 0) return fail(B200_EINVAL, "b200_clamped_glu: bad sizes");
+  if (rows == 0) return 0;
+  if (!y || !gu) return fail(B200_EINVAL, "b200_clamped_glu: null pointer");
+  const bool eight = ff % 8 == 0 && all16(y, gu);
+  const int64_t n = rows * ff / (eight ? 8 : 1);
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, kNumSMs * 16));
+  return rows_by_dtype(dtype, "b200_clamped_glu", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    auto launch = [&](auto kern) {
+      kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<T*>(y), static_cast<const T*>(gu), rows, ff, limit, alpha);
+    };
+    if (eight) launch(clamped_glu_kernel<T, 8>);
+    else launch(clamped_glu_kernel<T, 1>);
+    return check_launch("b200_clamped_glu");
+  });
+}
+
+int b200_expert_combine(float* out, const void* ys, const int64_t* where, int64_t n_tok, int top, int width, int dtype,
+                        void* stream) {
+  if (n_tok < 0 || top <= 0 || width <= 0) return fail(B200_EINVAL, "b200_expert_combine: bad sizes");
+  if (n_tok == 0) return 0;
+  if (!out || !ys || !where) return fail(B200_EINVAL, "b200_expert_combine: null pointer");
+  return rows_by_dtype(dtype, "b200_expert_combine", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    auto launch = [&](auto kern) {
+      kern<<<static_cast<unsigned>(n_tok), 128, 0, static_cast<cudaStream_t>(stream)>>>(out, static_cast<const T*>(ys), where, top, width);
+    };
+    if (width % 8 == 0 && all16(out, ys)) launch(expert_combine_kernel<T, 8>);
+    else launch(expert_combine_kernel<T, 1>);
+    return check_launch("b200_expert_combine");
+  });
+}
+
+}  // extern "C"

@@ -1,6 +1,7 @@
 // Attention of prompt portions over the paged cache on the fifth-generation tensor cores (16-bit storage types).
 //
-// A CTA serves 256 query rows of one sequence and one kv head (128 where the head sizes leave no room for more): up to 256 / rep
+// A CTA serves 256 query rows of one sequence and one kv head (128 where the head sizes leave no room for more, and two such CTAs
+// per SM in small steps): up to 256 / rep
 // consecutive tokens x the rep = H / G query heads that read this kv head, so a key tile is fetched once for all of them.  Keys are
 // walked in tiles of 64.
 //
@@ -177,11 +178,12 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 // shared memory of one CTA, from a 1024-byte boundary
-template <int DK, int DV, bool ALIAS>
+template <int DK, int DV, bool ALIAS, int HALVES>
 struct Plan {
-  static constexpr int kHalves = DK <= 128 ? 2 : 1;     // sets of 128 rows
+  static constexpr int kHalves = HALVES;                // sets of 128 rows
+  static constexpr int kCtas = HALVES == 1 && DK <= 128 ? 2 : 1;   // per SM
   static constexpr int kSoft = kHalves * kRows, kNT = kSoft + kLoad + 32;
-  static constexpr int kBufs = 3;                       // of keys, and of values
+  static constexpr int kBufs = kCtas == 2 ? 2 : 3;      // of keys, and of values
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + kHalves * (DK / 64) * kRows * 128;
   static constexpr int kV = kK + kBufs * (DK / 64) * kBlk;
@@ -190,15 +192,15 @@ struct Plan {
   static constexpr int kPage = kBar + 256;             // int [2][2][64]: rows of the pools that a tile's keys / values are in (-1: none)
   static constexpr int kLut = kPage + 2 * 2 * kKeys * 4;  // float [4][rep][pitch]: biases of the tiles' distances
   static constexpr int kO = 2 * kKeys;                 // columns of tensor memory per half: S0 | S1 | O
-  static constexpr int kHalfTm = kHalves == 2 ? 256 : 512;
-  static constexpr int kTm = 512;
+  static constexpr int kHalfTm = kHalves == 2 || kCtas == 2 ? 256 : 512;
+  static constexpr int kTm = kHalves * kHalfTm;
   static_assert(kO + DV <= kHalfTm, "tensor memory");
 };
 
-template <typename T, int DK, int DV, bool ALIAS, bool BIAS>
-__global__ void __launch_bounds__(Plan<DK, DV, ALIAS>::kNT, 1)
+template <typename T, int DK, int DV, bool ALIAS, bool BIAS, int HALVES>
+__global__ void __launch_bounds__(Plan<DK, DV, ALIAS, HALVES>::kNT, Plan<DK, DV, ALIAS, HALVES>::kCtas)
 tile_attn_kernel(const TileAttn A) {
-  using P = Plan<DK, DV, ALIAS>;
+  using P = Plan<DK, DV, ALIAS, HALVES>;
   constexpr int NB = P::kBufs, kSoft = P::kSoft;
   extern __shared__ unsigned char raw_smem[];
   unsigned char* sm = raw_smem + ((1024 - (smem_u32(raw_smem) & 1023)) & 1023);
@@ -566,31 +568,35 @@ tile_attn_kernel(const TileAttn A) {
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "n"(P::kTm));
 }
 
-template <typename T, int DK, int DV, bool ALIAS, bool BIAS>
+template <typename T, int DK, int DV, bool ALIAS, bool BIAS, int HALVES>
 int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stream) {
-  using P = Plan<DK, DV, ALIAS>;
+  using P = Plan<DK, DV, ALIAS, HALVES>;
   const int rep = A.H / A.G;
   size_t smem = 1024 + P::kLut;
   if (BIAS) smem += sizeof(float) * 4 * rep * (((P::kSoft / rep + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep));
-  smem = std::max<size_t>(smem, 120 * 1024);      // a CTA takes all of an SM's tensor memory: one per SM
+  smem = std::max<size_t>(smem, P::kCtas == 2 ? 80 * 1024 : 120 * 1024);   // no more CTAs per SM than tensor memory has room for
   if (smem > 227 * 1024) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
-  auto kern = tile_attn_kernel<T, DK, DV, ALIAS, BIAS>;
+  auto kern = tile_attn_kernel<T, DK, DV, ALIAS, BIAS, HALVES>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   kern<<<dim3(n_tiles, A.G, n_splits), P::kNT, smem, stream>>>(A);
   return check_launch("b200_tile_attn");
 }
 
 template <typename T>
-int launch_shape(const TileAttn& A, int dk, int dv, bool alias, int n_tiles, int n_splits, cudaStream_t stream) {
-  if (A.bias_lut) {
-    if (!alias && dk == 128 && dv == 128) return launch_tiles<T, 128, 128, false, true>(A, n_tiles, n_splits, stream);
-    if (!alias && dk == 64 && dv == 64) return launch_tiles<T, 64, 64, false, true>(A, n_tiles, n_splits, stream);
-  } else {
-    if (!alias && dk == 128 && dv == 128) return launch_tiles<T, 128, 128, false, false>(A, n_tiles, n_splits, stream);
-    if (!alias && dk == 64 && dv == 64) return launch_tiles<T, 64, 64, false, false>(A, n_tiles, n_splits, stream);
-    if (alias && dk == 256 && dv == 256) return launch_tiles<T, 256, 256, true, false>(A, n_tiles, n_splits, stream);
-    if (alias && dk == 320 && dv == 256) return launch_tiles<T, 320, 256, true, false>(A, n_tiles, n_splits, stream);
-  }
+int launch_shape(const TileAttn& A, int dk, int dv, bool alias, int rows, int n_tiles, int n_splits, cudaStream_t stream) {
+  auto grouped = [&](auto size) {
+    constexpr int D = decltype(size)::value;
+    if (rows == kRows) {
+      return A.bias_lut ? launch_tiles<T, D, D, false, true, 1>(A, n_tiles, n_splits, stream)
+                        : launch_tiles<T, D, D, false, false, 1>(A, n_tiles, n_splits, stream);
+    }
+    return A.bias_lut ? launch_tiles<T, D, D, false, true, 2>(A, n_tiles, n_splits, stream)
+                      : launch_tiles<T, D, D, false, false, 2>(A, n_tiles, n_splits, stream);
+  };
+  if (!alias && dk == 128 && dv == 128) return grouped(std::integral_constant<int, 128>{});
+  if (!alias && dk == 64 && dv == 64) return grouped(std::integral_constant<int, 64>{});
+  if (alias && dk == 256 && dv == 256) return launch_tiles<T, 256, 256, true, false, 1>(A, n_tiles, n_splits, stream);
+  if (alias && dk == 320 && dv == 256) return launch_tiles<T, 320, 256, true, false, 1>(A, n_tiles, n_splits, stream);
   return fail(B200_ESHAPE, "b200_tile_attn: head sizes %d / %d are not built", dk, dv);
 }
 
@@ -603,18 +609,26 @@ bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, in
   return dk == dv && (dk == 64 || dk == 128);
 }
 
-int tile_attn_rows(int dk) { return dk <= 128 ? 2 * kTileRows : kTileRows; }
-
-int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk) {
-  (void)dk;
-  const int64_t ctas = static_cast<int64_t>(n_tiles) * G;
-  if (ctas <= 0 || ctas * 2 > kNumSMs) return 1;
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({16, kNumSMs / ctas, key_tiles / 3})));
+// 256 rows share a fetched key tile, but only one such CTA runs per SM and nothing covers its beginning and end: worth it from three
+// rounds of them on (8 x 2048 tokens, 16 heads over 4, 7 rounds: 209 us against 242 with 128 rows and two CTAs per SM; 5 portions of up
+// to 1024 tokens under a window of 512, 1.4 rounds: 79 against 63).
+int tile_attn_rows(int rep, int G, int dk, int n_tokens) {
+  const int64_t ctas = static_cast<int64_t>(n_tokens) * rep / (2 * kTileRows) * G;
+  return dk <= 128 && ctas >= 3 * kNumSMs ? 2 * kTileRows : kTileRows;
 }
 
-int tile_attn_launch(const TileAttn& A, int dk, int dv, bool alias, int n_tiles, int n_splits, int dtype, cudaStream_t stream) {
-  return dtype == B200_DTYPE_BF16 ? launch_shape<__nv_bfloat16>(A, dk, dv, alias, n_tiles, n_splits, stream)
-                                  : launch_shape<__half>(A, dk, dv, alias, n_tiles, n_splits, stream);
+// Keys are divided while the chip has room for more CTAs, a share being worth its part of the merge: three tiles of 64 keys where
+// few rows are merged, eight otherwise.
+int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int rows) {
+  const int64_t ctas = static_cast<int64_t>(n_tiles) * G, room = (rows == kTileRows && dk <= 128 ? 2 : 1) * kNumSMs;
+  if (ctas <= 0 || ctas * 2 > room) return 1;
+  const int share = ctas * rows <= 4096 ? 3 : 8;
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({16, room / ctas, key_tiles / share})));
+}
+
+int tile_attn_launch(const TileAttn& A, int dk, int dv, bool alias, int rows, int n_tiles, int n_splits, int dtype, cudaStream_t stream) {
+  return dtype == B200_DTYPE_BF16 ? launch_shape<__nv_bfloat16>(A, dk, dv, alias, rows, n_tiles, n_splits, stream)
+                                  : launch_shape<__half>(A, dk, dv, alias, rows, n_tiles, n_splits, stream);
 }
 
 }  // namespace b200

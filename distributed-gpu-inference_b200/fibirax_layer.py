@@ -182,7 +182,7 @@ class ParallelMixer(nn.Module):
             args = (attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables)
             kw = dict(sink=self.sink, window=self.window, max_context=st.max_context(), softcap=self.softcap)
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
             if rest is not None:
                 mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
         else:
@@ -224,19 +224,12 @@ class GroupedSoftmaxMoE(nn.Module):
             self.w_down = _param(torch.stack([t[f"e{e}.down"] for e in range(self.E)]), device, dtype)  # [E, W, ff]
         self.grouped = bool(self.E) and (mixer_ops.grouped_linear_supported(self.w_gu.shape[2], self.w_gu.dtype)
                                          and mixer_ops.grouped_linear_supported(self.w_down.shape[2], self.w_down.dtype))
-        self._ar: Optional[torch.Tensor] = None
         self.shared_limit = 0.0
         self.ws_gu = self.ws_down = None
         if spec.get("shared"):
             self.shared_limit = float(spec["shared"]["limit"])
             self.ws_gu = _param(torch.cat([t["shared.gate"], t["shared.up"]], dim=0), device, dtype)
             self.ws_down = _param(t["shared.down"], device, dtype)
-
-    def _arange(self, n: int, device) -> torch.Tensor:
-        """``arange(n)`` on the device, cut from a cached longer one."""
-        if self._ar is None or self._ar.numel() < n or self._ar.device != device:
-            self._ar = torch.arange(max(n, 4096), device=device)
-        return self._ar[:n]
 
     def _route(self, x: torch.Tensor):
         """``(expert ids int32 [n, top], weights fp32 [n, top])`` from the fp32 residual rows."""
@@ -253,15 +246,11 @@ class GroupedSoftmaxMoE(nn.Module):
         """The chosen experts' outputs: ``(ys [n * top, width] in expert order, where int64 [n * top])``; entry ``k`` of
         token ``n`` is row ``where[n * top + k]``."""
         n, top, E = h.shape[0], self.top, self.E
-        # rows in expert order; where each expert's rows start comes from the sorted ids themselves (a search, not a
-        # count: no value ever travels to the host)
-        # 16-bit keys: the radix sort takes two passes where 64-bit keys take eight (expert counts stay far below 2^15)
-        sorted_ids, order = torch.sort(ids.reshape(-1).to(torch.int16), stable=True)
-        where = torch.empty_like(order)
-        where[order] = self._arange(n * top, h.device)
+        # rows in expert order, and where each expert's rows start: no value ever travels to the host
+        order, where, offsets = mixer_ops.expert_order(ids, E + self.ident)
+        offsets = offsets[:E + 1]
         ys = h.new_empty((0, h.shape[1]))
         if E:
-            offsets = torch.searchsorted(sorted_ids, self._arange(E + 1, h.device).to(torch.int16)).to(torch.int32)
             xs = mixer_ops.gather_rows(h, order, top)      # identity rows ride at the end and are never multiplied
             if self.grouped and n * top <= self.GROUPED_MAX_ROWS:
                 y = self._activate(mixer_ops.grouped_linear(xs, self.w_gu, offsets))

@@ -249,6 +249,29 @@ def sigmoid_topk(logits: torch.Tensor, top: int):
 
 
 @_timed
+def expert_order(ids: torch.Tensor, n_experts: int):
+    """``(order int64 [n * top], where int64 [n * top], offsets int32 [n_experts + 1])`` for ``ids`` int32 ``[n, top]`` in ``0 ..
+    n_experts - 1``: the pairs in stable expert order, the inverse, and where each expert's rows start.  Nothing travels to the host."""
+    _need_cuda(ids)
+    if ids.dtype != torch.int32 or not ids.is_contiguous():
+        raise TypeError("expert ids are contiguous int32")
+    n, lib = ids.numel(), _lib_()
+    if not lib.b200_expert_order_supported(n, int(n_experts)):     # more pairs or experts than the one-CTA sort holds
+        flat = ids.reshape(-1)
+        sorted_ids, order = torch.sort(flat.to(torch.int16) if n_experts < 1 << 15 else flat, stable=True)
+        where = torch.empty_like(order)
+        where[order] = torch.arange(n, device=ids.device)
+        bounds = torch.arange(n_experts + 1, device=ids.device).to(sorted_ids.dtype)
+        return order, where, torch.searchsorted(sorted_ids, bounds).to(torch.int32)
+    order = torch.empty((n,), dtype=torch.int64, device=ids.device)
+    where = torch.empty_like(order)
+    offsets = torch.empty((n_experts + 1,), dtype=torch.int32, device=ids.device)
+    rc = lib.b200_expert_order(order.data_ptr(), where.data_ptr(), offsets.data_ptr(), ids.data_ptr(), n, int(n_experts), _stream())
+    _lib.check_mixers(rc, "b200_expert_order")
+    return order, where, offsets
+
+
+@_timed
 def scaled_gather(h: torch.Tensor, weights: torch.Tensor, src: torch.Tensor, top: int) -> torch.Tensor:
     _need_cuda(h, weights, src)
     if not h.is_contiguous() or src.dtype != torch.int64 or weights.dtype != torch.float32:
@@ -530,9 +553,9 @@ def mixed_prompt_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Ten
     _lib.check_mixers(rc, "b200_mixed_prompt_attn")
 
 
-def tile_tokens(H: int, G: int, dk: int) -> int:
-    """Tokens of one sequence a CTA of ``tile_attention`` serves: 256 rows over the heads of a kv group, 128 for the widest heads."""
-    return max(1, int(_lib_().b200_tile_attn_rows(int(dk))) // (H // G))
+def tile_rows(H: int, G: int, dk: int, n_tokens: int) -> int:
+    """Query rows (tokens x heads of a kv group) of a ``tile_attention`` tile for portions of ``n_tokens`` tokens in all."""
+    return int(_lib_().b200_tile_attn_rows(H // G, int(G), int(dk), int(n_tokens)))
 
 
 def tile_attention_supported(H: int, G: int, dk: int, dv: int, same_pool: bool, bias: bool, dtype: torch.dtype) -> bool:
@@ -554,9 +577,9 @@ def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_p
                    tiles: torch.Tensor, tok_pos: torch.Tensor, scale: float, sink: Optional[torch.Tensor] = None, window: int = 0,
                    keep_first: int = 0, gate: Optional[torch.Tensor] = None, max_context: int = 0, softcap: float = 0.0, chunk: int = 0,
                    value_width: Optional[int] = None, value_div: int = 1, bias_lut: Optional[torch.Tensor] = None,
-                   temp_coef: float = 0.0, temp_every: int = 1) -> None:
+                   temp_coef: float = 0.0, temp_every: int = 1, rows: int = 128) -> None:
     """``mixed_prompt_attention`` (or, with ``bias_lut``, ``biased_prompt_attention``) for prompt portions in tiles of up to
-    128 or 256 rows: ``tiles`` int32 ``[n_tiles, 3]`` with up to ``tile_tokens(H, G, dk)`` consecutive tokens of one sequence each.
+    ``rows`` rows (see ``tile_rows``): ``tiles`` int32 ``[n_tiles, 3]`` with up to ``rows // (H // G)`` consecutive tokens of one sequence each.
     Only the tiles' rows of ``out`` are written, so the other portions of a step may go through another kernel."""
     _need_cuda(out, q, k_pool, v_pool, block_tables, tiles, tok_pos)
     nb, G, bs, dk = k_pool.shape
@@ -579,11 +602,11 @@ def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_p
     seen = min(max_context, window + keep_first + 128) if window > 0 else max_context
     if chunk > 0:
         seen = min(seen, chunk + 128)
-    splits = lib.b200_tile_attn_splits(tiles.shape[0], (seen + 63) // 64, G, dk) if max_context > 0 else 1
+    splits = lib.b200_tile_attn_splits(tiles.shape[0], (seen + 63) // 64, G, dk, int(rows)) if max_context > 0 else 1
     ws = torch.empty((splits, n, H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
     rc = lib.b200_tile_attn(out.data_ptr(), out.stride(0), out.stride(1), q.data_ptr(), q.stride(0), q.stride(1), _ptr(gate),
                             _rows2(gate) if gate is not None else 0, per_channel, k_pool.data_ptr(), v_pool.data_ptr(),
-                            block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), tiles.shape[0], tok_pos.data_ptr(), n,
+                            block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), tiles.shape[0], int(rows), tok_pos.data_ptr(), n,
                             _ptr(sink), _ptr(bias_lut), bias_lut.shape[1] if bias_lut is not None else 0, float(scale), float(softcap),
                             float(temp_coef), int(temp_every), int(window), int(keep_first), int(chunk), H, G, dk, dv, v_row,
                             int(value_div), int(out.dtype == torch.float32), bs, int(splits), _ptr(ws), DTYPE_ID[q.dtype], _stream())

@@ -228,14 +228,17 @@ class RaggedBatchState:
         return self._plan(("prompt", cap, at_least, below), cap, lambda count: count >= at_least and (below <= 0 or count < below))
 
     def attention_tiles(self, H: int, G: int, dk: int, cap: int, whole: bool):
-        """How an attention layer of H heads over G kv heads of key size ``dk`` serves the step: ``(tiles, rest)``.  ``tiles``: the long portions for
-        ``mixer_ops.tile_attention`` (None: none, or not ``whole``: the layer's sizes are not served there); ``rest``:
-        ``prompt_tiles`` of up to ``cap`` tokens over the others (None: none)."""
+        """How an attention layer of H heads over G kv heads of key size ``dk`` serves the step: ``(tiles, rest)``.  ``tiles``: the
+        long portions for ``mixer_ops.tile_attention``, ``(tile list, rows per tile)`` (None: none, or not ``whole``: the layer's
+        sizes are not served there); ``rest``: ``prompt_tiles`` of up to ``cap`` tokens over the others (None: none)."""
         from . import mixer_ops
 
         cut = mixer_ops.tile_attention_from(H, G) if whole else 1 << 30
         counts = [count for _first, count, _row, _past in self.spans]
-        tiles = self.prompt_tiles(cut, mixer_ops.tile_tokens(H, G, dk))[0] if max(counts) >= cut else None
+        tiles, most = None, max(counts)
+        if most >= cut:
+            rows = mixer_ops.tile_rows(H, G, dk, sum(c for c in counts if c >= cut))
+            tiles = self.prompt_tiles(cut, max(1, rows // (H // G)))[0], rows
         return tiles, self.prompt_tiles(1, cap, cut) if min(counts) < cut else None
 
     def scan_plan(self, ctas_per_seq: int = 0, segment: int = 0, at_least: int = 512):

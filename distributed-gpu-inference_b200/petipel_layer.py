@@ -171,7 +171,7 @@ class BiasedPagedAttention(nn.Module):
             tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.prompt_tile_tokens(H, G), self.in_tiles)
             if tiles is not None:
                 mixer_ops.tile_attention(attn.view(-1, H, dv), q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
-                                         tiles, st.tok_pos, self.scale, gate=gate, max_context=st.max_context(),
+                                         tiles[0], st.tok_pos, self.scale, gate=gate, rows=tiles[1], max_context=st.max_context(),
                                          bias_lut=self.bias_lut, temp_coef=self.temp_coef, temp_every=self.temp_every)
             if rest is not None:
                 mixer_ops.biased_prompt_attention(attn, q, gate, cache.k_pool, cache.v_pool, st.block_tables, rest[0], st.tok_pos,
@@ -219,7 +219,7 @@ class PolyNormMLP(nn.Module):
 
 
 class SigmoidTopKMoE(nn.Module):
-    """Router in fp32; tokens are sorted by expert, scaled by their score on the way in, pushed through the experts'
+    """Router in fp32 (sums in an order fixed by the width); tokens are sorted by expert, scaled by their score on the way in, pushed through the experts'
     clamped GLUs and summed per token in fp32.  ``GLU_ALPHA`` is fixed by the design."""
 
     GLU_ALPHA = 1.702
@@ -238,35 +238,29 @@ class SigmoidTopKMoE(nn.Module):
 
     def forward(self, h: torch.Tensor) -> torch.Tensor:
         n, top = h.shape[0], self.top
-        ids, w = mixer_ops.sigmoid_topk(F.linear(h.to(torch.float32), self.w_router), top)
-        flat = ids.reshape(-1).to(torch.int64)
-        order = torch.argsort(flat, stable=True)
-        counts = torch.bincount(flat, minlength=self.E)
+        ids, w = mixer_ops.sigmoid_topk(mixer_ops.router_logits(h, self.w_router), top)
+        order, where, offsets = mixer_ops.expert_order(ids, self.E)
         xs = mixer_ops.scaled_gather(h, w.reshape(-1), order, top)
         if self.grouped and n * top <= self.GROUPED_MAX_ROWS:
-            # all experts in one launch each way, offsets stay on the device: no host copy, no per-expert calls
-            offsets = torch.zeros(self.E + 1, dtype=torch.int32, device=h.device)
-            offsets[1:] = torch.cumsum(counts, 0)
+            # all experts in one launch each way
             y = mixer_ops.clamped_glu(mixer_ops.grouped_linear(xs, self.w_gu, offsets), self.limit, self.GLU_ALPHA)
             ys = mixer_ops.grouped_linear(y, self.w_down, offsets)
+        elif self.grouped and h.dtype == torch.bfloat16 and hasattr(torch, "_grouped_mm"):
+            # long prompt steps: the vendor's grouped GEMM, which also reads the offsets on the device
+            y = mixer_ops.clamped_glu(torch._grouped_mm(xs, self.w_gu.transpose(1, 2), offs=offsets[1:]), self.limit, self.GLU_ALPHA)
+            ys = torch._grouped_mm(y, self.w_down.transpose(1, 2), offs=offsets[1:])
         else:
-            # long prompt steps (and fp32): one vendor GEMM per expert each way; the counts come to the host once
-            counts = counts.tolist()
+            # other dtypes, or sizes off the 16-byte grid: one vendor GEMM per expert each way; the counts come to the host once
+            bounds = offsets.tolist()
             gu = torch.empty((n * top, self.w_gu.shape[1]), dtype=h.dtype, device=h.device)
-            lo = 0
-            for e, c in enumerate(counts):
-                if c:
-                    torch.mm(xs[lo:lo + c], self.w_gu[e].t(), out=gu[lo:lo + c])
-                    lo += c
+            for e, (lo, hi) in enumerate(zip(bounds[:-1], bounds[1:])):
+                if hi > lo:
+                    torch.mm(xs[lo:hi], self.w_gu[e].t(), out=gu[lo:hi])
             y = mixer_ops.clamped_glu(gu, self.limit, self.GLU_ALPHA)
             ys = torch.empty((n * top, h.shape[1]), dtype=h.dtype, device=h.device)
-            lo = 0
-            for e, c in enumerate(counts):
-                if c:
-                    torch.mm(y[lo:lo + c], self.w_down[e].t(), out=ys[lo:lo + c])
-                    lo += c
-        where = torch.empty_like(order)
-        where[order] = torch.arange(n * top, device=h.device)
+            for e, (lo, hi) in enumerate(zip(bounds[:-1], bounds[1:])):
+                if hi > lo:
+                    torch.mm(y[lo:hi], self.w_down[e].t(), out=ys[lo:hi])
         return mixer_ops.expert_combine(ys, where, n, top)
 
 

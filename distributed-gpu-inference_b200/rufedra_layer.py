@@ -207,7 +207,7 @@ class KeyValueSelectiveMixer(nn.Module):
             args = (attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables)
             kw = dict(window=self.window, gate=gate, max_context=st.max_context())
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
             if rest is not None:
                 mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale,
                                                  heads_as_rows=self.rows and st.max_count() == 1, **kw)

@@ -218,7 +218,7 @@ class LatentAttention(nn.Module):
             args = (o_lat.transpose(0, 1), q_lat.transpose(0, 1), cache.k_pool, cache.k_pool, st.block_tables)
             kw = dict(gate=proj[:, c[2]:c[2] + H], max_context=st.max_context())
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
             if rest is not None:
                 mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
         else:

@@ -176,7 +176,7 @@ class LatentRotaryAttention(nn.Module):
             args = (o_lat.transpose(0, 1), q_lat, cache.k_pool, cache.k_pool, st.block_tables)
             kw = dict(sink=self.sink, window=self.window, max_context=st.max_context(), value_width=r)
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
             if rest is not None:    # single tokens: all heads read the same rows, so 16 heads share a tensor-core tile
                 mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale,
                                                  heads_as_rows=H >= self.HEADS_AS_ROWS_FROM and st.max_count() == 1, **kw)
@@ -241,7 +241,7 @@ class DifferentialAttention(nn.Module):
             args = (maps, q.unflatten(1, (2 * H, dk)), k_pool, cache.v_pool, st.block_tables)
             kw = dict(chunk=self.chunk, max_context=st.max_context(), value_div=2)
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles, st.tok_pos, self.scale, **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
             if rest is not None:
                 mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
         else:
@@ -270,7 +270,6 @@ class SquaredReluMoE(GroupedSoftmaxMoE):
         self.w_down = _param(torch.stack([t[f"e{e}.down"] for e in range(self.E)]), device, dtype)    # [E, W, ff]
         self.grouped = (mixer_ops.grouped_linear_supported(self.w_gu.shape[2], self.w_gu.dtype)
                         and mixer_ops.grouped_linear_supported(self.w_down.shape[2], self.w_down.dtype))
-        self._ar = None
         self.ws_gu = self.ws_down = None
 
     def _route(self, x: torch.Tensor):

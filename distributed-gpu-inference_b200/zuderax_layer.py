@@ -271,7 +271,6 @@ class SigmoidGroupMoE(GroupedSoftmaxMoE):
         self.w_down = _param(torch.stack([t[f"e{e}.down"] for e in range(self.E)]), device, dtype)  # [E, W, ff]
         self.grouped = (mixer_ops.grouped_linear_supported(self.w_gu.shape[2], self.w_gu.dtype)
                         and mixer_ops.grouped_linear_supported(self.w_down.shape[2], self.w_down.dtype))
-        self._ar = None
 
     def _activate(self, z: torch.Tensor) -> torch.Tensor:
         return mixer_ops.silu_glu(z)

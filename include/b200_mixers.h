@@ -101,6 +101,11 @@ int b200_polynorm(void* out, const void* z, int64_t z_stride, const void* coef, 
 /* The `top` largest of E fp32 logits per token (ties: lowest index); weights = sigmoid(logit). */
 int b200_sigmoid_topk(int32_t* ids, float* weights, const float* logits, int n_tok, int E, int top, void* stream);
 
+/* Stable order of (token, choice) pairs by expert: order int64 [n_pairs] (pair of every sorted row), where int64 [n_pairs] (its inverse),
+ * offsets int32 [n_experts + 1] (first sorted row of every expert).  ids int32 [n_pairs] in 0 .. n_experts - 1. */
+int b200_expert_order_supported(int64_t n_pairs, int n_experts);
+int b200_expert_order(int64_t* order, int64_t* where, int32_t* offsets, const int32_t* ids, int64_t n_pairs, int n_experts, void* stream);
+
 /* xs[r] = T(weights[src[r]] * h[src[r] / top]): the expert-sorted, input-scaled rows. */
 int b200_scaled_gather(void* xs, const void* h, const float* weights, const int64_t* src, int64_t n_rows, int top,
                        int width, int dtype, void* stream);
@@ -472,16 +477,16 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
                                 float* workspace, int dtype, void* stream);
 
 /* b200_mixed_prompt_attn_ext2 and b200_biased_prompt_attn for prompt portions on the fifth-generation tensor cores: tiles of up to
- * b200_tile_attn_rows(dk) / (H / G) tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
+ * tile_rows / (H / G) tokens, tile_rows 128 or (dk <= 128) 256, as b200_tile_attn_rows picks for n_tokens tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
  * touched.  bias_lut fp32 [H][lut_len] with temp_coef / temp_every as in b200_biased_prompt_attn, or NULL.  The values are v_pool's
  * rows, or the first dv columns of the key rows when v_pool == k_pool.  n_splits > 1 divides the keys over as many CTAs and needs a
  * workspace fp32 [n_splits][n_tok][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte aligned query rows. */
 int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bias, int dtype);
-int b200_tile_attn_rows(int dk);
-int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk);
+int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens);
+int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows);
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,
-                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, const int32_t* tok_pos, int n_tok,
+                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, int tile_rows, const int32_t* tok_pos, int n_tok,
                    const float* sink, const float* bias_lut, int lut_len, float scale, float softcap, float temp_coef, int temp_every,
                    int window, int keep_first, int chunk, int H, int G, int dk, int dv, int v_row, int v_div, int out_f32, int block_size,
                    int n_splits, float* workspace, int dtype, void* stream);

@@ -1,0 +1,90 @@
+"""Row kernels at the edges of their register tiles (a piece of eight per lane, one, four or eight warps per row) and off the 16-byte
+grid, and the one-CTA expert order around its chunk sizes."""
+import pytest
+import torch
+
+from dgi_b200 import mixer_ops
+
+pytestmark = pytest.mark.gpu
+
+F64 = torch.float64
+EPS = 1e-5
+WIDTHS = [8, 64, 504, 512, 520, 1024, 1032, 2048, 4088, 4104, 8192, 8200, 16384, 16392, 1, 30, 1001]
+TOL = {torch.float32: 2e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10}     # one rounding of the result; fp32: its own sums
+
+
+def _unit(x):
+    return x / torch.sqrt((x * x).mean(-1, keepdim=True) + EPS)
+
+
+def _close(got, want, dtype):
+    return ((got.to(F64) - want).abs() <= TOL[dtype] * (want.abs() + want.square().mean().sqrt())).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("width", WIDTHS)
+def test_norms_and_polynorm(width, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(width)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    rows = 5
+    x, w, w2 = rnd(rows, width) * 3, (rnd(width) * 0.2).to(dtype), (rnd(width) * 0.2).to(dtype)
+    assert _close(mixer_ops.offset_rmsnorm(x, w, EPS), _unit(x.to(F64)) * (1 + w.to(F64)), dtype)
+    y = rnd(rows, width + 8).to(dtype)[:, :width]                       # rows of a wider projection
+    new = x.to(F64) + 0.7 * _unit(y.to(F64)) * (1 + w.to(F64))
+    out = mixer_ops.postnorm_residual(x, y, w, 0.7, EPS, w_next=w2)
+    assert _close(x, new, torch.float32)
+    assert _close(out, _unit(new) * (1 + w2.to(F64)), dtype)
+    coef = torch.tensor([0.6, 0.3, -0.2, 0.05], device="cuda").to(dtype)
+    z, c = y.to(F64), coef.to(F64)
+    assert _close(mixer_ops.polynorm(y, coef, EPS), c[0] * _unit(z) + c[1] * _unit(z * z) + c[2] * _unit(z ** 3) + c[3], dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("G,dk,dv,odd", [(4, 128, 128, 0), (1, 16, 260, 0), (3, 30, 7, 0), (2, 64, 64, 1), (5, 132, 4, 0)])
+def test_value_prep(G, dk, dv, odd, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(G * dk)
+    n, bs = 9, 4
+    wide = torch.randn(n, G * (dk + dv) + 8 + odd, generator=gen, device="cuda").to(dtype)
+    k, v = wide[:, odd:odd + G * dk], wide[:, odd + G * dk:odd + G * (dk + dv)]
+    kp, vp = torch.zeros(4, G, bs, dk, device="cuda", dtype=dtype), torch.zeros(4, G, bs, dv, device="cuda", dtype=dtype)
+    slots = torch.tensor([15, 0, -1, 7, 3, 16, 9, 10, 2], device="cuda")     # one unused, one beyond the pool
+    prev, keep = torch.randn(n, G * dv, generator=gen, device="cuda").to(dtype), torch.empty(n, G * dv, device="cuda", dtype=dtype)
+    mixer_ops.value_prep_append(k, v, kp, vp, slots, EPS, v_prev=prev, lam=0.3, v_keep=keep)
+    want = 0.7 * _unit(v.to(F64).reshape(n, G, dv)) + 0.3 * prev.to(F64).view(n, G, dv)
+    assert _close(keep.view(n, G, dv), want, dtype)
+    for i, s in enumerate(slots.tolist()):
+        if 0 <= s < 16:
+            assert torch.equal(kp[s // bs, :, s % bs], k[i].view(G, dk)) and torch.equal(vp[s // bs, :, s % bs], keep[i].view(G, dv))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("dv", [128, 4, 512, 132, 516, 33])
+def test_head_norm(dv, dtype):
+    x = torch.randn(11, 3, dv, device="cuda")
+    w = (1 + 0.1 * torch.randn(dv, device="cuda")).to(dtype)
+    assert _close(mixer_ops.head_rmsnorm(x, w, EPS), _unit(x.to(F64)) * w.to(F64), dtype)
+
+
+@pytest.mark.parametrize("n,top,E", [(1, 1, 1), (5, 3, 7), (512, 2, 8), (513, 2, 8), (4099, 2, 48), (1000, 4, 49), (70000, 2, 3)])
+def test_expert_order(n, top, E):
+    ids = torch.randint(0, E, (n, top), dtype=torch.int32, device="cuda")
+    if E > 2:
+        ids[ids == 1] = 0                                             # an expert without rows
+    order, where, offsets = mixer_ops.expert_order(ids, E)
+    want = torch.argsort(ids.reshape(-1), stable=True)
+    assert torch.equal(order, want) and torch.equal(where[order], torch.arange(n * top, device="cuda"))
+    assert offsets.tolist() == [0] + torch.bincount(ids.reshape(-1), minlength=E).cumsum(0).tolist()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("width", [8, 1024, 1032, 100])
+def test_expert_rows(width, dtype):
+    n, top, E = 37, 2, 5
+    h, wts = torch.randn(n, width, device="cuda").to(dtype), torch.rand(n, top, device="cuda")
+    order, where, _ = mixer_ops.expert_order(torch.randint(0, E, (n, top), dtype=torch.int32, device="cuda"), E)
+    xs = mixer_ops.scaled_gather(h, wts.reshape(-1), order, top)
+    assert _close(xs, wts.reshape(-1)[order].to(F64)[:, None] * h.to(F64)[order // top], dtype)
+    g, u = (xs.to(F64)[:, i * (width // 2):(i + 1) * (width // 2)] for i in range(2))
+    g, u = g.clamp(max=0.8), u.clamp(-0.8, 0.8)
+    assert _close(mixer_ops.clamped_glu(xs, 0.8, 1.7), g * torch.sigmoid(1.7 * g) * (u + 1), dtype)
+    assert _close(mixer_ops.expert_combine(xs, where, n, top), xs.to(F64)[where].view(n, top, width).sum(1), torch.float32)

@@ -88,10 +88,13 @@ OPTIONS = {
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("portions,page", [(EDGES, 16), (EDGES, 7), ([(40, 900)], 16), ([(300, 0), (17, 300)], 32)], ids=["edges", "page7", "split", "long"])
+@pytest.mark.parametrize("rows", [128, 256])
 @pytest.mark.parametrize("name", OPTIONS)
-def test_tile_attention(name, portions, page, dtype):
+def test_tile_attention(name, rows, portions, page, dtype):
     layout, opt = OPTIONS[name]
     H, G, dk, dv, div = layout
+    if rows > 128 and dk > 128:
+        pytest.skip("wide heads have tiles of 128 rows")
     opt = dict(opt)
     q, k_pool, v_pool, st, rnd = _case(layout, portions, page, dtype)
     n, D, scale = q.shape[0], dv or 256, dk ** -0.5
@@ -103,9 +106,9 @@ def test_tile_attention(name, portions, page, dtype):
     bias = rnd(H, opt["bias"]) if "bias" in opt else None
     extra = dict(bias_lut=bias, temp_coef=opt["temp"][0], temp_every=opt["temp"][1]) if "temp" in opt else dict(bias_lut=bias)
     out = torch.full((n, H, D), 7.0, dtype=torch.float32 if opt.get("fp32") else dtype, device="cuda")
-    tiles = st.prompt_tiles(2, mixer_ops.tile_tokens(H, G, dk))[0]
+    tiles = st.prompt_tiles(2, rows // (H // G))[0]
     mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, scale, max_context=st.max_context(),
-                             value_width=D, value_div=div, **kw, **extra)
+                             value_width=D, value_div=div, rows=rows, **kw, **extra)
     want = _reference(q, k_pool, v_pool, st, D, div, scale, bias=bias, temp=opt.get("temp"), **kw)
     ours = torch.cat([torch.arange(f, f + c) for f, c, _b, _p in st.spans if c > 1]).cuda()
     # weights rounded to 8 (bf16) or 11 bits, summed with random signs: one rounding of the result and a share of one per weight
@@ -123,8 +126,8 @@ def test_steep_scores_and_rescaling():
     st.block_tables[0, :36] = torch.arange(36, dtype=torch.int32, device="cuda")
     k_pool[:36] *= torch.linspace(0.01, 12, 36, device="cuda").to(k_pool.dtype)[:, None, None, None]
     out = torch.empty(64, 8, 128, dtype=torch.bfloat16, device="cuda")
-    tiles = st.prompt_tiles(2, mixer_ops.tile_tokens(8, 2, 128))[0]
-    for window in (0, 60):
-        mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, 0.5, window=window)
+    for window, rows in ((0, 128), (60, 128), (0, 256), (60, 256)):
+        tiles = st.prompt_tiles(2, rows // 4)[0]
+        mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, 0.5, window=window, rows=rows)
         want = _reference(q, k_pool, v_pool, st, 128, 1, 0.5, window=window)
         assert (out.to(F64) - want).norm() / want.norm() <= 1.5 * 2.0 ** -8
