@@ -430,6 +430,11 @@ int b200_argmax_keys_decode(int64_t* out, const int64_t* keys, int64_t rows, voi
   return argmax_keys_decode(out, keys, rows, static_cast<cudaStream_t>(stream));
 }
 
+int b200_rope_tables(void* cos_out, void* sin_out, const int64_t* pos, const float* inv_freq, int64_t n, int D, float scaling, int dtype,
+                     void* stream) {
+  return rope_tables(cos_out, sin_out, pos, inv_freq, n, D, scaling, dtype, static_cast<cudaStream_t>(stream));
+}
+
 int b200_silu_mul(void* out, const void* gate, const void* up, int64_t rows, int cols, int64_t gate_row_stride,
                   int64_t up_row_stride, int dtype, void* stream) {
   return silu_mul(out, gate, up, rows, cols, gate_row_stride, up_row_stride, dtype, static_cast<cudaStream_t>(stream));

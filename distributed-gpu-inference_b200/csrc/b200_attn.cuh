@@ -87,6 +87,8 @@ int argmax_rows(int64_t* out, const void* x, int64_t rows, int64_t cols, int64_t
 int argmax_rows_keys(int64_t* keys, const void* x, int64_t rows, int64_t cols, int64_t row_stride, int64_t col_offset,
                      int dtype, cudaStream_t s);
 int argmax_keys_decode(int64_t* out, const int64_t* keys, int64_t rows, cudaStream_t s);
+int rope_tables(void* cos_out, void* sin_out, const int64_t* pos, const float* inv_freq, int64_t n, int D, float scaling, int dtype,
+                cudaStream_t s);
 int silu_mul(void* out, const void* gate, const void* up, int64_t rows, int cols, int64_t g_stride, int64_t u_stride,
              int dtype, cudaStream_t s);
 

@@ -323,6 +323,22 @@ argmax_rows_kernel(int64_t* __restrict__ out, const T* __restrict__ x, int cols,
   }
 }
 
+// ---- RoPE tables of a call's positions: launch-bound (seven launches of the torch recipe, once per layer where the caller has no
+// tables; 4 layers of a small model's decode step: 28 of its 75 launches), so one thread per (position, frequency) writes all four entries
+template <typename T>
+__global__ void __launch_bounds__(128)
+rope_tables_kernel(T* __restrict__ cos_out, T* __restrict__ sin_out, const int64_t* __restrict__ pos, const float* __restrict__ inv_freq,
+                   int64_t total, int half, float scaling) {
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * 128 + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * 128) {
+    const int64_t n = i / half;
+    const int j = static_cast<int>(i - n * half);
+    const float angle = __fmul_rn(static_cast<float>(pos[n]), inv_freq[j]);
+    const T c = Cvt<T>::from_f32(__fmul_rn(cosf(angle), scaling)), s = Cvt<T>::from_f32(__fmul_rn(sinf(angle), scaling));
+    cos_out[n * 2 * half + j] = cos_out[n * 2 * half + half + j] = c;
+    sin_out[n * 2 * half + j] = sin_out[n * 2 * half + half + j] = s;
+  }
+}
+
 template <typename F>
 int by_dtype(int dtype, const char* name, F&& f) {
   switch (dtype) {
@@ -392,6 +408,20 @@ int rope_kv_append(void* q, int64_t q_stride, const void* k, int64_t k_stride, v
                                                 static_cast<T*>(v_pool), slot_mapping, n_tok, Hq, Hkv, D, block_size,
                                                 max_blocks);
     return check_launch("b200_rope_kv_append");
+  });
+}
+
+int rope_tables(void* cos_out, void* sin_out, const int64_t* pos, const float* inv_freq, int64_t n, int D, float scaling, int dtype,
+                cudaStream_t s) {
+  if (n < 0 || D <= 0 || D % 2) return fail(B200_EINVAL, "b200_rope_tables: bad sizes");
+  if (n == 0) return 0;
+  if (!cos_out || !sin_out || !pos || !inv_freq) return fail(B200_EINVAL, "b200_rope_tables: null pointer");
+  const int64_t total = n * (D / 2);
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((total + 127) / 128, kNumSMs * 32));
+  return by_dtype(dtype, "b200_rope_tables", [&](auto* tag) {
+    using T = std::remove_pointer_t<decltype(tag)>;
+    rope_tables_kernel<T><<<grid, 128, 0, s>>>(static_cast<T*>(cos_out), static_cast<T*>(sin_out), pos, inv_freq, total, D / 2, scaling);
+    return check_launch("b200_rope_tables");
   });
 }
 

@@ -433,6 +433,20 @@ polynorm_kernel(T* __restrict__ out, const T* __restrict__ z, int64_t z_stride, 
   }
 }
 
+// ---- blocks of several pools set to zero (the pages of a finished request, all layers in one launch) -------------------
+// The slots travel as a kernel argument: no copy to the device and nothing to keep until it has run.
+constexpr int kZeroPools = 32, kZeroSlots = 640;
+struct ZeroBlocks {
+  char* pool[kZeroPools];
+  int64_t bytes[kZeroPools];     // of a block, a multiple of 16
+  int32_t slot[kZeroSlots];
+};
+__global__ void __launch_bounds__(256) zero_blocks_kernel(const __grid_constant__ ZeroBlocks A) {
+  const int64_t n = A.bytes[blockIdx.y];
+  uint4* dst = reinterpret_cast<uint4*>(A.pool[blockIdx.y] + A.slot[blockIdx.x] * n);
+  for (int64_t i = threadIdx.x; i < n / 16; i += blockDim.x) dst[i] = make_uint4(0, 0, 0, 0);
+}
+
 // ---- expert order -------------------------------------------------------------------------------------------------
 // One CTA of 1024 threads; thread t owns the pairs of a contiguous chunk.  count[e][t] pairs of expert e in chunk t -> their running
 // sums over the chunks (a warp per expert) -> where every chunk's pairs of every expert start: a stable counting sort.  The ids are
@@ -678,6 +692,28 @@ int b200_polynorm(void* out, const void* z, int64_t z_stride, const void* coef, 
       polynorm_kernel<T><<<rows, 256, 0, s>>>(static_cast<T*>(out), static_cast<const T*>(z), z_stride, static_cast<const T*>(coef), eps, ff);
     return check_launch("b200_polynorm");
   });
+}
+
+int b200_zero_blocks(void* const* pools, const int64_t* block_bytes, int n_pools, const int32_t* slots, int n_slots, void* stream) {
+  if (n_pools < 0 || n_slots < 0) return fail(B200_EINVAL, "b200_zero_blocks: bad sizes");
+  if (n_pools == 0 || n_slots == 0) return 0;
+  if (!pools || !block_bytes || !slots) return fail(B200_EINVAL, "b200_zero_blocks: null pointer");
+  for (int p0 = 0; p0 < n_pools; p0 += kZeroPools) {
+    ZeroBlocks A{};
+    const int np = std::min(kZeroPools, n_pools - p0);
+    for (int i = 0; i < np; ++i) {
+      A.pool[i] = static_cast<char*>(pools[p0 + i]);
+      A.bytes[i] = block_bytes[p0 + i];
+      if (!A.pool[i] || !aligned16(A.pool[i]) || A.bytes[i] < 0 || A.bytes[i] % 16)
+        return fail(B200_ESHAPE, "b200_zero_blocks: blocks are whole 16-byte words");
+    }
+    for (int s0 = 0; s0 < n_slots; s0 += kZeroSlots) {
+      const int ns = std::min(kZeroSlots, n_slots - s0);
+      for (int i = 0; i < ns; ++i) A.slot[i] = slots[s0 + i];
+      zero_blocks_kernel<<<dim3(ns, np), 256, 0, static_cast<cudaStream_t>(stream)>>>(A);
+    }
+  }
+  return check_launch("b200_zero_blocks");
 }
 
 int b200_expert_order_supported(int64_t n_pairs, int n_experts) {

@@ -248,6 +248,17 @@ def sigmoid_topk(logits: torch.Tensor, top: int):
     return ids, w
 
 
+def zero_blocks(pools, slots) -> None:
+    """Blocks ``slots`` (a host list) of every tensor of ``pools`` (contiguous ``[blocks, ...]``) set to zero in one launch."""
+    import ctypes
+
+    n, m = len(pools), len(slots)
+    rc = _lib_().b200_zero_blocks((ctypes.c_void_p * n)(*[p.data_ptr() for p in pools]),
+                                  (ctypes.c_int64 * n)(*[p.stride(0) * p.element_size() for p in pools]), n,
+                                  (ctypes.c_int32 * m)(*slots), m, _stream())
+    _lib.check_mixers(rc, "b200_zero_blocks")
+
+
 @_timed
 def expert_order(ids: torch.Tensor, n_experts: int):
     """``(order int64 [n * top], where int64 [n * top], offsets int32 [n_experts + 1])`` for ``ids`` int32 ``[n, top]`` in ``0 ..

@@ -39,7 +39,7 @@ def _need_cuda(*tensors: torch.Tensor) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())    # current_stream() builds an object per call
 
 
 def _pool_dims(pool: torch.Tensor):
@@ -136,6 +136,20 @@ def rope_kv_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch
         cos.data_ptr(), sin.data_ptr(), k_pool.data_ptr(), v_pool.data_ptr(), slot_mapping.data_ptr(), n, Hq, Hkv, D, bs,
         max_blocks, _dtype_id(k_pool), _stream())
     _lib.check(rc, "b200_rope_kv_append")
+
+
+def rope_tables(pos: torch.Tensor, inv_freq: torch.Tensor, dtype: torch.dtype, scaling: float):
+    """``cos, sin [*pos.shape, 2 * len(inv_freq)]`` for int64 positions and fp32 frequencies (``cos(float(pos) * f) * scaling``)."""
+    _need_cuda(pos, inv_freq)
+    if pos.dtype != torch.int64 or inv_freq.dtype != torch.float32 or not pos.is_contiguous() or not inv_freq.is_contiguous():
+        raise ValueError("positions are contiguous int64, frequencies contiguous fp32")
+    D = 2 * inv_freq.numel()
+    cos = torch.empty((*pos.shape, D), dtype=dtype, device=pos.device)
+    sin = torch.empty_like(cos)
+    rc = _lib.load().b200_rope_tables(cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), inv_freq.data_ptr(), pos.numel(), D, float(scaling),
+                                      DTYPE_ID[dtype], _stream())
+    _lib.check(rc, "b200_rope_tables")
+    return cos, sin
 
 
 def silu_mul(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:

@@ -64,6 +64,9 @@ class RMSNorm(nn.Module):
 def rope_tables(position_ids: torch.Tensor, inv_freq: torch.Tensor, dtype: torch.dtype, scaling: float = 1.0):
     """``position_ids [B, T]`` → ``cos, sin [B, T, D]`` (fp32 math, times the RoPE variant's attention factor, cast to
     ``dtype`` — transformers' ``LlamaRotaryEmbedding.forward``)."""
+    if (position_ids.is_cuda and inv_freq.is_cuda and position_ids.dtype == torch.int64 and inv_freq.dtype == torch.float32
+            and position_ids.is_contiguous() and inv_freq.is_contiguous() and dtype in ops.DTYPE_ID):
+        return ops.rope_tables(position_ids, inv_freq, dtype, scaling)
     freqs = position_ids.to(torch.float32)[:, :, None] * inv_freq[None, None, :]
     emb = torch.cat((freqs, freqs), dim=-1)
     if scaling != 1.0:
@@ -233,13 +236,18 @@ class RaggedBatchState:
         sizes are not served there); ``rest``: ``prompt_tiles`` of up to ``cap`` tokens over the others (None: none)."""
         from . import mixer_ops
 
-        cut = mixer_ops.tile_attention_from(H, G) if whole else 1 << 30
-        counts = [count for _first, count, _row, _past in self.spans]
-        tiles, most = None, max(counts)
-        if most >= cut:
-            rows = mixer_ops.tile_rows(H, G, dk, sum(c for c in counts if c >= cut))
-            tiles = self.prompt_tiles(cut, max(1, rows // (H // G)))[0], rows
-        return tiles, self.prompt_tiles(1, cap, cut) if min(counts) < cut else None
+        if self._tiles is None:
+            self._tiles = {}
+        key = ("attention", H, G, dk, cap, whole)
+        if key not in self._tiles:      # the step's layers of one layout share it
+            cut = mixer_ops.tile_attention_from(H, G) if whole else 1 << 30
+            counts = [count for _first, count, _row, _past in self.spans]
+            tiles = None
+            if max(counts) >= cut:
+                rows = mixer_ops.tile_rows(H, G, dk, sum(c for c in counts if c >= cut))
+                tiles = self.prompt_tiles(cut, max(1, rows // (H // G)))[0], rows
+            self._tiles[key] = tiles, self.prompt_tiles(1, cap, cut) if min(counts) < cut else None
+        return self._tiles[key]
 
     def scan_plan(self, ctas_per_seq: int = 0, segment: int = 0, at_least: int = 512):
         """For recurrences whose carry can be added afterwards (a fixed decay): the step's portions of ``at_least`` tokens

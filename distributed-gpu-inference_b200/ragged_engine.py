@@ -23,6 +23,7 @@ import numpy as np
 import torch
 import torch.nn.functional as F
 
+from . import mixer_ops
 from .paged_layer import RaggedBatchState, RaggedLayerCache
 from .worker.distributed.kv_cache import CacheBlock, KVCachePool, RecurrentStatePool
 from .worker.distributed.model_shard import ModelShard
@@ -35,6 +36,27 @@ class _Request:
     blocks: List[Optional[List[List[CacheBlock]]]]     # per shard: per attention layer, its blocks (None: no pool)
     length: int = 0                                    # tokens already in cache / state
     table: List[int] = field(default_factory=list)     # pool slots of its blocks
+
+
+def _token_ids(toks: Sequence[int]) -> np.ndarray:
+    if isinstance(toks, list) and type(toks[0]) is int:
+        return np.array(toks, dtype=np.int64)
+    return np.fromiter((int(t) for t in toks), dtype=np.int64, count=len(toks))
+
+
+def _upload(device: torch.device, arrays: Sequence[np.ndarray]) -> List[torch.Tensor]:
+    """The arrays (8-byte elements before 4-byte ones) on the device, as views of one buffer filled by one copy."""
+    at, total = [], 0
+    for a in arrays:
+        at.append(total)
+        total += a.nbytes + (-a.nbytes % 16)
+    host = torch.empty(total, dtype=torch.uint8, pin_memory=True)
+    raw = host.numpy()
+    for o, a in zip(at, arrays):
+        raw[o:o + a.nbytes] = np.ascontiguousarray(a).reshape(-1).view(np.uint8)
+    buf = host.to(device, non_blocking=True)
+    kinds = {np.dtype(np.int64): torch.int64, np.dtype(np.int32): torch.int32}
+    return [buf[o:o + a.nbytes].view(kinds[a.dtype]).view(a.shape) for o, a in zip(at, arrays)]
 
 
 class RaggedStepEngine:
@@ -113,7 +135,7 @@ class RaggedStepEngine:
             if pool is not None:
                 for li, layer_blocks in enumerate(blocks):
                     pool.layer(li).unpin(b.block_id for b in layer_blocks)
-                pool.free_sequence(blocks)
+                pool.free_sequence(blocks, mixer_ops.zero_blocks)
         for sp in self.state_pools:
             if sp is not None:
                 sp.free(req.slot)
@@ -153,7 +175,8 @@ class RaggedStepEngine:
         wanted)``; unknown ids are admitted.  Returns fp32 logits ``[wanted, vocab]`` on the device in the order of
         the entries and their indices, or None when nothing was wanted."""
         bs = self.block_size
-        ids: List[int] = []
+        n_tok = 0
+        ids: List[np.ndarray] = []
         pos_l: List[np.ndarray] = []
         slot_l: List[np.ndarray] = []
         spans, scans, wanted, rows = [], [], [], []
@@ -183,14 +206,15 @@ class RaggedStepEngine:
             table = np.asarray(req.table, dtype=np.int64)
             pos_l.append(p)
             slot_l.append(table[p // bs] * bs + p % bs)
-            first = len(ids)
+            first = n_tok
             spans.append((first, n, len(rows), req.length))
             scans.append((first, n, req.slot, 1 if req.length == 0 else 0))
             wanted.extend(first + int(w) for w in want)
             rows.append(req.table)
-            ids.extend(int(t) for t in toks)
+            ids.append(_token_ids(toks))
+            n_tok += n
             req.length += n
-        if not ids:
+        if n_tok == 0:
             return None
         dev = self.device
         width = max(len(r) for r in rows)
@@ -198,19 +222,14 @@ class RaggedStepEngine:
         for b, r in enumerate(rows):
             tables[b, :len(r)] = r
 
-        def up(a):
-            return torch.from_numpy(np.ascontiguousarray(a)).to(dev, non_blocking=True)
-
-        st = RaggedBatchState(
-            tok_pos=up(np.concatenate(pos_l).astype(np.int32)),
-            slot_mapping=up(np.concatenate(slot_l)),
-            block_tables=up(tables),
-            scan_seqs=up(np.asarray(scans, dtype=np.int32)),
-            spans=spans,
-            tok_row=up(np.repeat(np.arange(len(spans), dtype=np.int32), [sp[1] for sp in spans])),
-            scan_host=scans,
-        )
-        h = up(np.asarray(ids, dtype=np.int64))
+        # everything the step's layers read travels in one copy from pinned memory: a copy per table from pageable memory cost
+        # as much host time as the tables themselves
+        slot_mapping, h, picked, tok_pos, scan_seqs, tok_row, block_tables = _upload(dev, (
+            np.concatenate(slot_l), np.concatenate(ids), np.asarray(wanted, dtype=np.int64),
+            np.concatenate(pos_l).astype(np.int32), np.asarray(scans, dtype=np.int32),
+            np.repeat(np.arange(len(spans), dtype=np.int32), [sp[1] for sp in spans]), tables))
+        st = RaggedBatchState(tok_pos=tok_pos, slot_mapping=slot_mapping, block_tables=block_tables, scan_seqs=scan_seqs, spans=spans,
+                              tok_row=tok_row, scan_host=scans)
         st.token_ids = h
         for si, shard in enumerate(self.shards):
             handles = []
@@ -225,8 +244,7 @@ class RaggedStepEngine:
                 h, _ = shard.forward(h, past_key_values=handles, use_cache=True)
         if not wanted:
             return None
-        sel = h.index_select(0, torch.tensor(wanted, dtype=torch.int64, device=dev))
-        return self._logits(sel)
+        return self._logits(h.index_select(0, picked))
 
     def _forward_traced(self, shard: ModelShard, h: torch.Tensor, handles) -> torch.Tensor:
         """``shard.forward`` unrolled so that the residual stream after every layer can be recorded."""

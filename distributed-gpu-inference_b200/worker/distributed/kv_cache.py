@@ -33,7 +33,7 @@ import time
 from collections import OrderedDict
 from dataclasses import dataclass, field  # noqa: F401
 from enum import Enum
-from typing import Any, Dict, Iterable, List, Optional, Sequence, Tuple
+from typing import Callable, Any, Dict, Iterable, List, Optional, Sequence, Tuple
 
 import torch
 
@@ -254,10 +254,13 @@ class PagedKVCache:
         if self._on_free is not None:
             self._on_free(block_id)
 
-    def free_blocks(self, block_ids: Iterable[str]) -> None:
+    def free_blocks(self, block_ids: Iterable[str], dead: Optional[List[int]] = None) -> None:
         """``free_block`` for many ids with the same observable result, but the pool rows that reach ref-count 0
-        are zeroed with one ``index_fill_`` per pool instead of two launches per block (SURVEY.md §9 #10)."""
-        dead: List[int] = []
+        are zeroed with one ``index_fill_`` per pool instead of two launches per block.  With ``dead``
+        those rows are appended to it instead and the caller zeroes them."""
+        owed = dead is not None
+        if dead is None:
+            dead = []
         blocks, slots, lru, pinned, free = self._blocks, self._block_to_slot, self._lru_queue, self._pinned, self._free_blocks
         on_free = self._on_free
         for block_id in block_ids:
@@ -277,7 +280,7 @@ class PagedKVCache:
             free.append(block_id)
             if on_free is not None:
                 on_free(block_id)
-        if dead:
+        if dead and not owed:
             idx = torch.tensor(dead, dtype=torch.int64, device=self._key_pool.device)
             self._key_pool.index_fill_(0, idx, 0)
             self._value_pool.index_fill_(0, idx, 0)
@@ -465,9 +468,27 @@ class KVCachePool:
             # this call releases for good loses its pin entry together with everything else (free_blocks)
             cache.free_blocks([blk.block_id for blk in layer_blocks])
 
-    def free_sequence(self, blocks: List[List[CacheBlock]]) -> None:
-        """Public spelling of the reference's private ``_free_sequence_blocks``."""
-        self._free_sequence_blocks(blocks)
+    def free_sequence(self, blocks: List[List[CacheBlock]], zero: Optional[Callable] = None) -> None:
+        """Public spelling of the reference's private ``_free_sequence_blocks``.  ``zero(pools, slots)`` (CUDA engines) sets the
+        rows that reach ref-count 0 to zero for all layers at once, where the layers' rows agree."""
+        if zero is None:
+            self._free_sequence_blocks(blocks)
+            return
+        dead: List[List[int]] = []
+        for cache, layer_blocks in zip(self._layer_caches, blocks):
+            dead.append([])
+            cache.free_blocks([blk.block_id for blk in layer_blocks], dead[-1])
+        groups: Dict[Tuple[int, ...], List[torch.Tensor]] = {}
+        for cache, slots in zip(self._layer_caches, dead):
+            if slots:
+                groups.setdefault(tuple(slots), []).extend(p for p in (cache.key_pool, cache.value_pool) if p.numel())
+        for slots, pools in groups.items():
+            whole = [p for p in pools if p.stride(0) * p.element_size() % 16 == 0 and p.data_ptr() % 16 == 0]
+            if whole:
+                zero(whole, slots)
+            for p in pools:
+                if not any(p is w for w in whole):
+                    p.index_fill_(0, torch.tensor(slots, dtype=torch.int64, device=p.device), 0)
 
     def get_total_memory_gb(self) -> float:
         return sum(c._get_pool_memory_gb() for c in self._layer_caches)

@@ -235,6 +235,10 @@ int b200_rope_kv_append_prompt(void* q, int64_t q_row_stride, void* k, int64_t k
                                const void* v, int64_t v_row_stride, const void* cos_table, const void* sin_table,
                                void* k_pool, void* v_pool, const int64_t* slot_mapping, int n_tok,
                                int Hq, int Hkv, int D, int block_size, int64_t max_blocks, int dtype, void* stream);
+/* RoPE tables: cos_out / sin_out [n, D] (storage dtype) = T(cos(float(pos[i]) * inv_freq[j]) * scaling), columns j and j + D/2 alike;
+ * inv_freq fp32 [D/2], pos int64 [n].  Replaces the seven launches of the torch recipe. */
+int b200_rope_tables(void* cos_out, void* sin_out, const int64_t* pos, const float* inv_freq, int64_t n, int D, float scaling, int dtype,
+                     void* stream);
 int b200_silu_mul(void* out, const void* gate, const void* up, int64_t rows, int cols,
                   int64_t gate_row_stride, int64_t up_row_stride, int dtype, void* stream);
 /* Greedy token: out[r] = argmax over x[r, 0..cols) — largest value, smallest index among equals, NaN largest, i.e.

@@ -88,3 +88,25 @@ def test_expert_rows(width, dtype):
     g, u = g.clamp(max=0.8), u.clamp(-0.8, 0.8)
     assert _close(mixer_ops.clamped_glu(xs, 0.8, 1.7), g * torch.sigmoid(1.7 * g) * (u + 1), dtype)
     assert _close(mixer_ops.expert_combine(xs, where, n, top), xs.to(F64)[where].view(n, top, width).sum(1), torch.float32)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("B,T,D,scaling", [(1, 1, 2, 1.0), (4, 1, 64, 1.0), (3, 7, 128, 1.2), (1, 300, 96, 1.0)])
+def test_rope_tables(B, T, D, scaling, dtype):
+    from dgi_b200 import paged_layer
+
+    pos = torch.randint(0, 100000, (B, T), device="cuda")
+    inv = 10000.0 ** (-torch.arange(0, D, 2, device="cuda", dtype=torch.float32) / D)
+    ang = pos.to(torch.float32)[:, :, None] * inv
+    ang = torch.cat((ang, ang), dim=-1)
+    cos, sin = paged_layer.rope_tables(pos, inv, dtype, scaling)
+    want = [(f * scaling).to(dtype) if scaling != 1.0 else f.to(dtype) for f in (ang.cos(), ang.sin())]
+    assert torch.equal(cos, want[0]) and torch.equal(sin, want[1])     # the same fp32 operations, rounded once
+
+
+@pytest.mark.parametrize("layers,blocks,slots", [(1, 3, [1]), (33, 700, list(range(0, 700, 1))), (2, 50, [49, 0, 7])])
+def test_zero_blocks(layers, blocks, slots):
+    pools = [torch.ones(blocks, 2, 4, 8 * (1 + i % 3), device="cuda", dtype=torch.bfloat16) for i in range(layers)]
+    mixer_ops.zero_blocks(pools, slots)
+    for p in pools:
+        assert (p[slots] == 0).all() and p.float().sum() == (blocks - len(slots)) * p[0].numel()
