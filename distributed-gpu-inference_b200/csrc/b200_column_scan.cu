@@ -15,9 +15,9 @@
 // column) pairs at once: seven shuffles instead of three per pair.
 //
 // Measured on B200, bf16, 64 x 128 states, against four lanes per column that prepare their own inputs: delta, 8 x 2048 tokens of 8
-// heads 2302 -> 540 us; gated, 6 portions of up to 1900 tokens of 16 heads 1228 -> 430 us; retention, 5 portions of up to 1024 tokens
-// of 16 heads 474 -> 190 us.  With one warp per scheduler a token is a chain of about 290 clocks (shared-memory reads, the packed
-// multiply-adds at two clocks each, the shuffles of the delta rule); larger steps overlap the chains of several CTAs.
+// heads 2302 -> 469 us; gated, 6 portions of up to 1900 tokens of 16 heads 1228 -> 396 us; retention, 5 portions of up to 1024 tokens
+// of 16 heads 474 -> 157 us.  A token of one warp per scheduler takes 250 - 470 clocks, of which the packed multiply-adds are 130 - 190:
+// what is left is the latency of a token's dependent steps, and larger steps overlap the chains of several CTAs.
 #include <type_traits>
 
 #include "b200_column_scan.cuh"
@@ -323,13 +323,10 @@ column_scan_kernel(const ColArgs A) {
       for (int c = 0; c < C; ++c) x[i][c] = 0.f;
       if (!sq.fresh && row < dk) {
         const float* src = sp + static_cast<int64_t>(row) * dv + col;
-        if (C == 4 && A.vec_s && col < dv) {
-          const float4 f = *reinterpret_cast<const float4*>(src);
-          x[i][0] = f.x;
-          if constexpr (C == 4) {
-            x[i][1] = f.y;
-            x[i][2] = f.z;
-            x[i][3] = f.w;
+        if (C == 4 && A.vec_s) {
+          if (col < dv) {
+            const float4 f = *reinterpret_cast<const float4*>(src);
+            x[i][0] = f.x, x[i][1 % C] = f.y, x[i][2 % C] = f.z, x[i][3 % C] = f.w;
           }
         } else {
 #pragma unroll
@@ -352,18 +349,36 @@ column_scan_kernel(const ColArgs A) {
   float* op = A.o + (static_cast<int64_t>(sq.tok0) * H + h) * dv + col + my_c;
   const int64_t o_tok = static_cast<int64_t>(H) * dv;
 
-  auto token = [&](const S_t& st, int tt, float (&out)[C]) {
+  // a token's rows as this lane needs them: read while the token before is computed
+  constexpr int kSections = S_t::kSections;
+  struct Rows {
+    f32x2 x[kSections][2 * NJ];      // q | f or k | 1 - f or g - 1
+    float v[C], beta;
+  };
+  auto read = [&](Rows& r4, const S_t& st, int tt) {
     const float* row = st.rows[tt] + 4 * r;
-    float v[C];
+#pragma unroll
+    for (int n = 0; n < kSections; ++n) {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(row + n * DK + 32 * j);
+        r4.x[n][2 * j] = w.x, r4.x[n][2 * j + 1] = w.y;
+      }
+    }
     if constexpr (C == 4) {
       const float4 f = *reinterpret_cast<const float4*>(&st.v[tt][cw]);
-      v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+      r4.v[0] = f.x, r4.v[1] = f.y, r4.v[2] = f.z, r4.v[3] = f.w;
     } else if constexpr (C == 2) {
       const float2 f = *reinterpret_cast<const float2*>(&st.v[tt][cw]);
-      v[0] = f.x, v[1] = f.y;
+      r4.v[0] = f.x, r4.v[1] = f.y;
     } else {
-      v[0] = st.v[tt][cw];
+      r4.v[0] = st.v[tt][cw];
     }
+    if constexpr (RULE == kDelta) r4.beta = st.beta[tt];
+  };
+  // The passes over the tile are written one after the other, every step of a pass on another pair: what a warp alone on its scheduler
+  // waits for is the latency of dependent multiply-adds.
+  auto token = [&](const Rows& in, float (&out)[C]) {
     f32x2 o2[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) o2[c] = 0ull;
@@ -372,16 +387,14 @@ column_scan_kernel(const ColArgs A) {
 #pragma unroll
       for (int c = 0; c < C; ++c) d2[c] = 0ull;
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(row + DK + 32 * j);
-        const ulonglong2 g4 = *reinterpret_cast<const ulonglong2*>(row + 2 * DK + 32 * j);
+      for (int i = 0; i < 2 * NJ; ++i) {
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-          S[c][2 * j] = fma2(g4.x, S[c][2 * j], S[c][2 * j]);
-          d2[c] = fma2(S[c][2 * j], k4.x, d2[c]);
-          S[c][2 * j + 1] = fma2(g4.y, S[c][2 * j + 1], S[c][2 * j + 1]);
-          d2[c] = fma2(S[c][2 * j + 1], k4.y, d2[c]);
-        }
+        for (int c = 0; c < C; ++c) S[c][i] = fma2(in.x[2][i], S[c][i], S[c][i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 2 * NJ; ++i) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) d2[c] = fma2(S[c][i], in.x[1][i], d2[c]);
       }
       float u[C];
 #pragma unroll
@@ -394,44 +407,34 @@ column_scan_kernel(const ColArgs A) {
 #pragma unroll
         for (int c = 0; c < C; ++c) u[c] += __shfl_xor_sync(0xffffffffu, u[c], x);
       }
-      const float beta = st.beta[tt];
       f32x2 uu[C];
 #pragma unroll
       for (int c = 0; c < C; ++c) {
-        u[c] = beta * (v[c] - u[c]);
+        u[c] = in.beta * (in.v[c] - u[c]);
         uu[c] = pair(u[c], u[c]);
       }
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(row + DK + 32 * j);
-        const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(row + 32 * j);
+      for (int i = 0; i < 2 * NJ; ++i) {
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-          S[c][2 * j] = fma2(k4.x, uu[c], S[c][2 * j]);
-          o2[c] = fma2(S[c][2 * j], q4.x, o2[c]);
-          S[c][2 * j + 1] = fma2(k4.y, uu[c], S[c][2 * j + 1]);
-          o2[c] = fma2(S[c][2 * j + 1], q4.y, o2[c]);
-        }
+        for (int c = 0; c < C; ++c) S[c][i] = fma2(in.x[1][i], uu[c], S[c][i]);
       }
     } else {
       f32x2 vv[C];
 #pragma unroll
-      for (int c = 0; c < C; ++c) vv[c] = pair(v[c], v[c]);
+      for (int c = 0; c < C; ++c) vv[c] = pair(in.v[c], in.v[c]);
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(row + 32 * j);
-        const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(row + DK + 32 * j);   // f, or the scaled k
-        ulonglong2 w4 = m4;
-        if constexpr (RULE == kGated) w4 = *reinterpret_cast<const ulonglong2*>(row + 2 * DK + 32 * j);
-        const f32x2 fx = RULE == kGated ? m4.x : dd, fy = RULE == kGated ? m4.y : dd;
+      for (int i = 0; i < 2 * NJ; ++i) {
+        f32x2 w[C];
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-          S[c][2 * j] = fma2(fx, S[c][2 * j], mul2(w4.x, vv[c]));
-          o2[c] = fma2(S[c][2 * j], q4.x, o2[c]);
-          S[c][2 * j + 1] = fma2(fy, S[c][2 * j + 1], mul2(w4.y, vv[c]));
-          o2[c] = fma2(S[c][2 * j + 1], q4.y, o2[c]);
-        }
+        for (int c = 0; c < C; ++c) w[c] = mul2(in.x[RULE == kGated ? 2 : 1][i], vv[c]);
+#pragma unroll
+        for (int c = 0; c < C; ++c) S[c][i] = fma2(RULE == kGated ? in.x[1][i] : dd, S[c][i], w[c]);
       }
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * NJ; ++i) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) o2[c] = fma2(S[c][i], in.x[0][i], o2[c]);
     }
 #pragma unroll
     for (int c = 0; c < C; ++c) {
@@ -462,13 +465,16 @@ column_scan_kernel(const ColArgs A) {
     const S_t& st = stage[s & 1];
     const int n = min(kStage, sq.count - s * kStage);
     if (n == kStage) {
+      Rows rows[2];
+      read(rows[0], st, 0);
 #pragma unroll
       for (int t0 = 0; t0 < kStage; t0 += kTok) {
         float part[8];
 #pragma unroll
         for (int t = 0; t < kTok; ++t) {
           float o[C];
-          token(st, t0 + t, o);
+          if (t0 + t + 1 < kStage) read(rows[(t0 + t + 1) & 1], st, t0 + t + 1);
+          token(rows[(t0 + t) & 1], o);
 #pragma unroll
           for (int c = 0; c < C; ++c) part[t * C + c] = o[c];
         }
@@ -479,7 +485,9 @@ column_scan_kernel(const ColArgs A) {
 #pragma unroll 1
       for (int t = 0; t < n; ++t) {
         float o[C], part[8];
-        token(st, t, o);
+        Rows one;
+        read(one, st, t);
+        token(one, o);
 #pragma unroll
         for (int i = 0; i < 8; ++i) part[i] = i < C ? o[i < C ? i : 0] : 0.f;
         const float sum = read_outs(part);
@@ -501,8 +509,8 @@ column_scan_kernel(const ColArgs A) {
       const int row = 32 * j + 4 * r + i;
       if (row >= dk) continue;
       float* dst = sp + static_cast<int64_t>(row) * dv + col;
-      if (C == 4 && A.vec_s && col < dv) {
-        *reinterpret_cast<float4*>(dst) = make_float4(x[i][0], x[i][C > 1 ? 1 : 0], x[i][C > 2 ? 2 : 0], x[i][C > 3 ? 3 : 0]);
+      if (C == 4 && A.vec_s) {
+        if (col < dv) *reinterpret_cast<float4*>(dst) = make_float4(x[i][0], x[i][1 % C], x[i][2 % C], x[i][3 % C]);
       } else {
 #pragma unroll
         for (int c = 0; c < C; ++c) {
@@ -513,8 +521,11 @@ column_scan_kernel(const ColArgs A) {
   }
 }
 
-// Columns per lane: four where the step's columns then still give half the schedulers of the chip a warp, fewer for small steps (a
-// shorter token per warp) and for key sizes whose tile would not fit the registers.
+// Columns per lane: two give a lone warp per scheduler a shorter token, four read shared memory half as often; which is ahead changes
+// with how many CTAs of two an SM gets (B200, 64 x 128 states, ns per token, gated / delta / retention; two against four columns): one
+// 134 / 193 / 102 against 157 / 245 / 137, two 175 / 257 / 141 against 158 / 245 / 136, three 241 / 366 / 190 against 246 / 374 / 213, four
+// 349 / 490 / 270 against 246 / 374 / 213, seven 555 / 805 / 434 against 469 / 721 / 405 (eight columns: 439 / 770 / 399, and 273 / 425 / 257
+// from the first CTA on).  Key sizes whose tile would not fit the registers take fewer.
 template <int RULE, typename T, int DK>
 int launch_columns(ColArgs& A, int n_seqs, cudaStream_t stream, const char* name) {
   auto go = [&](auto cols) {
@@ -527,8 +538,11 @@ int launch_columns(ColArgs& A, int n_seqs, cudaStream_t stream, const char* name
     return check_launch(name);
   };
   const int64_t columns = static_cast<int64_t>(n_seqs) * A.H * A.dv;
-  if constexpr (DK <= 128) {
-    if (columns >= 16 * 4 * kNumSMs / 2) return go(std::integral_constant<int, 4>{});
+  const int64_t per_sm = (columns + 32 * kNumSMs - 1) / (32 * kNumSMs);
+  if constexpr (DK <= 64) {
+    if (per_sm != 1 && per_sm != 3) return go(std::integral_constant<int, 4>{});
+  } else if constexpr (DK <= 128) {
+    if (per_sm > 1) return go(std::integral_constant<int, 4>{});
   }
   if constexpr (DK <= 256) {
     return go(std::integral_constant<int, 2>{});
