@@ -17,7 +17,6 @@
 //                               live sequence are carried in a slot pool
 //   gated delta rule            S <- diag(g) S;  u = beta (v - S^T k);  S <- S + k u^T;  o = S^T q  with a decay per
 //                               key channel, the fp32 state carried per sequence in a slot pool
-//   gated head norm             o * rsqrt(mean(o^2) + eps) * w * sigmoid(gate)
 //
 // Every size and constant of a design is a parameter.  Scores, softmax, norms, decays, the state and the residual
 // are fp32 whatever the storage dtype T is.  The order in which a position's sums are formed depends only on that
@@ -58,7 +57,6 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   return warp_sum(t);
 }
 
-__device__ __forceinline__ float sigmoid_(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float softplus_(float z) { return z > 20.0f ? z : log1pf(expf(z)); }
 
 // ---- RMS norm ----------------------------------------------------------------------------------------------------
@@ -273,7 +271,7 @@ struct AttnArgs {
 
 template <typename T>
 __device__ __forceinline__ float gate_at(const AttnArgs& A, const T* gate, int64_t n, int h, int c) {
-  return sigmoid_(Cvt<T>::to_f32(gate[n * A.gate_stride + (A.gate_dim ? h * A.gate_dim + c : h)]));
+  return logistic(Cvt<T>::to_f32(gate[n * A.gate_stride + (A.gate_dim ? h * A.gate_dim + c : h)]));
 }
 
 // first key a position sees (the kept first tokens of a window aside)
@@ -456,7 +454,7 @@ mixed_paged_attn_kernel(const AttnArgs A) {
       const float u = res[hl * dv + a], w = res[hl * dv + b];
       float ya = u * cf + w * sf, yb = w * cf - u * sf;        // the rotation by -p
       if (gate) {
-        const float gt = sigmoid_(Cvt<T>::to_f32(gate[static_cast<int64_t>(n) * A.gate_stride + h0 + hl]));
+        const float gt = logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(n) * A.gate_stride + h0 + hl]));
         ya *= gt; yb *= gt;
       }
       T* orow = out + (h0 + hl) * A.out_head_stride;
@@ -833,7 +831,7 @@ mixed_prompt_attn_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, co
           f = 1.0f / l;
         }
         if (gate && !A.unrotate && !(GATED && A.gate_dim))
-          f *= sigmoid_(Cvt<T>::to_f32(gate[static_cast<int64_t>(RH ? row0 : row0 + row) * A.gate_stride + (RH ? head0(h) + row : h)]));
+          f *= logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(RH ? row0 : row0 + row) * A.gate_stride + (RH ? head0(h) + row : h)]));
       }
 #pragma unroll
       for (int nt = 0; nt < DV8; ++nt) {
@@ -882,7 +880,7 @@ mixed_prompt_attn_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, co
         const float u = slab[row * DVP + a], w = slab[row * DVP + b];
         float ya = u * cf + w * sf, yb = w * cf - u * sf;       // the rotation by minus the position
         if (gate) {
-          const float gt = sigmoid_(Cvt<T>::to_f32(gate[static_cast<int64_t>(row0 + row) * A.gate_stride + h]));
+          const float gt = logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(row0 + row) * A.gate_stride + h]));
           ya *= gt;
           yb *= gt;
         }
@@ -932,7 +930,7 @@ attn_split_combine_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, c
       const float u = res[h * dv + a], w = res[h * dv + b];
       float ya = u * cf + w * sf, yb = w * cf - u * sf;
       if (gate) {
-        const float gt = sigmoid_(Cvt<T>::to_f32(gate[static_cast<int64_t>(n) * A.gate_stride + h]));
+        const float gt = logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(n) * A.gate_stride + h]));
         ya *= gt;
         yb *= gt;
       }
@@ -993,16 +991,25 @@ struct SeqSpan {
 
 constexpr int kConvTokens = 64;   // tokens per CTA; at least taps - 1, so only a sequence's first CTA reads the carried inputs
 
+// A thread's inputs are read kConvAhead tokens before they are used: what bounds the kernel is bytes in flight.  B200, 8 x 2048 tokens of
+// 2048 channels, bf16, four taps: 67 -> 47 us (the bytes alone: 20; with a check of the end at every token 104).
+constexpr int kConvAhead = 8;
+
+template <typename T, int V>
+using ConvRaw = std::conditional_t<V == 4, uint2, T>;
+template <typename T, int V>
+__device__ __forceinline__ ConvRaw<T, V> conv_raw(const T* p) {
+  return *reinterpret_cast<const ConvRaw<T, V>*>(p);
+}
+template <typename T, int V>
+__device__ __forceinline__ void conv_widen(float (&dst)[V], const ConvRaw<T, V>& raw) {
+  const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+  for (int u = 0; u < V; ++u) dst[u] = Cvt<T>::to_f32(e[u]);
+}
 template <typename T, int V>
 __device__ __forceinline__ void conv_load(float (&dst)[V], const T* p) {
-  if constexpr (V == 4) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p);
-    const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) dst[u] = Cvt<T>::to_f32(e[u]);
-  } else {
-    dst[0] = Cvt<T>::to_f32(p[0]);
-  }
+  conv_widen<T, V>(dst, conv_raw<T, V>(p));
 }
 
 template <typename T, int TAPS, int V>
@@ -1040,15 +1047,9 @@ causal_conv_silu_kernel(T* __restrict__ out, int64_t out_stride, const T* __rest
 #pragma unroll
       for (int u = 0; u < V; ++u) win[i][u] = tl[static_cast<int64_t>(i - pad) * C + u];
   }
-  float first[TAPS][V];                       // the carry itself, for the update below
-#pragma unroll
-  for (int i = 0; i < TAPS; ++i)
-#pragma unroll
-    for (int u = 0; u < V; ++u) first[i][u] = win[i][u];
   const int t1 = min(sq.count, t0 + kConvTokens);
-#pragma unroll 4
-  for (int t = t0; t < t1; ++t) {
-    conv_load<T, V>(win[TAPS - 1], xc + static_cast<int64_t>(t) * x_stride);
+  auto step = [&](int t, const ConvRaw<T, V>& raw) {
+    conv_widen<T, V>(win[TAPS - 1], raw);
     float y[V];
 #pragma unroll
     for (int u = 0; u < V; ++u) {
@@ -1056,7 +1057,7 @@ causal_conv_silu_kernel(T* __restrict__ out, int64_t out_stride, const T* __rest
 #pragma unroll
       for (int i = 0; i < TAPS; ++i) y[u] = fmaf(wr[i][u], win[i][u], y[u]);
       y[u] += b[u];
-      y[u] *= sigmoid_(y[u]);
+      y[u] *= logistic(y[u]);
 #pragma unroll
       for (int i = 0; i < TAPS - 1; ++i) win[i][u] = win[i + 1][u];
     }
@@ -1070,9 +1071,27 @@ causal_conv_silu_kernel(T* __restrict__ out, int64_t out_stride, const T* __rest
     } else {
       dst[0] = Cvt<T>::from_f32(y[0]);
     }
-  }
+  };
+  ConvRaw<T, V> ahead[kConvAhead];
+#pragma unroll
+  for (int j = 0; j < kConvAhead; ++j)
+    if (t0 + j < t1) ahead[j] = conv_raw<T, V>(xc + static_cast<int64_t>(t0 + j) * x_stride);
+  auto group = [&](int t, auto whole) {         // whole: neither this group nor the next is cut short
+    constexpr bool kWhole = decltype(whole)::value;
+#pragma unroll
+    for (int j = 0; j < kConvAhead; ++j) {
+      if (!kWhole && t + j >= t1) break;
+      const ConvRaw<T, V> raw = ahead[j];
+      if (kWhole || t + j + kConvAhead < t1) ahead[j] = conv_raw<T, V>(xc + static_cast<int64_t>(t + j + kConvAhead) * x_stride);
+      step(t + j, raw);
+    }
+  };
+  int t = t0;
+  for (; t + 2 * kConvAhead <= t1; t += kConvAhead) group(t, std::true_type{});
+  for (; t < t1; t += kConvAhead) group(t, std::false_type{});
   if (t0 == 0) {
-    // the new carry: the portion's last taps - 1 inputs (older ones come from the old carry when the portion is short)
+    // the new carry: the portion's last taps - 1 inputs; a short portion moves older ones down, each from a later place to an earlier
+    // one, so that none is overwritten before it is read
 #pragma unroll
     for (int i = 0; i < TAPS - 1; ++i) {
       if (i < pad) continue;
@@ -1080,40 +1099,13 @@ causal_conv_silu_kernel(T* __restrict__ out, int64_t out_stride, const T* __rest
       float nw[V];
       if (t >= 0) {
         conv_load<T, V>(nw, xc + static_cast<int64_t>(t) * x_stride);
-      } else {                                // slot TAPS - 1 + t of the window before token 0
+      } else {
 #pragma unroll
-        for (int u = 0; u < V; ++u) {
-          nw[u] = 0.f;
-#pragma unroll
-          for (int j = 0; j < TAPS - 1; ++j)
-            if (j == TAPS - 1 + t) nw[u] = first[j][u];
-        }
+        for (int u = 0; u < V; ++u) nw[u] = sq.fresh ? 0.f : tl[static_cast<int64_t>(TAPS - 1 + t - pad) * C + u];
       }
 #pragma unroll
       for (int u = 0; u < V; ++u) tl[static_cast<int64_t>(i - pad) * C + u] = nw[u];
     }
-  }
-}
-
-// ---- o * rsqrt(mean(o^2) + eps) * w * sigmoid(gate); one warp per (token, head) ------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256)
-head_rmsnorm_gated_kernel(T* __restrict__ out, const float* __restrict__ x, const T* __restrict__ w,
-                          const T* __restrict__ gate, int64_t gate_stride, float eps, int64_t rows, int H, int dv) {
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const float* xr = x + row * dv;
-  float ss = 0.f;
-  for (int i = lane; i < dv; i += 32) ss = fmaf(xr[i], xr[i], ss);
-  const float inv = rsqrtf(warp_sum(ss) / static_cast<float>(dv) + eps);
-  const int64_t n = row / H;
-  const int h = static_cast<int>(row - n * H);
-  const T* gr = gate ? gate + n * gate_stride + static_cast<int64_t>(h) * dv : nullptr;
-  for (int i = lane; i < dv; i += 32) {
-    float y = xr[i] * inv * Cvt<T>::to_f32(w[i]);
-    if (gr) y *= sigmoid_(Cvt<T>::to_f32(gr[i]));
-    out[row * dv + i] = Cvt<T>::from_f32(y);
   }
 }
 
@@ -1528,20 +1520,6 @@ int b200_delta_scan_ext(float* o_raw, const void* q, const void* k, const void* 
     return fail(B200_EINVAL, "b200_delta_scan: null pointer");
   return delta_column_scan(o_raw, ScanRows{q, k, v, in_stride}, beta_logit, beta_stride, a_logit, a_stride, dt_bias, a_log, per_channel != 0,
                            state, seqs, ScanShape{n_seqs, H, G, dk, dv}, unit_eps, q_scale, dtype, static_cast<cudaStream_t>(stream));
-}
-
-int b200_head_rmsnorm_gated(void* out, const float* x, const void* weight, const void* gate, int64_t gate_stride, float eps,
-                            int64_t n_tok, int H, int dv, int dtype, void* stream) {
-  if (n_tok < 0 || H <= 0 || dv <= 0) return fail(B200_EINVAL, "b200_head_rmsnorm_gated: bad sizes");
-  if (n_tok == 0) return 0;
-  if (!out || !x || !weight) return fail(B200_EINVAL, "b200_head_rmsnorm_gated: null pointer");
-  const int64_t rows = n_tok * H;
-  return hybrid_by_dtype(dtype, "b200_head_rmsnorm_gated", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    head_rmsnorm_gated_kernel<T><<<static_cast<unsigned>((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<T*>(out), x, static_cast<const T*>(weight), static_cast<const T*>(gate), gate_stride, eps, rows, H, dv);
-    return check_launch("b200_head_rmsnorm_gated");
-  });
 }
 
 }  // extern "C"

@@ -7,7 +7,6 @@
 //   retention scan              S_t = d_h S_(t-1) + (c k_t) v_t^T,  o_t = S_t^T q_t  with a fixed decay per head, the fp32
 //                               state carried per sequence in a slot pool; long portions run as parallel segments
 //                               whose missing carry is added afterwards
-//   head norm with a gate       o * rsqrt(mean(o^2) + eps) [* w] * act(gate) * out_scale, act = sigmoid or SiLU
 //   branch post-norm residual   y = sa a + sb b;  x += ls * w * y * rsqrt(mean(y^2) + eps);  optional copy of x in T
 //   grouped softmax routing     softmax scores, choice by score + bias inside the best expert groups, weights = chosen
 //                               scores over their sum
@@ -49,8 +48,6 @@ __device__ __forceinline__ float block_total(float v, float* red) {
   float t = (lane < nw) ? red[lane] : 0.f;
   return warp_sum(t);
 }
-
-__device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + expf(-z)); }
 
 // ---- q/k norm + rotary + append ------------------------------------------------------------------------------------
 // One CTA per token, one warp per head in turn (q heads, then k heads, then the value rows).  A head's row is read into
@@ -205,35 +202,6 @@ retention_apply_carry_kernel(float* __restrict__ o_raw, const T* __restrict__ q,
   }
 }
 
-// ---- head norm with a gate ------------------------------------------------------------------------------------------
-// one warp per (token, head) row of fp32 read-outs
-template <typename T>
-__global__ void __launch_bounds__(256)
-head_norm_act_gate_kernel(T* __restrict__ out, int64_t out_stride, const float* __restrict__ x, const T* __restrict__ w,
-                          const T* __restrict__ gate, int64_t gate_stride, int gate_act, float out_scale, float eps,
-                          int64_t rows, int H, int dv) {
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const float* xr = x + row * dv;
-  float ss = 0.f;
-  for (int i = lane; i < dv; i += 32) ss = fmaf(xr[i], xr[i], ss);
-  const float inv = rsqrtf(warp_sum(ss) / static_cast<float>(dv) + eps);
-  const int64_t n = row / H;
-  const int h = static_cast<int>(row - n * H);
-  const T* gr = gate ? gate + n * gate_stride + static_cast<int64_t>(h) * dv : nullptr;
-  T* orow = out + n * out_stride + static_cast<int64_t>(h) * dv;
-  for (int i = lane; i < dv; i += 32) {
-    float y = xr[i] * inv;
-    if (w) y *= Cvt<T>::to_f32(w[i]);
-    if (gr) {
-      const float g = Cvt<T>::to_f32(gr[i]);
-      y *= gate_act == 1 ? g * sigm(g) : sigm(g);
-    }
-    orow[i] = Cvt<T>::from_f32(y * out_scale);
-  }
-}
-
 // ---- branch post-norm residual --------------------------------------------------------------------------------------
 template <typename T, typename A>
 __global__ void __launch_bounds__(256)
@@ -301,7 +269,7 @@ group_topk_kernel(int32_t* __restrict__ ids, float* __restrict__ weights, const 
   const float* z = logits + static_cast<int64_t>(tok) * logit_stride;
   if (sigmoid_scores) {
     for (int e = lane; e < E; e += 32) {
-      const float s = sigm(z[e]);
+      const float s = logistic(z[e]);
       score[e] = s;
       choice[e] = s + (correction ? correction[e] : 0.f);
     }
@@ -511,23 +479,6 @@ int b200_retention_apply_carry(float* o_raw, const void* q, int64_t in_stride, c
     kern<<<grid, 128, smem, static_cast<cudaStream_t>(stream)>>>(o_raw, static_cast<const T*>(q), in_stride, seg_state,
                                                                  reinterpret_cast<const RetSeq*>(seg_spans), decay, H, dk, dv);
     return check_launch("b200_retention_apply_carry");
-  });
-}
-
-int b200_head_norm_act_gate(void* out, int64_t out_stride, const float* x, const void* weight, const void* gate,
-                            int64_t gate_stride, int gate_act, float out_scale, float eps, int64_t n_tok, int H, int dv,
-                            int dtype, void* stream) {
-  if (n_tok < 0 || H <= 0 || dv <= 0 || gate_act < 0 || gate_act > 1)
-    return fail(B200_EINVAL, "b200_head_norm_act_gate: bad sizes");
-  if (n_tok == 0) return 0;
-  if (!out || !x) return fail(B200_EINVAL, "b200_head_norm_act_gate: null pointer");
-  const int64_t rows = n_tok * H;
-  return parallel_by_dtype(dtype, "b200_head_norm_act_gate", [&](auto* tag) {
-    using T = std::remove_pointer_t<decltype(tag)>;
-    head_norm_act_gate_kernel<T><<<static_cast<unsigned>((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<T*>(out), out_stride, x, static_cast<const T*>(weight), static_cast<const T*>(gate), gate_stride,
-        gate_act, out_scale, eps, rows, H, dv);
-    return check_launch("b200_head_norm_act_gate");
   });
 }
 

@@ -110,3 +110,37 @@ def test_zero_blocks(layers, blocks, slots):
     mixer_ops.zero_blocks(pools, slots)
     for p in pools:
         assert (p[slots] == 0).all() and p.float().sum() == (blocks - len(slots)) * p[0].numel()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("dv,odd", [(128, 0), (8, 0), (72, 0), (256, 0), (264, 0), (512, 0), (516, 0), (33, 0), (128, 1)])
+@pytest.mark.parametrize("weight,gate,act", [(True, True, "sigmoid"), (False, True, "silu"), (False, False, "sigmoid")])
+def test_gated_head_norm(dv, odd, weight, gate, act, dtype):
+    n, H = 7, 5                                                        # 35 rows: the last warp's are cut short
+    x = torch.randn(n, H, dv, device="cuda")
+    w = (1 + 0.1 * torch.randn(dv, device="cuda")).to(dtype) if weight else None
+    g = torch.randn(n, H * dv + 8 + odd, device="cuda").to(dtype)[:, odd:odd + H * dv] if gate else None
+    g64 = g.to(F64).reshape(n, H, dv) if gate else None
+    want = _unit(x.to(F64)) * (w.to(F64) if weight else 1)
+    gated = want if not gate else want * torch.sigmoid(g64) * (g64 if act == "silu" else 1)
+    got = mixer_ops.head_norm_act_gate(x, w, g, EPS, dtype, gate_act=act, out_scale=-0.7)
+    assert _close(got.view(n, H, dv), -0.7 * gated, dtype)
+    if weight:
+        got = mixer_ops.head_rmsnorm_gated(x, w, g, EPS)
+        assert _close(got.view(n, H, dv), gated, dtype)
+
+
+@pytest.mark.parametrize("dtype,C", [(torch.bfloat16, 8), (torch.bfloat16, 7), (torch.float32, 6)])
+@pytest.mark.parametrize("taps", [1, 4, 6, 16])
+@pytest.mark.parametrize("cuts", [(1, 1, 2, 1, 9), (8, 7, 3), (64, 1, 65), (130,)])
+def test_causal_conv_portions(cuts, taps, dtype, C):
+    x, w = torch.randn(sum(cuts), C, device="cuda").to(dtype), torch.randn(C, taps, device="cuda").to(dtype)
+    tail, got, at = torch.full((2, taps - 1, C), 9.0, device="cuda"), [], 0
+    for cut in cuts:
+        seqs = torch.tensor([[0, cut, 1, int(at == 0)]], dtype=torch.int32, device="cuda")
+        got.append(mixer_ops.causal_conv_silu(x[at:at + cut], w, tail, seqs, cut))
+        at += cut
+    pad = torch.cat((torch.zeros(taps - 1, C, device="cuda", dtype=F64), x.to(F64)))
+    y = sum(pad[i:i + sum(cuts)] * w[:, i].to(F64) for i in range(taps))
+    tol = {torch.bfloat16: 2.0 ** -8, torch.float32: 4e-6}[dtype]       # taps products of up to ~ 10, then one rounding
+    assert ((torch.cat(got).to(F64) - y * torch.sigmoid(y)).abs() <= tol * (y.abs() + 1)).all()
