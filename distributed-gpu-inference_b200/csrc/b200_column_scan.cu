@@ -74,6 +74,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   return r;
 }
 
+__device__ __forceinline__ float logistic(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float soft_plus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
 // N consecutive elements of a row, `left` of which exist, into shared memory: without a register in between where the caller

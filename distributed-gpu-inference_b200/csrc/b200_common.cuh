@@ -91,15 +91,16 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // 1 / (1 + e^-z) as n / d with t = e^-|z|, d = 1 + t in [1, 2], n = 1 or t.  The quotient is an approximate reciprocal's, put right by one
-// Newton step on its remainder; d needs no care for overflow, so there is no branch between the elements of a row, whose chains then
-// overlap.  (A general division branches: row kernels with one sigmoid per element were bound by it, with the wider pieces 52 -> 34 us for 16384 x 8 gated rows of 128, bf16.)  Infinities give 0 and 1, NaN NaN.
-__device__ __forceinline__ float logistic(float z) {
+// Newton step on its remainder, which counts what d lost in its rounding (Dekker's sum); d needs no care for overflow, so there is no branch between the elements of a row, whose chains then
+// overlap.  (A general division branches: row kernels with one sigmoid per element were bound by it, with the wider pieces 52 -> 35 us for 16384 x 8 gated rows of 128, bf16.)  Infinities give 0 and 1, NaN NaN.
+// z times this over 2^20 points of -80 .. 80 against 64 bits: largest relative error 2.11e-7, mean 2.25e-8 (by division 2.25e-7, 2.56e-8).
+__device__ __forceinline__ float row_logistic(float z) {
   const float t = expf(-fabsf(z));
   const float d = 1.0f + t, n = z < 0.f ? t : 1.0f;
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float q = n * r;
-  return fmaf(fmaf(-q, d, n), r, q);
+  const float q = n * r, lost = t - (d - 1.0f);
+  return fmaf(fmaf(-q, lost, fmaf(-q, d, n)), r, q);
 }
 
 constexpr int kNumSMs = 148;  // B200

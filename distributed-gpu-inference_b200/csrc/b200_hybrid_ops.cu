@@ -271,7 +271,7 @@ struct AttnArgs {
 
 template <typename T>
 __device__ __forceinline__ float gate_at(const AttnArgs& A, const T* gate, int64_t n, int h, int c) {
-  return logistic(Cvt<T>::to_f32(gate[n * A.gate_stride + (A.gate_dim ? h * A.gate_dim + c : h)]));
+  return row_logistic(Cvt<T>::to_f32(gate[n * A.gate_stride + (A.gate_dim ? h * A.gate_dim + c : h)]));
 }
 
 // first key a position sees (the kept first tokens of a window aside)
@@ -454,7 +454,7 @@ mixed_paged_attn_kernel(const AttnArgs A) {
       const float u = res[hl * dv + a], w = res[hl * dv + b];
       float ya = u * cf + w * sf, yb = w * cf - u * sf;        // the rotation by -p
       if (gate) {
-        const float gt = logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(n) * A.gate_stride + h0 + hl]));
+        const float gt = row_logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(n) * A.gate_stride + h0 + hl]));
         ya *= gt; yb *= gt;
       }
       T* orow = out + (h0 + hl) * A.out_head_stride;
@@ -831,7 +831,7 @@ mixed_prompt_attn_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, co
           f = 1.0f / l;
         }
         if (gate && !A.unrotate && !(GATED && A.gate_dim))
-          f *= logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(RH ? row0 : row0 + row) * A.gate_stride + (RH ? head0(h) + row : h)]));
+          f *= row_logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(RH ? row0 : row0 + row) * A.gate_stride + (RH ? head0(h) + row : h)]));
       }
 #pragma unroll
       for (int nt = 0; nt < DV8; ++nt) {
@@ -880,7 +880,7 @@ mixed_prompt_attn_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, co
         const float u = slab[row * DVP + a], w = slab[row * DVP + b];
         float ya = u * cf + w * sf, yb = w * cf - u * sf;       // the rotation by minus the position
         if (gate) {
-          const float gt = logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(row0 + row) * A.gate_stride + h]));
+          const float gt = row_logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(row0 + row) * A.gate_stride + h]));
           ya *= gt;
           yb *= gt;
         }
@@ -930,7 +930,7 @@ attn_split_combine_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, c
       const float u = res[h * dv + a], w = res[h * dv + b];
       float ya = u * cf + w * sf, yb = w * cf - u * sf;
       if (gate) {
-        const float gt = logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(n) * A.gate_stride + h]));
+        const float gt = row_logistic(Cvt<T>::to_f32(gate[static_cast<int64_t>(n) * A.gate_stride + h]));
         ya *= gt;
         yb *= gt;
       }
@@ -992,7 +992,7 @@ struct SeqSpan {
 constexpr int kConvTokens = 64;   // tokens per CTA; at least taps - 1, so only a sequence's first CTA reads the carried inputs
 
 // A thread's inputs are read kConvAhead tokens before they are used: what bounds the kernel is bytes in flight.  B200, 8 x 2048 tokens of
-// 2048 channels, bf16, four taps: 67 -> 47 us (the bytes alone: 20; with a check of the end at every token 104).
+// 2048 channels, bf16, four taps: 67 -> 48 us (the bytes alone: 20; with a check of the end at every token 104).
 constexpr int kConvAhead = 8;
 
 template <typename T, int V>
@@ -1057,7 +1057,7 @@ causal_conv_silu_kernel(T* __restrict__ out, int64_t out_stride, const T* __rest
 #pragma unroll
       for (int i = 0; i < TAPS; ++i) y[u] = fmaf(wr[i][u], win[i][u], y[u]);
       y[u] += b[u];
-      y[u] *= logistic(y[u]);
+      y[u] *= row_logistic(y[u]);
 #pragma unroll
       for (int i = 0; i < TAPS - 1; ++i) win[i][u] = win[i + 1][u];
     }

@@ -269,7 +269,7 @@ group_topk_kernel(int32_t* __restrict__ ids, float* __restrict__ weights, const 
   const float* z = logits + static_cast<int64_t>(tok) * logit_stride;
   if (sigmoid_scores) {
     for (int e = lane; e < E; e += 32) {
-      const float s = logistic(z[e]);
+      const float s = row_logistic(z[e]);
       score[e] = s;
       choice[e] = s + (correction ? correction[e] : 0.f);
     }

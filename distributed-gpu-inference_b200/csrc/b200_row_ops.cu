@@ -323,7 +323,7 @@ value_prep_append_kernel(const T* __restrict__ k, int64_t k_stride, const T* __r
 // Bound by bytes and, with a gate, nearly as much by the instructions of its sigmoids.  LPR lanes per row, eight elements per lane and
 // piece; the rows of kHeadRows passes are under way before the first is waited for, and a row's token and head are counted on from the
 // warp's first row (a division per row of four elements per lane was a sixth of the instructions).
-// B200, bf16, 16384 x 8 rows of 128 with a gate: 52 -> 34 us (copying as many bytes: 29); without one 29 -> 27.
+// B200, bf16, 16384 x 8 rows of 128 with a gate: 52 -> 35 us (copying as many bytes: 29); without one 29 -> 27.
 constexpr int kHeadRows = 2;
 
 struct HeadNorm {
@@ -396,7 +396,7 @@ head_norm_rows(const HeadNorm A) {
         if (A.w) y *= Cvt<T>::to_f32(w[j].e[u]);
         if (A.gate) {
           const float z = Cvt<T>::to_f32(g[r][j].e[u]);
-          y *= A.act == 1 ? z * logistic(z) : logistic(z);
+          y *= A.act == 1 ? z * row_logistic(z) : row_logistic(z);
         }
         v[r][j][u] = y * A.out_scale;
       }
@@ -425,7 +425,7 @@ head_norm_kernel(const HeadNorm A) {
     if (w) y *= Cvt<T>::to_f32(w[i]);
     if (gr) {
       const float g = Cvt<T>::to_f32(gr[i]);
-      y *= A.act == 1 ? g * logistic(g) : logistic(g);
+      y *= A.act == 1 ? g * row_logistic(g) : row_logistic(g);
     }
     orow[i] = Cvt<T>::from_f32(y * A.out_scale);
   }
@@ -608,7 +608,7 @@ clamped_glu_kernel(T* __restrict__ y, const T* __restrict__ gu, int64_t rows, in
     for (int u = 0; u < N; ++u) {
       const float g = fminf(a[u], limit);
       const float up = fminf(fmaxf(b[u], -limit), limit);
-      a[u] = g * logistic(alpha * g) * (up + 1.0f);
+      a[u] = g * row_logistic(alpha * g) * (up + 1.0f);
     }
     if constexpr (N == 1) y[i] = Cvt<T>::from_f32(a[0]);
     else put(y + r * ff + c, a);
