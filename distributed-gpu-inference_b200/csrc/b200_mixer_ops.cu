@@ -713,7 +713,8 @@ grouped_linear_kernel(T* __restrict__ out, const T* __restrict__ xs, const T* __
 }
 
 // ---- routing ----------------------------------------------------------------------------------------------------
-// One warp per token: the `top` largest logits (ties: lowest index), weight = sigmoid(logit).
+// One warp per token: the `top` largest logits (ties: lowest index), weight = sigmoid(logit).  NaN logits are chosen last, the lowest
+// index first: the ids address experts and rows, so a token of NaNs has to have some, and its weights are NaN.
 __global__ void __launch_bounds__(128)
 sigmoid_topk_kernel(int32_t* __restrict__ ids, float* __restrict__ weights, const float* __restrict__ logits, int n_tok,
                     int E, int top) {
@@ -743,6 +744,15 @@ sigmoid_topk_kernel(int32_t* __restrict__ ids, float* __restrict__ weights, cons
       }
     }
     if (lane == 0) {
+      if (bi == 0x7fffffff) {        // what is left is NaN
+        auto taken = [&](int e) {
+          for (int j = 0; j < k; ++j)
+            if (ids[static_cast<int64_t>(tok) * top + j] == e) return true;
+          return false;
+        };
+        for (bi = 0; taken(bi);) ++bi;
+        best = z[bi];
+      }
       ids[static_cast<int64_t>(tok) * top + k] = bi;
       weights[static_cast<int64_t>(tok) * top + k] = sigmoidf_(best);
     }

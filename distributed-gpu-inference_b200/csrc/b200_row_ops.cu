@@ -518,23 +518,22 @@ __global__ void __launch_bounds__(256) zero_blocks_kernel(const __grid_constant_
 // ---- expert order -------------------------------------------------------------------------------------------------
 // One CTA of 1024 threads; thread t owns the pairs of a contiguous chunk.  count[e][t] pairs of expert e in chunk t -> their running
 // sums over the chunks (a warp per expert) -> where every chunk's pairs of every expert start: a stable counting sort.  The ids are
-// read twice and every output is written once; a radix sort of the same pairs is eight launches.
+// read twice and every output is written once; a radix sort of the same pairs is eight launches.  Ids outside 0 .. E - 1 sort behind
+// the last expert, so that order and where are permutations whatever the ids are: they index rows in the kernels that follow.
 constexpr int kOrderNT = 1024;
 constexpr int kOrderExperts = 48;
 __global__ void __launch_bounds__(kOrderNT)
 expert_order_kernel(int64_t* __restrict__ order, int64_t* __restrict__ where, int32_t* __restrict__ offsets, const int32_t* __restrict__ ids,
                     int n_pairs, int E) {
-  extern __shared__ int count[];          // [E][1024], then [E + 1]
-  int* start = count + E * kOrderNT;
+  extern __shared__ int count[];          // [E + 1][1024] (the last for ids of no expert), then [E + 2]
+  int* start = count + (E + 1) * kOrderNT;
+  auto bin = [&](int i) { return static_cast<int>(min(static_cast<unsigned>(ids[i]), static_cast<unsigned>(E))); };
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int per = (n_pairs + kOrderNT - 1) / kOrderNT, lo = min(t * per, n_pairs), hi = min(lo + per, n_pairs);
-  for (int e = 0; e < E; ++e) count[e * kOrderNT + t] = 0;
-  for (int i = lo; i < hi; ++i) {
-    const int e = ids[i];
-    if (e >= 0 && e < E) ++count[e * kOrderNT + t];
-  }
+  for (int e = 0; e <= E; ++e) count[e * kOrderNT + t] = 0;
+  for (int i = lo; i < hi; ++i) ++count[bin(i) * kOrderNT + t];
   __syncthreads();
-  for (int e = warp; e < E; e += kOrderNT / 32) {
+  for (int e = warp; e <= E; e += kOrderNT / 32) {
     int run = 0;
     for (int c = lane; c < kOrderNT; c += 32) {
       const int v = count[e * kOrderNT + c];
@@ -552,13 +551,12 @@ expert_order_kernel(int64_t* __restrict__ order, int64_t* __restrict__ where, in
   __syncthreads();
   if (t == 0) {
     start[0] = 0;
-    for (int e = 0; e < E; ++e) start[e + 1] += start[e];
+    for (int e = 0; e <= E; ++e) start[e + 1] += start[e];
   }
   __syncthreads();
   if (t <= E) offsets[t] = start[t];
   for (int i = lo; i < hi; ++i) {
-    const int e = ids[i];
-    if (e < 0 || e >= E) continue;
+    const int e = bin(i);
     const int at = start[e] + count[e * kOrderNT + t]++;
     order[at] = i;
     where[i] = at;
@@ -823,7 +821,7 @@ int b200_expert_order_supported(int64_t n_pairs, int n_experts) {
 int b200_expert_order(int64_t* order, int64_t* where, int32_t* offsets, const int32_t* ids, int64_t n_pairs, int n_experts, void* stream) {
   if (!b200_expert_order_supported(n_pairs, n_experts)) return fail(B200_ESHAPE, "b200_expert_order: up to %d pairs and %d experts", 1 << 17, kOrderExperts);
   if (!offsets || (n_pairs > 0 && (!order || !where || !ids))) return fail(B200_EINVAL, "b200_expert_order: null pointer");
-  const size_t smem = sizeof(int) * (static_cast<size_t>(n_experts) * kOrderNT + n_experts + 1);
+  const size_t smem = sizeof(int) * (static_cast<size_t>(n_experts + 1) * kOrderNT + n_experts + 2);
   if (smem > 48 * 1024) cudaFuncSetAttribute(expert_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   expert_order_kernel<<<1, kOrderNT, smem, static_cast<cudaStream_t>(stream)>>>(order, where, offsets, ids, static_cast<int>(n_pairs), n_experts);
   return check_launch("b200_expert_order");

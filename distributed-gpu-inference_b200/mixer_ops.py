@@ -262,13 +262,14 @@ def zero_blocks(pools, slots) -> None:
 @_timed
 def expert_order(ids: torch.Tensor, n_experts: int):
     """``(order int64 [n * top], where int64 [n * top], offsets int32 [n_experts + 1])`` for ``ids`` int32 ``[n, top]`` in ``0 ..
-    n_experts - 1``: the pairs in stable expert order, the inverse, and where each expert's rows start.  Nothing travels to the host."""
+    n_experts - 1``: the pairs in stable expert order, the inverse, and where each expert's rows start.  Other ids come behind the last
+    expert, so that ``order`` and ``where`` are permutations whatever the ids are.  Nothing travels to the host."""
     _need_cuda(ids)
     if ids.dtype != torch.int32 or not ids.is_contiguous():
         raise TypeError("expert ids are contiguous int32")
     n, lib = ids.numel(), _lib_()
     if not lib.b200_expert_order_supported(n, int(n_experts)):     # more pairs or experts than the one-CTA sort holds
-        flat = ids.reshape(-1)
+        flat = torch.where((ids < 0) | (ids > n_experts), n_experts, ids).reshape(-1)
         sorted_ids, order = torch.sort(flat.to(torch.int16) if n_experts < 1 << 15 else flat, stable=True)
         where = torch.empty_like(order)
         where[order] = torch.arange(n, device=ids.device)

@@ -98,14 +98,15 @@ int b200_head_rmsnorm(void* out, const float* x, const void* weight, float eps, 
 int b200_polynorm(void* out, const void* z, int64_t z_stride, const void* coef, float eps, int rows, int ff, int dtype,
                   void* stream);
 
-/* The `top` largest of E fp32 logits per token (ties: lowest index); weights = sigmoid(logit). */
+/* The `top` largest of E fp32 logits per token (ties: lowest index; NaN last); weights = sigmoid(logit). */
 int b200_sigmoid_topk(int32_t* ids, float* weights, const float* logits, int n_tok, int E, int top, void* stream);
 
 /* Block slots[i] of every pool set to zero: pools and block_bytes (a multiple of 16) are HOST arrays of n_pools, slots a HOST array. */
 int b200_zero_blocks(void* const* pools, const int64_t* block_bytes, int n_pools, const int32_t* slots, int n_slots, void* stream);
 
 /* Stable order of (token, choice) pairs by expert: order int64 [n_pairs] (pair of every sorted row), where int64 [n_pairs] (its inverse),
- * offsets int32 [n_experts + 1] (first sorted row of every expert).  ids int32 [n_pairs] in 0 .. n_experts - 1. */
+ * offsets int32 [n_experts + 1] (first sorted row of every expert).  ids int32 [n_pairs] in 0 .. n_experts - 1; others sort behind the
+ * last expert, so order and where are permutations whatever the ids are. */
 int b200_expert_order_supported(int64_t n_pairs, int n_experts);
 int b200_expert_order(int64_t* order, int64_t* where, int32_t* offsets, const int32_t* ids, int64_t n_pairs, int n_experts, void* stream);
 

@@ -76,6 +76,51 @@ def test_expert_order(n, top, E):
     assert offsets.tolist() == [0] + torch.bincount(ids.reshape(-1), minlength=E).cumsum(0).tolist()
 
 
+@pytest.mark.parametrize("n,top,E", [(7, 2, 5), (513, 2, 48), (700, 2, 49), (70000, 2, 3)])
+def test_expert_order_is_a_permutation_whatever_the_ids(n, top, E):
+    """Pairs of no expert come behind the last one: rows are addressed by ``order`` and ``where``."""
+    gen = torch.Generator().manual_seed(n)
+    ids = torch.randint(0, E, (n, top), dtype=torch.int32, generator=gen)
+    ids[::3, 0] = 0x7fffffff
+    ids[1::5, 1] = -1
+    ids[2::7, 0] = E
+    flat = torch.where((ids < 0) | (ids >= E), E, ids).reshape(-1)
+    want = torch.argsort(flat, stable=True)
+    order, where, offsets = (t.cpu() for t in mixer_ops.expert_order(ids.cuda(), E))
+    assert torch.equal(order, want) and torch.equal(where, torch.argsort(want))
+    assert offsets.tolist() == [0] + torch.bincount(flat, minlength=E + 1)[:E].cumsum(0).tolist()
+
+
+def test_sigmoid_topk_names_experts_for_tokens_of_nans():
+    nan, inf = float("nan"), float("inf")
+    rows = [[nan] * 40, [nan] * 39 + [1.0], [-inf] * 40, [0.0] * 20 + [nan] * 20, [nan, -inf] * 20]
+    ids, w = (t.cpu() for t in mixer_ops.sigmoid_topk(torch.tensor(rows, device="cuda"), 3))
+    assert ids.tolist() == [[0, 1, 2], [39, 0, 1], [0, 1, 2], [0, 1, 2], [1, 3, 5]]
+    assert w[0].isnan().all() and w[1, 1:].isnan().all()
+    assert abs(w[1, 0].item() - 1 / (1 + 2.718281828459045 ** -1)) < 2.0 ** -22      # e^-1, a sum and a quotient, each rounded once or twice
+    assert (w[2] == 0).all() and (w[3] == 0.5).all() and (w[4] == 0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n", [9, 1500])
+def test_a_token_of_nans_stays_its_own(n, dtype):
+    """Routed experts, the grouped kernel's sizes and the library's: the other tokens' rows are what they are without it."""
+    from dgi_b200.petipel_layer import SigmoidTopKMoE
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    E, W, ff = 5, 64, 32
+    lin = lambda o, i: torch.randn(o, i, generator=gen, device="cuda") / i ** 0.5  # noqa: E731
+    t = {f"e{e}.{k}": lin(*s) for e in range(E) for k, s in (("gate", (ff, W)), ("up", (ff, W)), ("down", (W, ff)))}
+    moe = SigmoidTopKMoE({"router": {"experts": E, "top": 2}, "expert": {"limit": 7.0}}, dict(t, router=lin(E, W)), "cuda", dtype)
+    h = torch.randn(n, W, generator=gen, device="cuda").to(dtype)
+    bad = h.clone()
+    bad[4] = float("nan")
+    out, want = moe(bad), moe(h)
+    rest = torch.arange(n, device="cuda") != 4
+    # another token's pairs move to other rows of the same products: their sums keep their order, or differ by its rounding
+    assert ((out - want)[rest].norm() / want[rest].norm()) <= {torch.float32: 1e-6}.get(dtype, 4 * TOL[dtype])
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("width", [8, 1024, 1032, 100])
 def test_expert_rows(width, dtype):
