@@ -240,8 +240,11 @@ cast_rows_kernel(T* __restrict__ out, const float* __restrict__ x, int64_t n) {
 }
 
 // ---- grouped routing: softmax or sigmoid scores ------------------------------------------------------------------------------------------
-// One warp per token.  Shared memory per warp: score[E], choice[E], group best[groups].  Ties go to the lowest index.
+// One warp per token.  Shared memory per warp: score[E], choice[E], group best[groups].  Ties go to the lowest index.  A score of NaN
+// counts as the lowest choice (NaN there marks an expert already taken), so that a token of NaNs has experts too: ids address rows.
 constexpr int kRouteWarps = 4;
+
+__device__ __forceinline__ float choice_of(float c) { return c == c ? c : -INFINITY; }
 
 __device__ __forceinline__ void warp_argmax(float& best, int& bi) {
 #pragma unroll
@@ -271,7 +274,7 @@ group_topk_kernel(int32_t* __restrict__ ids, float* __restrict__ weights, const 
     for (int e = lane; e < E; e += 32) {
       const float s = row_logistic(z[e]);
       score[e] = s;
-      choice[e] = s + (correction ? correction[e] : 0.f);
+      choice[e] = choice_of(s + (correction ? correction[e] : 0.f));
     }
   } else {
     float m = -INFINITY;
@@ -287,7 +290,7 @@ group_topk_kernel(int32_t* __restrict__ ids, float* __restrict__ weights, const 
     for (int e = lane; e < E; e += 32) {
       const float s = score[e] / sum;
       score[e] = s;
-      choice[e] = s + (correction ? correction[e] : 0.f);
+      choice[e] = choice_of(s + (correction ? correction[e] : 0.f));
     }
   }
   __syncwarp();

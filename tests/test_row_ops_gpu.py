@@ -101,6 +101,24 @@ def test_sigmoid_topk_names_experts_for_tokens_of_nans():
     assert (w[2] == 0).all() and (w[3] == 0.5).all() and (w[4] == 0).all()
 
 
+@pytest.mark.parametrize("groups,keep", [(1, 1), (4, 2)])
+@pytest.mark.parametrize("scores", ["softmax", "sigmoid"])
+def test_group_topk_names_experts_for_tokens_of_nans(scores, groups, keep):
+    E, top, nan = 40, 3, float("nan")
+    gen = torch.Generator(device="cuda").manual_seed(E)
+    z = torch.randn(6, E, generator=gen, device="cuda")
+    plain = z.clone()
+    z[1], z[3] = nan, nan
+    z[4, 5:] = nan
+    call = {"softmax": lambda x: mixer_ops.softmax_group_topk(x, None, top, groups, keep, sum_floor=1e-9),
+            "sigmoid": lambda x: mixer_ops.sigmoid_group_topk(x, None, E, top, groups, keep)}[scores]
+    (ids, w), (ids0, w0) = call(z), call(plain)
+    assert ((ids >= 0) & (ids < E)).all() and all(len(set(r)) == top for r in ids.tolist())
+    assert w[[1, 3]].isnan().all()
+    for r in (0, 2, 5):
+        assert torch.equal(ids[r], ids0[r]) and torch.equal(w[r], w0[r])
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("n", [9, 1500])
 def test_a_token_of_nans_stays_its_own(n, dtype):
