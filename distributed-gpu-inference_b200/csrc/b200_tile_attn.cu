@@ -190,7 +190,10 @@ struct Plan {
   static constexpr int kEnd = kV + (ALIAS ? 0 : kBufs * (DV / 64) * kBlk);
   static constexpr int kBar = kEnd;                    // barriers, the tensor memory's address, the failure flag
   static constexpr int kPage = kBar + 256;             // int [2][2][64]: rows of the pools that a tile's keys / values are in (-1: none)
-  static constexpr int kLut = kPage + 2 * 2 * kKeys * 4;  // float [4][rep][pitch]: biases of the tiles' distances
+  static constexpr int kLut = kPage + 2 * 2 * kKeys * 4;  // float [kLuts][rep][pitch]: biases of the tiles' distances
+  // A tile's biases are copied once S of the tile kBufs before it is done, hence P V of the one two before that, hence its softmax:
+  // the last reader known to be through is tile i - kBufs - 2.
+  static constexpr int kLuts = kBufs + 2;
   static constexpr int kO = 2 * kKeys;                 // columns of tensor memory per half: S0 | S1 | O
   static constexpr int kHalfTm = kHalves == 2 || kCtas == 2 ? 256 : 512;
   static constexpr int kTm = kHalves * kHalfTm;
@@ -311,7 +314,7 @@ tile_attn_kernel(const TileAttn A) {
       else move(std::integral_constant<int, DV>{});
       if (BIAS && !values) {      // entry [hh][x]: the bias of distance p0 - key0 - 63 + x
         const int d0 = p0 - key0(i) - (kKeys - 1), span = cnt + kKeys - 1;
-        const uint32_t dst = smem_u32(lut_s + (i & 3) * rep * pitch);
+        const uint32_t dst = smem_u32(lut_s + (i % P::kLuts) * rep * pitch);
         for (int hh = 0; hh < rep; ++hh) {
           const float* src = A.bias_lut + static_cast<int64_t>(g * rep + hh) * A.lut_len;
           for (int x = me; x < span; x += kTeam) cp4(dst + 4 * (hh * pitch + x), src + min(max(d0 + x, 0), A.lut_len - 1));
@@ -427,7 +430,7 @@ tile_attn_kernel(const TileAttn A) {
       tm_ld32(s[1], tm_row + (i & 1) * kKeys + 32);
       tc_wait_ld();
       if constexpr (BIAS) {
-        const float* b = lut_s + ((i & 3) * rep + (live ? hh : 0)) * pitch + (live ? t_row : 0) + kKeys - 1;
+        const float* b = lut_s + ((i % P::kLuts) * rep + (live ? hh : 0)) * pitch + (live ? t_row : 0) + kKeys - 1;
 #pragma unroll
         for (int c = 0; c < kKeys; ++c) s[c >> 5][c & 31] = fmaf(s[c >> 5][c & 31], mult, b[-c]);
       } else if (!plain) {
@@ -573,7 +576,7 @@ int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stre
   using P = Plan<DK, DV, ALIAS, HALVES>;
   const int rep = A.H / A.G;
   size_t smem = 1024 + P::kLut;
-  if (BIAS) smem += sizeof(float) * 4 * rep * (((P::kSoft / rep + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep));
+  if (BIAS) smem += sizeof(float) * P::kLuts * rep * (((P::kSoft / rep + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep));
   smem = std::max<size_t>(smem, P::kCtas == 2 ? 80 * 1024 : 120 * 1024);   // no more CTAs per SM than tensor memory has room for
   if (smem > 227 * 1024) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
   auto kern = tile_attn_kernel<T, DK, DV, ALIAS, BIAS, HALVES>;

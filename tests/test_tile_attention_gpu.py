@@ -131,3 +131,27 @@ def test_steep_scores_and_rescaling():
         mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, 0.5, window=window, rows=rows)
         want = _reference(q, k_pool, v_pool, st, 128, 1, 0.5, window=window)
         assert (out.to(F64) - want).norm() / want.norm() <= 1.5 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("layout,rows,bias", [(GROUPED, 128, 0), (GROUPED, 256, 0), (GROUPED, 128, 4000), (GROUPED, 256, 4000), (WIDE, 256, 4000),
+                                              (ONE, 256, 4000), (NARROW, 256, 4000), (LATENT, 128, 0), (LATENT_ROT, 128, 0)])
+def test_walks_of_many_key_tiles(layout, rows, bias):
+    """Every buffer, barrier and bias table is reused many times (no key splits); biases change sign and size from distance to distance,
+    so that another tile's table shows.  Several calls are the same to the bit."""
+    H, G, dk, dv, div = layout
+    q, k_pool, v_pool, st, rnd = _case(layout, [(600, 1500), (2 * rows + 5, 1900)], 16, torch.bfloat16)
+    lut = rnd(H, bias) * 3 if bias else None
+    D, scale = dv or 256, dk ** -0.5
+    out = torch.empty(q.shape[0], H, D, dtype=torch.bfloat16, device="cuda")
+    tiles = st.prompt_tiles(2, rows // (H // G))[0]
+    first = None
+    for _ in range(20):
+        out.fill_(7.0)
+        mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, scale, value_width=D, rows=rows, bias_lut=lut)
+        if first is None:
+            first = out.clone()
+            want = _reference(q, k_pool, v_pool, st, D, div, scale, bias=lut)
+            assert (out.to(F64) - want).norm() / want.norm() <= 1.5 * 2.0 ** -8
+            rows_err = (out.to(F64) - want).norm(dim=2) / want.norm(dim=2)
+            assert rows_err.max() <= 8 * 2.0 ** -8          # a row of wrong biases is off by its own size
+        assert torch.equal(out, first)
