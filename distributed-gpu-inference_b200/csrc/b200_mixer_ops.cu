@@ -539,14 +539,14 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int r = gq + 8 * i;
-      float mall = fmaxf(fmaxf(mg[r], mg[16 + r]), fmaxf(mg[32 + r], mg[48 + r]));
-      mall = mall == -INFINITY ? 0.f : mall;
+      const float seen = fmaxf(fmaxf(mg[r], mg[16 + r]), fmaxf(mg[32 + r], mg[48 + r]));   // -inf: none of these keys
+      const float mall = seen == -INFINITY ? 0.f : seen;
       const float w = expf(m[i] - mall);                  // this warp's weight in the merge
       float lsum = 0.f;
 #pragma unroll
       for (int w2 = 0; w2 < 4; ++w2) lsum += mg[64 + w2 * 16 + r] * expf(mg[w2 * 16 + r] - mall);
       l[i] = lsum;
-      m[i] = mall;
+      m[i] = seen;
 #pragma unroll
       for (int n = 0; n < DV8; ++n) {
         og[(warp * 16 + r) * dvp + n * 8 + 2 * tq] = o[n][2 * i] * w;
@@ -620,13 +620,15 @@ biased_split_merge_kernel(T* __restrict__ out, const float* __restrict__ ws, con
   float L = 0.f, O = 0.f;
 #pragma unroll 4
   for (int sp = 0; sp < splits; ++sp) {
-    const float f = expf(src[sp * step] - M);        // a row that saw none of a split's keys left sum 0 and output 0
+    const float f = expf(src[sp * step] - M);        // a row that saw none of a split's keys left maximum -inf, sum 0 and output 0
     L = fmaf(src[sp * step + 1], f, L);
     if (c < dv) O = fmaf(src[sp * step + 2 + c], f, O);
   }
   if (c >= dv) return;
+  // in the order of the launch without splits, whose result a row of one range repeats to the bit
   const float gt = gate ? sigmoidf_(Cvt<T>::to_f32(gate[n * gate_stride + h])) : 1.0f;
-  out[(n * H + h) * dv + c] = Cvt<T>::from_f32(O * gt / L);
+  const float inv = gt / L;
+  out[(n * H + h) * dv + c] = Cvt<T>::from_f32(O * inv);
 }
 
 // ---- grouped linear for expert-sorted rows (16-bit storage) ---------------------------------------------------------
