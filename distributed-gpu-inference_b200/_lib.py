@@ -122,7 +122,7 @@ MIXER_SIGNATURES = {
     "b200_biased_prompt_attn_ext": (
         c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
                 c_int, c_void_p, c_void_p, c_int, c_float, c_float, c_int, c_int, c_int, c_int, c_int, c_int,
-                c_int, c_void_p, c_int, c_int, c_void_p]),
+                c_int, c_void_p, c_int, c_void_p]),
     "b200_gated_scan": (
         c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                 c_int, c_int, c_int, c_int, c_void_p]),
@@ -279,13 +279,18 @@ MIXER_SIGNATURES = {
                 c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, c_int, c_int,
                 c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
                 c_int, c_void_p]),
+    "b200_mixed_prompt_attn_ext3": (
+        c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p,
+                c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, c_int, c_int,
+                c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p,
+                c_int, c_void_p]),
     # prompt portions on the fifth-generation tensor cores (csrc/b200_tile_attn.cu)
     "b200_tile_attn_supported": (c_int, [c_int] * 7),
     "b200_tile_attn_rows": (c_int, [c_int] * 4),
     "b200_tile_attn_splits": (c_int, [c_int] * 5),
     "b200_tile_attn": (
         c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p,
-                c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_float, c_float, c_int,
+                c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_float, c_float, c_int,
                 c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]),
     "b200_mixed_prompt_attn_rows_supported": (c_int, [c_int, c_int, c_int, c_int]),
     "b200_qknorm_rotary_append_ext2": (

@@ -267,6 +267,7 @@ struct AttnArgs {
   int out_f32 = 0;     // != 0: `out` is fp32 (same strides, in elements) whatever T is; plain outputs only (no turn back)
   int stage_q = 0;     // tensor-core kernel: a warp's 16 query rows are staged in shared memory once (always with row_heads)
   int gate_dim = 0;    // 0: one gate per head (rows of H); the value size: one per output channel (rows of H * dv)
+  int ws_tile = 0;     // key splits, > 0: the workspace holds this many rows per tile instead of one per packed row of the step
 };
 
 template <typename T>
@@ -536,7 +537,7 @@ constexpr int kTcPlain = 0, kTcGated = 1, kTcExt = 2;      // kTcExt carries eve
 template <typename T, int DV8, int HW, int MODE>
 __global__ void __launch_bounds__(kTcWarps * 32, (HW == 1 && DV8 <= 16) ? 2 : 1)
 mixed_prompt_attn_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, const float* __restrict__ rot_tab,
-                         float* __restrict__ ws, int n_tok, int stages) {
+                         float* __restrict__ ws, int ws_rows, int stages) {
   extern __shared__ __align__(16) unsigned char tc_smem[];
   constexpr bool EXT = MODE == kTcExt, GATED = MODE != kTcPlain;
   constexpr int HC = kTcWarps * HW;
@@ -796,8 +797,8 @@ mixed_prompt_attn_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, co
       for (int half = 0; half < 2; ++half) {
         const int row = qr + 8 * half;
         if (row >= rows_of(h)) continue;
-        float* dst = RH ? ws + ((static_cast<int64_t>(blockIdx.z) * n_tok + row0) * RH + head0(h) + row) * (DVP + 2)
-                        : ws + ((static_cast<int64_t>(blockIdx.z) * n_tok + row0 + row) * H + h) * (DVP + 2);
+        const int64_t at = static_cast<int64_t>(blockIdx.z) * ws_rows + (A.ws_tile > 0 ? static_cast<int>(blockIdx.x) * A.ws_tile : row0);
+        float* dst = RH ? ws + (at * RH + head0(h) + row) * (DVP + 2) : ws + ((at + row) * H + h) * (DVP + 2);
         if (qc == 0) {
           dst[0] = m_r[hw][half];
           dst[1] = l_r[hw][half];
@@ -900,18 +901,19 @@ mixed_prompt_attn_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, co
 // then the turn back and the gate, as in the single-CTA epilogue.
 template <typename T>
 __global__ void __launch_bounds__(256)
-attn_split_combine_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, const float* __restrict__ ws, int n_splits, int n_tok,
+attn_split_combine_kernel(const AttnArgs A, const int32_t* __restrict__ tiles, const float* __restrict__ ws, int n_splits, int ws_rows,
                           int dvp, const float* __restrict__ rot_tab) {
   extern __shared__ float res[];   // [H][dv]
   if (static_cast<int>(blockIdx.y) >= tiles[3 * blockIdx.x + 1]) return;
   const int n = tiles[3 * blockIdx.x] + blockIdx.y, H = A.H, dv = A.dv, stride = dvp + 2;
+  const int wr = A.ws_tile > 0 ? static_cast<int>(blockIdx.x) * A.ws_tile + blockIdx.y : n;
   for (int e = threadIdx.x; e < H * dv; e += blockDim.x) {
     const int h = e / dv, c = e - h * dv;
     float M = A.sink ? A.sink[h] : -INFINITY;
-    for (int sp = 0; sp < n_splits; ++sp) M = fmaxf(M, ws[((static_cast<int64_t>(sp) * n_tok + n) * H + h) * stride]);
+    for (int sp = 0; sp < n_splits; ++sp) M = fmaxf(M, ws[((static_cast<int64_t>(sp) * ws_rows + wr) * H + h) * stride]);
     float L = A.sink ? expf(A.sink[h] - M) : 0.f, O = 0.f;
     for (int sp = 0; sp < n_splits; ++sp) {
-      const float* src = ws + ((static_cast<int64_t>(sp) * n_tok + n) * H + h) * stride;
+      const float* src = ws + ((static_cast<int64_t>(sp) * ws_rows + wr) * H + h) * stride;
       const float f = src[0] == -INFINITY ? 0.f : expf(src[0] - M);
       L = fmaf(src[1], f, L);
       O = fmaf(src[2 + c], f, O);
@@ -1302,12 +1304,12 @@ int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_ro
 
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,
-                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, int tile_rows, const int32_t* tok_pos, int n_tok,
+                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, int tile_rows, const int32_t* tok_pos,
                    const float* sink, const float* bias_lut, int lut_len, float scale, float softcap, float temp_coef, int temp_every,
                    int window, int keep_first, int chunk, int H, int G, int dk, int dv, int v_row, int v_div, int out_f32, int block_size,
                    int n_splits, float* workspace, int dtype, void* stream) {
   const bool alias = k_pool == v_pool;
-  if (n_tiles < 0 || n_tok < 0 || H <= 0 || G <= 0 || H % G || block_size <= 0 || n_splits < 1 || n_splits > 64 || chunk < 0 ||
+  if (n_tiles < 0 || H <= 0 || G <= 0 || H % G || block_size <= 0 || n_splits < 1 || n_splits > 64 || chunk < 0 ||
       v_div < 1 || G % v_div || v_row < dv || v_row % 8 || (bias_lut && (lut_len <= 0 || softcap > 0.f)))
     return fail(B200_EINVAL, "b200_tile_attn: bad sizes");
   if (!tile_attn_supported(H, G, dk, dv, alias, bias_lut != nullptr, dtype) || (alias && (v_div != 1 || v_row != dk)))
@@ -1327,7 +1329,8 @@ int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, c
   A.gate = gate, A.gate_stride = gate_stride, A.gate_dim = gate_per_channel ? dv : 0;
   A.k_pool = k_pool, A.v_pool = v_pool, A.block_tables = block_tables, A.table_stride = table_stride;
   A.tiles = tiles, A.tok_pos = tok_pos, A.sink = sink, A.bias_lut = bias_lut, A.lut_len = lut_len, A.ws = workspace;
-  A.n_tok = n_tok, A.H = H, A.G = G, A.block_size = block_size, A.v_row = v_row, A.v_div = v_div;
+  const int per_tile = tile_rows / (H / G), ws_rows = n_tiles * per_tile;
+  A.H = H, A.G = G, A.block_size = block_size, A.v_row = v_row, A.v_div = v_div;
   A.window = window, A.keep_first = keep_first, A.chunk = chunk;
   A.out_f32 = out_f32, A.out_vec = aligned16(out) && ((out_tok_stride | out_head_stride) & 7) == 0;
   A.scale = scale, A.softcap = softcap, A.temp_coef = temp_coef, A.temp_every = temp_every;
@@ -1336,14 +1339,14 @@ int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, c
   if (rc != 0 || n_splits == 1) return rc;
   AttnArgs M{out, out_tok_stride, out_head_stride, q, q_tok_stride, q_head_stride, gate, gate_stride, k_pool, v_pool,
              block_tables, table_stride, nullptr, tok_pos, nullptr, sink, scale, window, keep_first, 0,
-             0, 0.0, H, G, dk, dv, block_size, softcap, chunk, v_row, v_div, 0, out_f32, 0, gate_per_channel ? dv : 0};
+             0, 0.0, H, G, dk, dv, block_size, softcap, chunk, v_row, v_div, 0, out_f32, 0, gate_per_channel ? dv : 0, per_tile};
   const size_t smem = sizeof(float) * static_cast<size_t>(H) * dv;
   if (smem > 200 * 1024) return fail(B200_ESHAPE, "b200_tile_attn: %d heads of %d are too many to merge", H, dv);
   return hybrid_by_dtype(dtype, "b200_tile_attn", [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
     auto merge = attn_split_combine_kernel<T>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    merge<<<dim3(n_tiles, tile_rows / (H / G)), 256, smem, s>>>(M, tiles, workspace, n_splits, n_tok, dv, nullptr);
+    merge<<<dim3(n_tiles, per_tile), 256, smem, s>>>(M, tiles, workspace, n_splits, ws_rows, dv, nullptr);
     return check_launch("b200_tile_attn (merge)");
   });
 }
@@ -1389,6 +1392,20 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
                                 int keep_first, int chunk, const float* value_rot, int interleaved, int H, int G, int dk,
                                 int dv, int v_row, int v_div, int heads_as_rows, int out_f32, int block_size, int n_splits,
                                 float* workspace, int dtype, void* stream) {
+  return b200_mixed_prompt_attn_ext3(out, out_tok_stride, out_head_stride, q, q_tok_stride, q_head_stride, gate, gate_stride,
+                                     gate_per_channel, k_pool, v_pool, block_tables, table_stride, tiles, n_tiles, 0, tok_pos, n_tok,
+                                     talk, sink, scale, softcap, window, keep_first, chunk, value_rot, interleaved, H, G, dk, dv,
+                                     v_row, v_div, heads_as_rows, out_f32, block_size, n_splits, workspace, dtype, stream);
+}
+
+int b200_mixed_prompt_attn_ext3(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q,
+                                int64_t q_tok_stride, int64_t q_head_stride, const void* gate, int64_t gate_stride,
+                                int gate_per_channel, const void* k_pool, const void* v_pool, const int32_t* block_tables,
+                                int table_stride, const int32_t* tiles, int n_tiles, int ws_tile, const int32_t* tok_pos, int n_tok,
+                                const float* talk, const float* sink, float scale, float softcap, int window,
+                                int keep_first, int chunk, const float* value_rot, int interleaved, int H, int G, int dk,
+                                int dv, int v_row, int v_div, int heads_as_rows, int out_f32, int block_size, int n_splits,
+                                float* workspace, int dtype, void* stream) {
   if (gate_per_channel && value_rot) return fail(B200_EINVAL, "b200_mixed_prompt_attn: a gate per channel is not turned back");
   if (out_f32 && value_rot) return fail(B200_EINVAL, "b200_mixed_prompt_attn: fp32 outputs are not turned back");
   if (chunk < 0 || v_row < dv || v_row % 8 || v_div < 1 || G % v_div)
@@ -1400,7 +1417,7 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
   const int H_real = H;
   if (heads_as_rows) H = (H + 15) / 16;      // the kernel's heads are groups of 16 rows
   if (n_tiles < 0 || n_tok < 0 || H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0 || block_size <= 0 || n_splits < 1 ||
-      n_splits > 64)
+      n_splits > 64 || ws_tile < 0 || ws_tile > kTcRows)
     return fail(B200_EINVAL, "b200_mixed_prompt_attn: bad sizes");
   if (n_tiles == 0) return 0;
   if (!out || !q || !k_pool || !v_pool || !block_tables || !tiles || !tok_pos || (n_splits > 1 && !workspace))
@@ -1420,7 +1437,8 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
   AttnArgs A{out, out_tok_stride, out_head_stride, q, q_tok_stride, q_head_stride, gate, gate_stride, k_pool, v_pool,
              block_tables, table_stride, nullptr, tok_pos, talk, sink, scale, window, keep_first, value_rot != nullptr,
              interleaved, 0.0, H, G, dk, dv, block_size, softcap, chunk, v_row, v_div, heads_as_rows ? H_real : 0,
-             out_f32, stage_q ? 1 : 0, gate_per_channel ? dv : 0};
+             out_f32, stage_q ? 1 : 0, gate_per_channel ? dv : 0, ws_tile};
+  const int ws_rows = ws_tile > 0 ? n_tiles * ws_tile : n_tok;
   const dim3 grid(n_tiles, (H + kTcWarps * plan.hw - 1) / (kTcWarps * plan.hw), n_splits);
   return hybrid_by_dtype(dtype, "b200_mixed_prompt_attn", [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
@@ -1432,7 +1450,7 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
         if (plan.smem > 48 * 1024)
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(plan.smem));
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        kern<<<grid, kTcWarps * 32, plan.smem, s>>>(A, tiles, value_rot, workspace, n_tok, plan.stages);
+        kern<<<grid, kTcWarps * 32, plan.smem, s>>>(A, tiles, value_rot, workspace, ws_rows, plan.stages);
       };
       auto pick = [&](auto mode) {
         constexpr int M = decltype(mode)::value;
@@ -1449,11 +1467,11 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
       if (rc != 0 || n_splits == 1) return rc;
       // the merge runs over the tiles' rows only: others of the step belong to another launch (as many tiles as rows: one each)
       A.H = H_real;
-      const dim3 rows(n_tiles, n_tiles == n_tok ? 1 : kTcRows);
+      const dim3 rows(n_tiles, ws_tile > 0 ? ws_tile : (n_tiles == n_tok ? 1 : kTcRows));
       const size_t smem_c = sizeof(float) * static_cast<size_t>(H_real) * dv;
       auto comb = attn_split_combine_kernel<T>;
       if (smem_c > 48 * 1024) cudaFuncSetAttribute(comb, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_c));
-      comb<<<rows, 256, smem_c, s>>>(A, tiles, workspace, n_splits, n_tok, plan.dv8 * 8, value_rot);
+      comb<<<rows, 256, smem_c, s>>>(A, tiles, workspace, n_splits, ws_rows, plan.dv8 * 8, value_rot);
       return check_launch("b200_mixed_prompt_attn (merge)");
     }
   });

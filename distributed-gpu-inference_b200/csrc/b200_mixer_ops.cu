@@ -323,7 +323,7 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
                               const AttnTile* __restrict__ tiles, const int32_t* __restrict__ tok_pos,
                               const float* __restrict__ bias_lut, int lut_len, int lut_in_smem, int q_vec, float scale,
                               float temp_coef, int temp_every, int H, int G, int dk, int dv, int block_size, float* __restrict__ ws,
-                              int n_tok) {
+                              int ws_tile) {
   // Row r of the CTA's 64 is (token r / rep, head g * rep + r % rep): the heads of a kv group share the K / V tiles.
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int dvp = DV8 * 8;
@@ -556,16 +556,17 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
     __syncthreads();
     if (!split && warp != 0) return;
     if (split) {     // (maximum, sum, output) of these keys, all warps: the merge kernel below reads them
+      const int64_t ws_row0 = (static_cast<int64_t>(blockIdx.z) * gridDim.x + blockIdx.x) * ws_tile;
       for (int e = threadIdx.x; e < n_rows * dv; e += blockDim.x) {
         const int r = e / dv, c = e - r * dv, t = r / rep;
-        float* dst = ws + ((static_cast<int64_t>(blockIdx.z) * n_tok + tile.tok0 + t) * H + g * rep + r - t * rep) * (dv + 2);
+        float* dst = ws + ((ws_row0 + t) * H + g * rep + r - t * rep) * (dv + 2);
         dst[2 + c] = (og[r * dvp + c] + og[(16 + r) * dvp + c]) + (og[(32 + r) * dvp + c] + og[(48 + r) * dvp + c]);
       }
       if (warp == 0 && tq == 0) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           if (gq + 8 * i >= n_rows) continue;
-          float* dst = ws + ((static_cast<int64_t>(blockIdx.z) * n_tok + tile.tok0 + tokr[i]) * H + headr[i]) * (dv + 2);
+          float* dst = ws + ((ws_row0 + tokr[i]) * H + headr[i]) * (dv + 2);
           dst[0] = m[i];
           dst[1] = l[i];
         }
@@ -607,14 +608,14 @@ biased_prompt_attn_mma_kernel(T* __restrict__ out, const T* __restrict__ q, int6
 template <typename T>
 __global__ void __launch_bounds__(128)
 biased_split_merge_kernel(T* __restrict__ out, const float* __restrict__ ws, const T* __restrict__ gate, int64_t gate_stride,
-                          const AttnTile* __restrict__ tiles, const int32_t* __restrict__ tok_pos, int n_tok, int H, int dv) {
+                          const AttnTile* __restrict__ tiles, const int32_t* __restrict__ tok_pos, int H, int dv) {
   const AttnTile tile = tiles[blockIdx.x];
   if (static_cast<int>(blockIdx.y) >= tile.count) return;
   const int64_t n = tile.tok0 + blockIdx.y;
   const int h = blockIdx.z, c = threadIdx.x;
   const int splits = (tok_pos[tile.tok0] + tile.count - 1) / kSplitKeys + 1;     // as the tile's CTAs cut its keys
-  const int64_t step = static_cast<int64_t>(n_tok) * H * (dv + 2);
-  const float* src = ws + (n * H + h) * (dv + 2);
+  const int64_t step = static_cast<int64_t>(gridDim.x) * gridDim.y * H * (dv + 2);
+  const float* src = ws + ((static_cast<int64_t>(blockIdx.x) * gridDim.y + blockIdx.y) * H + h) * (dv + 2);
   float M = -INFINITY;
   for (int sp = 0; sp < splits; ++sp) M = fmaxf(M, src[sp * step]);
   float L = 0.f, O = 0.f;
@@ -849,7 +850,7 @@ int b200_biased_prompt_attn(void* out, const void* q, int64_t q_stride, const vo
                             int block_size, int dtype, void* stream) {
   return b200_biased_prompt_attn_ext(out, q, q_stride, gate, gate_stride, k_pool, v_pool, block_tables, table_stride, tiles, n_tiles,
                                      max_tile_tokens, tok_pos, bias_lut, lut_len, scale, temp_coef, temp_every, H, G, dk, dv, block_size,
-                                     0, nullptr, 0, dtype, stream);
+                                     0, nullptr, dtype, stream);
 }
 
 int b200_biased_attn_split_keys(void) { return kSplitKeys; }
@@ -858,7 +859,7 @@ int b200_biased_prompt_attn_ext(void* out, const void* q, int64_t q_stride, cons
                             const void* k_pool, const void* v_pool, const int32_t* block_tables, int table_stride,
                             const int32_t* tiles, int n_tiles, int max_tile_tokens, const int32_t* tok_pos, const float* bias_lut,
                             int lut_len, float scale, float temp_coef, int temp_every, int H, int G, int dk, int dv,
-                            int block_size, int max_context, float* workspace, int n_tok, int dtype, void* stream) {
+                            int block_size, int max_context, float* workspace, int dtype, void* stream) {
   if (n_tiles < 0 || H <= 0 || G <= 0 || H % G || block_size <= 0 || lut_len <= 0)
     return fail(B200_EINVAL, "b200_biased_prompt_attn: bad sizes");
   if (!b200_biased_prompt_attn_supported(dk, dv, dtype))
@@ -893,7 +894,7 @@ int b200_biased_prompt_attn_ext(void* out, const void* q, int64_t q_stride, cons
             static_cast<T*>(out), static_cast<const T*>(q), q_stride, static_cast<const T*>(gate), gate_stride,
             static_cast<const T*>(k_pool), static_cast<const T*>(v_pool), block_tables, table_stride,
             reinterpret_cast<const AttnTile*>(tiles), tok_pos, bias_lut, lut_len, lut_in_smem, q_vec, scale, temp_coef,
-            temp_every, H, G, dk, dv, block_size, ws, n_tok);
+            temp_every, H, G, dk, dv, block_size, ws, max_tile_tokens);
       };
       if (ksplit) {
         if (dv8 == 4) launch(biased_prompt_attn_mma_kernel<T, 4, true>);
@@ -907,7 +908,7 @@ int b200_biased_prompt_attn_ext(void* out, const void* q, int64_t q_stride, cons
       const int rc = check_launch("b200_biased_prompt_attn");
       if (rc != 0 || !ws) return rc;
       biased_split_merge_kernel<T><<<dim3(n_tiles, max_tile_tokens, H), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-          static_cast<T*>(out), ws, static_cast<const T*>(gate), gate_stride, reinterpret_cast<const AttnTile*>(tiles), tok_pos, n_tok, H, dv);
+          static_cast<T*>(out), ws, static_cast<const T*>(gate), gate_stride, reinterpret_cast<const AttnTile*>(tiles), tok_pos, H, dv);
       return check_launch("b200_biased_prompt_attn (merge)");
     }
   });

@@ -499,7 +499,8 @@ tile_attn_kernel(const TileAttn A) {
     const float m_nat = m_ref * kLn2;
     const int64_t n = tok0 + t_row;
     if (gridDim.z > 1) {
-      float* dst = A.ws + ((static_cast<int64_t>(blockIdx.z) * A.n_tok + n) * A.H + h_row) * (DV + 2);
+      const int64_t wr = (static_cast<int64_t>(blockIdx.z) * gridDim.x + blockIdx.x) * (kSoft / rep) + t_row;
+      float* dst = A.ws + (wr * A.H + h_row) * (DV + 2);
       if (live) {
         dst[0] = ok ? m_nat : NAN;
         dst[1] = l;

@@ -18,8 +18,8 @@ struct TileAttn {
   const int32_t* tiles; const int32_t* tok_pos;
   const float* sink;
   const float* bias_lut; int lut_len;        // distance biases [H][lut_len], or null
-  float* ws;                                 // key splits: [split][n_tok][H][dv + 2]
-  int n_tok, H, G, block_size, v_row, v_div;
+  float* ws;                                 // key splits: [split][tile][token of the tile][H][dv + 2]
+  int H, G, block_size, v_row, v_div;
   int window, keep_first, chunk;
   int gate_dim, out_f32, out_vec;            // gates per channel: the value size; 16-byte stores possible
   float scale, softcap, temp_coef;

@@ -180,11 +180,11 @@ class ParallelMixer(nn.Module):
         if self.tensor_cores:
             tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
             args = (attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables)
-            kw = dict(sink=self.sink, window=self.window, max_context=st.max_context(), softcap=self.softcap)
+            kw = dict(sink=self.sink, window=self.window, softcap=self.softcap)
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], max_context=tiles[2], **kw)
             if rest is not None:
-                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, max_tile_tokens=rest[1], max_context=rest[2], **kw)
         else:
             mixer_ops.mixed_paged_attention(attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
                                             st.tok_row, st.tok_pos, self.scale, sink=self.sink, window=self.window,

@@ -149,6 +149,11 @@ def prompt_attention_supported(dk: int, dv: int, dtype: torch.dtype) -> bool:
     return bool(_lib_().b200_biased_prompt_attn_supported(int(dk), int(dv), DTYPE_ID[dtype]))
 
 
+# Bytes up to which ``biased_prompt_attention`` divides keys over CTAs.  Steps beyond (256 sequences of 16 heads, one of them at 130000
+# tokens) have CTAs enough without; dividing always at multiples of the same size is what keeps a row's sums its own.
+SPLIT_WORKSPACE = 1 << 30
+
+
 @_timed
 def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[torch.Tensor], k_pool: torch.Tensor,
                             v_pool: torch.Tensor, block_tables: torch.Tensor, tiles: torch.Tensor, tok_pos: torch.Tensor,
@@ -157,7 +162,7 @@ def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[t
     """``biased_paged_attention`` on the tensor cores, for prompt portions and decoded tokens alike; writes the tiles'
     rows of ``out`` ``[n, H*dv]`` (16-bit dtypes, see ``prompt_attention_supported``).  ``tiles``: up to
     ``prompt_tile_tokens(H, G)`` tokens each; ``max_tile_tokens``: the largest tile (0 = unknown) — steps of decoded
-    tokens only take the variant whose warps split the keys; with ``max_context`` (a bound on the step's contexts) its CTAs do too."""
+    tokens only take the variant whose warps split the keys; with ``max_context`` (a bound on the tiles' contexts) its CTAs do too."""
     _need_cuda(out, q, k_pool, v_pool, block_tables, tiles, tok_pos, bias_lut)
     nb, G, bs, dk = k_pool.shape
     dv = v_pool.shape[3]
@@ -174,12 +179,14 @@ def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[t
     ws = None
     if 0 < max_tile_tokens * (H // G) <= 16 and max_context > lib.b200_biased_attn_split_keys():
         splits = -(-max_context // lib.b200_biased_attn_split_keys())
-        ws = torch.empty((splits, n, H, dv + 2), dtype=torch.float32, device=q.device)
+        rows = tiles.shape[0] * max_tile_tokens     # the tiles' own: a step's prompts beside them are another launch's
+        if splits * rows * H * (dv + 2) * 4 <= SPLIT_WORKSPACE:
+            ws = torch.empty((splits, rows, H, dv + 2), dtype=torch.float32, device=q.device)
     rc = lib.b200_biased_prompt_attn_ext(out.data_ptr(), q.data_ptr(), _rows2(q), _ptr(gate),
                                          _rows2(gate) if gate is not None else 0, k_pool.data_ptr(), v_pool.data_ptr(),
                                          block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), tiles.shape[0],
                                          int(max_tile_tokens), tok_pos.data_ptr(), bias_lut.data_ptr(), bias_lut.shape[1], float(scale),
-                                         float(temp_coef), int(temp_every), H, G, dk, dv, bs, int(max_context), _ptr(ws), n, DTYPE_ID[q.dtype], _stream())
+                                         float(temp_coef), int(temp_every), H, G, dk, dv, bs, int(max_context), _ptr(ws), DTYPE_ID[q.dtype], _stream())
     _lib.check_mixers(rc, "b200_biased_prompt_attn")
 
 
@@ -515,12 +522,12 @@ def mixed_prompt_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Ten
                            keep_first: int = 0, value_rot: Optional[torch.Tensor] = None, interleaved: bool = False,
                            gate: Optional[torch.Tensor] = None, max_context: int = 0, softcap: float = 0.0,
                            chunk: int = 0, value_width: Optional[int] = None, value_div: int = 1,
-                           heads_as_rows: bool = False) -> None:
+                           heads_as_rows: bool = False, max_tile_tokens: int = PROMPT_TILE_TOKENS) -> None:
     """``mixed_paged_attention`` on the tensor cores for prompt portions and decoded tokens alike (16-bit dtypes, see
     ``mixed_prompt_attention_supported``).  ``tiles`` int32 ``[n_tiles, 3]``: up to ``PROMPT_TILE_TOKENS`` consecutive
-    tokens of one sequence each, together covering every row of ``q``; ``value_rot``: the table ``rotary_kv_append``
-    returned for this step's tokens; ``max_context``: the longest context of the step (a hint: steps of few tokens over
-    long contexts divide the keys over several CTAs and merge); ``chunk``, ``value_width`` and ``value_div`` as in
+    tokens of one sequence each (``max_tile_tokens`` bounds them); only their rows of ``out`` are written; ``value_rot``: the table
+    ``rotary_kv_append`` returned for this step's tokens; ``max_context``: the longest context of the tiles (a hint: few tokens
+    over long contexts divide the keys over several CTAs and merge); ``chunk``, ``value_width`` and ``value_div`` as in
     ``mixed_paged_attention``, as are the kinds of ``gate``.  ``heads_as_rows`` (steps of single tokens over one kv head,
     no talk / value_rot; see ``heads_as_rows_supported``): the 16 rows of a tensor-core tile are 16 query heads of one token
     instead of 16 tokens of one head."""
@@ -544,6 +551,10 @@ def mixed_prompt_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Ten
     per_channel = _gate_kind(gate, n, H, dv, q.dtype)
     if heads_as_rows and (G != 1 or talk is not None or value_rot is not None):
         raise ValueError("heads_as_rows needs one kv head and no talk or value_rot")
+    if not 1 <= max_tile_tokens <= PROMPT_TILE_TOKENS:
+        raise ValueError(f"tiles have 1 to {PROMPT_TILE_TOKENS} tokens")
+    if heads_as_rows:
+        max_tile_tokens = 1
     lib = _lib_()
     seen = min(max_context, window + keep_first + PROMPT_TILE_TOKENS) if window > 0 else max_context
     if chunk > 0:
@@ -554,11 +565,12 @@ def mixed_prompt_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Ten
                                                DTYPE_ID[q.dtype]) if max_context > 0 else 1
     ws = None
     if splits > 1:
-        ws = torch.empty(lib.b200_mixed_prompt_attn_workspace(splits, n, H, dv) // 4, dtype=torch.float32, device=q.device)
-    rc = lib.b200_mixed_prompt_attn_ext2(out.data_ptr(), out.stride(0), out.stride(1), q.data_ptr(), q.stride(0),
+        ws = torch.empty(lib.b200_mixed_prompt_attn_workspace(splits, tiles.shape[0] * max_tile_tokens, H, dv) // 4, dtype=torch.float32,
+                         device=q.device)
+    rc = lib.b200_mixed_prompt_attn_ext3(out.data_ptr(), out.stride(0), out.stride(1), q.data_ptr(), q.stride(0),
                                         q.stride(1), _ptr(gate), _rows2(gate) if gate is not None else 0, per_channel, k_pool.data_ptr(),
                                         v_pool.data_ptr(), block_tables.data_ptr(), block_tables.stride(0),
-                                        tiles.data_ptr(), tiles.shape[0], tok_pos.data_ptr(), n, _ptr(talk), _ptr(sink),
+                                        tiles.data_ptr(), tiles.shape[0], int(max_tile_tokens), tok_pos.data_ptr(), n, _ptr(talk), _ptr(sink),
                                         float(scale), float(softcap), int(window), int(keep_first), int(chunk),
                                         _ptr(value_rot), int(interleaved), H, G, dk, dv, v_row, int(value_div),
                                         int(heads_as_rows), out_f32, bs, int(splits), _ptr(ws), DTYPE_ID[q.dtype], _stream())
@@ -615,10 +627,10 @@ def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_p
     if chunk > 0:
         seen = min(seen, chunk + 128)
     splits = lib.b200_tile_attn_splits(tiles.shape[0], (seen + 63) // 64, G, dk, int(rows)) if max_context > 0 else 1
-    ws = torch.empty((splits, n, H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+    ws = torch.empty((splits, tiles.shape[0] * (rows // (H // G)), H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
     rc = lib.b200_tile_attn(out.data_ptr(), out.stride(0), out.stride(1), q.data_ptr(), q.stride(0), q.stride(1), _ptr(gate),
                             _rows2(gate) if gate is not None else 0, per_channel, k_pool.data_ptr(), v_pool.data_ptr(),
-                            block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), tiles.shape[0], int(rows), tok_pos.data_ptr(), n,
+                            block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), tiles.shape[0], int(rows), tok_pos.data_ptr(),
                             _ptr(sink), _ptr(bias_lut), bias_lut.shape[1] if bias_lut is not None else 0, float(scale), float(softcap),
                             float(temp_coef), int(temp_every), int(window), int(keep_first), int(chunk), H, G, dk, dv, v_row,
                             int(value_div), int(out.dtype == torch.float32), bs, int(splits), _ptr(ws), DTYPE_ID[q.dtype], _stream())

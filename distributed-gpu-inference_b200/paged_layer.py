@@ -232,8 +232,9 @@ class RaggedBatchState:
 
     def attention_tiles(self, H: int, G: int, dk: int, cap: int, whole: bool):
         """How an attention layer of H heads over G kv heads of key size ``dk`` serves the step: ``(tiles, rest)``.  ``tiles``: the
-        long portions for ``mixer_ops.tile_attention``, ``(tile list, rows per tile)`` (None: none, or not ``whole``: the layer's
-        sizes are not served there); ``rest``: ``prompt_tiles`` of up to ``cap`` tokens over the others (None: none)."""
+        long portions for ``mixer_ops.tile_attention``, ``(tile list, rows per tile, longest context of these)`` (None: none, or not
+        ``whole``: the layer's sizes are not served there); ``rest``: the others in tiles of up to ``cap`` tokens, ``(tile list, most
+        tokens of a tile, longest context of these)`` (None: none)."""
         from . import mixer_ops
 
         if self._tiles is None:
@@ -241,12 +242,15 @@ class RaggedBatchState:
         key = ("attention", H, G, dk, cap, whole)
         if key not in self._tiles:      # the step's layers of one layout share it
             cut = mixer_ops.tile_attention_from(H, G) if whole else 1 << 30
-            counts = [count for _first, count, _row, _past in self.spans]
-            tiles = None
-            if max(counts) >= cut:
-                rows = mixer_ops.tile_rows(H, G, dk, sum(c for c in counts if c >= cut))
-                tiles = self.prompt_tiles(cut, max(1, rows // (H // G)))[0], rows
-            self._tiles[key] = tiles, self.prompt_tiles(1, cap, cut) if min(counts) < cut else None
+            long = [(count, past + count) for _first, count, _row, past in self.spans if count >= cut]
+            short = [past + count for _first, count, _row, past in self.spans if count < cut]
+            tiles = rest = None
+            if long:
+                rows = mixer_ops.tile_rows(H, G, dk, sum(c for c, _ in long))
+                tiles = self.prompt_tiles(cut, max(1, rows // (H // G)))[0], rows, max(t for _, t in long)
+            if short:
+                rest = *self.prompt_tiles(1, cap, cut), max(short)
+            self._tiles[key] = tiles, rest
         return self._tiles[key]
 
     def scan_plan(self, ctas_per_seq: int = 0, segment: int = 0, at_least: int = 512):

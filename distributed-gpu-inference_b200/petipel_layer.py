@@ -171,12 +171,12 @@ class BiasedPagedAttention(nn.Module):
             tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.prompt_tile_tokens(H, G), self.in_tiles)
             if tiles is not None:
                 mixer_ops.tile_attention(attn.view(-1, H, dv), q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
-                                         tiles[0], st.tok_pos, self.scale, gate=gate, rows=tiles[1], max_context=st.max_context(),
+                                         tiles[0], st.tok_pos, self.scale, gate=gate, rows=tiles[1], max_context=tiles[2],
                                          bias_lut=self.bias_lut, temp_coef=self.temp_coef, temp_every=self.temp_every)
             if rest is not None:
                 mixer_ops.biased_prompt_attention(attn, q, gate, cache.k_pool, cache.v_pool, st.block_tables, rest[0], st.tok_pos,
                                                   self.bias_lut, self.scale, self.temp_coef, self.temp_every, H,
-                                                  max_tile_tokens=rest[1], max_context=st.max_context())
+                                                  max_tile_tokens=rest[1], max_context=rest[2])
         else:                         # fp32, or head sizes off the tensor-core grid: the row kernel
             tiles, most = st.tiles_for(H, G)
             mixer_ops.biased_paged_attention(q, gate, cache.k_pool, cache.v_pool, st.block_tables, tiles, most,

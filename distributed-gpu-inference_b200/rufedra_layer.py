@@ -205,11 +205,11 @@ class KeyValueSelectiveMixer(nn.Module):
         if self.tensor_cores:
             tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
             args = (attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables)
-            kw = dict(window=self.window, gate=gate, max_context=st.max_context())
+            kw = dict(window=self.window, gate=gate)
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], max_context=tiles[2], **kw)
             if rest is not None:
-                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale,
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, max_tile_tokens=rest[1], max_context=rest[2],
                                                  heads_as_rows=self.rows and st.max_count() == 1, **kw)
         else:
             mixer_ops.mixed_paged_attention(attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,

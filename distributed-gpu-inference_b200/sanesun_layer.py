@@ -216,11 +216,11 @@ class LatentAttention(nn.Module):
         if self.tensor_cores:
             tiles, rest = st.attention_tiles(H, 1, r, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
             args = (o_lat.transpose(0, 1), q_lat.transpose(0, 1), cache.k_pool, cache.k_pool, st.block_tables)
-            kw = dict(gate=proj[:, c[2]:c[2] + H], max_context=st.max_context())
+            kw = dict(gate=proj[:, c[2]:c[2] + H])
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], max_context=tiles[2], **kw)
             if rest is not None:
-                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, max_tile_tokens=rest[1], max_context=rest[2], **kw)
         else:
             mixer_ops.mixed_paged_attention(o_lat.transpose(0, 1), q_lat.transpose(0, 1), cache.k_pool, cache.k_pool,
                                             st.block_tables, st.tok_row, st.tok_pos, self.scale,

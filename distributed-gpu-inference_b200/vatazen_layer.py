@@ -174,11 +174,11 @@ class LatentRotaryAttention(nn.Module):
         if self.tensor_cores:
             tiles, rest = st.attention_tiles(H, 1, r + dr, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
             args = (o_lat.transpose(0, 1), q_lat, cache.k_pool, cache.k_pool, st.block_tables)
-            kw = dict(sink=self.sink, window=self.window, max_context=st.max_context(), value_width=r)
+            kw = dict(sink=self.sink, window=self.window, value_width=r)
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], max_context=tiles[2], **kw)
             if rest is not None:    # single tokens: all heads read the same rows, so 16 heads share a tensor-core tile
-                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale,
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, max_tile_tokens=rest[1], max_context=rest[2],
                                                  heads_as_rows=H >= self.HEADS_AS_ROWS_FROM and st.max_count() == 1, **kw)
         else:
             mixer_ops.mixed_paged_attention(o_lat.transpose(0, 1), q_lat, cache.k_pool, cache.k_pool, st.block_tables,
@@ -239,11 +239,11 @@ class DifferentialAttention(nn.Module):
         if self.tensor_cores:
             tiles, rest = st.attention_tiles(2 * H, 2 * G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
             args = (maps, q.unflatten(1, (2 * H, dk)), k_pool, cache.v_pool, st.block_tables)
-            kw = dict(chunk=self.chunk, max_context=st.max_context(), value_div=2)
+            kw = dict(chunk=self.chunk, value_div=2)
             if tiles is not None:
-                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], **kw)
+                mixer_ops.tile_attention(*args, tiles[0], st.tok_pos, self.scale, rows=tiles[1], max_context=tiles[2], **kw)
             if rest is not None:
-                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, **kw)
+                mixer_ops.mixed_prompt_attention(*args, rest[0], st.tok_pos, self.scale, max_tile_tokens=rest[1], max_context=rest[2], **kw)
         else:
             mixer_ops.mixed_paged_attention(maps, q.unflatten(1, (2 * H, dk)), k_pool, cache.v_pool, st.block_tables,
                                             st.tok_row, st.tok_pos, self.scale, chunk=self.chunk, value_div=2)

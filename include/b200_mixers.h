@@ -72,13 +72,13 @@ int b200_biased_prompt_attn(void* out, const void* q, int64_t q_stride, const vo
                             const float* bias_lut, int lut_len, float scale, float temp_coef, int temp_every, int H, int G,
                             int dk, int dv, int block_size, int dtype, void* stream);
 /* The same; tiles of at most 16 rows (decoded tokens) whose longest context (max_context, a bound) exceeds b200_biased_attn_split_keys()
- * divide their keys over CTAs when workspace is given: fp32 [ceil(max_context / split keys)][n_tok][H][dv + 2], n_tok the packed rows. */
+ * divide their keys over CTAs when workspace is given: fp32 [ceil(max_context / split keys)][n_tiles][max_tile_tokens][H][dv + 2]. */
 int b200_biased_attn_split_keys(void);
 int b200_biased_prompt_attn_ext(void* out, const void* q, int64_t q_stride, const void* gate, int64_t gate_stride,
                             const void* k_pool, const void* v_pool, const int32_t* block_tables, int table_stride,
                             const int32_t* tiles, int n_tiles, int max_tile_tokens, const int32_t* tok_pos,
                             const float* bias_lut, int lut_len, float scale, float temp_coef, int temp_every, int H, int G,
-                            int dk, int dv, int block_size, int max_context, float* workspace, int n_tok, int dtype, void* stream);
+                            int dk, int dv, int block_size, int max_context, float* workspace, int dtype, void* stream);
 
 /* Gated linear recurrence per (sequence, head) over the sequence's tokens of this step, in order:
  *   q = silu(zq), f = lower + (1 - lower) * sigmoid(zf + f_bias), S <- diag(f) S + (1 - f) v^T, o = S^T q.
@@ -479,18 +479,28 @@ int b200_mixed_prompt_attn_ext2(void* out, int64_t out_tok_stride, int64_t out_h
                                 int keep_first, int chunk, const float* value_rot, int interleaved, int H, int G, int dk,
                                 int dv, int v_row, int v_div, int heads_as_rows, int out_f32, int block_size, int n_splits,
                                 float* workspace, int dtype, void* stream);
+/* b200_mixed_prompt_attn_ext2 whose workspace (n_splits > 1) holds ws_tile rows per tile, the most tokens a tile has (up to 16), instead of
+ * one per packed row: b200_mixed_prompt_attn_workspace with n_tiles * ws_tile for n_tok.  0: per packed row. */
+int b200_mixed_prompt_attn_ext3(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q,
+                                int64_t q_tok_stride, int64_t q_head_stride, const void* gate, int64_t gate_stride,
+                                int gate_per_channel, const void* k_pool, const void* v_pool, const int32_t* block_tables,
+                                int table_stride, const int32_t* tiles, int n_tiles, int ws_tile, const int32_t* tok_pos, int n_tok,
+                                const float* talk, const float* sink, float scale, float softcap, int window,
+                                int keep_first, int chunk, const float* value_rot, int interleaved, int H, int G, int dk,
+                                int dv, int v_row, int v_div, int heads_as_rows, int out_f32, int block_size, int n_splits,
+                                float* workspace, int dtype, void* stream);
 
 /* b200_mixed_prompt_attn_ext2 and b200_biased_prompt_attn for prompt portions on the fifth-generation tensor cores: tiles of up to
  * tile_rows / (H / G) tokens, tile_rows 128 or (dk <= 128) 256, as b200_tile_attn_rows picks for n_tokens tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
  * touched.  bias_lut fp32 [H][lut_len] with temp_coef / temp_every as in b200_biased_prompt_attn, or NULL.  The values are v_pool's
  * rows, or the first dv columns of the key rows when v_pool == k_pool.  n_splits > 1 divides the keys over as many CTAs and needs a
- * workspace fp32 [n_splits][n_tok][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte aligned query rows. */
+ * workspace fp32 [n_splits][n_tiles][tile_rows / (H / G)][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte aligned query rows. */
 int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bias, int dtype);
 int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens);
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows);
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,
-                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, int tile_rows, const int32_t* tok_pos, int n_tok,
+                   const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, int tile_rows, const int32_t* tok_pos,
                    const float* sink, const float* bias_lut, int lut_len, float scale, float softcap, float temp_coef, int temp_every,
                    int window, int keep_first, int chunk, int H, int G, int dk, int dv, int v_row, int v_div, int out_f32, int block_size,
                    int n_splits, float* workspace, int dtype, void* stream);

@@ -173,3 +173,23 @@ def test_weights_of_steep_rows(layout, spread):
         want = _reference(q, k_pool, v_pool, st, D, div, scale)
         # 1.4: a sample of 64 x H rows, and scores summed in fp32
         assert (out.to(F64) - want).norm() / want.norm() <= 1.4 * (5e-4 if spread < 10 else 3.3e-4)
+
+
+@pytest.mark.parametrize("layout,heads_as_rows", [(GROUPED, False), (WIDE, False), (WIDE, True), (LATENT, False), (PAIRED, False)])
+@pytest.mark.parametrize("most", [1, 16])
+def test_few_tokens_beside_a_prompt(layout, heads_as_rows, most):
+    """The 16-row kernel over part of a step, keys divided over CTAs: its workspace has a place for each of its tiles' rows."""
+    H, G, dk, dv, div = layout
+    q, k_pool, v_pool, st, _ = _case(layout, [(300, 0), (1, 2500), (150, 40), (1, 17)], 16, torch.bfloat16)
+    D, scale = dv or 256, dk ** -0.5
+    q = q.contiguous()
+    tiles = torch.tensor([(300, 1, 1), (451, 1, 3)], dtype=torch.int32, device="cuda")
+    out = torch.full((q.shape[0], H, D), 7.0, dtype=torch.bfloat16, device="cuda")
+    mixer_ops.mixed_prompt_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, scale, max_context=2501, value_width=D,
+                                     value_div=div, heads_as_rows=heads_as_rows, max_tile_tokens=most)
+    want = _reference(q, k_pool, v_pool, st, D, div, scale)
+    rows = torch.tensor([300, 451], device="cuda")
+    assert ((out[rows].to(F64) - want[rows]).norm(dim=(1, 2)) / want[rows].norm(dim=(1, 2))).max() <= 1.5 * 2.0 ** -8
+    left = torch.ones(q.shape[0], dtype=torch.bool, device="cuda")
+    left[rows] = False
+    assert (out[left] == 7).all()
