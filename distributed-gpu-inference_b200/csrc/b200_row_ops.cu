@@ -520,8 +520,10 @@ __global__ void __launch_bounds__(256) zero_blocks_kernel(const __grid_constant_
 // sums over the chunks (a warp per expert) -> where every chunk's pairs of every expert start: a stable counting sort.  The ids are
 // read twice and every output is written once; a radix sort of the same pairs is eight launches.  Ids outside 0 .. E - 1 sort behind
 // the last expert, so that order and where are permutations whatever the ids are: they index rows in the kernels that follow.
+// B200, 4 .. 48 experts, against a radix sort with its inverse and a search: 2048 pairs 5 .. 12 us against 29, 8192 14 .. 21 against 49, 16384 33 .. 44
+// against 52, 32768 83 .. 107 against 46 (a thread's ids are read one after the other): the library's sort from there on.
 constexpr int kOrderNT = 1024;
-constexpr int kOrderExperts = 48;
+constexpr int kOrderExperts = 48, kOrderPairs = 16384;
 __global__ void __launch_bounds__(kOrderNT)
 expert_order_kernel(int64_t* __restrict__ order, int64_t* __restrict__ where, int32_t* __restrict__ offsets, const int32_t* __restrict__ ids,
                     int n_pairs, int E) {
@@ -815,11 +817,11 @@ int b200_zero_blocks(void* const* pools, const int64_t* block_bytes, int n_pools
 }
 
 int b200_expert_order_supported(int64_t n_pairs, int n_experts) {
-  return n_pairs >= 0 && n_pairs <= (1 << 17) && n_experts > 0 && n_experts <= kOrderExperts;
+  return n_pairs >= 0 && n_pairs <= kOrderPairs && n_experts > 0 && n_experts <= kOrderExperts;
 }
 
 int b200_expert_order(int64_t* order, int64_t* where, int32_t* offsets, const int32_t* ids, int64_t n_pairs, int n_experts, void* stream) {
-  if (!b200_expert_order_supported(n_pairs, n_experts)) return fail(B200_ESHAPE, "b200_expert_order: up to %d pairs and %d experts", 1 << 17, kOrderExperts);
+  if (!b200_expert_order_supported(n_pairs, n_experts)) return fail(B200_ESHAPE, "b200_expert_order: up to %d pairs and %d experts", kOrderPairs, kOrderExperts);
   if (!offsets || (n_pairs > 0 && (!order || !where || !ids))) return fail(B200_EINVAL, "b200_expert_order: null pointer");
   const size_t smem = sizeof(int) * (static_cast<size_t>(n_experts + 1) * kOrderNT + n_experts + 2);
   if (smem > 48 * 1024) cudaFuncSetAttribute(expert_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));

@@ -276,7 +276,7 @@ def expert_order(ids: torch.Tensor, n_experts: int):
         raise TypeError("expert ids are contiguous int32")
     n, lib = ids.numel(), _lib_()
     if not lib.b200_expert_order_supported(n, int(n_experts)):     # more pairs or experts than the one-CTA sort holds
-        flat = torch.where((ids < 0) | (ids > n_experts), n_experts, ids).reshape(-1)
+        flat = ids.reshape(-1).clamp(-1, n_experts).remainder_(n_experts + 1)     # ids of no expert: n_experts
         sorted_ids, order = torch.sort(flat.to(torch.int16) if n_experts < 1 << 15 else flat, stable=True)
         where = torch.empty_like(order)
         where[order] = torch.arange(n, device=ids.device)

@@ -65,7 +65,7 @@ def test_head_norm(dv, dtype):
     assert _close(mixer_ops.head_rmsnorm(x, w, EPS), _unit(x.to(F64)) * w.to(F64), dtype)
 
 
-@pytest.mark.parametrize("n,top,E", [(1, 1, 1), (5, 3, 7), (512, 2, 8), (513, 2, 8), (4099, 2, 48), (1000, 4, 49), (70000, 2, 3)])
+@pytest.mark.parametrize("n,top,E", [(1, 1, 1), (5, 3, 7), (512, 2, 8), (513, 2, 8), (4099, 2, 48), (8192, 2, 5), (8193, 2, 5), (1000, 4, 49), (70000, 2, 3)])
 def test_expert_order(n, top, E):
     ids = torch.randint(0, E, (n, top), dtype=torch.int32, device="cuda")
     if E > 2:
