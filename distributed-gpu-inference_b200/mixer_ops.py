@@ -587,13 +587,26 @@ def tile_attention_supported(H: int, G: int, dk: int, dv: int, same_pool: bool, 
     return bool(_lib_().b200_tile_attn_supported(int(H), int(G), int(dk), int(dv), int(same_pool), int(bias), DTYPE_ID[dtype]))
 
 
-def tile_attention_from(H: int, G: int) -> int:
-    """Tokens from which a portion goes to ``tile_attention``: from two tokens and 8 rows (tokens x heads of a kv group) on.  Most of
-    the 128 rows of a product are padding then, but the walk is as long as one of the 16-row kernels and divides the keys over as
-    many CTAs (B200, 16 heads over 4: two tokens per sequence, 8 sequences at 4000: 44 us, 50 with biases, against 96 / 183 us in 16-row
-    tiles; 48 sequences: 197 / 255 against 346 / 225; nothing cached: level at launch latency; 32 tokens, 48 sequences at 1000: 61 / 75
-    against 262 / 207)."""
-    return max(2, 8 // (H // G))
+def tile_attention_from(H: int, G: int, bias: bool = False) -> int:
+    """Tokens from which a portion goes to ``tile_attention``.  Most of the 128 rows of a product are padding for a few tokens, but the walk
+    is as long as one of the 16-row kernels and divides the keys over CTAs.  Without biases: from two tokens and 8 rows (tokens x heads of
+    a kv group) on (B200, 16 heads over 4, two tokens per sequence, 16-row kernel against tile: 8 sequences at 500 32 and 21 us, at 2000 55
+    and 37; 48 sequences at 2000 177 and 79).  With biases the 16-row kernel divides the keys of its 16 rows over CTAs too and starts sooner,
+    so that it keeps them (as above: 8 sequences at 100 10 and 12 us, at 2000 23 and 42; 48 at 2000 85 and 113; from 17 rows on 145 and 46),
+    except where every head has its own keys (12 over 12, 8 sequences at 100: 15 and 11; 48 at 2000: 363 and 210)."""
+    rep = H // G
+    return 16 // rep + 1 if bias and rep > 1 else max(2, 8 // rep)
+
+
+# A portion of up to 16 tokens whose context is up to 32 keys is one step of the 16-row kernel's walk; the tile kernel's fixed beginning (tensor
+# memory, more warps, more shared memory) is hidden while an SM holds one or two of its CTAs.  B200, 16-row against tile, 8 tokens
+# each: 16 heads over 4, 20 sequences 7.6 and 7.1 us, 40: 7.7 and 8.9, 160: 15.6 and 20.3; 16 over 16, 12 sequences 11.2 and 8.9, 40: 11.4 and 20.0.
+TINY_TOKENS, TINY_CONTEXT = 16, 32
+
+
+def tiny_to_tiles(n_portions: int, H: int, G: int) -> bool:
+    """Whether ``n_portions`` of up to ``TINY_TOKENS`` tokens and ``TINY_CONTEXT`` keys still go to ``tile_attention``."""
+    return n_portions * G <= (148 if H // G > 2 else 296)
 
 
 @_timed

@@ -224,13 +224,13 @@ class RaggedBatchState:
         from . import mixer_ops
 
         cap = mixer_ops.attn_tile_tokens(1 << 20, num_heads, num_kv_heads)
-        return self._plan(("row", cap, below), cap, lambda count: below <= 0 or count < below)
+        return self._plan(("row", cap, below), cap, lambda count, _context: below <= 0 or count < below)
 
-    def prompt_tiles(self, at_least: int, cap: int, below: int = 0):
-        """Tiles of up to ``cap`` tokens over the portions of ``at_least`` tokens or more (and, ``below`` > 0, fewer than that)."""
-        return self._plan(("prompt", cap, at_least, below), cap, lambda count: count >= at_least and (below <= 0 or count < below))
+    def prompt_tiles(self, at_least: int, cap: int):
+        """Tiles of up to ``cap`` tokens over the portions of ``at_least`` tokens or more (tensor-core prompt kernel)."""
+        return self._plan(("prompt", cap, at_least), cap, lambda count, _context: count >= at_least)
 
-    def attention_tiles(self, H: int, G: int, dk: int, cap: int, whole: bool):
+    def attention_tiles(self, H: int, G: int, dk: int, cap: int, whole: bool, bias: bool = False):
         """How an attention layer of H heads over G kv heads of key size ``dk`` serves the step: ``(tiles, rest)``.  ``tiles``: the
         long portions for ``mixer_ops.tile_attention``, ``(tile list, rows per tile, longest context of these)`` (None: none, or not
         ``whole``: the layer's sizes are not served there); ``rest``: the others in tiles of up to ``cap`` tokens, ``(tile list, most
@@ -239,17 +239,26 @@ class RaggedBatchState:
 
         if self._tiles is None:
             self._tiles = {}
-        key = ("attention", H, G, dk, cap, whole)
+        key = ("attention", H, G, dk, cap, whole, bias)
         if key not in self._tiles:      # the step's layers of one layout share it
-            cut = mixer_ops.tile_attention_from(H, G) if whole else 1 << 30
-            long = [(count, past + count) for _first, count, _row, past in self.spans if count >= cut]
-            short = [past + count for _first, count, _row, past in self.spans if count < cut]
+            cut = mixer_ops.tile_attention_from(H, G, bias) if whole else 1 << 30
+
+            def tiny(count, context):
+                return count <= mixer_ops.TINY_TOKENS and context <= mixer_ops.TINY_CONTEXT
+
+            shapes = [(count, past + count) for _first, count, _row, past in self.spans]
+            leave = not bias and not mixer_ops.tiny_to_tiles(sum(n >= cut and tiny(n, t) for n, t in shapes), H, G)
+
+            def takes(count, context):
+                return count >= cut and not (leave and tiny(count, context))
+
+            long, short = [s for s in shapes if takes(*s)], [t for n, t in shapes if not takes(n, t)]
             tiles = rest = None
             if long:
-                rows = mixer_ops.tile_rows(H, G, dk, sum(c for c, _ in long))
-                tiles = self.prompt_tiles(cut, max(1, rows // (H // G)))[0], rows, max(t for _, t in long)
+                rows = mixer_ops.tile_rows(H, G, dk, sum(n for n, _ in long))
+                tiles = self._plan((key, "tiles"), max(1, rows // (H // G)), takes)[0], rows, max(t for _, t in long)
             if short:
-                rest = *self.prompt_tiles(1, cap, cut), max(short)
+                rest = *self._plan((key, "rest"), cap, lambda n, t: not takes(n, t)), max(short)
             self._tiles[key] = tiles, rest
         return self._tiles[key]
 
@@ -291,7 +300,7 @@ class RaggedBatchState:
         if key not in self._tiles:
             rows, most = [], 1
             for first, count, table_row, past in self.spans:
-                if not keep(count):
+                if not keep(count, past + count):
                     continue
                 for lo in range(0, count, cap):
                     n = min(cap, count - lo)

@@ -29,6 +29,25 @@ def test_portions_go_to_one_kernel_each_with_their_own_contexts():
     assert _step([]).attention_tiles(16, 4, 128, 16, True) == (None, None)
 
 
+@pytest.mark.parametrize("H,G,bias,cut", [(16, 4, False, 2), (16, 4, True, 5), (16, 16, False, 8), (16, 16, True, 8), (8, 4, True, 9), (16, 1, True, 2),
+                                          (6, 2, False, 2), (6, 2, True, 6)])
+def test_short_portions_stay_with_the_16_row_kernels(H, G, bias, cut):
+    assert mixer_ops.tile_attention_from(H, G, bias) == cut
+    st = _step([(cut - 1, 900), (cut, 900), (1, 40)])
+    tiles, rest = st.attention_tiles(H, G, 128, 16, True, bias)
+    assert [n for _f, n, _b in tiles[0].tolist()] == [cut] and sorted(n for _f, n, _b in rest[0].tolist()) == sorted([cut - 1, 1])
+
+
+@pytest.mark.parametrize("H,G,few,many", [(16, 4, 37, 38), (16, 16, 18, 19), (16, 8, 37, 38)])
+def test_many_tiny_prompts_stay_with_the_16_row_kernel(H, G, few, many):
+    for n, left in ((few, False), (many, True)):
+        st = _step([(16, 16)] * n + [(17, 15), (12, 21), (100, 0)])       # one token or key too many, and a prompt
+        tiles, rest = st.attention_tiles(H, G, 128, 16, True)
+        assert (rest is not None and len(rest[0]) == n and rest[2] == 32) == left
+        assert sum(c for _f, c, _b in tiles[0].tolist()) == 129 + (0 if left else 16 * n)
+        assert st.attention_tiles(H, G, 128, 16, True, bias=True)[1] is None      # biases: by rows alone
+
+
 class _Recorder:
     """Stands in for the library: sizes and rules are the real ones, launches are noted and not made."""
 
