@@ -104,5 +104,7 @@ __device__ __forceinline__ float row_logistic(float z) {
 }
 
 constexpr int kNumSMs = 148;  // B200
+constexpr int kMaxSmem = 227 * 1024;   // a CTA's shared memory: the limit to set where launches of one kernel differ in size (another
+                                       // thread's smaller one between setting it and the launch would make that fail)
 
 }  // namespace b200

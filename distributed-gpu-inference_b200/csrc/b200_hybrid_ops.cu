@@ -1316,6 +1316,8 @@ int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, c
     return fail(B200_ESHAPE, "b200_tile_attn: head layout (%d over %d, %d / %d) is not served", H, G, dk, dv);
   if (tile_rows != kTileRows && (tile_rows != 2 * kTileRows || dk > 128))
     return fail(B200_EINVAL, "b200_tile_attn: tiles have %d rows", kTileRows);
+  if (n_splits > 1 && sizeof(float) * static_cast<size_t>(H) * dv > kMaxSmem)
+    return fail(B200_ESHAPE, "b200_tile_attn: %d heads of %d are too many to merge", H, dv);
   if (n_tiles == 0) return 0;
   if (!out || !q || !k_pool || !v_pool || !block_tables || !tiles || !tok_pos || (n_splits > 1 && !workspace))
     return fail(B200_EINVAL, "b200_tile_attn: null pointer");
@@ -1341,11 +1343,10 @@ int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, c
              block_tables, table_stride, nullptr, tok_pos, nullptr, sink, scale, window, keep_first, 0,
              0, 0.0, H, G, dk, dv, block_size, softcap, chunk, v_row, v_div, 0, out_f32, 0, gate_per_channel ? dv : 0, per_tile};
   const size_t smem = sizeof(float) * static_cast<size_t>(H) * dv;
-  if (smem > 200 * 1024) return fail(B200_ESHAPE, "b200_tile_attn: %d heads of %d are too many to merge", H, dv);
   return hybrid_by_dtype(dtype, "b200_tile_attn", [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
     auto merge = attn_split_combine_kernel<T>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (smem > 48 * 1024) cudaFuncSetAttribute(merge, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     merge<<<dim3(n_tiles, per_tile), 256, smem, s>>>(M, tiles, workspace, n_splits, ws_rows, dv, nullptr);
     return check_launch("b200_tile_attn (merge)");
   });
@@ -1470,7 +1471,7 @@ int b200_mixed_prompt_attn_ext3(void* out, int64_t out_tok_stride, int64_t out_h
       const dim3 rows(n_tiles, ws_tile > 0 ? ws_tile : (n_tiles == n_tok ? 1 : kTcRows));
       const size_t smem_c = sizeof(float) * static_cast<size_t>(H_real) * dv;
       auto comb = attn_split_combine_kernel<T>;
-      if (smem_c > 48 * 1024) cudaFuncSetAttribute(comb, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_c));
+      if (smem_c > 48 * 1024) cudaFuncSetAttribute(comb, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
       comb<<<rows, 256, smem_c, s>>>(A, tiles, workspace, n_splits, ws_rows, plan.dv8 * 8, value_rot);
       return check_launch("b200_mixed_prompt_attn (merge)");
     }

@@ -824,7 +824,7 @@ int b200_expert_order(int64_t* order, int64_t* where, int32_t* offsets, const in
   if (!b200_expert_order_supported(n_pairs, n_experts)) return fail(B200_ESHAPE, "b200_expert_order: up to %d pairs and %d experts", kOrderPairs, kOrderExperts);
   if (!offsets || (n_pairs > 0 && (!order || !where || !ids))) return fail(B200_EINVAL, "b200_expert_order: null pointer");
   const size_t smem = sizeof(int) * (static_cast<size_t>(n_experts + 1) * kOrderNT + n_experts + 2);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(expert_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (smem > 48 * 1024) cudaFuncSetAttribute(expert_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   expert_order_kernel<<<1, kOrderNT, smem, static_cast<cudaStream_t>(stream)>>>(order, where, offsets, ids, static_cast<int>(n_pairs), n_experts);
   return check_launch("b200_expert_order");
 }

@@ -574,9 +574,9 @@ int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stre
   size_t smem = 1024 + P::kLut;
   if (BIAS) smem += sizeof(float) * P::kLuts * rep * (((P::kSoft / rep + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep));
   smem = std::max<size_t>(smem, P::kCtas == 2 ? 80 * 1024 : 120 * 1024);   // no more CTAs per SM than tensor memory has room for
-  if (smem > 227 * 1024) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
+  if (smem > kMaxSmem) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
   auto kern = tile_attn_kernel<T, DK, DV, ALIAS, BIAS, HALVES>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   kern<<<dim3(n_tiles, A.G, n_splits), P::kNT, smem, stream>>>(A);
   return check_launch("b200_tile_attn");
 }

@@ -640,6 +640,8 @@ def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_p
     if chunk > 0:
         seen = min(seen, chunk + 128)
     splits = lib.b200_tile_attn_splits(tiles.shape[0], (seen + 63) // 64, G, dk, int(rows)) if max_context > 0 else 1
+    if H * dv * 4 > 227 * 1024:     # more than the merge of splits holds
+        splits = 1
     ws = torch.empty((splits, tiles.shape[0] * (rows // (H // G)), H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
     rc = lib.b200_tile_attn(out.data_ptr(), out.stride(0), out.stride(1), q.data_ptr(), q.stride(0), q.stride(1), _ptr(gate),
                             _rows2(gate) if gate is not None else 0, per_channel, k_pool.data_ptr(), v_pool.data_ptr(),

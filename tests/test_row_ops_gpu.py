@@ -207,3 +207,29 @@ def test_causal_conv_portions(cuts, taps, dtype, C):
     y = sum(pad[i:i + sum(cuts)] * w[:, i].to(F64) for i in range(taps))
     tol = {torch.bfloat16: 2.0 ** -8, torch.float32: 4e-6}[dtype]       # taps products of up to ~ 10, then one rounding
     assert ((torch.cat(got).to(F64) - y * torch.sigmoid(y)).abs() <= tol * (y.abs() + 1)).all()
+
+
+def test_launches_of_different_sizes_from_two_threads():
+    """One kernel, dynamic shared memory by the call: another thread's smaller launch must not lower the limit in between."""
+    import threading
+
+    ids = {E: torch.randint(0, E, (500, 2), dtype=torch.int32, device="cuda") for E in (13, 24, 40, 48)}
+    torch.cuda.synchronize()      # the threads' streams start from here
+    failed = []
+
+    def work(sizes):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in range(1500):
+                    E = sizes[i % 2]
+                    last = mixer_ops.expert_order(ids[E], E)
+                assert torch.equal(last[0], torch.argsort(ids[E].reshape(-1), stable=True))
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in ((13, 48), (40, 24), (48, 40), (13, 24))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
