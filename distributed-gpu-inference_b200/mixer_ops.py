@@ -256,13 +256,22 @@ def sigmoid_topk(logits: torch.Tensor, top: int):
 
 
 def zero_blocks(pools, slots) -> None:
-    """Blocks ``slots`` (a host list) of every tensor of ``pools`` (contiguous ``[blocks, ...]``) set to zero in one launch."""
+    """Blocks ``slots`` (a host list) of every tensor of ``pools`` (contiguous ``[blocks, ...]`` on one device) set to zero in one launch
+    there, whatever the current device is."""
     import ctypes
 
     n, m = len(pools), len(slots)
-    rc = _lib_().b200_zero_blocks((ctypes.c_void_p * n)(*[p.data_ptr() for p in pools]),
-                                  (ctypes.c_int64 * n)(*[p.stride(0) * p.element_size() for p in pools]), n,
-                                  (ctypes.c_int32 * m)(*slots), m, _stream())
+    if not n or not m:
+        return
+    _need_cuda(*pools)
+    if any(p.device != pools[0].device or not p.is_contiguous() for p in pools):
+        raise ValueError("pools are contiguous and on one device")
+    if min(slots) < 0 or max(slots) >= min(p.shape[0] for p in pools):
+        raise IndexError(f"block slots {min(slots)} .. {max(slots)} of pools of {min(p.shape[0] for p in pools)} blocks")
+    with torch.cuda.device(pools[0].device):
+        rc = _lib_().b200_zero_blocks((ctypes.c_void_p * n)(*[p.data_ptr() for p in pools]),
+                                      (ctypes.c_int64 * n)(*[p.stride(0) * p.element_size() for p in pools]), n,
+                                      (ctypes.c_int32 * m)(*slots), m, _stream())
     _lib.check_mixers(rc, "b200_zero_blocks")
 
 
