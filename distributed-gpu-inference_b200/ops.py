@@ -141,13 +141,15 @@ def rope_kv_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch
 def rope_tables(pos: torch.Tensor, inv_freq: torch.Tensor, dtype: torch.dtype, scaling: float):
     """``cos, sin [*pos.shape, 2 * len(inv_freq)]`` for int64 positions and fp32 frequencies (``cos(float(pos) * f) * scaling``)."""
     _need_cuda(pos, inv_freq)
-    if pos.dtype != torch.int64 or inv_freq.dtype != torch.float32 or not pos.is_contiguous() or not inv_freq.is_contiguous():
-        raise ValueError("positions are contiguous int64, frequencies contiguous fp32")
+    if pos.dtype != torch.int64 or inv_freq.dtype != torch.float32 or not pos.is_contiguous() or not inv_freq.is_contiguous() \
+            or inv_freq.dim() != 1 or inv_freq.device != pos.device:
+        raise ValueError("positions are contiguous int64, frequencies a contiguous fp32 vector on the same device")
     D = 2 * inv_freq.numel()
     cos = torch.empty((*pos.shape, D), dtype=dtype, device=pos.device)
     sin = torch.empty_like(cos)
-    rc = _lib.load().b200_rope_tables(cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), inv_freq.data_ptr(), pos.numel(), D, float(scaling),
-                                      DTYPE_ID[dtype], _stream())
+    with torch.cuda.device(pos.device):      # the tables belong to the positions' device, whatever the current one is
+        rc = _lib.load().b200_rope_tables(cos.data_ptr(), sin.data_ptr(), pos.data_ptr(), inv_freq.data_ptr(), pos.numel(), D, float(scaling),
+                                          DTYPE_ID[dtype], _stream())
     _lib.check(rc, "b200_rope_tables")
     return cos, sin
 

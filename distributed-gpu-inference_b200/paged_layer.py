@@ -64,8 +64,9 @@ class RMSNorm(nn.Module):
 def rope_tables(position_ids: torch.Tensor, inv_freq: torch.Tensor, dtype: torch.dtype, scaling: float = 1.0):
     """``position_ids [B, T]`` → ``cos, sin [B, T, D]`` (fp32 math, times the RoPE variant's attention factor, cast to
     ``dtype`` — transformers' ``LlamaRotaryEmbedding.forward``)."""
-    if (position_ids.is_cuda and inv_freq.is_cuda and position_ids.dtype == torch.int64 and inv_freq.dtype == torch.float32
-            and position_ids.is_contiguous() and inv_freq.is_contiguous() and dtype in ops.DTYPE_ID):
+    if (position_ids.is_cuda and inv_freq.device == position_ids.device and position_ids.dim() == 2 and inv_freq.dim() == 1
+            and position_ids.dtype == torch.int64 and inv_freq.dtype == torch.float32 and position_ids.is_contiguous()
+            and inv_freq.is_contiguous() and inv_freq.numel() and not inv_freq.requires_grad and dtype in ops.DTYPE_ID):
         return ops.rope_tables(position_ids, inv_freq, dtype, scaling)
     freqs = position_ids.to(torch.float32)[:, :, None] * inv_freq[None, None, :]
     emb = torch.cat((freqs, freqs), dim=-1)

@@ -51,3 +51,12 @@ def test_zeroed_blocks_follow_their_pools(recorded):
 def test_zeroed_blocks_are_on_a_gpu():
     with pytest.raises(_lib.B200LibraryError):
         mixer_ops.zero_blocks([torch.ones(4, 2, 8)], [0])
+
+
+def test_rope_tables_follow_their_positions(recorded):
+    pos, freqs = torch.zeros(2, 3, dtype=torch.int64), torch.ones(4)
+    cos, sin = ops.rope_tables(pos, freqs, torch.bfloat16, 1.0)
+    assert cos.shape == sin.shape == (2, 3, 8) and recorded == [(torch.device("cpu"), "b200_rope_tables")]
+    for bad in (freqs.view(2, 2), freqs.double(), torch.ones(4, device="meta")):
+        with pytest.raises(ValueError):
+            ops.rope_tables(pos, bad, torch.bfloat16, 1.0)
