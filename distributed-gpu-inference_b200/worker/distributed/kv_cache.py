@@ -33,7 +33,7 @@ import time
 from collections import OrderedDict
 from dataclasses import dataclass, field  # noqa: F401
 from enum import Enum
-from typing import Callable, Any, Dict, Iterable, List, Optional, Sequence, Tuple
+from typing import Any, Callable, Dict, Iterable, List, Optional, Sequence, Tuple
 
 import torch
 
@@ -475,9 +475,14 @@ class KVCachePool:
             self._free_sequence_blocks(blocks)
             return
         dead: List[List[int]] = []
-        for cache, layer_blocks in zip(self._layer_caches, blocks):
-            dead.append([])
-            cache.free_blocks([blk.block_id for blk in layer_blocks], dead[-1])
+        try:
+            for cache, layer_blocks in zip(self._layer_caches, blocks):
+                dead.append([])
+                cache.free_blocks([blk.block_id for blk in layer_blocks], dead[-1])
+        finally:      # what was freed is zeroed also when a later layer fails
+            self._zero_rows(dead, zero)
+
+    def _zero_rows(self, dead: List[List[int]], zero: Callable) -> None:
         groups: Dict[Tuple[int, ...], List[torch.Tensor]] = {}
         for cache, slots in zip(self._layer_caches, dead):
             if slots:

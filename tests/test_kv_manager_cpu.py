@@ -197,3 +197,28 @@ def test_unreachable_tail_of_a_broken_chain_is_released_on_lookup():
     assert pool.layer(0).get_stats()["free_blocks"] == 6
     assert idx.match(toks)[0] == 1                      # only the head is usable ...
     assert pool.layer(0).get_stats()["free_blocks"] == 7  # ... and the block behind the gap was given back
+
+
+def test_rows_freed_before_a_failure_are_zeroed():
+    """One zeroing pass for all layers: when a later layer's hook raises, what was freed until then must not keep its contents."""
+    pool = kv.KVCachePool(3, 2, 8, 4, 8, device="cpu")
+    seq = pool.allocate_sequence(10)
+    slots = [[b.slot for b in layer] for layer in seq]
+    for c in pool._layer_caches:
+        c.key_pool.fill_(1.0)
+        c.value_pool.fill_(1.0)
+
+    def hook(_block_id):
+        raise RuntimeError("index is gone")
+
+    pool._layer_caches[1]._on_free = hook
+
+    def zero(pools, rows):
+        for p in pools:
+            p[list(rows)] = 0
+
+    with pytest.raises(RuntimeError):
+        pool.free_sequence(seq, zero)
+    first, second = pool._layer_caches[:2]
+    assert (first.key_pool[slots[0]] == 0).all() and (first.value_pool[slots[0]] == 0).all() and first.key_pool.sum() == 5 * 64
+    assert (second.key_pool[slots[1][:1]] == 0).all()      # the block whose hook raised had been freed
