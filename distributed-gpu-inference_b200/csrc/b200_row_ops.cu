@@ -730,8 +730,9 @@ int b200_value_prep_append(const void* k, int64_t k_stride, const void* v, int64
   if (n_tok < 0 || G <= 0 || dk <= 0 || dv <= 0 || block_size <= 0) return fail(B200_EINVAL, "b200_value_prep_append: bad sizes");
   if (n_tok == 0) return 0;
   if (!k || !v || !k_pool || !v_pool || !slot_mapping) return fail(B200_EINVAL, "b200_value_prep_append: null pointer");
-  const bool four = dk % 4 == 0 && dv % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 && all16(v_prev, v_keep, k_pool, v_pool) &&
-                    reinterpret_cast<uintptr_t>(k) % (4 * dtype_size(dtype)) == 0 && reinterpret_cast<uintptr_t>(v) % (4 * dtype_size(dtype)) == 0;
+  const int es = dtype_size(dtype);       // 0: refused below
+  const bool four = es && dk % 4 == 0 && dv % 4 == 0 && k_stride % 4 == 0 && v_stride % 4 == 0 && all16(v_prev, v_keep, k_pool, v_pool) &&
+                    reinterpret_cast<uintptr_t>(k) % (4 * es) == 0 && reinterpret_cast<uintptr_t>(v) % (4 * es) == 0;
   const unsigned grid = static_cast<unsigned>((static_cast<int64_t>(n_tok) * G + 7) / 8);
   return rows_by_dtype(dtype, "b200_value_prep_append", [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;

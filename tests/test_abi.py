@@ -143,3 +143,17 @@ int main(void) {
     assert res.returncode == 0, res.stderr
     run = subprocess.run([str(exe)], capture_output=True, text=True)
     assert run.returncode == 0 and run.stdout.startswith("ok "), (run.returncode, run.stdout, run.stderr)
+
+
+def test_unknown_types_are_refused_before_any_arithmetic_on_their_size():
+    """In a process of its own: a size of 0 in an alignment test would end it."""
+    import subprocess
+    import sys
+
+    code = ("from dgi_b200 import _lib\n"
+            "lib = _lib.load_mixers()\n"
+            "p = 4096\n"
+            "rc = lib.b200_value_prep_append(p, 64, p, 64, None, None, 0.0, 1e-5, p, p, p, 1, 1, 64, 64, 16, 4, 99, None)\n"
+            "print('rc', rc)\n")
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert out.returncode == 0 and "rc " in out.stdout and "rc 0" not in out.stdout, (out.returncode, out.stdout, out.stderr[-500:])
