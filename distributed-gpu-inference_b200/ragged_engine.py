@@ -40,7 +40,10 @@ class _Request:
 
 def _token_ids(toks: Sequence[int]) -> np.ndarray:
     if isinstance(toks, list) and type(toks[0]) is int:
-        return np.array(toks, dtype=np.int64)
+        try:
+            return np.array(toks, dtype=np.int64)
+        except (TypeError, ValueError):     # ints beside device scalars: one by one
+            pass
     return np.fromiter((int(t) for t in toks), dtype=np.int64, count=len(toks))
 
 

@@ -134,3 +134,24 @@ def test_oracle_recurrence_carries_its_state():
     assert torch.allclose(torch.cat([a, b]), whole, atol=1e-6) and torch.allclose(Sb, S, atol=1e-6)
     logits = R.forward(CFG, P.random_checkpoint(cfg, seed=2, bias_rows=10), [1, 2, 3, 4, 5, 6, 7])
     assert logits.shape == (7, 29) and torch.isfinite(logits).all()
+
+
+def test_token_ids_of_any_whole_numbers():
+    """Plain lists go through numpy at once; ints beside scalars that numpy cannot read (on a device) one by one."""
+    import numpy as np
+
+    from dgi_b200.ragged_engine import _token_ids
+
+    class OnDevice:
+        def __array__(self, *a, **k):
+            raise TypeError("can't convert a device tensor to numpy")
+
+        def __int__(self):
+            return 7
+
+    for toks, want in (([1, 2, 3], [1, 2, 3]), ([1, OnDevice(), np.int32(4), torch.tensor(9)], [1, 7, 4, 9]), ((5, OnDevice()), [5, 7]),
+                       (np.arange(3), [0, 1, 2]), (torch.tensor([4, 5]), [4, 5])):
+        got = _token_ids(toks)
+        assert got.dtype == np.int64 and got.tolist() == want
+    with pytest.raises((TypeError, ValueError)):
+        _token_ids([1, None])
