@@ -83,3 +83,27 @@ def test_recurrence_edges(rule, shape, dtype, odd):
     # fp32 sums of dk products, at most 65 tokens deep: 16 units of 2^-24 per level of a sum of 256 leave 1e-5 of the largest entry
     for x, y in ((got, want), (state, want_state)):
         assert (x.to(F64) - y).abs().max() <= 1e-5 * y.abs().max() + 1e-7
+
+
+@pytest.mark.parametrize("rule", ["gated", "retention"])
+def test_a_sequence_of_nans_stays_its_own(rule):
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    H, dk, dv, counts = 2, 64, 40, (19, 30, 1)
+    n = sum(counts)
+    x = torch.randn(n, H * (2 * dk + dv), generator=gen, device="cuda")
+    seqs = torch.tensor([(sum(counts[:i]), c, i, 0) for i, c in enumerate(counts)], dtype=torch.int32, device="cuda")
+    state = torch.randn(3, H, dk, dv, generator=gen, device="cuda")
+    bias, lower, decay = torch.randn(H * dk, generator=gen, device="cuda"), torch.rand(H * dk, device="cuda") * 0.9, torch.tensor([0.9, 0.99], device="cuda")
+
+    def run(rows):
+        s = state.clone()
+        a, b, v = rows[:, :H * dk], rows[:, H * dk:2 * H * dk], rows[:, 2 * H * dk:]
+        o = mixer_ops.gated_scan(a, b, v, bias, lower, s, seqs, H) if rule == "gated" else mixer_ops.retention_scan(a, b, v, decay, 0.1, s, seqs)
+        return o, s
+
+    bad = x.clone()
+    bad[19 + 11] = float("nan")
+    (o, s), (o0, s0) = run(bad), run(x)
+    clean = [t for t in range(n) if not 30 <= t < 49]
+    assert torch.equal(o[clean], o0[clean]) and torch.equal(s[[0, 2]], s0[[0, 2]])
+    assert o[30:49].isnan().all() and s[1].isnan().all()

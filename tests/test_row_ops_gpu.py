@@ -233,3 +233,47 @@ def test_launches_of_different_sizes_from_two_threads():
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("width", [64, 1032, 30])
+def test_rows_of_nans_and_infinities_stay_their_own(width, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(width)
+    x = torch.randn(6, width, generator=gen, device="cuda")
+    w = (torch.randn(width, generator=gen, device="cuda") * 0.2).to(dtype)
+    coef = torch.tensor([0.6, 0.3, -0.2, 0.05], device="cuda").to(dtype)
+    bad = x.clone()
+    bad[1], bad[3, 2] = float("nan"), float("inf")
+    rest = [0, 2, 4, 5]
+    for op in (lambda v: mixer_ops.offset_rmsnorm(v, w, EPS), lambda v: mixer_ops.polynorm(v.to(dtype), coef, EPS),
+               lambda v: mixer_ops.head_rmsnorm(v.view(6, 1, width), w, EPS).view(6, -1),
+               lambda v: mixer_ops.postnorm_residual(v.clone(), v.to(dtype), w, 0.7, EPS, w_next=w)):
+        got, want = op(bad), op(x)
+        assert torch.equal(got[rest], want[rest]) and got[1].isnan().all() and got[3, 2].isnan()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n", [1, 9, 1023, 1500])
+def test_routed_experts_of_every_path(n, dtype):
+    """The grouped kernel up to 2048 pairs, beyond it the library's grouped GEMM (bf16) or one GEMM per expert (fp16, fp32)."""
+    from dgi_b200.petipel_layer import SigmoidTopKMoE
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    E, W, ff, limit = 5, 64, 32, 1.5
+    lin = lambda o, i: (torch.randn(o, i, generator=gen, device="cuda") / i ** 0.5).to(dtype)  # noqa: E731
+    t = {f"e{e}.{k}": lin(*s) for e in range(E) for k, s in (("gate", (ff, W)), ("up", (ff, W)), ("down", (W, ff)))}
+    t["router"] = lin(E, W)
+    moe = SigmoidTopKMoE({"router": {"experts": E, "top": 2}, "expert": {"limit": limit}}, t, "cuda", dtype)
+    h = torch.randn(n, W, generator=gen, device="cuda").to(dtype)
+    z = h.to(F64) @ t["router"].to(F64).T
+    top, ids = z.topk(2, dim=1)
+    want = torch.zeros(n, W, dtype=F64, device="cuda")
+    for k in range(2):
+        for e in range(E):
+            rows = ids[:, k] == e
+            xs = (torch.sigmoid(top[rows, k])[:, None] * h[rows].to(F64)).to(dtype).to(F64)
+            g = (xs @ t[f"e{e}.gate"].to(F64).T).clamp(max=limit)
+            u = (xs @ t[f"e{e}.up"].to(F64).T).clamp(-limit, limit)
+            want[rows] += (g * torch.sigmoid(1.702 * g) * (u + 1)) @ t[f"e{e}.down"].to(F64).T
+    # inputs, products, activations and outputs of an expert each rounded once
+    assert (moe(h) - want).norm() / want.norm() <= {torch.float32: 2e-6}.get(dtype, 4 * TOL[dtype])

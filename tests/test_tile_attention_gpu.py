@@ -193,3 +193,50 @@ def test_few_tokens_beside_a_prompt(layout, heads_as_rows, most):
     left = torch.ones(q.shape[0], dtype=torch.bool, device="cuda")
     left[rows] = False
     assert (out[left] == 7).all()
+
+
+@pytest.mark.parametrize("layout,rows", [(GROUPED, 128), (GROUPED, 256), (LATENT, 128)])
+def test_a_query_of_nans_stays_its_own(layout, rows):
+    H, G, dk, dv, div = layout
+    q, k_pool, v_pool, st, _ = _case(layout, [(70, 300), (40, 0)], 16, torch.bfloat16)
+    D = dv or 256
+    tiles = st.prompt_tiles(2, rows // (H // G))[0]
+
+    def run(x):
+        out = torch.empty(q.shape[0], H, D, dtype=torch.bfloat16, device="cuda")
+        mixer_ops.tile_attention(out, x, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, 0.1, value_width=D, rows=rows)
+        return out
+
+    bad = q.clone()
+    bad[5, 1], bad[80] = float("nan"), float("inf")
+    got, want = run(bad), run(q)
+    hit = torch.zeros(q.shape[0], H, dtype=torch.bool, device="cuda")
+    hit[5, 1], hit[80] = True, True
+    assert torch.equal(got[~hit], want[~hit]) and got[hit].isnan().all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bias", [False, True])
+def test_a_sequence_alone_in_a_step_and_in_portions(bias, dtype):
+    """How the keys are divided, how many rows a tile has and which kernel takes a portion change with the step and the cut: a position's
+    result changes by roundings of its weights and of itself, no more; without key splits it is the same to the bit."""
+    H, G, dk, dv, _ = GROUPED
+    q, k_pool, v_pool, st, rnd = _case(GROUPED, [(200, 400)] + [(90, 0)] * 3, 16, dtype)
+    lut = rnd(H, 500) if bias else None
+
+    def run(tokens, max_context, rows=128):      # the first sequence's tokens in portions of these sizes
+        out = torch.full((q.shape[0], H, dk), 7.0, dtype=dtype, device="cuda")
+        first = 0
+        for n in tokens:
+            cap = rows // (H // G)
+            tiles = torch.tensor([(first + lo, min(cap, n - lo), 0) for lo in range(0, n, cap)], dtype=torch.int32, device="cuda")
+            mixer_ops.tile_attention(out, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, 0.09, rows=rows, bias_lut=lut,
+                                     max_context=max_context)
+            first += n
+        return out[:200]
+
+    whole = run([200], 0)
+    assert torch.equal(whole, run([200], 0, 256)) and torch.equal(whole, run([70, 1, 129], 0)) and torch.equal(whole, run([64] * 3 + [8], 0, 256))
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for other in (run([200], 600), run([70, 1, 129], 600), run([33, 167], 600, 256)):
+        assert (other.to(F64) - whole.to(F64)).norm() / whole.to(F64).norm() <= 2 * eps
