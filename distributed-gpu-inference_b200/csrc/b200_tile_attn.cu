@@ -16,15 +16,16 @@
 // another one issues the products; they meet at mbarriers only.  While the softmax works on tile i the tensor cores run S of tile i + 1 and
 // P V of tile i - 1.  256 rows per fetched tile halve what two CTAs of 128 rows per SM ask of L2 (32 KB per 64 keys and 4.2 MFLOP).
 //
-// Measured on B200 (bf16, 8 x 2048 tokens, 16 heads over 4 kv heads of 128): 212 us plain, 261 us with distance biases (the mma.sync
-// kernel: 1419), 141 us with a window of 512; latent 320 / 256, 4 x 1500 tokens of 16 heads behind 700, window 512: 142 us (417).
-// A tile of 64 keys x 256 rows takes about 2200 clocks: 1280 of the tensor cores (S with 64 columns is bound by reading Q from shared
-// memory), 1000 of exponentials (two warps per scheduler at four per clock), the copies 2000 (64 threads per pool); about a third of
-// the launch is the CTAs' beginnings and ends, which nothing covers with one CTA per SM.  128 rows and two CTAs: 242 and 321 us.
+// Measured on B200 (bf16, 8 x 2048 tokens, 16 heads over 4 kv heads of 128): 237 us plain, 274 us with distance biases (the mma.sync
+// kernel: 1419), 156 us with a window of 512; latent 320 / 256, 4 portions of up to 1500 tokens of 16 heads behind 700, window 512: 104 us
+// (417).  A tile of 64 keys x 256 rows took about 2200 clocks before O was rescaled at every new maximum (212 / 261 / 141 us): 1280 of the
+// tensor cores (S with 64 columns is bound by reading Q from shared memory), 1000 of exponentials (two warps per scheduler at four per
+// clock), the copies 2000 (64 threads per pool); about a third of the launch is the CTAs' beginnings and ends, which nothing covers
+// with one CTA per SM.  128 rows and two CTAs: 250 and 338 us.
 //
 // Weights are taken relative to the row's running maximum, so that the largest is 1 and loses nothing when P is rounded to the storage
-// type; O is scaled down whenever a row of the warp has a new maximum, after the tile's weights are written, so that P V of the tile before
-// runs under the exponentials.  (Scaling only once the maximum has grown by 2^8 leaves the largest weight anywhere in 1 .. 256, rounded
+// type; O is scaled down whenever a row of the warp has a new maximum (with the tile's weights already written, so that P V of the tile
+// before runs under the exponentials).  (Scaling only once the maximum has grown by 2^8 leaves the largest weight anywhere in 1 .. 256, rounded
 // like any other while the sum is not: scores of standard deviation 4 and 10 over 2048 keys came out 0.0013 and 0.0011 from float64 before
 // the output's own rounding, 0.0005 and 0.0003 this way.)  A latent cache (values = the first DV columns of the key rows) is fetched once
 // and read through both descriptors.
@@ -135,6 +136,14 @@ __device__ __forceinline__ void tm_ld32(float (&r)[32], uint32_t addr) {
         "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]), "=r"(u[19]),
         "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]), "=r"(u[28]), "=r"(u[29]),
         "=r"(u[30]), "=r"(u[31])
+      : "r"(addr));
+}
+__device__ __forceinline__ void tm_ld16(float (&r)[16], uint32_t addr) {
+  uint32_t* u = reinterpret_cast<uint32_t*>(r);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]),
+        "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
       : "r"(addr));
 }
 __device__ __forceinline__ void tm_st16(uint32_t addr, const uint32_t (&u)[16]) {
@@ -415,6 +424,30 @@ tile_attn_kernel(const TileAttn A) {
     float m_ref = -INFINITY, l = 0.f;       // in powers of two; -inf until the row sees a key
     bool ok = true;
 
+    // O of the tiles before tile i to the new maximum where a row of the warp has one: after the tile's weights, with P V of the tile before
+    // under them, or (kEarly) before, where the registers do not hold the factor as well (96 with two CTAs per SM, biases: 378 -> 338 us
+    // of 8 x 2048 tokens; the other forms lose 3 .. 10% that way)
+    constexpr bool kEarly = BIAS && HALVES == 1;
+    auto rescale = [&](int i, bool grow, float corr) {
+      if (i == 0 || !__any_sync(0xffffffffu, grow)) return;
+      ok = values_done(i - 1) && ok;
+      tc_fence_after();
+      constexpr int kW = kEarly ? 16 : 32;
+#pragma unroll 1
+      for (int c = 0; c < DV; c += kW) {
+        float o[kW];
+        if constexpr (kEarly) tm_ld16(o, tm_row + P::kO + c);
+        else tm_ld32(o, tm_row + P::kO + c);
+        tc_wait_ld();
+#pragma unroll
+        for (int x = 0; x < kW; x += 16) {
+          uint32_t w[16];
+#pragma unroll
+          for (int u = 0; u < 16; ++u) w[u] = __float_as_uint(o[x + u] * corr);
+          tm_st16(tm_row + P::kO + c + x, w);
+        }
+      }
+    };
     for (int i = 0; i < mine; ++i) {
       const int j0 = key0(i);
       ok = bar_wait(my_s + 8 * (i & 1), (i >> 1) & 1, dead) && ok;
@@ -450,6 +483,7 @@ tile_attn_kernel(const TileAttn A) {
       const bool grow = m_new > m_ref;
       const float corr = grow ? exp2_fast(m_ref - m_new) : 1.0f;      // 0 where nothing was seen before
       if (grow) m_ref = m_new;
+      if constexpr (kEarly) rescale(i, grow, corr);
       const f32x2 kk = both(k2), mm = both(m_ref == -INFINITY ? 0.f : -m_ref);     // a row that sees no key yet keeps weights 0
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -468,23 +502,7 @@ tile_attn_kernel(const TileAttn A) {
         tm_st16(tm_row + (i & 1) * kKeys + x * 16, w);
       }
       l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
-      if (i > 0 && __any_sync(0xffffffffu, grow)) {       // after the weights: P V of the tile before runs under them
-        ok = values_done(i - 1) && ok;
-        tc_fence_after();
-#pragma unroll 1
-        for (int c = 0; c < DV; c += 32) {
-          float o[32];
-          tm_ld32(o, tm_row + P::kO + c);
-          tc_wait_ld();
-#pragma unroll
-          for (int x = 0; x < 2; ++x) {
-            uint32_t w[16];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) w[u] = __float_as_uint(o[16 * x + u] * corr);
-            tm_st16(tm_row + P::kO + c + 16 * x, w);
-          }
-        }
-      }
+      if constexpr (!kEarly) rescale(i, grow, corr);
       tc_wait_st();
       tc_fence_before();
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(my_p + 8 * (i & 1)) : "memory");
@@ -609,8 +627,8 @@ bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, in
 }
 
 // 256 rows share a fetched key tile, but only one such CTA runs per SM and nothing covers its beginning and end: worth it from three
-// rounds of them on (8 x 2048 tokens, 16 heads over 4, 7 rounds: 209 us against 242 with 128 rows and two CTAs per SM; 5 portions of up
-// to 1024 tokens under a window of 512, 1.4 rounds: 79 against 63).
+// rounds of them on (8 x 2048 tokens, 16 heads over 4, 7 rounds: 237 us against 250 with 128 rows and two CTAs per SM, with biases 273 against
+// 338; 5 portions of up to 1024 tokens under a window of 512, 1.4 rounds: 41.9 against 40.3, with a soft cap 79 against 77).
 int tile_attn_rows(int rep, int G, int dk, int n_tokens) {
   const int64_t ctas = static_cast<int64_t>(n_tokens) * rep / (2 * kTileRows) * G;
   return dk <= 128 && ctas >= 3 * kNumSMs ? 2 * kTileRows : kTileRows;
