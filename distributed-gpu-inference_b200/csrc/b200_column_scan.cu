@@ -525,7 +525,8 @@ column_scan_kernel(const ColArgs A) {
 // with how many CTAs of two an SM gets (B200, 64 x 128 states, ns per token, gated / delta / retention; two against four columns): one
 // 134 / 193 / 102 against 157 / 245 / 137, two 175 / 257 / 141 against 158 / 245 / 136, three 241 / 366 / 190 against 246 / 374 / 213, four
 // 349 / 490 / 270 against 246 / 374 / 213, seven 555 / 805 / 434 against 469 / 721 / 405 (eight columns: 439 / 770 / 399, and 273 / 425 / 257
-// from the first CTA on).  Key sizes whose tile would not fit the registers take fewer.
+// from the first CTA on).  Keys of 65 .. 128 take four from two CTAs on without a table of their own; sizes whose tile would not fit the
+// registers take fewer.
 template <int RULE, typename T, int DK>
 int launch_columns(ColArgs& A, int n_seqs, cudaStream_t stream, const char* name) {
   auto go = [&](auto cols) {

@@ -11,8 +11,10 @@
 //
 // Every constant of a design (eps, multipliers, temperatures, limits, table sizes) is a parameter.  Scores, softmax,
 // norms, gates of the recurrence, the state and the residual are fp32 whatever the storage dtype T is.  Summation
-// orders depend only on a token's own position and sizes, never on how a batch was cut, so a position's result does
-// not change with its neighbours in the batch.
+// orders of the fp32 attention and of the recurrence depend only on a token's own position and sizes, never on how a batch was
+// cut, so a position's result does not change with its neighbours in the batch.  The 16-bit attention has one order for launches
+// of up to 16 rows per tile (decoded tokens: key ranges at fixed multiples) and one for longer tiles; which a token gets follows from
+// its portion and, where the prompt portions of a step share the launch, from those: rounding level.
 #include <algorithm>
 #include <type_traits>
 

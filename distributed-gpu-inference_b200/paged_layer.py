@@ -269,8 +269,10 @@ class RaggedBatchState:
         GPU as they are (``ctas_per_seq``: CTAs the scan launches per sequence; 0 = unknown, always cut).  ``.segs`` int32
         ``[n, 4]`` are scan rows (first row, count, scratch slot = the segment's index, fresh = 1), ``.parents`` int32
         ``[m, 4]`` = (first segment, segments, state slot, fresh), ``.direct`` the scan rows of the step's other sequences
-        (or None).  Measured on B200: the segments pay below about one CTA per SM (a lone 2048-token prompt: 3.5 x), and
-        cost time once the token-by-token launch has two CTAs per SM."""
+        (or None).  The lines at 64 and 160 CTAs were drawn with an older token-by-token kernel.  Measured on B200 with today's
+        (64 x 128 states, equal portions; token by token / segments of 128 / of 256 tokens, us): 16 CTAs, 2048 tokens 184 / 68 / 94,
+        1024 94 / 54 / 92, 512 49 / 51 / 89; 64 CTAs 186 / 135 / 149, 95 / 88 / 115, 49 / 67 / 94; 96 CTAs 186 / 205 / 191, 95 / 113 / 130,
+        49 / 77 / 112; 160 CTAs 255 / 341 / 289, 130 / 163 / 184, 67 / 107 / 128: segments pay up to about 64 CTAs and from about 1000 tokens."""
         if self.scan_host is None or not any(count >= at_least for _f, count, _s, _fr in self.scan_host):
             return None
         ctas = ctas_per_seq * len(self.scan_host)

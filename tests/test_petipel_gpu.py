@@ -616,7 +616,7 @@ def test_routed_feed_forward_16_bit_takes_the_grouped_kernel():
     h = torch.randn(50, W, generator=g).bfloat16()
     ref = R.moe_ff(h.float(), {k: v.float() for k, v in t.items()}, spec)
     got = mod(h.to(DEV)).cpu()
-    mod.GROUPED_MAX_ROWS = 0                      # the per-expert path on the same input
+    mod.GROUPED_MAX_ROWS = 0                      # the library's path on the same input (its grouped GEMM in bf16)
     loops = mod(h.to(DEV)).cpu()
     close(got, ref, 2e-2)
     close(loops, ref, 2e-2)
