@@ -609,13 +609,16 @@ def tile_attention_from(H: int, G: int, bias: bool = False) -> int:
 
 # A portion of up to 16 tokens whose context is up to 32 keys is one step of the 16-row kernel's walk; the tile kernel's fixed beginning (tensor
 # memory, more warps, more shared memory) is hidden while an SM holds one or two of its CTAs.  B200, 16-row against tile, 8 tokens
-# each: 16 heads over 4, 20 sequences 7.6 and 7.1 us, 40: 7.7 and 8.9, 160: 15.6 and 20.3; 16 over 16, 12 sequences 11.2 and 8.9, 40: 11.4 and 20.0.
+# each: 16 heads over 4, 20 sequences 7.6 and 7.1 us, 40: 7.7 and 8.9, 160: 15.6 and 20.3; 16 over 16, 12 sequences 11.2 and 8.9, 40: 11.4
+# and 20.0.  With more heads per kv head, or one kv head, the tile kernel has as few CTAs and stays level or ahead: 16 over 2, 200 sequences
+# 14.7 and 15.1; 16 over 1 19.1 and 11.2; latent 320 of 16 heads 34.9 and 25.9.
 TINY_TOKENS, TINY_CONTEXT = 16, 32
 
 
 def tiny_to_tiles(n_portions: int, H: int, G: int) -> bool:
     """Whether ``n_portions`` of up to ``TINY_TOKENS`` tokens and ``TINY_CONTEXT`` keys still go to ``tile_attention``."""
-    return n_portions * G <= (148 if H // G > 2 else 296)
+    rep = H // G
+    return G == 1 or rep > 4 or n_portions * G <= (148 if rep > 2 else 296)
 
 
 @_timed

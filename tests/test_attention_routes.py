@@ -48,6 +48,11 @@ def test_many_tiny_prompts_stay_with_the_16_row_kernel(H, G, few, many):
         assert st.attention_tiles(H, G, 128, 16, True, bias=True)[1] is None      # biases: by rows alone
 
 
+@pytest.mark.parametrize("H,G", [(16, 1), (4, 1), (16, 2), (1, 1)])
+def test_layouts_of_few_tiles_take_tiny_prompts_in_tiles(H, G):
+    assert mixer_ops.tiny_to_tiles(1000, H, G)
+
+
 class _Recorder:
     """Stands in for the library: sizes and rules are the real ones, launches are noted and not made."""
 
