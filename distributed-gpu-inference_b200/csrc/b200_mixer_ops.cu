@@ -952,7 +952,7 @@ int b200_gated_scan(float* o_raw, const void* zq, const void* zf, const void* v,
   if (n_seqs < 0 || H <= 0 || dk <= 0 || dv <= 0) return fail(B200_EINVAL, "b200_gated_scan: bad sizes");
   if (n_seqs == 0) return 0;
   if (!o_raw || !zq || !zf || !v || !f_bias || !lower || !state || !seqs) return fail(B200_EINVAL, "b200_gated_scan: null pointer");
-  (void)max_count;   // one kernel for portions of any length
+  (void)max_count;   // one kernel for portions of any length (b200_split_scan: in chunks)
   if (2 * dk + 32 > 1024) return fail(B200_ESHAPE, "b200_gated_scan: key size %d beyond 496", dk);
   return gated_column_scan(o_raw, ScanRows{zq, zf, v, in_stride}, f_bias, lower, state, seqs, ScanShape{n_seqs, H, H, dk, dv}, dtype,
                            static_cast<cudaStream_t>(stream));

@@ -190,12 +190,39 @@ def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[t
     _lib.check_mixers(rc, "b200_biased_prompt_attn")
 
 
+# Tokens of a step's longest portion from which the recurrences (gated, delta, retention) run in chunks on the tensor cores.  B200, bf16,
+# 64 x 128 states, us token by token / in chunks: 8 x 96 tokens of 4 heads gated 15.5 / 15.9, delta 21.4 / 21.5, retention 12.3 / 14.8;
+# 192 tokens 27.0 / 21.8, 38.7 / 30.4, 21.0 / 20.4; 2048 tokens 248 / 151, 379 / 233, 186 / 145; 8 x 64 tokens of 16 heads 20.3 / 18.8,
+# 29.8 / 27.0, 17.9 / 17.3.
+SPLIT_SCAN_FROM = (96, 96, 160)
+SPLIT_SCAN_WORKSPACE = 1 << 30      # bytes of chunk operands at most (one head's if that is more); the heads go in groups beyond
+
+
+def split_scan_takes(rule: int, max_count: int, dk: int, dtype: torch.dtype) -> bool:
+    """Whether a step whose longest portion has ``max_count`` tokens runs in chunks (rule 0: gated, 1: delta, 2: retention)."""
+    return max_count >= SPLIT_SCAN_FROM[rule] and bool(_lib_().b200_split_scan_supported(dk, DTYPE_ID[dtype]))
+
+
+def _split_scan(rule: int, o, q, k, v, stride: int, beta, a, bias, rate, decay, per_channel: bool, state, seqs, G: int, eps: float,
+                scale: float) -> None:
+    """``b200_split_scan`` into ``o``; ``beta`` and ``a`` are (tensor or None, row stride)."""
+    _, H, dk, dv = state.shape
+    lib, n, n_seqs = _lib_(), q.shape[0], seqs.shape[0]
+    one = lib.b200_split_scan_workspace(rule, n, n_seqs, 1)
+    ws = torch.empty(max(one, min(one * H, SPLIT_SCAN_WORKSPACE)), dtype=torch.uint8, device=q.device)
+    rc = lib.b200_split_scan(rule, o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), stride, _ptr(beta[0]), beta[1], _ptr(a[0]), a[1],
+                             _ptr(bias), _ptr(rate), _ptr(decay), int(per_channel), state.data_ptr(), seqs.data_ptr(), n_seqs, n, H, G, dk,
+                             dv, float(eps), float(scale), ws.data_ptr(), ws.numel(), DTYPE_ID[q.dtype], _stream())
+    _lib.check_mixers(rc, "b200_split_scan")
+
+
 @_timed
 def gated_scan(zq: torch.Tensor, zf: torch.Tensor, v: torch.Tensor, f_bias: torch.Tensor, lower: torch.Tensor,
                state: torch.Tensor, seqs: torch.Tensor, H: int, max_count: int = 1 << 20) -> torch.Tensor:
     """Gated linear recurrence over each sequence's tokens; ``state`` fp32 ``[slots, H, dk, dv]`` is read (unless the
     sequence is fresh) and written back.  ``zq / zf [n, H*dk]``, ``v [n, H*dv]`` are column slices of ONE projection
-    (same row stride).  ``max_count``: the largest token count in ``seqs`` (picks the kernel; a hint, not a bound).
+    (same row stride).  ``max_count``: the largest token count in ``seqs`` (picks the kernel; a hint, not a bound): 16-bit steps with a
+    portion of ``SPLIT_SCAN_FROM`` tokens or more and keys of up to 64 run in chunks on the tensor cores, others token by token.
     Returns the raw read-outs, fp32 ``[n, H, dv]``."""
     _need_cuda(zq, zf, v, state, seqs)
     n = zq.shape[0]
@@ -210,6 +237,9 @@ def gated_scan(zq: torch.Tensor, zf: torch.Tensor, v: torch.Tensor, f_bias: torc
     if seqs.dtype != torch.int32 or seqs.dim() != 2 or seqs.shape[1] != 4 or not seqs.is_contiguous():
         raise ValueError("seqs must be contiguous int32 [n_seqs, 4]")
     o = torch.empty((n, H, dv), dtype=torch.float32, device=zq.device)
+    if split_scan_takes(0, min(max_count, n), dk, zq.dtype):
+        _split_scan(0, o, zq, zf, v, stride, (None, 0), (None, 0), f_bias, lower, None, False, state, seqs, H, 0.0, 0.0)
+        return o
     rc = _lib_().b200_gated_scan(o.data_ptr(), zq.data_ptr(), zf.data_ptr(), v.data_ptr(), stride, f_bias.data_ptr(),
                                  lower.data_ptr(), state.data_ptr(), seqs.data_ptr(), seqs.shape[0], int(max_count), H, dk, dv,
                                  DTYPE_ID[zq.dtype], _stream())
@@ -696,8 +726,9 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_logit: to
     ``[H]``) over each sequence's tokens; ``state`` fp32 ``[slots, H, dk, dv]``
     is read (unless the sequence is fresh) and written back.  ``q / k [n, G*dk]`` and ``v [n, H*dv]`` are column
     slices of ONE tensor (same row stride), ``beta_logit [n, H]``.  Returns fp32 ``[n, H, dv]``.  ``max_count``: the
-    largest token count in ``seqs`` (0: unknown); with one decay per head it picks the kernel: steps of single tokens, bf16
-    steps with a portion of ``CHUNK_SCAN_FROM`` tokens or more in chunks on the tensor cores, others token by token."""
+    largest token count in ``seqs`` (0: unknown), picks the kernel.  One decay per head: steps of single tokens, and bf16 steps with a
+    portion of ``CHUNK_SCAN_FROM`` tokens or more in chunks of 64 on the tensor cores; otherwise, 16-bit steps with a portion of
+    ``SPLIT_SCAN_FROM`` tokens or more and keys of up to 64 in chunks of 16 at fp32 precision; others token by token."""
     _need_cuda(q, k, v, beta_logit, a_logit, dt_bias, a_log, state, seqs)
     n = q.shape[0]
     _, H, dk, dv = state.shape
@@ -727,6 +758,9 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_logit: to
         rc = lib.b200_delta_chunk_scan(*head, state.data_ptr(), seqs.data_ptr(), n_seqs, int(max_count), *tail, ws.data_ptr(), dt,
                                        _stream())
         _lib.check_mixers(rc, "b200_delta_chunk_scan")
+    elif split_scan_takes(1, min(max_count, n), dk, q.dtype):
+        _split_scan(1, o, q, k, v, stride, (beta_logit, _rows2(beta_logit)), (a_logit, _rows2(a_logit)), dt_bias, a_log, None,
+                    not one_decay, state, seqs, G, unit_eps, q_scale)
     else:
         rc = lib.b200_delta_scan_ext(*head, int(not one_decay), state.data_ptr(), seqs.data_ptr(), n_seqs, *tail, dt, _stream())
         _lib.check_mixers(rc, "b200_delta_scan")
@@ -794,7 +828,7 @@ def qknorm_rotary_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_no
 
 @_timed
 def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, k_scale: float,
-                   state: torch.Tensor, seqs: torch.Tensor, plan=None) -> torch.Tensor:
+                   state: torch.Tensor, seqs: torch.Tensor, plan=None, max_count: int = 0) -> torch.Tensor:
     """Fixed-decay linear attention over each sequence's tokens: ``S <- decay[h] S + (k_scale k) v^T``, ``o = S^T q``;
     ``state`` fp32 ``[slots, H, dk, dv]`` is read (unless the sequence is fresh) and written back.  ``q / k [n, H*dk]``
     and ``v [n, H*dv]`` are column slices of ONE tensor.  Returns fp32 ``[n, H, dv]``.
@@ -802,7 +836,8 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
     ``plan`` (``RaggedBatchState.scan_plan()``; None: every sequence runs token by token in one launch) names the long
     portions of the step as parallel segments: each segment runs as a fresh sequence against a scratch state, one launch
     chains the segments' end states into the state at every segment's start and the sequence's final state, and one adds
-    what each token missed, ``decay^(t - t0 + 1) P^T q_t``.  Short sequences of the same step run as before."""
+    what each token missed, ``decay^(t - t0 + 1) P^T q_t``.  Short sequences of the same step run as before.  Without a plan, ``max_count``
+    (the largest token count in ``seqs``, 0: unknown) picks the kernel as in ``gated_scan``."""
     _need_cuda(q, k, v, decay, state, seqs)
     n = q.shape[0]
     _, H, dk, dv = state.shape
@@ -817,6 +852,9 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
         raise ValueError("decay is contiguous fp32 [H]")
     _check_seqs(seqs)
     o = torch.empty((n, H, dv), dtype=torch.float32, device=q.device)
+    if plan is None and split_scan_takes(2, min(max_count, n), dk, q.dtype):
+        _split_scan(2, o, q, k, v, stride, (None, 0), (None, 0), None, None, decay, False, state, seqs, H, 0.0, k_scale)
+        return o
     lib, dt, st = _lib_(), DTYPE_ID[q.dtype], _stream()
 
     def scan(into: torch.Tensor, table: torch.Tensor) -> None:

@@ -257,12 +257,13 @@ class ChannelDeltaMixer(nn.Module):
         H, G, dk, dv, c = self.H, self.G, self.dk, self.dv, self.cuts
         state, tail = cache.rstate
         proj = F.linear(h, self.w_in)
-        qkv = mixer_ops.causal_conv_silu(proj[:, :self.n_conv], self.w_conv, tail, st.scan_seqs,
-                                         max_count=max(sp[1] for sp in st.spans))
+        longest = st.max_count()
+        qkv = mixer_ops.causal_conv_silu(proj[:, :self.n_conv], self.w_conv, tail, st.scan_seqs, max_count=longest)
         a_logit = F.linear(proj[:, c[2]:c[2] + self.ra], self.w_a2)
         gate = F.linear(proj[:, c[3]:c[3] + self.rg], self.w_g2)
         o = mixer_ops.delta_scan(qkv[:, :G * dk], qkv[:, G * dk:2 * G * dk], qkv[:, 2 * G * dk:], proj[:, c[1]:c[1] + H],
-                                 a_logit, self.dt_bias, self.a_log, state, st.scan_seqs, G, UNIT_NORM_EPS, dk ** -0.5)
+                                 a_logit, self.dt_bias, self.a_log, state, st.scan_seqs, G, UNIT_NORM_EPS, dk ** -0.5,
+                                 max_count=longest)
         return F.linear(mixer_ops.head_rmsnorm_gated(o, self.norm_w, gate, self.eps), self.w_o)
 
 

@@ -523,6 +523,18 @@ int b200_delta_scan_ext(float* o_raw, const void* q, const void* k, const void* 
                         int per_channel, float* state, const int32_t* seqs, int n_seqs, int H, int G, int dk, int dv,
                         float unit_eps, float q_scale, int dtype, void* stream);
 
+/* The recurrences of b200_gated_scan (rule 0), b200_delta_scan_ext (1) and b200_retention_scan (2) in chunks of 16 tokens on the tensor
+ * cores at fp32 precision, for 16-bit inputs and key sizes up to 64: arguments as there (k: the forget gate's logits for rule 0, whose
+ * bias and rate are f_bias and lower; bias and rate of rule 1 are dt_bias and a_log; scale: q_scale or k_scale; what a rule does not
+ * have may be NULL or 0).  n_tok: at least the tokens that seqs names.  workspace: b200_split_scan_workspace(rule, n_tok, n_seqs,
+ * heads) bytes serve `heads` heads at once, 16-byte aligned; with fewer than H heads' the heads go in groups, one head's is needed. */
+int b200_split_scan_supported(int dk, int dtype);
+size_t b200_split_scan_workspace(int rule, int n_tok, int n_seqs, int heads);
+int b200_split_scan(int rule, float* o_raw, const void* q, const void* k, const void* v, int64_t in_stride, const void* beta_logit,
+                    int64_t beta_stride, const void* a_logit, int64_t a_stride, const void* bias, const void* rate, const float* decay,
+                    int per_channel, float* state, const int32_t* seqs, int n_seqs, int n_tok, int H, int G, int dk, int dv,
+                    float unit_eps, float scale, void* workspace, size_t workspace_bytes, int dtype, void* stream);
+
 /* ---- the delta rule with one decay per head in chunks, and per-channel selective state spaces ---------------------- */
 
 /* b200_delta_scan_ext with per_channel = 0 in chunks of 64 tokens on the tensor cores (bf16, dk <= 256): q, k and v enter the
