@@ -77,6 +77,15 @@ SIGNATURES = {
     "b200_argmax_rows_keys": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, c_void_p]),
     "b200_argmax_keys_decode": (c_int, [c_void_p, c_void_p, c_int64, c_void_p]),
     "b200_rope_tables": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_float, c_int, c_void_p]),
+    "b200_llama_decode_layer_supported": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int]),
+    "b200_llama_decode_layer_workspace": (
+        c_size_t, [c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int]),
+    "b200_llama_decode_layer": (
+        c_int,
+        [c_void_p, c_void_p, c_int64, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
+         c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
+         c_int, c_int, c_int, c_int, c_int64, c_int, c_int, c_void_p, c_size_t, c_int, c_uint, c_void_p],
+    ),
     "b200_silu_mul": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int64, c_int64, c_int, c_void_p]),
     "b200_kv_gather_dense": (
         c_int,

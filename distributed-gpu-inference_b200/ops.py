@@ -371,6 +371,66 @@ def rope_append_decode_attention(
     return out
 
 
+def one_call_batch(width: int, ff: int) -> int:
+    """Sequences up to which a decode step of a Llama layer is one call (``llama_decode_layer``) instead of its separate launches.  Its
+    projections have latencies, not bandwidth, in their favour: B200, bf16, 4 layers, us per step as a CUDA graph, separate / one call:
+    width 512, ff 1408: 135 / 68 with one sequence, 148 / 121 with 32; width 1024 185 / 90 and 181 / 164; width 2048, ff 5632 303 / 227,
+    300 / 247 with 8, 277 / 284 with 16; width 4096, ff 14336 563 / 712.  Launched from Python a layer takes 250 us of host time
+    separately, 70 in one call."""
+    return 0 if ff > 8192 else 32 if width <= 1024 else 8 if width <= 2048 else 0
+
+
+def llama_decode_layer(x: torch.Tensor, norm1: torch.Tensor, eps1: float, weights: Sequence[torch.Tensor], norm2: torch.Tensor, eps2: float,
+                       position_ids: Optional[torch.Tensor], inv_freq: Optional[torch.Tensor], rope_scaling: float,
+                       cos: Optional[torch.Tensor], sin: Optional[torch.Tensor], k_pool: torch.Tensor, v_pool: torch.Tensor,
+                       block_tables: torch.Tensor, context_lens: torch.Tensor, max_context_len: int, num_heads: int, num_splits: int = 0,
+                       flags: int = 0) -> torch.Tensor:
+    """One decoder layer over ``x [B, 1, W]`` (contiguous, f16 / bf16): norms, projections ``weights`` = q, k, v, o, gate, up, down
+    (contiguous ``[out, in]``), RoPE, append and paged attention, SiLU feed-forward, residuals, in five launches.  RoPE from ``cos / sin
+    [B, D]``, or from ``position_ids`` (int64 ``[B, 1]``) and ``inv_freq`` (fp32 ``[D / 2]``).  Returns ``[B, 1, W]``."""
+    _need_cuda(x, norm1, norm2, k_pool, v_pool, block_tables, context_lens, *weights)
+    max_blocks, Hkv, bs, D = _pool_dims(k_pool)
+    B, T, W = x.shape
+    ff, dt = weights[4].shape[0], DTYPE_ID[x.dtype]
+    if v_pool.shape != k_pool.shape or v_pool.dtype != k_pool.dtype or not v_pool.is_contiguous():
+        raise ValueError("k_pool and v_pool must match")
+    if x.dtype != k_pool.dtype:
+        raise TypeError("q dtype must equal the pool dtype")
+    shapes = ((num_heads * D, W), (Hkv * D, W), (Hkv * D, W), (W, num_heads * D), (ff, W), (ff, W), (W, ff))
+    if T != 1 or not x.is_contiguous() or tuple(tuple(w.shape) for w in weights) != shapes or norm1.numel() != W or norm2.numel() != W:
+        raise ValueError("inputs do not match the layer's sizes")
+    for t in (norm1, norm2, *weights):
+        if t.dtype != x.dtype or not t.is_contiguous():
+            raise ValueError("weights are contiguous in x's dtype")
+    if block_tables.dtype != torch.int32 or block_tables.dim() != 2 or block_tables.shape[0] != B:
+        raise ValueError("block_tables must be int32 [B, n]")
+    if block_tables.stride(1) != 1 and block_tables.shape[1] > 1:
+        raise ValueError("block_tables rows must be contiguous")
+    if context_lens.dtype != torch.int32 or context_lens.shape != (B,) or not context_lens.is_contiguous():
+        raise ValueError("context_lens must be a contiguous int32 [B]")
+    if cos is not None:
+        if cos.shape != (B, D) or sin.shape != (B, D) or not cos.is_contiguous() or not sin.is_contiguous():
+            raise ValueError("cos / sin must be contiguous [B, D]")
+        if cos.dtype != x.dtype or sin.dtype != x.dtype:
+            raise TypeError("q, k_new, v_new, cos and sin must share the pool dtype")
+        _need_cuda(cos, sin)
+    lib = _lib.load()
+    need = lib.b200_llama_decode_layer_workspace(B, W, ff, num_heads, Hkv, D, bs, int(max_context_len), int(num_splits), dt)
+    ws = torch.empty(max(need, 16), dtype=torch.uint8, device=x.device)
+    out = torch.empty_like(x)
+    with _timed():
+        rc = lib.b200_llama_decode_layer(
+            out.data_ptr(), x.data_ptr(), W, norm1.data_ptr(), float(eps1), weights[0].data_ptr(), weights[1].data_ptr(),
+            weights[2].data_ptr(), weights[3].data_ptr(), norm2.data_ptr(), float(eps2), weights[4].data_ptr(), weights[5].data_ptr(),
+            weights[6].data_ptr(), 0 if cos is not None else position_ids.data_ptr(), 0 if cos is not None else inv_freq.data_ptr(),
+            float(rope_scaling), cos.data_ptr() if cos is not None else 0, sin.data_ptr() if cos is not None else 0, k_pool.data_ptr(),
+            v_pool.data_ptr(), block_tables.data_ptr(), block_tables.stride(0) if B > 1 else block_tables.shape[1],
+            context_lens.data_ptr(), B, W, ff, num_heads, Hkv, D, bs, max_blocks, int(max_context_len), int(num_splits), ws.data_ptr(),
+            ws.numel(), dt, int(flags), _stream())
+    _lib.check(rc, "b200_llama_decode_layer")
+    return out
+
+
 def attn_prefix_plan(B: int, Hq: int, Hkv: int, D: int, block_size: int, prefix_blocks: int, max_context_len: int,
                      dtype: torch.dtype):
     """``(prefix_splits, suffix_splits)`` the library would choose for the shared-prefix variant."""

@@ -327,6 +327,22 @@ class RaggedLayerCache:
     state: RaggedBatchState
 
 
+def _plain_weight(w: torch.Tensor, dtype: torch.dtype, device: int) -> bool:
+    return type(w) is nn.Parameter and w.dtype == dtype and w.get_device() == device and w.is_contiguous() and w.data_ptr() % 16 == 0
+
+
+def _plain_modules(layer: nn.Module) -> bool:
+    """No hooks on the layer's modules, nor global ones: nothing would notice that a forward was not called."""
+    mod = nn.modules.module
+    if mod._global_forward_hooks or mod._global_forward_pre_hooks:
+        return False
+    a, m = layer._modules["self_attn"], layer._modules["mlp"]
+    for sub in (*a._modules.values(), *m._modules.values(), layer.input_layernorm, layer.post_attention_layernorm):
+        if sub._forward_hooks or sub._forward_pre_hooks or "forward" in sub.__dict__:
+            return False
+    return True
+
+
 class PagedLlamaDecoderLayer(nn.Module):
     """One Llama decoder layer; see the module docstring."""
 
@@ -408,6 +424,44 @@ class PagedLlamaDecoderLayer(nn.Module):
     _gu_w = None
     defer_residual = False
 
+    # ---- a decode step in one call -----------------------------------------------------------------
+    def _one_call(self, x: torch.Tensor, position_ids, handle: "PagedLayerKV", st: "PagedBatchState") -> Optional[torch.Tensor]:
+        """The layer's output for one new token per sequence through ``ops.llama_decode_layer``, or None where that does not apply:
+        a plain layer (its own modules, no hooks, no biases), 16-bit contiguous weights of x's dtype on the current device, no
+        gradients, no autocast."""
+        B = x.shape[0]
+        if B > ops.one_call_batch(self.hidden_size, self.mlp.gate_proj.weight.shape[0]) or x.dtype not in (torch.bfloat16, torch.float16) \
+                or torch.is_grad_enabled() or torch.is_autocast_enabled() or type(x) is not torch.Tensor or not x.is_cuda:
+            return None
+        dev = x.get_device()
+        if dev != torch.cuda.current_device() or not x.is_contiguous() or x.shape[2] != self.hidden_size or not _plain_modules(self):
+            return None
+        kp = handle.k_pool
+        if kp.dim() != 4 or not ops.fused_decode_supported(kp, self.num_heads) or kp.shape[1] != self.num_kv_heads or kp.shape[3] != self.head_dim:
+            return None
+        weights = []
+        for grp, name in self._LINEARS:
+            m = self._modules[grp]._modules[name]
+            if type(m) is not nn.Linear or m.bias is not None or not _plain_weight(m.weight, x.dtype, dev):
+                return None
+            weights.append(m.weight)
+        norms = (self.input_layernorm, self.post_attention_layernorm)
+        for m in norms:
+            if type(m) is not RMSNorm or not _plain_weight(m.weight, x.dtype, dev):
+                return None
+        cos, sin = st.cos, st.sin
+        if cos is None:
+            f = self.inv_freq
+            if position_ids is None or position_ids.dtype != torch.int64 or tuple(position_ids.shape) != (B, 1) or not position_ids.is_contiguous() \
+                    or position_ids.get_device() != dev or f.dtype != torch.float32 or not f.is_contiguous() or f.get_device() != dev \
+                    or 2 * f.numel() != self.head_dim:
+                return None
+        else:
+            cos, sin = cos.reshape(B, self.head_dim), sin.reshape(B, self.head_dim)
+        return ops.llama_decode_layer(x, norms[0].weight, norms[0].variance_epsilon, weights, norms[1].weight, norms[1].variance_epsilon,
+                                      position_ids, self.inv_freq, self.rope_attention_scaling, cos, sin, kp, handle.v_pool, st.block_tables,
+                                      st.context_lens, st.max_context_len, self.num_heads, num_splits=st.num_splits, flags=st.attn_flags)
+
     # ---- forward -----------------------------------------------------------------------------------
     def forward(
         self,
@@ -425,6 +479,11 @@ class PagedLlamaDecoderLayer(nn.Module):
         st = past_key_value.state
         B, T, _ = hidden_states.shape
         Hq, Hkv, D = self.num_heads, self.num_kv_heads, self.head_dim
+
+        if T == 1 and self._qkv_w is None and st.pending_residual is None and not self.defer_residual and st.prefix_blocks == 0:
+            h = self._one_call(hidden_states, position_ids, past_key_value, st)
+            if h is not None:
+                return h, (past_key_value if use_cache else None)
 
         if st.pending_residual is not None:
             # the previous layer of this shard left its last residual add to us: h_in = hidden + pending, and the

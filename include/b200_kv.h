@@ -239,6 +239,20 @@ int b200_rope_kv_append_prompt(void* q, int64_t q_row_stride, void* k, int64_t k
  * inv_freq fp32 [D/2], pos int64 [n].  Replaces the seven launches of the torch recipe. */
 int b200_rope_tables(void* cos_out, void* sin_out, const int64_t* pos, const float* inv_freq, int64_t n, int D, float scaling, int dtype,
                      void* stream);
+/* One Llama decoder layer of a decode step (one new token per sequence, its slot already counted in context_lens) for up to 32 sequences
+ * in f16 / bf16: x [B, W] (row stride x_stride) -> h_out [B, W], K and V appended to the pools.  Weights [rows, cols] contiguous, no
+ * biases: wq [Hq D, W], wk and wv [Hkv D, W], wo [W, Hq D], wg and wu [ff, W], wd [W, ff]; norm1, norm2 [W].  RoPE: cos_table / sin_table
+ * [B, D], or both NULL: from pos (int64 [B]), inv_freq (fp32 [D/2]) and rope_scaling.  Sums in fp32, rounded to the storage type where the
+ * separate entry points and a library GEMM in between round.  num_splits 0: the library's choice.  Operands 16-byte aligned. */
+int b200_llama_decode_layer_supported(int B, int W, int ff, int Hq, int Hkv, int D, int block_size, int dtype);
+size_t b200_llama_decode_layer_workspace(int B, int W, int ff, int Hq, int Hkv, int D, int block_size, int max_context_len, int num_splits,
+                                         int dtype);
+int b200_llama_decode_layer(void* h_out, const void* x, int64_t x_stride, const void* norm1, float eps1, const void* wq, const void* wk,
+                            const void* wv, const void* wo, const void* norm2, float eps2, const void* wg, const void* wu, const void* wd,
+                            const int64_t* pos, const float* inv_freq, float rope_scaling, const void* cos_table, const void* sin_table,
+                            void* k_pool, void* v_pool, const int32_t* block_tables, int table_stride, const int32_t* context_lens, int B,
+                            int W, int ff, int Hq, int Hkv, int D, int block_size, int64_t max_blocks, int max_context_len, int num_splits,
+                            void* workspace, size_t workspace_bytes, int dtype, unsigned attn_flags, void* stream);
 int b200_silu_mul(void* out, const void* gate, const void* up, int64_t rows, int cols,
                   int64_t gate_row_stride, int64_t up_row_stride, int dtype, void* stream);
 /* Greedy token: out[r] = argmax over x[r, 0..cols) — largest value, smallest index among equals, NaN largest, i.e.
