@@ -296,6 +296,7 @@ MIXER_SIGNATURES = {
     # prompt portions on the fifth-generation tensor cores (csrc/b200_tile_attn.cu)
     "b200_tile_attn_supported": (c_int, [c_int] * 7),
     "b200_tile_attn_rows": (c_int, [c_int] * 4),
+    "b200_tile_attn_rows_ext": (c_int, [c_int] * 5),
     "b200_tile_attn_splits": (c_int, [c_int] * 5),
     "b200_tile_attn": (
         c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p,

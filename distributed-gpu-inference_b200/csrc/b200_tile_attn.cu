@@ -12,16 +12,16 @@
 //   O += P V    tcgen05.mma with P from tensor memory; V lies in shared memory as the pool holds it (one line per key), read with the
 //               transposed descriptor; O stays in tensor memory in fp32 for the whole walk
 //
-// Four more warps copy pages (cp.async a tile or two ahead; any page size; rows past the sequence are zero-filled), one thread of a
-// another one issues the products; they meet at mbarriers only.  While the softmax works on tile i the tensor cores run S of tile i + 1 and
-// P V of tile i - 1.  256 rows per fetched tile halve what two CTAs of 128 rows per SM ask of L2 (32 KB per 64 keys and 4.2 MFLOP).
+// Four more warps copy pages a tile or two ahead - pages that divide 64 keys by the copy engine, one box of 64 columns per page and block of
+// columns, a sequence's last tile and other page sizes row by row with rows past the sequence zero-filled - and another one issues the
+// products; they meet at mbarriers only.  While the softmax works on tile i the tensor cores run S of tile i + 1 and P V of tile i - 1.
 //
-// Measured on B200 (bf16, 8 x 2048 tokens, 16 heads over 4 kv heads of 128): 237 us plain, 274 us with distance biases (the mma.sync
-// kernel: 1419), 156 us with a window of 512; latent 320 / 256, 4 portions of up to 1500 tokens of 16 heads behind 700, window 512: 104 us
-// (417).  A tile of 64 keys x 256 rows took about 2200 clocks before O was rescaled at every new maximum (212 / 261 / 141 us): 1280 of the
-// tensor cores (S with 64 columns is bound by reading Q from shared memory), 1000 of exponentials (two warps per scheduler at four per
-// clock), the copies 2000 (64 threads per pool); about a third of the launch is the CTAs' beginnings and ends, which nothing covers
-// with one CTA per SM.  128 rows and two CTAs: 250 and 338 us.
+// Measured on B200 (bf16, 8 x 2048 tokens, 16 heads over 4 kv heads of 128): 213 us plain, 257 us with distance biases (the mma.sync
+// kernel: 1419), 323 us with a soft cap, 156 us with a window of 512; latent 320 / 256, 4 portions of up to 1500 tokens of 16 heads behind
+// 700, window 512: 101 us (417).  Pages row by row by 64 threads per pool: 237, 274, 574 (with a soft cap by exponentials), 156, 104.  What a
+// tile of 64 keys x 256 rows takes: 1280 clocks of the tensor cores (S with 64 columns is bound by reading Q from shared memory), 1000 of
+// exponentials (two warps per scheduler at four per clock) beside as much of other work per score; about a third of the launch is the
+// CTAs' beginnings and ends.
 //
 // Weights are taken relative to the row's running maximum, so that the largest is 1 and loses nothing when P is rounded to the storage
 // type; O is scaled down whenever a row of the warp has a new maximum (with the tile's weights already written, so that P V of the tile
@@ -35,6 +35,8 @@
 //
 // Every wait is bounded: a barrier that does not complete within a second marks the launch as failed, the rest of the walk does not
 // wait, tensor memory is freed and the rows come out as NaN.
+#include <cuda.h>
+
 #include <algorithm>
 #include <type_traits>
 
@@ -205,7 +207,7 @@ struct Plan {
 
 template <typename T, int DK, int DV, bool ALIAS, bool BIAS, int HALVES>
 __global__ void __launch_bounds__(Plan<DK, DV, ALIAS, HALVES>::kNT, Plan<DK, DV, ALIAS, HALVES>::kCtas)
-tile_attn_kernel(const TileAttn A) {
+tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map) {
   using P = Plan<DK, DV, ALIAS, HALVES>;
   constexpr int NB = P::kBufs, kSoft = P::kSoft;
   extern __shared__ unsigned char raw_smem[];
@@ -285,12 +287,47 @@ tile_attn_kernel(const TileAttn A) {
     const int32_t* table = A.block_tables + static_cast<int64_t>(trow) * A.table_stride;
     const int shift = (bs & (bs - 1)) == 0 ? __ffs(bs) - 1 : -1;
     int* rows_s = reinterpret_cast<int*>(sm + P::kPage) + (values ? 2 * kKeys : 0);
-    // the page of one key of a tile, looked up by the team's first 64 threads a tile ahead of its copies
+    // A tile whose keys all exist and whose pages divide it is fetched page by page by the copy engine (boxes of 64 columns that land as
+    // `line` has them), the others (a sequence's last) row by row with zeros behind the last.
+    const bool boxes = A.boxes != 0;
+    const int n_pages = boxes ? kKeys / bs : 0;
+    auto whole = [&](int i) { return boxes && i < n_it && key0(i) + kKeys - 1 <= p_last; };
+    // the page of one key of a tile (or the tile's page number `me`), looked up by the team's first threads a tile ahead of its copies
     auto look_up = [&](int i) {
+      if (whole(i)) return me < n_pages ? table[key0(i) / bs + me] : -1;
       const int j = key0(i) + me;
       return me < kKeys && i < n_it && j <= p_last ? table[shift >= 0 ? j >> shift : j / bs] : -1;
     };
+    auto biases = [&](int i) {      // entry [hh][x]: the bias of distance p0 - key0 - 63 + x
+      const int d0 = p0 - key0(i) - (kKeys - 1), span = cnt + kKeys - 1;
+      const uint32_t dst = smem_u32(lut_s + (i % P::kLuts) * rep * pitch);
+      for (int hh = 0; hh < rep; ++hh) {
+        const float* src = A.bias_lut + static_cast<int64_t>(g * rep + hh) * A.lut_len;
+        for (int x = me; x < span; x += kTeam) cp4(dst + 4 * (hh * pitch + x), src + min(max(d0 + x, 0), A.lut_len - 1));
+      }
+    };
+    auto copy_pages = [&](int i, int page) {
+      if (me < n_pages) {
+        constexpr int kBox = 128;       // bytes of a box's row
+        const int cols = values ? DV / 64 : DK / 64;
+        const uint32_t base = (values ? sm0 + P::kV + (i % NB) * (DV / 64) * kBlk : sm0 + P::kK + (i % NB) * (DK / 64) * kBlk) + me * bs * kBox;
+        if (page >= 0) {
+          const uint32_t bar = (values ? bar_v : bar_k) + 8 * (i % NB);
+          asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(cols * bs * kBox) : "memory");
+          for (int c = 0; c < cols; ++c)
+            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(base + c * kBlk),
+                         "l"(values ? &v_map : &k_map), "r"(64 * c), "r"((page * heads + head) * bs), "r"(bar) : "memory");
+        } else {                        // no page: zeros
+          for (int c = 0; c < cols; ++c) {
+            for (int b = 0; b < bs * kBox; b += 16) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(base + c * kBlk + b), "r"(0) : "memory");
+          }
+        }
+      }
+      if (BIAS && !values) biases(i);
+      cp_commit();
+    };
     auto copy = [&](int i, int page) {
+      if (whole(i)) return copy_pages(i, page);
       if (me < kKeys) {
         const int j = key0(i) + me, off = shift >= 0 ? j & (bs - 1) : j % bs;
         rows_s[(i & 1) * kKeys + me] = page < 0 ? -1 : (page * heads + head) * bs + off;
@@ -315,14 +352,7 @@ tile_attn_kernel(const TileAttn A) {
       };
       if (DK == DV || !values) move(std::integral_constant<int, DK>{});
       else move(std::integral_constant<int, DV>{});
-      if (BIAS && !values) {      // entry [hh][x]: the bias of distance p0 - key0 - 63 + x
-        const int d0 = p0 - key0(i) - (kKeys - 1), span = cnt + kKeys - 1;
-        const uint32_t dst = smem_u32(lut_s + (i % P::kLuts) * rep * pitch);
-        for (int hh = 0; hh < rep; ++hh) {
-          const float* src = A.bias_lut + static_cast<int64_t>(g * rep + hh) * A.lut_len;
-          for (int x = me; x < span; x += kTeam) cp4(dst + 4 * (hh * pitch + x), src + min(max(d0 + x, 0), A.lut_len - 1));
-        }
-      }
+      if (BIAS && !values) biases(i);
       cp_commit();
     };
     auto arrived = [&](int i) {     // this thread's copies of the tile are in shared memory, for the tensor cores too
@@ -461,11 +491,33 @@ tile_attn_kernel(const TileAttn A) {
 #pragma unroll
         for (int c = 0; c < kKeys; ++c) s[c >> 5][c & 31] = fmaf(s[c >> 5][c & 31], mult, b[-c]);
       } else if (!plain) {
+        float far = A.softcap > 0.f ? 0.f : INFINITY;
 #pragma unroll
         for (int c = 0; c < kKeys; ++c) {
-          float x = s[c >> 5][c & 31] * mult;
-          if (A.softcap > 0.f) x = A.softcap * (1.0f - __fdividef(2.0f, __expf(x * two_over_cap) + 1.0f));
-          s[c >> 5][c & 31] = x;
+          s[c >> 5][c & 31] *= mult;
+          far = fmaxf(far, fabsf(s[c >> 5][c & 31]));
+        }
+        if (!__any_sync(0xffffffffu, far > 0.5f * A.softcap)) {
+          // all within half the cap: x tanh(u) / u, u = x / cap, by its series in u^2 (Chebyshev nodes on 0 .. 1/4, 3e-10): 1 / (1 + e^x) and
+          // the difference from 1 took three times as long (5 x 1024 tokens of 16 heads, window 512: 99 us against 56) and lost the last
+          // digits of small scores
+          const float per_cap = 0.5f * two_over_cap;
+#pragma unroll
+          for (int c = 0; c < kKeys; ++c) {
+            float& x = s[c >> 5][c & 31];
+            const float u = x * per_cap, t = u * u;
+            float q = fmaf(t, -0x1.b12a58p-8f, 0x1.5c8676p-6f);
+            q = fmaf(t, q, -0x1.b97d94p-5f);
+            q = fmaf(t, q, 0x1.110ec8p-3f);
+            q = fmaf(t, q, -0x1.555550p-2f);
+            x = fmaf(x * t, q, x);
+          }
+        } else if (A.softcap > 0.f) {
+#pragma unroll
+          for (int c = 0; c < kKeys; ++c) {
+            float& x = s[c >> 5][c & 31];
+            x = A.softcap * (1.0f - __fdividef(2.0f, __expf(x * two_over_cap) + 1.0f));
+          }
         }
       }
       // keys in sight of every token of the tile need no mask
@@ -585,6 +637,26 @@ tile_attn_kernel(const TileAttn A) {
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "n"(P::kTm));
 }
 
+// The pool as rows of `width` elements, fetched in boxes of 64 columns x one page; made for the launch (a microsecond) and not kept.
+// Its height is the largest a row's number allows: which rows are read is the block tables' business, as with plain loads.
+template <typename T>
+bool page_map(CUtensorMap* map, const void* pool, int width, int block_size) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult qr;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess) p = nullptr;
+    return reinterpret_cast<Encode>(p);
+  }();
+  if (!encode || !aligned16(pool)) return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(width), 0x7fffffffu}, strides[1] = {2ull * width};
+  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(block_size)}, step[2] = {1, 1};
+  return encode(map, std::is_same_v<T, __nv_bfloat16> ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(pool),
+                dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <typename T, int DK, int DV, bool ALIAS, bool BIAS, int HALVES>
 int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stream) {
   using P = Plan<DK, DV, ALIAS, HALVES>;
@@ -595,7 +667,12 @@ int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stre
   if (smem > kMaxSmem) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
   auto kern = tile_attn_kernel<T, DK, DV, ALIAS, BIAS, HALVES>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-  kern<<<dim3(n_tiles, A.G, n_splits), P::kNT, smem, stream>>>(A);
+  TileAttn B = A;
+  CUtensorMap k_map{}, v_map{};
+  // pages that divide a tile of keys, rows that start on 16 bytes
+  B.boxes = A.block_size % 8 == 0 && kKeys % A.block_size == 0 && page_map<T>(&k_map, A.k_pool, DK, A.block_size) &&
+            (ALIAS || (A.v_row % 8 == 0 && page_map<T>(&v_map, A.v_pool, A.v_row, A.block_size)));
+  kern<<<dim3(n_tiles, A.G, n_splits), P::kNT, smem, stream>>>(B, k_map, v_map);
   return check_launch("b200_tile_attn");
 }
 
@@ -626,12 +703,13 @@ bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, in
   return dk == dv && (dk == 64 || dk == 128);
 }
 
-// 256 rows share a fetched key tile, but only one such CTA runs per SM and nothing covers its beginning and end: worth it from three
-// rounds of them on (8 x 2048 tokens, 16 heads over 4, 7 rounds: 237 us against 250 with 128 rows and two CTAs per SM, with biases 273 against
-// 338; 5 portions of up to 1024 tokens under a window of 512, 1.4 rounds: 41.9 against 40.3, with a soft cap 79 against 77).
-int tile_attn_rows(int rep, int G, int dk, int n_tokens) {
+// 256 rows share a fetched key tile and its biases, but only one such CTA runs per SM and nothing covers its beginning and end; with pages
+// by the copy engine two CTAs of 128 rows are ahead where the softmax does no more than scale (8 x 2048 tokens, 16 heads over 4: 213 us
+// against 225; 5 x 1024 under a window of 512: 44.6 / 46.0), 256 rows where it also adds biases or caps (257 against 285, 323 against 369;
+// 8 x 700 tokens of 8 heads, 1.2 rounds of CTAs, biases: 36.3 / 39.6) and the step fills the SMs once.
+int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy) {
   const int64_t ctas = static_cast<int64_t>(n_tokens) * rep / (2 * kTileRows) * G;
-  return dk <= 128 && ctas >= 3 * kNumSMs ? 2 * kTileRows : kTileRows;
+  return heavy && dk <= 128 && ctas >= kNumSMs ? 2 * kTileRows : kTileRows;
 }
 
 // Keys are divided while the chip has room for more CTAs, a share being worth its part of the merge: three tiles of 64 keys where

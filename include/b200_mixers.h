@@ -497,6 +497,7 @@ int b200_mixed_prompt_attn_ext3(void* out, int64_t out_tok_stride, int64_t out_h
  * workspace fp32 [n_splits][n_tiles][tile_rows / (H / G)][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte aligned query rows. */
 int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bias, int dtype);
 int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens);
+int b200_tile_attn_rows_ext(int rep, int G, int dk, int n_tokens, int heavy);   /* heavy: with distance biases or a soft cap */
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows);
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,
