@@ -15,6 +15,7 @@ What it owns
 """
 from __future__ import annotations
 
+from array import array
 from collections import deque
 from dataclasses import dataclass, field
 from typing import Any, Dict, List, Optional, Sequence, Tuple
@@ -36,13 +37,14 @@ class _Request:
     blocks: List[Optional[List[List[CacheBlock]]]]     # per shard: per attention layer, its blocks (None: no pool)
     length: int = 0                                    # tokens already in cache / state
     table: List[int] = field(default_factory=list)     # pool slots of its blocks
+    leases: Dict[int, Tuple[List[str], List[int]]] = field(default_factory=dict)   # per pool: (ids, slots) of blocks held without block objects
 
 
 def _token_ids(toks: Sequence[int]) -> np.ndarray:
     if isinstance(toks, list) and type(toks[0]) is int:
         try:
-            return np.array(toks, dtype=np.int64)
-        except (TypeError, ValueError):     # ints beside device scalars: one by one
+            return np.frombuffer(array("q", toks), dtype=np.int64)      # half the time of np.array
+        except (TypeError, ValueError, OverflowError):     # ints beside device scalars: one by one
             pass
     return np.fromiter((int(t) for t in toks), dtype=np.int64, count=len(toks))
 
@@ -56,10 +58,14 @@ def _upload(device: torch.device, arrays: Sequence[np.ndarray]) -> List[torch.Te
     host = torch.empty(total, dtype=torch.uint8, pin_memory=True)
     raw = host.numpy()
     for o, a in zip(at, arrays):
-        raw[o:o + a.nbytes] = np.ascontiguousarray(a).reshape(-1).view(np.uint8)
+        raw[o:o + a.nbytes].view(a.dtype)[...] = a.reshape(-1)
     buf = host.to(device, non_blocking=True)
-    kinds = {np.dtype(np.int64): torch.int64, np.dtype(np.int32): torch.int32}
-    return [buf[o:o + a.nbytes].view(kinds[a.dtype]).view(a.shape) for o, a in zip(at, arrays)]
+    whole = {np.dtype(np.int64): buf.view(torch.int64), np.dtype(np.int32): buf.view(torch.int32)}
+    out = []
+    for o, a in zip(at, arrays):
+        t = whole[a.dtype].narrow(0, o // a.itemsize, a.size)
+        out.append(t if a.ndim == 1 else t.view(a.shape))
+    return out
 
 
 class RaggedStepEngine:
@@ -134,8 +140,10 @@ class RaggedStepEngine:
 
     def finish(self, rid: Any) -> None:
         req = self.requests.pop(rid)
-        for pool, blocks in zip(self.kv_pools, req.blocks):
-            if pool is not None:
+        for i, (pool, blocks) in enumerate(zip(self.kv_pools, req.blocks)):
+            if i in req.leases:
+                pool.give_back(*req.leases[i], mixer_ops.zero_blocks)
+            if pool is not None and any(blocks):
                 for li, layer_blocks in enumerate(blocks):
                     pool.layer(li).unpin(b.block_id for b in layer_blocks)
                 pool.free_sequence(blocks, mixer_ops.zero_blocks)
@@ -156,13 +164,26 @@ class RaggedStepEngine:
         if need - have > self.free_blocks:
             raise RuntimeError(f"KV pages exhausted: request needs {need - have} more, {self.free_blocks} free")
         row = None
-        for pool, blocks in zip(self.kv_pools, req.blocks):
+        for i, (pool, blocks) in enumerate(zip(self.kv_pools, req.blocks)):
             if pool is None:
                 continue
-            pool.extend_sequence(blocks, new_len)
+            got = pool.lease(need - have) if not any(blocks) else None
+            if got is not None:
+                held = req.leases.setdefault(i, ([], []))
+                held[0].extend(got[0])
+                held[1].extend(got[1])
+                if row is None:
+                    row = got[1]
+                elif got[1] != row:
+                    raise RuntimeError("layers disagree on block slots; per-layer tables are not supported here")
+                continue
+            # the layers' free lists differ, or the request has such blocks already: block by block
+            leased = len(req.leases[i][1]) if i in req.leases else 0
+            pool.extend_sequence(blocks, new_len - leased * self.block_size)
+            have_here = have - leased
             for li, layer_blocks in enumerate(blocks):
-                pool.layer(li).pin(b.block_id for b in layer_blocks[have:])   # a live request's pages are not evictable
-                got = [b.slot for b in layer_blocks[have:]]
+                pool.layer(li).pin(b.block_id for b in layer_blocks[have_here:])   # a live request's pages are not evictable
+                got = [b.slot for b in layer_blocks[have_here:]]
                 if row is None:
                     row = got
                 elif got != row:
@@ -180,8 +201,6 @@ class RaggedStepEngine:
         bs = self.block_size
         n_tok = 0
         ids: List[np.ndarray] = []
-        pos_l: List[np.ndarray] = []
-        slot_l: List[np.ndarray] = []
         spans, scans, wanted, rows = [], [], [], []
         # refuse the whole step before touching anything when its pages or slots do not fit
         new_blocks, new_seqs, seen = 0, 0, set()
@@ -205,10 +224,6 @@ class RaggedStepEngine:
                 continue
             req = self.requests.get(rid) or self.admit(rid)
             self._grow(req, req.length + n)
-            p = np.arange(req.length, req.length + n, dtype=np.int64)
-            table = np.asarray(req.table, dtype=np.int64)
-            pos_l.append(p)
-            slot_l.append(table[p // bs] * bs + p % bs)
             first = n_tok
             spans.append((first, n, len(rows), req.length))
             scans.append((first, n, req.slot, 1 if req.length == 0 else 0))
@@ -227,10 +242,14 @@ class RaggedStepEngine:
 
         # everything the step's layers read travels in one copy from pinned memory: a copy per table from pageable memory cost
         # as much host time as the tables themselves
+        scan = np.array(scans, dtype=np.int32)
+        row_of = np.repeat(np.arange(len(spans), dtype=np.int32), scan[:, 1])
+        past = np.array([sp[3] for sp in spans], dtype=np.int64)
+        pos = np.arange(n_tok, dtype=np.int64) + (past - scan[:, 0])[row_of]
+        page, offset = np.divmod(pos, bs)
+        slots = tables[row_of, page].astype(np.int64) * bs + offset
         slot_mapping, h, picked, tok_pos, scan_seqs, tok_row, block_tables = _upload(dev, (
-            np.concatenate(slot_l), np.concatenate(ids), np.asarray(wanted, dtype=np.int64),
-            np.concatenate(pos_l).astype(np.int32), np.asarray(scans, dtype=np.int32),
-            np.repeat(np.arange(len(spans), dtype=np.int32), [sp[1] for sp in spans]), tables))
+            slots, np.concatenate(ids), np.array(wanted, dtype=np.int64), pos.astype(np.int32), scan, row_of, tables))
         st = RaggedBatchState(tok_pos=tok_pos, slot_mapping=slot_mapping, block_tables=block_tables, scan_seqs=scan_seqs, spans=spans,
                               tok_row=tok_row, scan_host=scans)
         st.token_ids = h

@@ -155,3 +155,29 @@ def test_token_ids_of_any_whole_numbers():
         assert got.dtype == np.int64 and got.tolist() == want
     with pytest.raises((TypeError, ValueError)):
         _token_ids([1, None])
+
+
+def test_leased_blocks_beside_block_objects():
+    """Leases take what ``allocate_sequence`` would take, count as blocks in use, are never evicted, come back zeroed in order; layers whose
+    free lists differ give none."""
+    def pool():
+        return KVCachePool(num_layers=2, num_heads=0, head_dim=0, block_size=4, max_blocks_per_layer=6, device="cpu", dtype=torch.float32,
+                           layer_shapes=[(1, 8, 8), (2, 4, 8)])
+
+    a, b = pool(), pool()
+    want = [blk.slot for blk in a.allocate_sequence(11)[0]]
+    ids, slots = b.lease(3)
+    assert slots == want and ids == [f"block_{s}" for s in slots]
+    assert [c.get_stats()["total_blocks"] for c in b._layer_caches] == [3, 3] and len(b.layer(0)._free_blocks) == 3
+    assert b.lease(4) is None and b.lease(0) is None and b.layer(0).get_stats()["allocations"] == 3
+    rest = b.allocate_sequence(12)
+    assert not {blk.slot for blk in rest[0]} & set(slots)
+    with pytest.raises(RuntimeError):       # the other sequence's blocks are evicted for this one, the lease is not
+        b.allocate_sequence(16)
+    b.layer(0).key_pool.fill_(1.0)
+    zeroed = []
+    b.give_back(ids, slots, lambda pools, s: zeroed.append((len(pools), list(s))) or [p.index_fill_(0, torch.tensor(s), 0) for p in pools])
+    assert zeroed == [(4, slots)] and not b.layer(0).key_pool[slots].any() and b.layer(0)._free_blocks[-3:] == ids
+    c = pool()
+    c.layer(1)._free_blocks.reverse()
+    assert c.lease(2) is None and [x.get_stats()["free_blocks"] for x in c._layer_caches] == [6, 6]
