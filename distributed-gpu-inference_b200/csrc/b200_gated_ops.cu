@@ -23,6 +23,7 @@
 
 #include "../../include/b200_mixers.h"
 #include "b200_common.cuh"
+#include "b200_rotary_rows.cuh"
 
 namespace b200 {
 namespace {
@@ -93,6 +94,7 @@ token_shift_kernel(T* __restrict__ out, int64_t out_stride, T* __restrict__ x_ca
 }
 
 // ---- latent rotary append ------------------------------------------------------------------------------------------
+// Rows that cannot be moved in 16-byte pieces, and fp32 (b200_rotary_rows.cu has the others).
 // One CTA per token.  (cos, sin) * gain of the token's angles are formed once (double precision angles) and serve the
 // shared key part and every query head.
 template <typename T>
@@ -395,6 +397,10 @@ int b200_latent_rotary_append_ext(const void* q_rot, int64_t q_tok_stride, int64
   if (n_tok == 0) return 0;
   if (!q_rot || !q_out || !dkv || !c_norm || !pool || !slot_mapping || !tok_pos || (rot_dims > 0 && !freqs))
     return fail(B200_EINVAL, "b200_latent_rotary_append: null pointer");
+  if (latent_rows(LatentRows{q_rot, q_tok_stride, q_head_stride, q_out, qo_tok_stride, qo_head_stride, dkv, dkv_stride, c_norm, eps, freqs,
+                             gain, rot_dims, interleaved, pool, slot_mapping, tok_pos, n_tok, H, rot_width, rank}, dtype,
+                  static_cast<cudaStream_t>(stream)))
+    return check_launch("b200_latent_rotary_append");
   const size_t smem = sizeof(float) * std::max(rot_dims, 2);
   return gated_by_dtype(dtype, "b200_latent_rotary_append", [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;

@@ -20,6 +20,7 @@
 
 #include "../../include/b200_mixers.h"
 #include "b200_column_scan.cuh"
+#include "b200_rotary_rows.cuh"
 #include "b200_common.cuh"
 
 namespace b200 {
@@ -50,6 +51,7 @@ __device__ __forceinline__ float block_total(float v, float* red) {
 }
 
 // ---- q/k norm + rotary + append ------------------------------------------------------------------------------------
+// Rows that cannot be moved in 16-byte pieces, and fp32 (b200_rotary_rows.cu has the others).
 // One CTA per token, one warp per head in turn (q heads, then k heads, then the value rows).  A head's row is read into
 // the warp's fp32 slab, normed there, and written out with its rotated pairs.
 constexpr int kQkWarps = 8;
@@ -428,6 +430,9 @@ int b200_qknorm_rotary_append_ext2(void* q, int64_t q_stride, const void* k, int
   if (n_tok == 0) return 0;
   if (!q || !k || !v || !k_pool || !v_pool || !slot_mapping || !tok_pos || (rot_dims > 0 && !freqs))
     return fail(B200_EINVAL, "b200_qknorm_rotary_append: null pointer");
+  if (qk_rows(QkRows{q, q_stride, k, k_stride, v, v_stride, q_norm, k_norm, unit_norm, eps, freqs, rot_dims, interleaved, k_pool, v_pool,
+                     slot_mapping, tok_pos, n_tok, H, G, Gv, dk, dv, block_size}, dtype, static_cast<cudaStream_t>(stream)))
+    return check_launch("b200_qknorm_rotary_append");
   const size_t smem = sizeof(float) * (static_cast<size_t>(rot_dims) + static_cast<size_t>(kQkWarps) * dk);
   if (smem > 200 * 1024) return fail(B200_ESHAPE, "b200_qknorm_rotary_append: head size %d too large", dk);
   return parallel_by_dtype(dtype, "b200_qknorm_rotary_append", [&](auto* tag) {

@@ -1058,6 +1058,18 @@ def latent_rotary_append(q_rot: torch.Tensor, q_out: torch.Tensor, dkv: torch.Te
     _lib.check_mixers(rc, "b200_latent_rotary_append")
 
 
+def heads_by_token(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """``a [H, n, r] @ w [H, r, dv]`` per head -> ``[n, H * dv]``, a token's heads side by side: the GEMMs write them there (a
+    copy behind them took 16 us at 3900 tokens of 16 heads of 128), unless a gradient is asked for, which ``out=`` does not
+    allow."""
+    (H, n, _), dv = a.shape, w.shape[2]
+    if torch.is_grad_enabled() and (a.requires_grad or w.requires_grad):
+        return torch.bmm(a, w).transpose(0, 1).reshape(n, H * dv)
+    o = torch.empty((n, H, dv), dtype=a.dtype, device=a.device)
+    torch.bmm(a, w, out=o.transpose(0, 1))
+    return o.view(n, H * dv)
+
+
 @_timed
 def head_diff_norm(a: torch.Tensor, lam: float, out_scale: float, eps: float, rep: int, dtype: Optional[torch.dtype] = None,
                    out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -225,8 +225,7 @@ class LatentAttention(nn.Module):
             mixer_ops.mixed_paged_attention(o_lat.transpose(0, 1), q_lat.transpose(0, 1), cache.k_pool, cache.k_pool,
                                             st.block_tables, st.tok_row, st.tok_pos, self.scale,
                                             gate=proj[:, c[2]:c[2] + H])
-        o = torch.bmm(o_lat, self.w_uv)                                          # [H, n, dv]
-        return F.linear(o.transpose(0, 1).reshape(n, H * self.dv), self.w_o)
+        return F.linear(mixer_ops.heads_by_token(o_lat, self.w_uv), self.w_o)
 
 
 class ChannelDeltaMixer(nn.Module):

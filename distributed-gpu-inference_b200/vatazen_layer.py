@@ -184,8 +184,7 @@ class LatentRotaryAttention(nn.Module):
             mixer_ops.mixed_paged_attention(o_lat.transpose(0, 1), q_lat, cache.k_pool, cache.k_pool, st.block_tables,
                                             st.tok_row, st.tok_pos, self.scale, sink=self.sink, window=self.window,
                                             value_width=r)
-        o = torch.bmm(o_lat, self.w_uv)                                           # [H, n, dv]
-        return F.linear(o.transpose(0, 1).reshape(n, H * self.dv), self.w_o)
+        return F.linear(mixer_ops.heads_by_token(o_lat, self.w_uv), self.w_o)
 
 
 class DifferentialAttention(nn.Module):
