@@ -21,6 +21,7 @@
 #include "../../include/b200_mixers.h"
 #include "b200_column_scan.cuh"
 #include "b200_common.cuh"
+#include "b200_decode_rows.cuh"
 
 namespace b200 {
 
@@ -611,21 +612,28 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 biased_split_merge_kernel(T* __restrict__ out, const float* __restrict__ ws, const T* __restrict__ gate, int64_t gate_stride,
                           const AttnTile* __restrict__ tiles, const int32_t* __restrict__ tok_pos, int H, int dv) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const AttnTile tile = tiles[blockIdx.x];
   if (static_cast<int>(blockIdx.y) >= tile.count) return;
   const int64_t n = tile.tok0 + blockIdx.y;
-  const int h = blockIdx.z, c = threadIdx.x;
+  const int h = blockIdx.z, c = threadIdx.x, lane = threadIdx.x & 31;
   const int splits = (tok_pos[tile.tok0] + tile.count - 1) / kSplitKeys + 1;     // as the tile's CTAs cut its keys
   const int64_t step = static_cast<int64_t>(gridDim.x) * gridDim.y * H * (dv + 2);
   const float* src = ws + ((static_cast<int64_t>(blockIdx.x) * gridDim.y + blockIdx.y) * H + h) * (dv + 2);
-  float M = -INFINITY;
-  for (int sp = 0; sp < splits; ++sp) M = fmaxf(M, src[sp * step]);
+  float M = -INFINITY;      // a lane per split: one trip to memory for all maxima and sums
+  for (int sp = lane; sp < splits; sp += 32) M = fmaxf(M, src[sp * step]);
+  M = warp_max(M);
   float L = 0.f, O = 0.f;
-#pragma unroll 4
-  for (int sp = 0; sp < splits; ++sp) {
-    const float f = expf(src[sp * step] - M);        // a row that saw none of a split's keys left maximum -inf, sum 0 and output 0
-    L = fmaf(src[sp * step + 1], f, L);
-    if (c < dv) O = fmaf(src[sp * step + 2 + c], f, O);
+  for (int base = 0; base < splits; base += 32) {
+    const int sp = base + lane, here = min(32, splits - base);
+    const float f = sp < splits ? expf(src[sp * step] - M) : 0.f;      // a row that saw none of a split's keys left -inf, 0 and 0
+    const float lf = sp < splits ? src[sp * step + 1] * f : 0.f;
+    L += warp_sum(lf);
+#pragma unroll 8
+    for (int u = 0; u < here; ++u) {
+      const float fu = __shfl_sync(0xffffffffu, f, u);
+      if (c < dv) O = fmaf(src[(base + u) * step + 2 + c], fu, O);
+    }
   }
   if (c >= dv) return;
   // in the order of the launch without splits, whose result a row of one range repeats to the bit
@@ -898,7 +906,13 @@ int b200_biased_prompt_attn_ext(void* out, const void* q, int64_t q_stride, cons
             reinterpret_cast<const AttnTile*>(tiles), tok_pos, bias_lut, lut_len, lut_in_smem, q_vec, scale, temp_coef,
             temp_every, H, G, dk, dv, block_size, ws, max_tile_tokens);
       };
-      if (ksplit) {
+      // decoded tokens over pages of whole 16-token tiles: b200_decode_rows.cu, where both sides' times stand
+      const bool rows = ksplit && decode_rows(DecodeRows{out, q, q_stride, gate, gate_stride, k_pool, v_pool, block_tables, table_stride, tiles,
+                                                         tok_pos, bias_lut, lut_len, scale, temp_coef, temp_every, H, G, block_size, ws,
+                                                         max_tile_tokens, kSplitKeys},
+                                              dk, dv, max_tile_tokens, n_tiles, n_splits, dtype, static_cast<cudaStream_t>(stream)) == 0;
+      if (rows) {
+      } else if (ksplit) {
         if (dv8 == 4) launch(biased_prompt_attn_mma_kernel<T, 4, true>);
         else if (dv8 == 8) launch(biased_prompt_attn_mma_kernel<T, 8, true>);
         else launch(biased_prompt_attn_mma_kernel<T, 16, true>);
@@ -909,8 +923,18 @@ int b200_biased_prompt_attn_ext(void* out, const void* q, int64_t q_stride, cons
       }
       const int rc = check_launch("b200_biased_prompt_attn");
       if (rc != 0 || !ws) return rc;
-      biased_split_merge_kernel<T><<<dim3(n_tiles, max_tile_tokens, H), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-          static_cast<T*>(out), ws, static_cast<const T*>(gate), gate_stride, reinterpret_cast<const AttnTile*>(tiles), tok_pos, H, dv);
+      // launched while the CTAs above run; it waits for them on the device
+      cudaLaunchAttribute early{};
+      early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      early.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(n_tiles, max_tile_tokens, H);
+      cfg.blockDim = dim3(128);
+      cfg.stream = static_cast<cudaStream_t>(stream);
+      cfg.attrs = &early;
+      cfg.numAttrs = 1;
+      cudaLaunchKernelEx(&cfg, biased_split_merge_kernel<T>, static_cast<T*>(out), static_cast<const float*>(ws), static_cast<const T*>(gate),
+                         gate_stride, reinterpret_cast<const AttnTile*>(tiles), tok_pos, H, dv);
       return check_launch("b200_biased_prompt_attn (merge)");
     }
   });

@@ -80,3 +80,18 @@ def test_keys_divided_over_ctas(H, G, dk, dv, portions, level, dtype):
         alone = _run(c, past + n, rows=[i])
         assert torch.equal(alone[f:f + n], got[f:f + n])
         assert (alone[:f] == 7).all() and (alone[f + n:] == 7).all()
+
+
+@pytest.mark.parametrize("page", [16, 48, 64, 24])       # the last one is not whole tiles of 16
+@pytest.mark.parametrize("H,G,dk,dv,portions", [(8, 1, 64, 128, CONTEXTS), (16, 1, 128, 64, CONTEXTS), (4, 2, 64, 64, [(8, 0), (1, 17), (3, 300), (2, 4000)]),
+                                                (1, 1, 128, 128, [(1, 0), (16, 250), (9, 1015)])])
+def test_page_sizes_row_counts_and_unwritten_rows(H, G, dk, dv, portions, page):
+    c = _case(H, G, dk, dv, portions, torch.bfloat16, page=page)
+    want = _reference(c)
+    for f, n, b, past in c["spans"]:                  # what nobody wrote may hold anything
+        j = torch.arange(past + n, -(-(past + n) // page) * page, device="cuda")
+        for pool in (c["k"], c["v"]):
+            pool[c["tables"][b, j // page].long(), :, j % page] = float("nan")
+    most = max(p + n for n, p in portions)
+    tol = 3 * 2.0 ** -8                               # weights and result rounded to 8 bits, scores within 2^-20
+    assert _off(_run(c, most), want) <= tol and _off(_run(c, 0), want) <= tol
