@@ -10,6 +10,7 @@
 // SM keep 192 KB under way.  Same case: 49.9 us.
 #include <cuda.h>
 
+#include <atomic>
 #include <type_traits>
 
 #include "b200_common.cuh"
@@ -284,13 +285,20 @@ template <typename T, int DK, int DV>
 int launch(const DecodeRows& A, int rows, dim3 grid, cudaStream_t stream) {
   CUtensorMap k_map, v_map;
   if (!tile_map<T>(&k_map, A.k_pool, DK) || !tile_map<T>(&v_map, A.v_pool, DV)) return 1;
-  auto go = [&](auto kern) {
+  auto go = [&](auto nb) {      // a body, and so a flag, per kernel
     constexpr int smem = Ring<DK, DV>::kSmem;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const auto kern = decode_rows_kernel<T, DK, DV, decltype(nb)::value>;
+    static std::atomic<uint64_t> ready{0};      // a bit per device: the limit is always the same, a call need not set it again
+    int device = 0;
+    cudaGetDevice(&device);
+    if (device >= 64 || !(ready.load(std::memory_order_acquire) >> device & 1)) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (device < 64) ready.fetch_or(1ull << device, std::memory_order_release);
+    }
     kern<<<grid, kWarps * 32, smem, stream>>>(A, k_map, v_map);
   };
-  if (rows <= 8) go(decode_rows_kernel<T, DK, DV, 1>);
-  else go(decode_rows_kernel<T, DK, DV, 2>);
+  if (rows <= 8) go(std::integral_constant<int, 1>{});
+  else go(std::integral_constant<int, 2>{});
   return 0;
 }
 
