@@ -73,11 +73,12 @@ decode_rows_kernel(const DecodeRows A, const __grid_constant__ CUtensorMap k_map
   const int n_tiles = (keys + kTok - 1) / kTok, n_mine = n_tiles > warp ? (n_tiles - warp + kWarps - 1) / kWarps : 0;
   const int per_page = A.block_size / kTok, first = key_from / kTok + warp;      // tiles of the sequence: first, first + 4, ...
   const int32_t* table = A.block_tables + static_cast<int64_t>(seq) * A.table_stride;
-  // lane l: the pool row (in tiles) of this warp's tile base + l
+  // lane l: the pool row (in tiles) of this warp's tile base + l; behind the context's last key the table is not read (its stride says
+  // nothing about its width: one row may serve all sequences with stride 0)
   int base = 0;
   auto look_up = [&] {
     const int t = first + (base + lane) * kWarps;
-    return t / per_page < A.table_stride ? (table[t / per_page] * A.G + g) * per_page + t % per_page : 0;
+    return t * kTok <= p_last ? (table[t / per_page] * A.G + g) * per_page + t % per_page : 0;
   };
   int rows16 = look_up();
   auto fetch = [&](int j) {

@@ -95,3 +95,24 @@ def test_page_sizes_row_counts_and_unwritten_rows(H, G, dk, dv, portions, page):
     most = max(p + n for n, p in portions)
     tol = 3 * 2.0 ** -8                               # weights and result rounded to 8 bits, scores within 2^-20
     assert _off(_run(c, most), want) <= tol and _off(_run(c, 0), want) <= tol
+
+
+@pytest.mark.parametrize("form", ["expanded", "one_row_transposed", "columns_of_a_wider_one", "wider_than_contexts"])
+def test_block_tables_whose_stride_is_not_their_width(form):
+    """A table's stride finds its rows and is no bound of its columns."""
+    c = _case(8, 2, 128, 128, [(1, 1300)] if form == "one_row_transposed" else CONTEXTS, torch.bfloat16)
+    t = c["tables"]
+    if form == "expanded":                          # every sequence reads the pages of the longest
+        c["tables"] = t[-1:].contiguous().expand(t.shape[0], -1)
+    elif form == "one_row_transposed":
+        c["tables"] = t[0].contiguous()[:, None].t()
+        assert c["tables"].stride() == (1, 1)
+    elif form == "columns_of_a_wider_one":
+        wide = torch.full((t.shape[0], t.shape[1] + 5), -1, dtype=torch.int32, device="cuda")
+        wide[:, 5:] = t
+        c["tables"] = wide[:, 5:]
+    else:
+        c["tables"] = torch.cat([t, torch.full_like(t, -1)], 1)
+    most, want = max(p + n for _f, n, _b, p in c["spans"]), _reference(c)
+    tol = 3 * 2.0 ** -8                             # as above
+    assert _off(_run(c, most), want) <= tol and _off(_run(c, 0), want) <= tol
