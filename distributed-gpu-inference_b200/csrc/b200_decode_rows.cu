@@ -8,6 +8,9 @@
 // the copy engine into its own ring of two (no block barrier before the merge); keys stand where the matrix instruction has 16 rows and
 // the query rows where it has eight columns; the bias of the next tile is asked for before this one is waited for.  Three CTAs per
 // SM keep 192 KB under way.  Same case: 49.9 us.
+//
+// Every wait is bounded: a copy that does not land within a second ends its warp's walk, the copies still under way are waited for (a
+// second again) before the merge takes their place, and the CTA's rows come out as NaN.
 #include <cuda.h>
 
 #include <atomic>
@@ -142,9 +145,14 @@ decode_rows_kernel(const DecodeRows A, const __grid_constant__ CUtensorMap k_map
   biases(0);
   const int mat = lane >> 3, mrow = lane & 7;
   const int k_row = (mat & 1) * 8 + mrow, k_chunk = mat >> 1, v_row = (mat >> 1) * 8 + mrow, v_chunk = mat & 1;
+  bool lost = false;
   for (int i = 0; i < n_mine; ++i) {
     const uint32_t kt = ring + i % kStages * R::kStage, vt = kt + R::kK;
-    if (!__all_sync(0xffffffffu, landed(bars + i % kStages * 8, (i / kStages) & 1))) break;
+    if (!__all_sync(0xffffffffu, landed(bars + i % kStages * 8, (i / kStages) & 1))) {
+      for (int j = i; j < min(i + kStages, n_mine); ++j) landed(bars + j % kStages * 8, (j / kStages) & 1);
+      lost = true;
+      break;
+    }
     const int key0 = (first + i * kWarps) * kTok;
     if (key0 + kTok > p_last + 1) zero_v_tail<DV>(vt, p_last + 1 - key0, lane);      // rows that nobody wrote
     float s[NB][4];
@@ -215,7 +223,7 @@ decode_rows_kernel(const DecodeRows A, const __grid_constant__ CUtensorMap k_map
     }
   }
   // the warps' (maximum, sum, output) over the rings, taken together in their order
-  __syncthreads();
+  const bool failed = __syncthreads_or(lost);
   float* o_s = reinterpret_cast<float*>(smem);      // [4][ROWS][DV]
   float* m_s = o_s + kWarps * ROWS * DV;
   float* l_s = m_s + kWarps * ROWS;
@@ -238,7 +246,7 @@ decode_rows_kernel(const DecodeRows A, const __grid_constant__ CUtensorMap k_map
   const int64_t ws_row = (static_cast<int64_t>(blockIdx.z) * gridDim.x + blockIdx.x) * A.ws_tile;
   for (int i = threadIdx.x; i < n_rows * DV; i += kWarps * 32) {
     const int r = i / DV, c = i % DV, t = r / rep, h = g * rep + r - t * rep;
-    float M = -INFINITY, L = 0.f, O = 0.f;
+    float M = -INFINITY, L = 0.f, O = failed ? NAN : 0.f;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) M = fmaxf(M, m_s[w * ROWS + r]);
 #pragma unroll
