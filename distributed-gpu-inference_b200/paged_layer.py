@@ -331,16 +331,22 @@ def _plain_weight(w: torch.Tensor, dtype: torch.dtype, device: int) -> bool:
     return type(w) is nn.Parameter and w.dtype == dtype and w.get_device() == device and w.is_contiguous() and w.data_ptr() % 16 == 0
 
 
-def _plain_modules(layer: nn.Module) -> bool:
-    """No hooks on the layer's modules, nor global ones: nothing would notice that a forward was not called."""
+def _plain_modules(layer: nn.Module):
+    """``(projections, norms)`` of the layer where they are ``nn.Linear`` without bias and ``RMSNorm`` and have no hooks, nor are there
+    global ones: nothing would notice that a forward was not called.  None otherwise (a module in a projection's place need only be
+    callable: it may have no weight)."""
     mod = nn.modules.module
     if mod._global_forward_hooks or mod._global_forward_pre_hooks:
-        return False
-    a, m = layer._modules["self_attn"], layer._modules["mlp"]
-    for sub in (*a._modules.values(), *m._modules.values(), layer.input_layernorm, layer.post_attention_layernorm):
+        return None
+    a, m = layer._modules["self_attn"]._modules, layer._modules["mlp"]._modules
+    linears = [(a if grp == "self_attn" else m).get(name) for grp, name in layer._LINEARS]
+    norms = (layer._modules.get("input_layernorm"), layer._modules.get("post_attention_layernorm"))
+    if any(type(sub) is not nn.Linear or sub.bias is not None for sub in linears) or any(type(sub) is not RMSNorm for sub in norms):
+        return None
+    for sub in (*linears, *norms):
         if sub._forward_hooks or sub._forward_pre_hooks or "forward" in sub.__dict__:
-            return False
-    return True
+            return None
+    return linears, norms
 
 
 class PagedLlamaDecoderLayer(nn.Module):
@@ -430,24 +436,24 @@ class PagedLlamaDecoderLayer(nn.Module):
         a plain layer (its own modules, no hooks, no biases), 16-bit contiguous weights of x's dtype on the current device, no
         gradients, no autocast."""
         B = x.shape[0]
-        if B > ops.one_call_batch(self.hidden_size, self.mlp.gate_proj.weight.shape[0]) or x.dtype not in (torch.bfloat16, torch.float16) \
-                or torch.is_grad_enabled() or torch.is_autocast_enabled() or type(x) is not torch.Tensor or not x.is_cuda:
+        if B > ops.one_call_batch(self.hidden_size, 0) or x.dtype not in (torch.bfloat16, torch.float16) or torch.is_grad_enabled() \
+                or torch.is_autocast_enabled() or type(x) is not torch.Tensor or not x.is_cuda:
             return None
         dev = x.get_device()
-        if dev != torch.cuda.current_device() or not x.is_contiguous() or x.shape[2] != self.hidden_size or not _plain_modules(self):
+        if dev != torch.cuda.current_device() or not x.is_contiguous() or x.shape[2] != self.hidden_size:
             return None
         kp = handle.k_pool
         if kp.dim() != 4 or not ops.fused_decode_supported(kp, self.num_heads) or kp.shape[1] != self.num_kv_heads or kp.shape[3] != self.head_dim:
             return None
-        weights = []
-        for grp, name in self._LINEARS:
-            m = self._modules[grp]._modules[name]
-            if type(m) is not nn.Linear or m.bias is not None or not _plain_weight(m.weight, x.dtype, dev):
-                return None
-            weights.append(m.weight)
-        norms = (self.input_layernorm, self.post_attention_layernorm)
-        for m in norms:
-            if type(m) is not RMSNorm or not _plain_weight(m.weight, x.dtype, dev):
+        parts = _plain_modules(self)
+        if parts is None:
+            return None
+        linears, norms = parts
+        weights = [m.weight for m in linears]
+        if B > ops.one_call_batch(self.hidden_size, weights[4].shape[0]):
+            return None
+        for w in (*weights, norms[0].weight, norms[1].weight):
+            if not _plain_weight(w, x.dtype, dev):
                 return None
         cos, sin = st.cos, st.sin
         if cos is None:

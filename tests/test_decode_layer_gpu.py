@@ -112,3 +112,25 @@ def test_who_keeps_the_separate_launches(monkeypatch):
     layer.mlp.up_proj = torch.nn.Linear(256, 704, bias=True, device="cuda", dtype=torch.bfloat16)
     run()
     assert len(calls) == 1
+
+
+class _Callable(torch.nn.Module):
+    """What a projection's place needs: a forward, no weight."""
+
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, x):
+        return self.inner(x)
+
+
+@pytest.mark.parametrize("group,name", PagedLlamaDecoderLayer._LINEARS)
+def test_a_projection_need_only_be_callable(group, name, monkeypatch):
+    layer, x, pos, k, v, st, lens = _case(256, 4, 2, 704, 4, torch.bfloat16)
+    want, _, _ = _exact(layer, x, pos, k, v, st, lens)
+    monkeypatch.setattr(ops, "llama_decode_layer", lambda *a, **kw: pytest.fail("a wrapped projection was passed by"))
+    setattr(getattr(layer, group), name, _Callable(getattr(getattr(layer, group), name)))
+    with torch.no_grad():
+        got, _ = layer(x, position_ids=pos, past_key_value=PagedLayerKV(k, v, st))
+    assert (got[:, 0].to(F64) - want).norm() <= 3 * 2.0 ** -9 * want.norm()      # as above
