@@ -6,6 +6,7 @@ anything itself and none falls back to torch: a missing library or a non-CUDA te
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional, Sequence
 
 import torch
@@ -378,6 +379,12 @@ def one_call_batch(width: int, ff: int) -> int:
     300 / 247 with 8, 277 / 284 with 16; width 4096, ff 14336 563 / 712.  Launched from Python a layer takes 250 us of host time
     separately, 70 in one call."""
     return 0 if ff > 8192 else 32 if width <= 1024 else 8 if width <= 2048 else 0
+
+
+@functools.lru_cache(maxsize=256)
+def llama_decode_layer_supported(B: int, width: int, ff: int, Hq: int, Hkv: int, D: int, block_size: int, dtype: torch.dtype) -> bool:
+    """Whether ``llama_decode_layer`` serves these sizes (width and ff in 32s, and what ``fused_decode_supported`` asks for)."""
+    return bool(_lib.load().b200_llama_decode_layer_supported(B, width, ff, Hq, Hkv, D, block_size, DTYPE_ID[dtype]))
 
 
 def llama_decode_layer(x: torch.Tensor, norm1: torch.Tensor, eps1: float, weights: Sequence[torch.Tensor], norm2: torch.Tensor, eps2: float,

@@ -433,8 +433,8 @@ class PagedLlamaDecoderLayer(nn.Module):
     # ---- a decode step in one call -----------------------------------------------------------------
     def _one_call(self, x: torch.Tensor, position_ids, handle: "PagedLayerKV", st: "PagedBatchState") -> Optional[torch.Tensor]:
         """The layer's output for one new token per sequence through ``ops.llama_decode_layer``, or None where that does not apply:
-        a plain layer (its own modules, no hooks, no biases), 16-bit contiguous weights of x's dtype on the current device, no
-        gradients, no autocast."""
+        a plain layer (its own modules, no hooks, no biases) of sizes that the library serves, 16-bit contiguous weights of x's dtype on
+        the current device, no gradients, no autocast."""
         B = x.shape[0]
         if B > ops.one_call_batch(self.hidden_size, 0) or x.dtype not in (torch.bfloat16, torch.float16) or torch.is_grad_enabled() \
                 or torch.is_autocast_enabled() or type(x) is not torch.Tensor or not x.is_cuda:
@@ -450,7 +450,9 @@ class PagedLlamaDecoderLayer(nn.Module):
             return None
         linears, norms = parts
         weights = [m.weight for m in linears]
-        if B > ops.one_call_batch(self.hidden_size, weights[4].shape[0]):
+        ff = weights[4].shape[0]
+        if B > ops.one_call_batch(self.hidden_size, ff) or not ops.llama_decode_layer_supported(
+                B, self.hidden_size, ff, self.num_heads, self.num_kv_heads, self.head_dim, kp.shape[2], x.dtype):
             return None
         for w in (*weights, norms[0].weight, norms[1].weight):
             if not _plain_weight(w, x.dtype, dev):

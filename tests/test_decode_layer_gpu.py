@@ -13,11 +13,12 @@ pytestmark = pytest.mark.gpu
 F64 = torch.float64
 
 
-def _case(W, heads, kv, ff, B, dtype, seed=0, context=70):
+def _case(W, heads, kv, ff, B, dtype, seed=0, context=70, head_dim=None):
     gen = torch.Generator(device="cuda").manual_seed(seed)
-    cfg = LlamaShapeConfig(hidden_size=W, num_attention_heads=heads, num_key_value_heads=kv, intermediate_size=ff, vocab_size=64, num_hidden_layers=1)
+    cfg = LlamaShapeConfig(hidden_size=W, num_attention_heads=heads, num_key_value_heads=kv, intermediate_size=ff, vocab_size=64, num_hidden_layers=1,
+                           head_dim=head_dim)
     layer = PagedLlamaDecoderLayer(cfg, 0, "cuda", dtype)
-    D = W // heads
+    D = layer.head_dim
     with torch.no_grad():
         for p in layer.parameters():
             p.copy_(torch.randn(p.shape, generator=gen, device="cuda") * (p.shape[-1] ** -0.5 if p.dim() == 2 else 0.1) + (p.dim() == 1))
@@ -134,3 +135,15 @@ def test_a_projection_need_only_be_callable(group, name, monkeypatch):
     with torch.no_grad():
         got, _ = layer(x, position_ids=pos, past_key_value=PagedLayerKV(k, v, st))
     assert (got[:, 0].to(F64) - want).norm() <= 3 * 2.0 ** -9 * want.norm()      # as above
+
+
+@pytest.mark.parametrize("W,heads,ff,B,head_dim", [(256, 2, 688, 4, None), (512, 4, 1000, 1, None), (128, 2, 344, 9, None), (144, 2, 704, 3, 64),
+                                                   (256, 4, 8, 32, None)])
+def test_sizes_that_are_no_multiples_of_32_keep_the_separate_launches(W, heads, ff, B, head_dim, monkeypatch):
+    layer, x, pos, k, v, st, lens = _case(W, heads, heads // 2, ff, B, torch.bfloat16, head_dim=head_dim)
+    want, want_k, want_v = _exact(layer, x, pos, k, v, st, lens)
+    monkeypatch.setattr(ops, "llama_decode_layer", lambda *a, **kw: pytest.fail("these sizes are not served"))
+    with torch.no_grad():
+        got, _ = layer(x, position_ids=pos, past_key_value=PagedLayerKV(k, v, st))
+    for a, b in ((got[:, 0], want), (k, want_k), (v, want_v)):
+        assert (a.to(F64) - b).norm() <= 3 * 2.0 ** -9 * b.norm()                # as above
