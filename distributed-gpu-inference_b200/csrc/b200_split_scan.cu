@@ -145,7 +145,7 @@ __device__ __forceinline__ void split3(float x, float y, float dx, float dy, uin
 // a preparing warp writes at once (as they come: 16 lanes to a bank).
 __device__ __forceinline__ int slot_of(int L, int kk) { return L ^ ((L >> 3) & 3) ^ ((kk & 1) << 2); }
 __device__ __forceinline__ bool tame(float x) { return fabsf(x) < kWild; }   // false for NaN
-__device__ __forceinline__ int chunks_of(int count) { return (count + kTok - 1) / kTok; }
+__device__ __forceinline__ int chunks_of(int count) { return (max(count, 0) + kTok - 1) / kTok; }
 
 // Chunks of the sequences before `seq` (a warp's work).
 __device__ __forceinline__ int chunks_before(const SplitSeq* seqs, int seq) {
@@ -651,7 +651,8 @@ split_chain_kernel(const SplitArgs A) {
   const int col_cta = blockIdx.z * kCols;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_chunks = chunks_of(sq.count);
-  const int64_t first = static_cast<int64_t>(chunks_before(A.seqs, blockIdx.x)) * A.heads + blockIdx.y;
+  const int before = chunks_before(A.seqs, blockIdx.x);
+  const int64_t first = static_cast<int64_t>(before) * A.heads + blockIdx.y;
 
   const int r = lane >> 2, c = lane & 3, m = lane >> 3, l8 = lane & 7;
   const int col = col_cta + 16 * warp + r;           // and col + 8
@@ -662,7 +663,8 @@ split_chain_kernel(const SplitArgs A) {
   const T* vp = static_cast<const T*>(A.v) + sq.tok0 * A.stride + static_cast<int64_t>(h) * dv + col_cta;
 
   float S[8][4];          // S^T: columns col, col + 8; channels 8 j + 2 c, + 1
-  bool odd = false;
+  const bool made = before + n_chunks <= A.n_chunks;      // sequences that share tokens may have more chunks than the workspace: no operands
+  bool odd = !made;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
 #pragma unroll
@@ -672,7 +674,7 @@ split_chain_kernel(const SplitArgs A) {
       odd = odd || !tame(S[j][i]);
     }
   }
-  for (int i = threadIdx.x; i < n_chunks; i += kChainNT) odd = odd || A.wild[first + static_cast<int64_t>(i) * A.heads];
+  for (int i = threadIdx.x; made && i < n_chunks; i += kChainNT) odd = odd || A.wild[first + static_cast<int64_t>(i) * A.heads];
   if (__syncthreads_or(odd)) {
     walk_tokens<RULE, T>(A, sq, h, sp, op, vp, 16 * warp + r, in0, in1, reinterpret_cast<float*>(chain_raw));
     return;

@@ -526,8 +526,9 @@ int b200_delta_scan_ext(float* o_raw, const void* q, const void* k, const void* 
 /* The recurrences of b200_gated_scan (rule 0), b200_delta_scan_ext (1) and b200_retention_scan (2) in chunks of 16 tokens on the tensor
  * cores at fp32 precision, for 16-bit inputs and key sizes up to 64: arguments as there (k: the forget gate's logits for rule 0, whose
  * bias and rate are f_bias and lower; bias and rate of rule 1 are dt_bias and a_log; scale: q_scale or k_scale; what a rule does not
- * have may be NULL or 0).  n_tok: at least the tokens that seqs names.  workspace: b200_split_scan_workspace(rule, n_tok, n_seqs,
- * heads) bytes serve `heads` heads at once, 16-byte aligned; with fewer than H heads' the heads go in groups, one head's is needed. */
+ * have may be NULL or 0).  n_tok: the tokens that seqs names (sequences beyond it, as some are when they share tokens, walk token by
+ * token).  workspace: b200_split_scan_workspace(rule, n_tok, n_seqs, heads) bytes serve `heads` heads at once, 16-byte aligned; with
+ * fewer than H heads' the heads go in groups, one head's is needed. */
 int b200_split_scan_supported(int dk, int dtype);
 size_t b200_split_scan_workspace(int rule, int n_tok, int n_seqs, int heads);
 int b200_split_scan(int rule, float* o_raw, const void* q, const void* k, const void* v, int64_t in_stride, const void* beta_logit,

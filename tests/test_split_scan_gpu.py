@@ -98,3 +98,19 @@ def test_values_that_cannot_be_split(rule, where, value):
     first, last = (0, 40) if where == "state" else (40, 141)
     assert torch.equal(got[:, keep], clean[:, keep])
     assert torch.equal(got[:first], clean[:first]) and torch.equal(got[last:], clean[last:])
+
+
+@pytest.mark.parametrize("rule", ["gated", "delta", "retention"])
+def test_sequences_that_share_tokens(rule, monkeypatch):
+    """Five states over the same tokens have more chunks than the tokens have: the read-outs and every state are a sequence's alone."""
+    monkeypatch.setattr(mixer_ops, "SPLIT_SCAN_FROM", (1, 1, 1))
+    dk, dv, H, n = 64, 72, 2, 41
+    parts, state, consts, _, _ = _inputs(dk, dv, H, H, [n], torch.bfloat16, False)
+    state = state[:1].repeat(6, 1, 1, 1)
+    alone = state.clone()
+    want = _run(rule, parts, consts, alone, torch.tensor([(0, n, 1, 0)], dtype=torch.int32, device="cuda"), H, H, n)
+    seqs = torch.tensor([(0, n, i, 0) for i in range(1, 6)], dtype=torch.int32, device="cuda")
+    got = _run(rule, parts, consts, state, seqs, H, H, n)
+    # some in chunks, some token by token: fp32 sums of dk and 16 products, as above
+    assert (got - want).abs().max() <= 2e-5 * want.abs().max() and (state[1:] - alone[1]).abs().max() <= 2e-5 * alone[1].abs().max()
+    assert torch.equal(state[0], alone[0])
