@@ -203,6 +203,11 @@ def split_scan_takes(rule: int, max_count: int, dk: int, dtype: torch.dtype) -> 
     return max_count >= SPLIT_SCAN_FROM[rule] and bool(_lib_().b200_split_scan_supported(dk, DTYPE_ID[dtype]))
 
 
+def _portion(max_count: int, n: int) -> int:
+    """The hint as a portion's length: beyond the step's ``n`` tokens it says nothing about the portions (0: unknown, token by token)."""
+    return max_count if max_count <= n else 0
+
+
 def _split_scan(rule: int, o, q, k, v, stride: int, beta, a, bias, rate, decay, per_channel: bool, state, seqs, G: int, eps: float,
                 scale: float) -> None:
     """``b200_split_scan`` into ``o``; ``beta`` and ``a`` are (tensor or None, row stride)."""
@@ -221,8 +226,9 @@ def gated_scan(zq: torch.Tensor, zf: torch.Tensor, v: torch.Tensor, f_bias: torc
                state: torch.Tensor, seqs: torch.Tensor, H: int, max_count: int = 1 << 20) -> torch.Tensor:
     """Gated linear recurrence over each sequence's tokens; ``state`` fp32 ``[slots, H, dk, dv]`` is read (unless the
     sequence is fresh) and written back.  ``zq / zf [n, H*dk]``, ``v [n, H*dv]`` are column slices of ONE projection
-    (same row stride).  ``max_count``: the largest token count in ``seqs`` (picks the kernel; a hint, not a bound): 16-bit steps with a
-    portion of ``SPLIT_SCAN_FROM`` tokens or more and keys of up to 64 run in chunks on the tensor cores, others token by token.
+    (same row stride).  ``max_count``: the largest token count in ``seqs`` (picks the kernel; a hint, not a bound; beyond ``n``: unknown):
+    16-bit steps with a portion of ``SPLIT_SCAN_FROM`` tokens or more and keys of up to 64 run in chunks on the tensor cores, others
+    token by token.
     Returns the raw read-outs, fp32 ``[n, H, dv]``."""
     _need_cuda(zq, zf, v, state, seqs)
     n = zq.shape[0]
@@ -237,7 +243,7 @@ def gated_scan(zq: torch.Tensor, zf: torch.Tensor, v: torch.Tensor, f_bias: torc
     if seqs.dtype != torch.int32 or seqs.dim() != 2 or seqs.shape[1] != 4 or not seqs.is_contiguous():
         raise ValueError("seqs must be contiguous int32 [n_seqs, 4]")
     o = torch.empty((n, H, dv), dtype=torch.float32, device=zq.device)
-    if split_scan_takes(0, min(max_count, n), dk, zq.dtype):
+    if split_scan_takes(0, _portion(max_count, n), dk, zq.dtype):
         _split_scan(0, o, zq, zf, v, stride, (None, 0), (None, 0), f_bias, lower, None, False, state, seqs, H, 0.0, 0.0)
         return o
     rc = _lib_().b200_gated_scan(o.data_ptr(), zq.data_ptr(), zf.data_ptr(), v.data_ptr(), stride, f_bias.data_ptr(),
@@ -758,7 +764,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_logit: to
         rc = lib.b200_delta_chunk_scan(*head, state.data_ptr(), seqs.data_ptr(), n_seqs, int(max_count), *tail, ws.data_ptr(), dt,
                                        _stream())
         _lib.check_mixers(rc, "b200_delta_chunk_scan")
-    elif split_scan_takes(1, min(max_count, n), dk, q.dtype):
+    elif split_scan_takes(1, _portion(max_count, n), dk, q.dtype):
         _split_scan(1, o, q, k, v, stride, (beta_logit, _rows2(beta_logit)), (a_logit, _rows2(a_logit)), dt_bias, a_log, None,
                     not one_decay, state, seqs, G, unit_eps, q_scale)
     else:
@@ -852,7 +858,7 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
         raise ValueError("decay is contiguous fp32 [H]")
     _check_seqs(seqs)
     o = torch.empty((n, H, dv), dtype=torch.float32, device=q.device)
-    if plan is None and split_scan_takes(2, min(max_count, n), dk, q.dtype):
+    if plan is None and split_scan_takes(2, _portion(max_count, n), dk, q.dtype):
         _split_scan(2, o, q, k, v, stride, (None, 0), (None, 0), None, None, decay, False, state, seqs, H, 0.0, k_scale)
         return o
     lib, dt, st = _lib_(), DTYPE_ID[q.dtype], _stream()

@@ -114,3 +114,12 @@ def test_sequences_that_share_tokens(rule, monkeypatch):
     # some in chunks, some token by token: fp32 sums of dk and 16 products, as above
     assert (got - want).abs().max() <= 2e-5 * want.abs().max() and (state[1:] - alone[1]).abs().max() <= 2e-5 * alone[1].abs().max()
     assert torch.equal(state[0], alone[0])
+
+
+@pytest.mark.parametrize("rule", ["gated", "delta", "retention"])
+def test_a_hint_beyond_the_step_is_no_portion(rule):
+    """160 single tokens without a usable hint walk token by token (in chunks of 16 each would be a chunk): the same bits."""
+    parts, state, consts, seqs, _ = _inputs(64, 48, 2, 2, [1] * 160, torch.bfloat16, False)
+    other = state.clone()
+    want = _run(rule, parts, consts, state, seqs, 2, 2, 1)
+    assert torch.equal(_run(rule, parts, consts, other, seqs, 2, 2, 1 << 20), want) and torch.equal(other, state)
