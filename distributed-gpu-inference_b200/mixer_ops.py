@@ -195,7 +195,8 @@ def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[t
 # 192 tokens 27.0 / 21.8, 38.7 / 30.4, 21.0 / 20.4; 2048 tokens 248 / 151, 379 / 233, 186 / 145; 8 x 64 tokens of 16 heads 20.3 / 18.8,
 # 29.8 / 27.0, 17.9 / 17.3.
 SPLIT_SCAN_FROM = (96, 96, 160)
-SPLIT_SCAN_WORKSPACE = 1 << 30      # bytes of chunk operands at most (one head's if that is more); the heads go in groups beyond
+SPLIT_SCAN_WORKSPACE = 1 << 30      # bytes of chunk operands at most (one head's if that is more); the heads go in groups beyond, smaller
+                                    # ones where memory is short, and token by token where one head's do not fit
 
 
 def split_scan_takes(rule: int, max_count: int, dk: int, dtype: torch.dtype) -> bool:
@@ -208,17 +209,31 @@ def _portion(max_count: int, n: int) -> int:
     return max_count if max_count <= n else 0
 
 
+def _chunk_workspace(one: int, H: int, device: torch.device) -> Optional[torch.Tensor]:
+    """Room for the chunk operands (``one`` bytes a head) of as many of ``H`` heads as the device still holds; None: not for one."""
+    heads = max(1, min(H, SPLIT_SCAN_WORKSPACE // one))
+    while heads:
+        try:
+            return torch.empty(heads * one, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:
+            heads //= 2
+    return None
+
+
 def _split_scan(rule: int, o, q, k, v, stride: int, beta, a, bias, rate, decay, per_channel: bool, state, seqs, G: int, eps: float,
-                scale: float) -> None:
-    """``b200_split_scan`` into ``o``; ``beta`` and ``a`` are (tensor or None, row stride)."""
+                scale: float) -> bool:
+    """``b200_split_scan`` into ``o``; ``beta`` and ``a`` are (tensor or None, row stride).  False, with nothing done, where the device
+    has no memory left for its workspace: the token-by-token scans need none."""
     _, H, dk, dv = state.shape
     lib, n, n_seqs = _lib_(), q.shape[0], seqs.shape[0]
-    one = lib.b200_split_scan_workspace(rule, n, n_seqs, 1)
-    ws = torch.empty(max(one, min(one * H, SPLIT_SCAN_WORKSPACE)), dtype=torch.uint8, device=q.device)
+    ws = _chunk_workspace(lib.b200_split_scan_workspace(rule, n, n_seqs, 1), H, q.device)
+    if ws is None:
+        return False
     rc = lib.b200_split_scan(rule, o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), stride, _ptr(beta[0]), beta[1], _ptr(a[0]), a[1],
                              _ptr(bias), _ptr(rate), _ptr(decay), int(per_channel), state.data_ptr(), seqs.data_ptr(), n_seqs, n, H, G, dk,
                              dv, float(eps), float(scale), ws.data_ptr(), ws.numel(), DTYPE_ID[q.dtype], _stream())
     _lib.check_mixers(rc, "b200_split_scan")
+    return True
 
 
 @_timed
@@ -243,8 +258,8 @@ def gated_scan(zq: torch.Tensor, zf: torch.Tensor, v: torch.Tensor, f_bias: torc
     if seqs.dtype != torch.int32 or seqs.dim() != 2 or seqs.shape[1] != 4 or not seqs.is_contiguous():
         raise ValueError("seqs must be contiguous int32 [n_seqs, 4]")
     o = torch.empty((n, H, dv), dtype=torch.float32, device=zq.device)
-    if split_scan_takes(0, _portion(max_count, n), dk, zq.dtype):
-        _split_scan(0, o, zq, zf, v, stride, (None, 0), (None, 0), f_bias, lower, None, False, state, seqs, H, 0.0, 0.0)
+    if split_scan_takes(0, _portion(max_count, n), dk, zq.dtype) and _split_scan(
+            0, o, zq, zf, v, stride, (None, 0), (None, 0), f_bias, lower, None, False, state, seqs, H, 0.0, 0.0):
         return o
     rc = _lib_().b200_gated_scan(o.data_ptr(), zq.data_ptr(), zf.data_ptr(), v.data_ptr(), stride, f_bias.data_ptr(),
                                  lower.data_ptr(), state.data_ptr(), seqs.data_ptr(), seqs.shape[0], int(max_count), H, dk, dv,
@@ -764,10 +779,9 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_logit: to
         rc = lib.b200_delta_chunk_scan(*head, state.data_ptr(), seqs.data_ptr(), n_seqs, int(max_count), *tail, ws.data_ptr(), dt,
                                        _stream())
         _lib.check_mixers(rc, "b200_delta_chunk_scan")
-    elif split_scan_takes(1, _portion(max_count, n), dk, q.dtype):
-        _split_scan(1, o, q, k, v, stride, (beta_logit, _rows2(beta_logit)), (a_logit, _rows2(a_logit)), dt_bias, a_log, None,
-                    not one_decay, state, seqs, G, unit_eps, q_scale)
-    else:
+    elif not (split_scan_takes(1, _portion(max_count, n), dk, q.dtype) and _split_scan(
+            1, o, q, k, v, stride, (beta_logit, _rows2(beta_logit)), (a_logit, _rows2(a_logit)), dt_bias, a_log, None, not one_decay,
+            state, seqs, G, unit_eps, q_scale)):
         rc = lib.b200_delta_scan_ext(*head, int(not one_decay), state.data_ptr(), seqs.data_ptr(), n_seqs, *tail, dt, _stream())
         _lib.check_mixers(rc, "b200_delta_scan")
     return o
@@ -858,8 +872,8 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
         raise ValueError("decay is contiguous fp32 [H]")
     _check_seqs(seqs)
     o = torch.empty((n, H, dv), dtype=torch.float32, device=q.device)
-    if plan is None and split_scan_takes(2, _portion(max_count, n), dk, q.dtype):
-        _split_scan(2, o, q, k, v, stride, (None, 0), (None, 0), None, None, decay, False, state, seqs, H, 0.0, k_scale)
+    if plan is None and split_scan_takes(2, _portion(max_count, n), dk, q.dtype) and _split_scan(
+            2, o, q, k, v, stride, (None, 0), (None, 0), None, None, decay, False, state, seqs, H, 0.0, k_scale):
         return o
     lib, dt, st = _lib_(), DTYPE_ID[q.dtype], _stream()
 

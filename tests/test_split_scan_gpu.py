@@ -123,3 +123,27 @@ def test_a_hint_beyond_the_step_is_no_portion(rule):
     other = state.clone()
     want = _run(rule, parts, consts, state, seqs, 2, 2, 1)
     assert torch.equal(_run(rule, parts, consts, other, seqs, 2, 2, 1 << 20), want) and torch.equal(other, state)
+
+
+@pytest.mark.parametrize("room", [2, 1, 0], ids=["two_heads", "one_head", "none"])
+@pytest.mark.parametrize("rule", ["gated", "delta", "retention"])
+def test_without_memory_for_the_workspace(rule, room, monkeypatch):
+    """Heads in smaller groups keep their bits; without room for one head's operands the scan walks token by token."""
+    dk, dv, H, lens = 64, 48, 4, [170, 20]
+    parts, state, consts, seqs, _ = _inputs(dk, dv, H, H, lens, torch.bfloat16, False)
+    states = [state.clone() for _ in range(2)]
+    want = _run(rule, parts, consts, states[0], seqs, H, H, max(lens) if room else 1)
+    one = mixer_ops._lib_().b200_split_scan_workspace(1 if rule == "delta" else 0, sum(lens), len(lens), 1)
+    real, asked = torch.empty, []
+
+    def empty(*size, **kw):
+        if kw.get("dtype") == torch.uint8:
+            asked.append(size[0])
+            if size[0] > room * one:
+                raise torch.OutOfMemoryError("no memory")
+        return real(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", empty)
+    got = _run(rule, parts, consts, states[1], seqs, H, H, max(lens))
+    assert asked == [h * one for h in ((4, 2, 1) if room < 2 else (4, 2))]
+    assert torch.equal(got, want) and torch.equal(states[1], states[0])
