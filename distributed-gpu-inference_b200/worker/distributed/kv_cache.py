@@ -504,14 +504,18 @@ class KVCachePool:
         return ids, [slot_of[i] for i in ids]
 
     def give_back(self, ids: List[str], slots: List[int], zero: Callable) -> None:
-        """Leased blocks become free again, their rows zeroed by ``zero(pools, slots)`` as in ``free_sequence``."""
+        """Leased blocks become free again in every layer, their rows zeroed by ``zero(pools, slots)`` as in ``free_sequence``, also when
+        an ``_on_free`` callback fails."""
         for cache in self._layer_caches:
             cache._free_blocks.extend(ids)
             cache._leased -= len(ids)
-            if cache._on_free is not None:
-                for block_id in ids:
-                    cache._on_free(block_id)
-        self._zero_rows([slots] * len(self._layer_caches), zero)
+        try:
+            for cache in self._layer_caches:
+                if cache._on_free is not None:
+                    for block_id in ids:
+                        cache._on_free(block_id)
+        finally:
+            self._zero_rows([slots] * len(self._layer_caches), zero)
 
     def _zero_rows(self, dead: List[List[int]], zero: Callable) -> None:
         groups: Dict[Tuple[int, ...], List[torch.Tensor]] = {}

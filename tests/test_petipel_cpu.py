@@ -181,3 +181,22 @@ def test_leased_blocks_beside_block_objects():
     c = pool()
     c.layer(1)._free_blocks.reverse()
     assert c.lease(2) is None and [x.get_stats()["free_blocks"] for x in c._layer_caches] == [6, 6]
+
+
+def test_leased_blocks_come_back_zeroed_when_a_callback_fails():
+    pool = KVCachePool(num_layers=2, num_heads=0, head_dim=0, block_size=4, max_blocks_per_layer=6, device="cpu", dtype=torch.float32,
+                       layer_shapes=[(1, 8, 8), (2, 4, 8)])
+    ids, slots = pool.lease(3)
+    for c in pool._layer_caches:
+        c.key_pool.fill_(1.0)
+        c.value_pool.fill_(1.0)
+
+    def fails(block_id):
+        raise KeyError(block_id)
+
+    pool.layer(0)._on_free = fails
+    with pytest.raises(KeyError):
+        pool.give_back(ids, slots, lambda pools, s: [p.index_fill_(0, torch.tensor(s), 0) for p in pools])
+    assert [c.get_stats()["free_blocks"] for c in pool._layer_caches] == [6, 6]
+    assert [c.get_stats()["total_blocks"] for c in pool._layer_caches] == [0, 0]
+    assert not any(p[slots].any() for c in pool._layer_caches for p in (c.key_pool, c.value_pool))
