@@ -105,3 +105,35 @@ def test_oracle_properties():
     full = torch.softmax(z, dim=-1).gather(1, ids)
     assert torch.allclose(w, full / full.sum(-1, keepdim=True)) and torch.allclose(w.sum(-1), torch.ones(50, dtype=F64))
     assert torch.equal(ids.sort(dim=1).values, z.topk(3, dim=-1).indices.sort(dim=1).values)
+
+
+@pytest.mark.parametrize("how", ["plain", "gradient", "tangent", "vmap", "jvp", "autocast"])
+def test_heads_by_token_under_transforms(how):
+    from dgi_b200 import mixer_ops
+    gen = torch.Generator().manual_seed(1)
+    a, w = torch.randn(2, 3, 4, generator=gen), torch.randn(2, 4, 5, generator=gen)
+
+    def plain(a, w):
+        return torch.bmm(a, w).transpose(0, 1).reshape(a.shape[1], -1)
+
+    def both(fn):
+        return fn(mixer_ops.heads_by_token), fn(plain)
+
+    with torch.set_grad_enabled(how == "gradient"):
+        if how == "plain":
+            got, want = both(lambda f: f(a, w))
+        elif how == "gradient":
+            p = w.clone().requires_grad_()
+            got, want = both(lambda f: torch.autograd.grad(f(a, p).sum(), p)[0])
+        elif how == "tangent":
+            fw = torch.autograd.forward_ad
+            with fw.dual_level():
+                got, want = both(lambda f: fw.unpack_dual(f(a, fw.make_dual(w, w + 1))).tangent)
+        elif how == "vmap":
+            got, want = both(lambda f: torch.vmap(lambda x: f(a, x))(torch.stack([w, w + 1])))
+        elif how == "jvp":
+            got, want = both(lambda f: torch.func.jvp(lambda x: f(a, x), (w,), (w + 1,))[1])
+        else:
+            with torch.autocast("cpu", dtype=torch.bfloat16):
+                got, want = both(lambda f: f(a.bfloat16(), w))
+    assert got.dtype == want.dtype and torch.equal(got, want)
