@@ -190,23 +190,39 @@ def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[t
     _lib.check_mixers(rc, "b200_biased_prompt_attn")
 
 
-# Tokens of a step's longest portion from which the recurrences (gated, delta, retention) run in chunks on the tensor cores.  B200, bf16,
-# 64 x 128 states, us token by token / in chunks: 8 x 96 tokens of 4 heads gated 15.5 / 15.9, delta 21.4 / 21.5, retention 12.3 / 14.8;
-# 192 tokens 27.0 / 21.8, 38.7 / 30.4, 21.0 / 20.4; 2048 tokens 248 / 151, 379 / 233, 186 / 145; 8 x 64 tokens of 16 heads 20.3 / 18.8,
-# 29.8 / 27.0, 17.9 / 17.3.
+# Tokens of a step's longest portion from which the recurrences (gated, delta, retention) may run in chunks on the tensor cores.  B200, bf16,
+# 64 x 128 states, us token by token / in chunks: 8 x 96 tokens of 4 heads gated 15.4 / 15.8, delta 21.9 / 21.4, retention 16.9 / 18.6; 192
+# tokens 27.4 / 22.2, 38.5 / 30.5, 25.2 / 24.9; 2048 tokens 248 / 154, 382 / 233, 191 / 151.
 SPLIT_SCAN_FROM = (96, 96, 160)
 SPLIT_SCAN_WORKSPACE = 1 << 30      # bytes of chunk operands at most (one head's if that is more); the heads go in groups beyond, smaller
                                     # ones where memory is short, and token by token where one head's do not fit
 
 
-def split_scan_takes(rule: int, max_count: int, dk: int, dtype: torch.dtype) -> bool:
-    """Whether a step whose longest portion has ``max_count`` tokens runs in chunks (rule 0: gated, 1: delta, 2: retention)."""
-    return max_count >= SPLIT_SCAN_FROM[rule] and bool(_lib_().b200_split_scan_supported(dk, DTYPE_ID[dtype]))
+def split_scan_pays(rule: int, longest: int, n: int, n_seqs: int, H: int, dk: int, dv: int) -> bool:
+    """Whether chunks are ahead for a step of ``n`` tokens in ``n_seqs`` portions, the longest of ``longest`` (rule 0: gated, 1: delta, 2:
+    retention; ``H`` states of ``dk`` x ``dv``).  A chunk's work does not shrink with the state (padded to 64 keys and 64-column blocks) nor
+    with the portion (a single token takes a chunk), what chunks shorten is the chain of a long portion.  B200, bf16, us token by token / in
+    chunks (gated):
+
+    64 x 128 states, whose chunks cost less than their tokens: 64 portions of 96, 16 heads 163 / 136; 512 beside 63 single tokens 107 / 74; but
+    96 beside 255, of 4, 16, 32 heads 38 / 46, 122 / 179, 232 / 351, 160 beside 63, 32 heads 77 / 97.
+    64 x 64, 16 heads: 8 of 512 77 / 70, 512 beside 63 95 / 59, but 64 of 96 85 / 100, of 256 205 / 222.  Smaller ones likewise from longer
+    portions on: 32 x 128 8 of 192 38 / 38, 64 of 256 284 / 316; 16 x 16 1 of 512 71 / 45, 8 of 192 29 / 33, 256 of 96 224 / 387.
+    Retention of up to 32 keys walks at 63 ns a token: 1 of 512 39 / 42, 8 of 2048 of 32 x 32 133 / 243."""
+    chunks = n // 16 + n_seqs
+    if longest < SPLIT_SCAN_FROM[rule]:
+        return False
+    if dk > 32 and 13 * dv >= 64 * (8 + 7 * -(-dv // 64)):
+        return 16 * chunks <= 2 * n or 8 * longest >= H * chunks
+    if dk <= 32 and rule == 2:
+        return False
+    return 2 * longest >= 3 * SPLIT_SCAN_FROM[rule] and 16 * chunks <= 4 * n and (16 if dv > 32 else 4) * longest >= H * chunks
 
 
-def _portion(max_count: int, n: int) -> int:
-    """The hint as a portion's length: beyond the step's ``n`` tokens it says nothing about the portions (0: unknown, token by token)."""
-    return max_count if max_count <= n else 0
+def split_scan_takes(rule: int, max_count: int, n: int, n_seqs: int, H: int, dk: int, dv: int, dtype: torch.dtype) -> bool:
+    """Whether such a step runs in chunks (``split_scan_pays``): ``max_count`` tokens in its longest portion, 0 or more than ``n``: unknown."""
+    return max_count <= n and split_scan_pays(rule, max_count, n, n_seqs, H, dk, dv) and \
+        bool(_lib_().b200_split_scan_supported(dk, DTYPE_ID[dtype]))
 
 
 def _chunk_workspace(one: int, H: int, device: torch.device) -> Optional[torch.Tensor]:
@@ -242,8 +258,7 @@ def gated_scan(zq: torch.Tensor, zf: torch.Tensor, v: torch.Tensor, f_bias: torc
     """Gated linear recurrence over each sequence's tokens; ``state`` fp32 ``[slots, H, dk, dv]`` is read (unless the
     sequence is fresh) and written back.  ``zq / zf [n, H*dk]``, ``v [n, H*dv]`` are column slices of ONE projection
     (same row stride).  ``max_count``: the largest token count in ``seqs`` (picks the kernel; a hint, not a bound; beyond ``n``: unknown):
-    16-bit steps with a portion of ``SPLIT_SCAN_FROM`` tokens or more and keys of up to 64 run in chunks on the tensor cores, others
-    token by token.
+    16-bit steps with long portions (``split_scan_pays``) and keys of up to 64 run in chunks on the tensor cores, others token by token.
     Returns the raw read-outs, fp32 ``[n, H, dv]``."""
     _need_cuda(zq, zf, v, state, seqs)
     n = zq.shape[0]
@@ -258,7 +273,7 @@ def gated_scan(zq: torch.Tensor, zf: torch.Tensor, v: torch.Tensor, f_bias: torc
     if seqs.dtype != torch.int32 or seqs.dim() != 2 or seqs.shape[1] != 4 or not seqs.is_contiguous():
         raise ValueError("seqs must be contiguous int32 [n_seqs, 4]")
     o = torch.empty((n, H, dv), dtype=torch.float32, device=zq.device)
-    if split_scan_takes(0, _portion(max_count, n), dk, zq.dtype) and _split_scan(
+    if split_scan_takes(0, max_count, n, seqs.shape[0], H, dk, dv, zq.dtype) and _split_scan(
             0, o, zq, zf, v, stride, (None, 0), (None, 0), f_bias, lower, None, False, state, seqs, H, 0.0, 0.0):
         return o
     rc = _lib_().b200_gated_scan(o.data_ptr(), zq.data_ptr(), zf.data_ptr(), v.data_ptr(), stride, f_bias.data_ptr(),
@@ -748,8 +763,8 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_logit: to
     is read (unless the sequence is fresh) and written back.  ``q / k [n, G*dk]`` and ``v [n, H*dv]`` are column
     slices of ONE tensor (same row stride), ``beta_logit [n, H]``.  Returns fp32 ``[n, H, dv]``.  ``max_count``: the
     largest token count in ``seqs`` (0: unknown), picks the kernel.  One decay per head: steps of single tokens, and bf16 steps with a
-    portion of ``CHUNK_SCAN_FROM`` tokens or more in chunks of 64 on the tensor cores; otherwise, 16-bit steps with a portion of
-    ``SPLIT_SCAN_FROM`` tokens or more and keys of up to 64 in chunks of 16 at fp32 precision; others token by token."""
+    portion of ``CHUNK_SCAN_FROM`` tokens or more in chunks of 64 on the tensor cores; otherwise, 16-bit steps with long
+    portions (``split_scan_pays``) and keys of up to 64 in chunks of 16 at fp32 precision; others token by token."""
     _need_cuda(q, k, v, beta_logit, a_logit, dt_bias, a_log, state, seqs)
     n = q.shape[0]
     _, H, dk, dv = state.shape
@@ -779,7 +794,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta_logit: to
         rc = lib.b200_delta_chunk_scan(*head, state.data_ptr(), seqs.data_ptr(), n_seqs, int(max_count), *tail, ws.data_ptr(), dt,
                                        _stream())
         _lib.check_mixers(rc, "b200_delta_chunk_scan")
-    elif not (split_scan_takes(1, _portion(max_count, n), dk, q.dtype) and _split_scan(
+    elif not (split_scan_takes(1, max_count, n, n_seqs, H, dk, dv, q.dtype) and _split_scan(
             1, o, q, k, v, stride, (beta_logit, _rows2(beta_logit)), (a_logit, _rows2(a_logit)), dt_bias, a_log, None, not one_decay,
             state, seqs, G, unit_eps, q_scale)):
         rc = lib.b200_delta_scan_ext(*head, int(not one_decay), state.data_ptr(), seqs.data_ptr(), n_seqs, *tail, dt, _stream())
@@ -872,7 +887,7 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
         raise ValueError("decay is contiguous fp32 [H]")
     _check_seqs(seqs)
     o = torch.empty((n, H, dv), dtype=torch.float32, device=q.device)
-    if plan is None and split_scan_takes(2, _portion(max_count, n), dk, q.dtype) and _split_scan(
+    if plan is None and split_scan_takes(2, max_count, n, seqs.shape[0], H, dk, dv, q.dtype) and _split_scan(
             2, o, q, k, v, stride, (None, 0), (None, 0), None, None, decay, False, state, seqs, H, 0.0, k_scale):
         return o
     lib, dt, st = _lib_(), DTYPE_ID[q.dtype], _stream()

@@ -200,3 +200,17 @@ def test_leased_blocks_come_back_zeroed_when_a_callback_fails():
     assert [c.get_stats()["free_blocks"] for c in pool._layer_caches] == [6, 6]
     assert [c.get_stats()["total_blocks"] for c in pool._layer_caches] == [0, 0]
     assert not any(p[slots].any() for c in pool._layer_caches for p in (c.key_pool, c.value_pool))
+
+
+@pytest.mark.parametrize("rule,state,heads,portions,chunks", [
+    # (rule, state, heads, portions, ahead in chunks), as measured
+    (0, (64, 128), 16, [1900] * 6, True), (1, (64, 128), 8, [2048] * 8, True), (2, (64, 128), 16, [1024] * 5, True),
+    (0, (64, 128), 4, [95] * 8, False), (2, (64, 128), 16, [159], False), (0, (64, 128), 16, [512] + [1] * 63, True),
+    (1, (64, 128), 32, [2048] + [1] * 255, True), (0, (64, 128), 16, [96] + [1] * 255, False), (1, (64, 128), 4, [96] + [1] * 255, False),
+    (0, (64, 128), 32, [160] + [1] * 63, False), (0, (64, 64), 16, [512] * 8, True), (0, (64, 64), 16, [96] * 64, False),
+    (1, (64, 72), 16, [256] * 64, False), (1, (32, 128), 16, [512], True), (1, (32, 128), 16, [256] * 64, False),
+    (0, (16, 16), 16, [512], True), (0, (16, 16), 16, [192] * 8, False), (0, (32, 32), 16, [2048] * 8, False),
+    (2, (32, 128), 16, [512], False), (2, (32, 32), 16, [2048] * 8, False), (2, (64, 64), 16, [512] * 8, True)])
+def test_which_steps_run_in_chunks(rule, state, heads, portions, chunks):
+    from dgi_b200 import mixer_ops
+    assert mixer_ops.split_scan_pays(rule, max(portions), sum(portions), len(portions), heads, *state) is chunks
