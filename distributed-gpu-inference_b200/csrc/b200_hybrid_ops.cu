@@ -1296,9 +1296,11 @@ int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bi
   return tile_attn_supported(H, G, dk, dv, same_pool != 0, bias != 0, dtype) ? 1 : 0;
 }
 
-int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens) { return tile_attn_rows(rep, G, dk, n_tokens, false); }
+int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens) { return tile_attn_rows(rep, G, dk, n_tokens, false, true); }
 
-int b200_tile_attn_rows_ext(int rep, int G, int dk, int n_tokens, int heavy) { return tile_attn_rows(rep, G, dk, n_tokens, heavy != 0); }
+int b200_tile_attn_rows_ext(int rep, int G, int dk, int n_tokens, int heavy) {
+  return tile_attn_rows(rep, G, dk, n_tokens, (heavy & 1) != 0, (heavy & 2) == 0);
+}
 
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows) {
   return tile_attn_splits(n_tiles, key_tiles, G, dk, tile_rows);

@@ -706,10 +706,12 @@ bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, in
 // 256 rows share a fetched key tile and its biases, but only one such CTA runs per SM and nothing covers its beginning and end; with pages
 // by the copy engine two CTAs of 128 rows are ahead where the softmax does no more than scale (8 x 2048 tokens, 16 heads over 4: 213 us
 // against 225; 5 x 1024 under a window of 512: 44.6 / 46.0), 256 rows where it also adds biases or caps (257 against 285, 323 against 369;
-// 8 x 700 tokens of 8 heads, 1.2 rounds of CTAs, biases: 36.3 / 39.6) and the step fills the SMs once.
-int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy) {
+// 8 x 700 tokens of 8 heads, 1.2 rounds of CTAs, biases: 36.3 / 39.6) and the step fills the SMs once.  Pages that come row by row keep 256
+// rows from three rounds on (8 x 1000 tokens of 16 heads, pages of 24: 82 us against 94).
+int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy, bool boxes) {
   const int64_t ctas = static_cast<int64_t>(n_tokens) * rep / (2 * kTileRows) * G;
-  return heavy && dk <= 128 && ctas >= kNumSMs ? 2 * kTileRows : kTileRows;
+  const bool wide = heavy ? ctas >= kNumSMs : !boxes && ctas >= 3 * kNumSMs;
+  return wide && dk <= 128 ? 2 * kTileRows : kTileRows;
 }
 
 // Keys are divided while the chip has room for more CTAs, a share being worth its part of the merge: three tiles of 64 keys where

@@ -178,7 +178,7 @@ class ParallelMixer(nn.Module):
                                        st.slot_mapping, st.tok_pos, H, interleaved=True)
         attn = buf[:, :self.Kl].unflatten(1, (H, dv))
         if self.tensor_cores:
-            tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles, softcap=self.softcap > 0)
+            tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles, softcap=self.softcap > 0, page=cache.k_pool.shape[2])
             args = (attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables)
             kw = dict(sink=self.sink, window=self.window, softcap=self.softcap)
             if tiles is not None:

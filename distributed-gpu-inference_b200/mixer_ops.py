@@ -652,9 +652,11 @@ def mixed_prompt_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Ten
     _lib.check_mixers(rc, "b200_mixed_prompt_attn")
 
 
-def tile_rows(H: int, G: int, dk: int, n_tokens: int, heavy: bool = False) -> int:
-    """Query rows (tokens x heads of a kv group) of a ``tile_attention`` tile for portions of ``n_tokens`` tokens in all."""
-    return int(_lib_().b200_tile_attn_rows_ext(H // G, int(G), int(dk), int(n_tokens), int(heavy)))
+def tile_rows(H: int, G: int, dk: int, n_tokens: int, heavy: bool = False, page: int = 16) -> int:
+    """Query rows (tokens x heads of a kv group) of a ``tile_attention`` tile for portions of ``n_tokens`` tokens in all (``heavy``: with
+    distance biases or a soft cap) over pages of ``page`` tokens."""
+    by_row = 2 if page % 8 or 64 % page else 0      # pages that the copy engine cannot fetch whole
+    return int(_lib_().b200_tile_attn_rows_ext(H // G, int(G), int(dk), int(n_tokens), int(heavy) | by_row))
 
 
 def tile_attention_supported(H: int, G: int, dk: int, dv: int, same_pool: bool, bias: bool, dtype: torch.dtype) -> bool:

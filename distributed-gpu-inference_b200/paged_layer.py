@@ -231,8 +231,9 @@ class RaggedBatchState:
         """Tiles of up to ``cap`` tokens over the portions of ``at_least`` tokens or more (tensor-core prompt kernel)."""
         return self._plan(("prompt", cap, at_least), cap, lambda count, _context: count >= at_least)
 
-    def attention_tiles(self, H: int, G: int, dk: int, cap: int, whole: bool, bias: bool = False, softcap: bool = False):
-        """How an attention layer of H heads over G kv heads of key size ``dk`` serves the step: ``(tiles, rest)``.  ``tiles``: the
+    def attention_tiles(self, H: int, G: int, dk: int, cap: int, whole: bool, bias: bool = False, softcap: bool = False,
+                        page: int = 16):
+        """How an attention layer of H heads over G kv heads of key size ``dk`` (pages of ``page`` tokens) serves the step: ``(tiles, rest)``.  ``tiles``: the
         long portions for ``mixer_ops.tile_attention``, ``(tile list, rows per tile, longest context of these)`` (None: none, or not
         ``whole``: the layer's sizes are not served there); ``rest``: the others in tiles of up to ``cap`` tokens, ``(tile list, most
         tokens of a tile, longest context of these)`` (None: none)."""
@@ -240,7 +241,7 @@ class RaggedBatchState:
 
         if self._tiles is None:
             self._tiles = {}
-        key = ("attention", H, G, dk, cap, whole, bias, softcap)
+        key = ("attention", H, G, dk, cap, whole, bias, softcap, page)
         if key not in self._tiles:      # the step's layers of one layout share it
             cut = mixer_ops.tile_attention_from(H, G, bias) if whole else 1 << 30
 
@@ -256,7 +257,7 @@ class RaggedBatchState:
             long, short = [s for s in shapes if takes(*s)], [t for n, t in shapes if not takes(n, t)]
             tiles = rest = None
             if long:
-                rows = mixer_ops.tile_rows(H, G, dk, sum(n for n, _ in long), bias or softcap)
+                rows = mixer_ops.tile_rows(H, G, dk, sum(n for n, _ in long), bias or softcap, page)
                 tiles = self._plan((key, "tiles"), max(1, rows // (H // G)), takes)[0], rows, max(t for _, t in long)
             if short:
                 rest = *self._plan((key, "rest"), cap, lambda n, t: not takes(n, t)), max(short)

@@ -168,7 +168,7 @@ class BiasedPagedAttention(nn.Module):
         q, gate = proj[:, :a], proj[:, c:c + H]
         attn = torch.empty((h.shape[0], H * dv), dtype=h.dtype, device=h.device)
         if self.tensor_core_prompt:   # 16-bit storage and sizes the tensor-core kernel takes: portions and single tokens
-            tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.prompt_tile_tokens(H, G), self.in_tiles, bias=True)
+            tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.prompt_tile_tokens(H, G), self.in_tiles, bias=True, page=cache.k_pool.shape[2])
             if tiles is not None:
                 mixer_ops.tile_attention(attn.view(-1, H, dv), q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
                                          tiles[0], st.tok_pos, self.scale, gate=gate, rows=tiles[1], max_context=tiles[2],

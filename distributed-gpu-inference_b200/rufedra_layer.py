@@ -203,7 +203,7 @@ class KeyValueSelectiveMixer(nn.Module):
                                        st.tok_pos, H, interleaved=False, unit_norm=True)
         attn = buf[:, :self.Kl].unflatten(1, (H, dk))
         if self.tensor_cores:
-            tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            tiles, rest = st.attention_tiles(H, G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles, page=cache.k_pool.shape[2])
             args = (attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables)
             kw = dict(window=self.window, gate=gate)
             if tiles is not None:

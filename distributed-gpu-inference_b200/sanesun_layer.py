@@ -214,7 +214,7 @@ class LatentAttention(nn.Module):
         q_lat = torch.bmm(q.transpose(0, 1), self.w_uk)                          # [H, n, r]
         o_lat = torch.empty((H, n, r), dtype=h.dtype, device=h.device)
         if self.tensor_cores:
-            tiles, rest = st.attention_tiles(H, 1, r, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            tiles, rest = st.attention_tiles(H, 1, r, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles, page=cache.k_pool.shape[2])
             args = (o_lat.transpose(0, 1), q_lat.transpose(0, 1), cache.k_pool, cache.k_pool, st.block_tables)
             kw = dict(gate=proj[:, c[2]:c[2] + H])
             if tiles is not None:

@@ -172,7 +172,7 @@ class LatentRotaryAttention(nn.Module):
         torch.bmm(q[:, :, :dn].transpose(0, 1), self.w_uk, out=q_lat[:, :, :r].transpose(0, 1))
         o_lat = torch.empty((H, n, r), dtype=h.dtype, device=h.device)
         if self.tensor_cores:
-            tiles, rest = st.attention_tiles(H, 1, r + dr, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            tiles, rest = st.attention_tiles(H, 1, r + dr, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles, page=cache.k_pool.shape[2])
             args = (o_lat.transpose(0, 1), q_lat, cache.k_pool, cache.k_pool, st.block_tables)
             kw = dict(sink=self.sink, window=self.window, value_width=r)
             if tiles is not None:
@@ -236,7 +236,7 @@ class DifferentialAttention(nn.Module):
                                        st.slot_mapping, st.tok_pos, 2 * H)
         maps = torch.empty((n, 2 * H, dv), dtype=torch.float32, device=h.device)    # rounded only after their difference
         if self.tensor_cores:
-            tiles, rest = st.attention_tiles(2 * H, 2 * G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles)
+            tiles, rest = st.attention_tiles(2 * H, 2 * G, dk, mixer_ops.PROMPT_TILE_TOKENS, self.in_tiles, page=cache.k_pool.shape[2])
             args = (maps, q.unflatten(1, (2 * H, dk)), k_pool, cache.v_pool, st.block_tables)
             kw = dict(chunk=self.chunk, value_div=2)
             if tiles is not None:

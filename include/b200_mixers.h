@@ -490,13 +490,16 @@ int b200_mixed_prompt_attn_ext3(void* out, int64_t out_tok_stride, int64_t out_h
                                 float* workspace, int dtype, void* stream);
 
 /* b200_mixed_prompt_attn_ext2 and b200_biased_prompt_attn for prompt portions on the fifth-generation tensor cores: tiles of up to
- * tile_rows / (H / G) tokens, tile_rows 128 or (dk <= 128) 256, as b200_tile_attn_rows picks for n_tokens tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
- * touched.  bias_lut fp32 [H][lut_len] with temp_coef / temp_every as in b200_biased_prompt_attn, or NULL.  The values are v_pool's
+ * tile_rows / (H / G) tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
+ * touched.  tile_rows: 128 or (dk <= 128) 256; b200_tile_attn_rows_ext picks for n_tokens tokens, heavy = 1 with distance biases or a
+ * soft cap, + 2 with pages other than 8, 16, 32 or 64 tokens (b200_tile_attn_rows: heavy = 0, for which 128 is ahead at every size).
+ * bias_lut fp32 [H][lut_len] with temp_coef / temp_every as in b200_biased_prompt_attn, or NULL.  The values are v_pool's
  * rows, or the first dv columns of the key rows when v_pool == k_pool.  n_splits > 1 divides the keys over as many CTAs and needs a
- * workspace fp32 [n_splits][n_tiles][tile_rows / (H / G)][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte aligned query rows. */
+ * workspace fp32 [n_splits][n_tiles][tile_rows / (H / G)][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte
+ * aligned query rows. */
 int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bias, int dtype);
 int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens);
-int b200_tile_attn_rows_ext(int rep, int G, int dk, int n_tokens, int heavy);   /* heavy: with distance biases or a soft cap */
+int b200_tile_attn_rows_ext(int rep, int G, int dk, int n_tokens, int heavy);
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows);
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,

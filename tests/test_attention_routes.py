@@ -117,3 +117,13 @@ def test_a_workspace_beyond_its_bound_is_not_allocated(workspaces):
     mixer_ops.biased_prompt_attention(p["out"].flatten(1), p["q"].flatten(1), None, p["k"], p["v"], st.block_tables, rest[0], st.tok_pos,
                                       torch.zeros(H, 8), 1.0, 0.0, 1, H, max_tile_tokens=rest[1], max_context=rest[2])
     assert workspaces == []
+
+
+@pytest.mark.parametrize("page,rows", [(8, 128), (16, 128), (64, 128), (24, 256), (7, 256), (128, 256)])
+def test_pages_that_come_row_by_row_share_wider_tiles(page, rows):
+    """Plain attention: 128 rows where the copy engine fetches whole pages; where it cannot, 256 from three rounds of CTAs on.  Biases and
+    caps: 256 from one round on, whatever the pages."""
+    assert mixer_ops.tile_rows(16, 4, 128, 8000, page=page) == rows and mixer_ops.tile_rows(16, 4, 128, 7000, page=page) == 128
+    assert mixer_ops.tile_rows(16, 4, 128, 2400, heavy=True, page=page) == 256 and mixer_ops.tile_rows(16, 4, 256, 8000, True, page) == 128
+    st = _step([(1000, 0)] * 8)
+    assert st.attention_tiles(16, 4, 128, 16, True, page=page)[0][1] == rows
