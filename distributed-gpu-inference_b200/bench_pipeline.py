@@ -1,4 +1,4 @@
-"""bench.py's multi-GPU leg: layer-sharded decode over N ranks (BASELINE config 4 by default).
+"""bench.py's multi-GPU leg: layer-sharded decode over N ranks (the 70B shape by default).
 
 Launched by torchrun, one rank per GPU.  Rank r builds layers ``get_layer_range_for_worker(L, N, r)`` of the
 named shape (random-init, same seed scheme on every partition), one ``PagedDecodeEngine`` per micro-batch, and
@@ -6,7 +6,7 @@ joins a ``LayerPipeline`` with a vocabulary-parallel head.  Timed region: K deco
 bracketed by barrier + synchronize, CUDA events on every rank, MAX over ranks.
 
 Every run also PROVES what it times (the ``parity`` object of the line):
-  * BASELINE config 1 (tiny fp32 model, real prompt pass, 64 greedy tokens) goes through the same N-rank pipeline
+  * the tiny model (fp32, real prompt pass, 64 greedy tokens) goes through the same N-rank pipeline
     and must reproduce the reference's golden tokens (tests/golden/tiny_decode.json for N <= 4 and the 8-layer
     fixture tiny8_decode.json for every N);
   * the first sequences of micro-batch 0 of each timed leg get a REAL prompt pass, and the tokens the pipeline
@@ -92,7 +92,7 @@ def _free():
 
 
 # -----------------------------------------------------------------------------------------------------------------
-# parity, part 1: BASELINE config 1 through the N-rank pipeline against the reference's golden tokens
+# parity, part 1: the tiny model through the N-rank pipeline against the reference's golden tokens
 # -----------------------------------------------------------------------------------------------------------------
 def _golden_through_pipeline(name, rank, world, dev, groups):
     """Decode the fixture's prompts (real prompt pass + 63 steps, fp32) through the N-rank pipeline with the
@@ -212,7 +212,7 @@ def _agreement_vs_single_gpu(cfg, prompts, pipe_tokens, ctx, dev, fuse):
 # P/D hand-off
 # -----------------------------------------------------------------------------------------------------------------
 def _measure_pd_handoff(rank, world, dev):
-    """Third part of BASELINE's metric: prefill -> decode KV hand-off, rank i -> rank i + N/2 on all pairs at once,
+    """Third part of the metric: prefill -> decode KV hand-off, rank i -> rank i + N/2 on all pairs at once,
     one fused peer-push launch per sequence (8B-shape blocks, 8 layers x 4 sequences of 4k tokens = 512 MiB per
     pair), CUDA events between barriers, max over ranks.  Afterwards every pair moves the same source blocks a
     second time through torch indexing + NCCL send/recv and the receiver compares them with what the push left in

@@ -132,7 +132,7 @@ def compute_prefix_hash(token_ids: List[int]) -> str:
 def compute_prefix_hash_wide(token_ids: List[int]) -> str:
     """Extension for real vocabularies: little-endian uint32 per token, same digest and truncation.
 
-    No reference counterpart (SURVEY.md §9 defect 7); equals ``compute_prefix_hash`` only for empty input.
+    No reference counterpart (the reference's hash fails for ids of 256 and more); equals ``compute_prefix_hash`` only for empty input.
     """
     buf = b"".join(int(t).to_bytes(4, "little", signed=False) for t in token_ids)
     return hashlib.sha256(buf).hexdigest()[:16]

@@ -14,7 +14,7 @@ namespace b200 {
 // append
 // ---------------------------------------------------------------------------------------------------------
 // A CTA takes TOKS consecutive tokens.  The first TOKS threads turn the tokens' slots into pool row offsets once (the
-// only divisions of the kernel; the flat-index version of round 1 spent two 64-bit divisions per 16-byte vector and
+// only divisions of the kernel; a flat index spent two 64-bit divisions per 16-byte vector and
 // was issue-bound at 62 % of the copy peak, profiles/r02_ncu_append.md); after that thread x owns 16-byte vector x of
 // the K|V row pair of every token of the CTA — TOKS independent loads in flight before the first store, consecutive
 // threads on consecutive vectors of one contiguous head row.

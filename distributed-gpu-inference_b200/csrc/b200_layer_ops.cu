@@ -105,7 +105,7 @@ add_rmsnorm_kernel(T* __restrict__ out, T* __restrict__ resid_out, const T* __re
 // Grid (groups of kRopeToks tokens, chunks of 128 work items); a thread handles one 16-byte vector of the first half of
 // a head together with its partner vector in the second half (rotate-half pairs d and d + D/2), for every token of
 // the CTA's group.  The tokens' slots are turned into pool row offsets once per CTA (shared memory), so the per-thread
-// work is loads, the rotation and stores; a CTA per token (round 1) spent its time on launch overhead and on two
+// work is loads, the rotation and stores; a CTA per token spent its time on launch overhead and on two
 // 64-bit divisions per thread (0.69 of the copy peak on a 16k-token prompt chunk).
 constexpr int kRopeToks = 4;
 

@@ -27,6 +27,7 @@
 // B200, bf16, 64 x 128 states, us token by token / here (operands + chain): gated, 6 portions of up to 1780 tokens of 16 heads 395 / 223
 // (68 + 155); delta, 8 x 2048 of 8 heads 467 / 304 (128 + 176); retention, 5 x 1024 of 16 heads 184 / 125 (36 + 89).
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "../../include/b200_mixers.h"
@@ -871,7 +872,13 @@ int launch_split(SplitArgs& A, void* workspace, size_t bytes, cudaStream_t strea
   constexpr size_t smem = sizeof(Chain<RULE, T>);
   static_assert(kStages == 3 && sizeof(Prep<RULE>) <= 48 * 1024 && smem <= static_cast<size_t>(kMaxSmem));
   auto chain = split_chain_kernel<RULE, T>;
-  cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  static std::atomic<uint64_t> ready{0};      // a bit per device: the limit is always the same, a call need not set it again
+  int device = 0;
+  cudaGetDevice(&device);
+  if (device >= 64 || !(ready.load(std::memory_order_acquire) >> device & 1)) {
+    cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (device < 64) ready.fetch_or(1ull << device, std::memory_order_release);
+  }
   for (A.h0 = 0; A.h0 < A.H; A.h0 += most) {
     A.heads = std::min(most, A.H - A.h0);
     A.ops = static_cast<unsigned char*>(workspace);

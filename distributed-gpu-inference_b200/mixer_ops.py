@@ -5,6 +5,7 @@ library, nothing here computes and nothing falls back to torch.  Activations of 
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -19,8 +20,6 @@ EVENTS: Optional[list] = None
 
 
 def _timed(fn):
-    import functools
-
     @functools.wraps(fn)
     def wrapper(*args, **kwargs):
         if EVENTS is None:
@@ -221,8 +220,18 @@ def split_scan_pays(rule: int, longest: int, n: int, n_seqs: int, H: int, dk: in
 
 def split_scan_takes(rule: int, max_count: int, n: int, n_seqs: int, H: int, dk: int, dv: int, dtype: torch.dtype) -> bool:
     """Whether such a step runs in chunks (``split_scan_pays``): ``max_count`` tokens in its longest portion, 0 or more than ``n``: unknown."""
-    return max_count <= n and split_scan_pays(rule, max_count, n, n_seqs, H, dk, dv) and \
-        bool(_lib_().b200_split_scan_supported(dk, DTYPE_ID[dtype]))
+    return max_count <= n and split_scan_pays(rule, max_count, n, n_seqs, H, dk, dv) and _split_scan_supported(dk, dtype)
+
+
+@functools.lru_cache(maxsize=None)
+def _split_scan_supported(dk: int, dtype: torch.dtype) -> bool:
+    return bool(_lib_().b200_split_scan_supported(dk, DTYPE_ID[dtype]))
+
+
+@functools.lru_cache(maxsize=None)
+def _chunk_bytes(rule: int) -> int:
+    """Workspace of one chunk and head."""
+    return int(_lib_().b200_split_scan_workspace(rule, 0, 1, 1))
 
 
 def _chunk_workspace(one: int, H: int, device: torch.device) -> Optional[torch.Tensor]:
@@ -242,7 +251,7 @@ def _split_scan(rule: int, o, q, k, v, stride: int, beta, a, bias, rate, decay, 
     has no memory left for its workspace: the token-by-token scans need none."""
     _, H, dk, dv = state.shape
     lib, n, n_seqs = _lib_(), q.shape[0], seqs.shape[0]
-    ws = _chunk_workspace(lib.b200_split_scan_workspace(rule, n, n_seqs, 1), H, q.device)
+    ws = _chunk_workspace((n // 16 + n_seqs) * _chunk_bytes(rule), H, q.device)
     if ws is None:
         return False
     rc = lib.b200_split_scan(rule, o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), stride, _ptr(beta[0]), beta[1], _ptr(a[0]), a[1],

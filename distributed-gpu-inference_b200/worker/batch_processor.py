@@ -7,7 +7,7 @@ results delivered through per-request futures.  The engine protocol is the refer
 ``inference_async(params)``, ``inference(params)``; an ``Exception`` instance in the returned list fails only that
 request (:237-242).  ``dgi_b200.engine.PagedDecodeEngine`` and ``dgi_b200.worker.engines.PagedLLMEngine`` provide
 ``batch_inference``, so a batch really runs as one batch on the GPU (in the reference no engine implements it and
-every batch degrades to the serial fallback, SURVEY.md §9 #12).
+every batch degrades to the serial fallback).
 """
 from __future__ import annotations
 

@@ -2,7 +2,7 @@
 
 Drop-in for the reference's ``worker/distributed/kv_cache.py``: same classes, constructor arguments, return
 values, ``get_stats()`` keys and — bit for bit — the same block-id sequence for any alloc/free/evict schedule
-(SURVEY.md Appendix A; pinned by tests/golden/allocator_*.json which were produced by the reference itself).
+(pinned by tests/golden/allocator_*.json which were produced by the reference itself).
 
 What is kept exactly
   * pool layout ``[max_blocks, num_heads, block_size, head_dim]`` for K and for V (reference :130-144)
@@ -12,7 +12,7 @@ What is kept exactly
   * ``KVCachePool.allocate_sequence``: ceil-div block count, layer-major (reference :283-313)
   * tier keys ``"{prefix_hash}:{layer}"``, CPU LRU capacity formula, pickle payload (reference :326-555)
 
-Deliberate deviations (each is listed in DESIGN.md)
+Deliberate deviations
   1. pools are created on any device, not only CUDA (#1) — the reference leaves CPU caches unusable
   2. ``KVCachePool`` / ``DistributedKVCacheManager`` accept ``dtype=`` (#2); default stays fp16
   3. blocks handed out earlier in the same ``allocate_sequence`` call, and blocks pinned with ``pin()``,
@@ -257,7 +257,7 @@ class PagedKVCache:
 
     def free_blocks(self, block_ids: Iterable[str], dead: Optional[List[int]] = None) -> None:
         """``free_block`` for many ids with the same observable result, but the pool rows that reach ref-count 0
-        are zeroed with one ``index_fill_`` per pool instead of two launches per block (SURVEY.md §9 #10).  With ``dead``
+        are zeroed with one ``index_fill_`` per pool instead of two launches per block.  With ``dead``
         those rows are appended to it instead and the caller zeroes them."""
         owed = dead is not None
         if dead is None:
@@ -310,7 +310,7 @@ class PagedKVCache:
         return self._block_to_slot[block_id]
 
     def pin(self, block_ids: Iterable[str]) -> None:
-        """Protect blocks of a live sequence from LRU eviction (SURVEY.md §9 #8).  Pins are counted: a block shared
+        """Protect blocks of a live sequence from LRU eviction.  Pins are counted: a block shared
         by several live sequences is pinned once per sequence and stays protected until each has called ``unpin``.
         Freeing a sequence lifts no pin of a block that survives the free — whoever pinned must unpin."""
         pinned = self._pinned
@@ -400,7 +400,7 @@ class KVCachePool:
                           shared_prefix: Optional[List[List[CacheBlock]]] = None) -> List[List[CacheBlock]]:
         """Blocks for ``seq_len`` tokens in every layer (reference :283-313).
 
-        ``shared_prefix`` (addition, SURVEY.md §8f row 3): per layer, blocks of an existing sequence that hold the
+        ``shared_prefix`` (addition): per layer, blocks of an existing sequence that hold the
         same leading tokens.  They are reused with ``add_ref`` — the copy-on-write sharing ``CacheBlock.ref_count``
         was designed for (reference :63-72) — and only the remainder is freshly allocated, so the sequences' block
         tables start with identical slots.  Shared blocks (ref_count > 1) are never evicted (reference :232-234).
@@ -743,7 +743,7 @@ class DistributedKVCacheManager:
 
 
 # ---------------------------------------------------------------------------------------------------------
-# Prefix reuse per block (SURVEY.md §8f row 3).  The reference keeps ONE block per (prefix hash, layer) in
+# Prefix reuse per block.  The reference keeps ONE block per (prefix hash, layer) in
 # ``_prefix_index`` and hashes ``bytes(token_ids)``, which fails for ids >= 256 (reference :384-387, :462).
 # ---------------------------------------------------------------------------------------------------------
 def chained_block_hashes(token_ids: Sequence[int], block_size: int) -> List[str]:

@@ -6,7 +6,7 @@ protobuf-like request objects and returning plain dicts, with the shard and the 
 constructor (:43-53).  Only the servicer is mirrored here; the transports around it (gRPC server, aiohttp routes,
 :399-560) are out of scope.
 
-What is different, and why (SURVEY.md §9 #4, #14):
+What is different, and why:
 
 * The reference's ``_forward`` (:351-374) calls ``model_shard.forward(h, position_ids=arange(pos, pos+T)[None],
   use_cache=True)`` with NO ``past_key_values`` and throws the returned KV away, so decoding through the servicer

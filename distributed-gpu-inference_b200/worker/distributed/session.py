@@ -9,7 +9,7 @@ Reference: worker/distributed/session.py.  Kept for callers:
   total_latency_ms, retries, avg_latency_ms, tokens_per_second``, the ``ValueError`` when ``max_length`` would be
   exceeded, and the per-hop retry loop with linear back-off (reference :198-395);
 * ``SessionManager`` (reference :398-455) — without the self-deadlock of the original, whose ``create_session``
-  holds the lock while ``_cleanup_expired_sessions`` re-acquires it through ``close_session`` (SURVEY.md §9 #6).
+  holds the lock while ``_cleanup_expired_sessions`` re-acquires it through ``close_session``.
 
 What changed: the reference's hop is an aiohttp POST of base64 JSON (:125-160).  Inside one box the hop is either
 an in-process call into a stage (``InProcessTransport``) or NCCL point-to-point (``dgi_b200.pipeline``), so

@@ -1,4 +1,4 @@
-"""``PagedLLMEngine`` — the paged decode path behind the reference's engine surface (SURVEY.md §8f row 2).
+"""``PagedLLMEngine`` — the paged decode path behind the reference's engine surface.
 
 Shape of the surface: ``BaseEngine`` (reference: worker/engines/base.py:11-57 — ``load_model / inference(params) /
 unload_model / get_status``) and ``LLMBaseEngine`` (reference: worker/engines/llm_base.py:45-188 — ``generate_async /
