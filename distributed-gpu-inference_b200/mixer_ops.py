@@ -193,6 +193,13 @@ def biased_prompt_attention(out: torch.Tensor, q: torch.Tensor, gate: Optional[t
 # 64 x 128 states, us token by token / in chunks: 8 x 96 tokens of 4 heads gated 15.4 / 15.8, delta 21.9 / 21.4, retention 16.9 / 18.6; 192
 # tokens 27.4 / 22.2, 38.5 / 30.5, 25.2 / 24.9; 2048 tokens 248 / 154, 382 / 233, 191 / 151.
 SPLIT_SCAN_FROM = (96, 96, 160)
+# Chunks take 8 - 10 us more of the host (a workspace, two launches): a step whose mixer leaves the device waiting walks until the walk is
+# longer than that, from ``SPLIT_SCAN_ALONE`` tokens in one portion or ``SPLIT_SCAN_WORK`` = longest portion x tokens x heads on.  The mixers
+# called from Python, us walking / in chunks: gated, width 512, 1 portion of 200 64 / 73, 300 64 / 73, 448 74 / 74, 576 89 / 75; width 2048, 4 of
+# 200 65 / 74, 4 of 300 87 / 78, 8 of 200 95 / 89.  Delta, width 512, 1 of 300 119 / 129, 448 128 / 130, 576 151 / 130; width 2048, 4 of 300
+# 151 / 132.  Retention, width 512, 1 of 448 140 / 148, 576 (in segments) 155 / 149; width 2048, 2 of 448 137 / 142, 4 of 448 192 / 178.
+SPLIT_SCAN_ALONE = (448, 448, 512)
+SPLIT_SCAN_WORK = (3600000, 3600000, 6500000)
 SPLIT_SCAN_WORKSPACE = 1 << 30      # bytes of chunk operands at most (one head's if that is more); the heads go in groups beyond, smaller
                                     # ones where memory is short, and token by token where one head's do not fit
 
@@ -209,7 +216,7 @@ def split_scan_pays(rule: int, longest: int, n: int, n_seqs: int, H: int, dk: in
     portions on: 32 x 128 8 of 192 38 / 38, 64 of 256 284 / 316; 16 x 16 1 of 512 71 / 45, 8 of 192 29 / 33, 256 of 96 224 / 387.
     Retention of up to 32 keys walks at 63 ns a token: 1 of 512 39 / 42, 8 of 2048 of 32 x 32 133 / 243."""
     chunks = n // 16 + n_seqs
-    if longest < SPLIT_SCAN_FROM[rule]:
+    if longest < SPLIT_SCAN_ALONE[rule] and (longest < SPLIT_SCAN_FROM[rule] or longest * n * H < SPLIT_SCAN_WORK[rule]):
         return False
     if dk > 32 and 13 * dv >= 64 * (8 + 7 * -(-dv // 64)):
         return 16 * chunks <= 2 * n or 8 * longest >= H * chunks

@@ -208,7 +208,9 @@ def test_leased_blocks_come_back_zeroed_when_a_callback_fails():
     (0, (64, 128), 4, [95] * 8, False), (2, (64, 128), 16, [159], False), (0, (64, 128), 16, [512] + [1] * 63, True),
     (1, (64, 128), 32, [2048] + [1] * 255, True), (0, (64, 128), 16, [96] + [1] * 255, False), (1, (64, 128), 4, [96] + [1] * 255, False),
     (0, (64, 128), 32, [160] + [1] * 63, False), (0, (64, 64), 16, [512] * 8, True), (0, (64, 64), 16, [96] * 64, False),
-    (1, (64, 72), 16, [256] * 64, False), (1, (32, 128), 16, [512], True), (1, (32, 128), 16, [256] * 64, False),
+    (1, (64, 72), 16, [256] * 64, False), (1, (32, 128), 16, [512], True), (0, (64, 128), 4, [300], False), (0, (64, 128), 4, [448], True),
+    (0, (64, 128), 16, [200] * 4, False), (0, (64, 128), 16, [300] * 4, True), (1, (64, 128), 16, [200] * 8, True), (1, (64, 128), 8, [200] * 8, False),
+    (2, (64, 128), 4, [448] * 8, False), (2, (64, 128), 4, [576], True), (2, (64, 128), 16, [448] * 4, True), (2, (64, 128), 16, [448] * 2, False), (1, (32, 128), 16, [256] * 64, False),
     (0, (16, 16), 16, [512], True), (0, (16, 16), 16, [192] * 8, False), (0, (32, 32), 16, [2048] * 8, False),
     (2, (32, 128), 16, [512], False), (2, (32, 32), 16, [2048] * 8, False), (2, (64, 64), 16, [512] * 8, True)])
 def test_which_steps_run_in_chunks(rule, state, heads, portions, chunks):
