@@ -373,12 +373,15 @@ def rope_append_decode_attention(
 
 
 def one_call_batch(width: int, ff: int) -> int:
-    """Sequences up to which a decode step of a Llama layer is one call (``llama_decode_layer``) instead of its separate launches.  Its
-    projections have latencies, not bandwidth, in their favour: B200, bf16, 4 layers, us per step as a CUDA graph, separate / one call:
-    width 512, ff 1408: 135 / 68 with one sequence, 148 / 121 with 32; width 1024 185 / 90 and 181 / 164; width 2048, ff 5632 303 / 227,
-    300 / 247 with 8, 277 / 284 with 16; width 4096, ff 14336 563 / 712.  Launched from Python a layer takes 250 us of host time
-    separately, 70 in one call."""
-    return 0 if ff > 8192 else 32 if width <= 1024 else 8 if width <= 2048 else 0
+    """Sequences up to which a decode step of a Llama layer (separate projections) is one call (``llama_decode_layer``) instead of its
+    separate launches.  Its projections have latencies, not bandwidth, in their favour.  B200, bf16, 2 layers, us per step as a CUDA
+    graph, separate / one call: width 512, ff 1408 72 / 35 with one sequence, 79 / 46 with 16, 74 / 61 with 32; width 1024, ff 1408 95 / 59 and
+    87 / 82, ff 2816 100 / 70 with 16, 93 / 92 with 17, 92 / 103 with 32, ff 8192 143 / 128 and 127 / 200; width 2048, ff 5632 149 / 124 with 8,
+    137 / 138 with 9, ff 8192 167 / 141 and 147 / 158; 4 layers of width 4096, ff 14336, with one 563 / 712.  Launched from Python a layer takes
+    250 us of host time separately, 70 in one call, checks and allocations included."""
+    if ff > 8192 or width > 2048:      # beyond 8192 not measured
+        return 0
+    return 8 if width > 1024 else 32 if ff + 2 * width <= 3584 else 16
 
 
 @functools.lru_cache(maxsize=256)

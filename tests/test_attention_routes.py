@@ -127,3 +127,10 @@ def test_pages_that_come_row_by_row_share_wider_tiles(page, rows):
     assert mixer_ops.tile_rows(16, 4, 128, 2400, heavy=True, page=page) == 256 and mixer_ops.tile_rows(16, 4, 256, 8000, True, page) == 128
     st = _step([(1000, 0)] * 8)
     assert st.attention_tiles(16, 4, 128, 16, True, page=page)[0][1] == rows
+
+
+@pytest.mark.parametrize("width,ff,most", [(256, 1024, 32), (512, 1408, 32), (512, 2048, 32), (1024, 1408, 32), (1024, 2816, 16), (512, 8192, 16),
+                                           (1024, 8192, 16), (2048, 5632, 8), (2048, 8192, 8), (1024, 8224, 0), (4096, 1408, 0)])
+def test_how_many_sequences_a_decode_layer_takes_in_one_call(width, ff, most):
+    from dgi_b200 import ops
+    assert ops.one_call_batch(width, ff) == most
