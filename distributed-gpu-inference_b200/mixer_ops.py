@@ -1116,13 +1116,14 @@ def heads_by_token(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     copy behind them took 16 us at 3900 tokens of 16 heads of 128), except for one token, whose heads lie so already, and where
     ``out=`` does not go: gradients, forward-mode tangents, functorch's transforms, and autocast, which does not see it."""
     (H, n, _), dv = a.shape, w.shape[2]
-    wrapped, tangent = torch._C._functorch.is_functorch_wrapped_tensor, torch.autograd.forward_ad.unpack_dual
-    if n == 1 or torch.is_grad_enabled() and (a.requires_grad or w.requires_grad) or torch.is_autocast_enabled(a.device.type) \
-            or wrapped(a) or wrapped(w) or tangent(a).tangent is not None or tangent(w).tangent is not None:
-        return torch.bmm(a, w).transpose(0, 1).reshape(n, H * dv)
-    o = torch.empty((n, H, dv), dtype=a.dtype, device=a.device)
-    torch.bmm(a, w, out=o.transpose(0, 1))
-    return o.view(n, H * dv)
+    if n > 1 and not (torch.is_grad_enabled() and (a.requires_grad or w.requires_grad)) and not torch.is_autocast_enabled(a.device.type):
+        o = torch.empty((n, H, dv), dtype=a.dtype, device=a.device)
+        try:
+            torch.bmm(a, w, out=o.transpose(0, 1))
+            return o.view(n, H * dv)
+        except RuntimeError:      # a tangent or a transform: refused before anything ran (looking for them first takes 4 us of the host)
+            pass
+    return torch.bmm(a, w).transpose(0, 1).reshape(n, H * dv)
 
 
 @_timed
