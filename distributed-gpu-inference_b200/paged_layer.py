@@ -339,8 +339,10 @@ def _plain_modules(layer: nn.Module):
     mod = nn.modules.module
     if mod._global_forward_hooks or mod._global_forward_pre_hooks:
         return None
-    a, m = layer._modules["self_attn"]._modules, layer._modules["mlp"]._modules
-    linears = [(a if grp == "self_attn" else m).get(name) for grp, name in layer._LINEARS]
+    groups = {grp: layer._modules.get(grp) for grp in ("self_attn", "mlp")}
+    if None in groups.values():
+        return None
+    linears = [groups[grp]._modules.get(name) for grp, name in layer._LINEARS]
     norms = (layer._modules.get("input_layernorm"), layer._modules.get("post_attention_layernorm"))
     if any(type(sub) is not nn.Linear or sub.bias is not None for sub in linears) or any(type(sub) is not RMSNorm for sub in norms):
         return None

@@ -153,3 +153,26 @@ def test_paged_layer_refuses_what_it_does_not_implement():
     layer = PagedLlamaDecoderLayer(LlamaShapeConfig(**base), 0, "cpu", torch.float32)
     want = 1.0 / (500000.0 ** (torch.arange(0, 64, 2, dtype=torch.int64).float() / 64))
     assert torch.equal(layer.inv_freq, want) and layer.rope_attention_scaling == 1.0
+
+
+def test_a_layer_without_its_own_modules_is_no_plain_layer():
+    """What the one-call decode form looks at: projections that are no modules of the layer, or none at all, are left to the layer."""
+    from dgi_b200 import paged_layer
+    from dgi_b200.testing import LlamaShapeConfig
+
+    cfg = LlamaShapeConfig(hidden_size=128, num_attention_heads=2, num_key_value_heads=1, intermediate_size=96, vocab_size=8, num_hidden_layers=1)
+
+    def layer():
+        return paged_layer.PagedLlamaDecoderLayer(cfg, 0, "cpu", torch.bfloat16)
+
+    assert paged_layer._plain_modules(layer()) is not None
+    for grp, name in paged_layer.PagedLlamaDecoderLayer._LINEARS:
+        one = layer()
+        inner = getattr(getattr(one, grp), name)
+        delattr(getattr(one, grp), name)
+        setattr(getattr(one, grp), name, lambda x: inner(x))
+        assert paged_layer._plain_modules(one) is None
+        one = layer()
+        delattr(one, grp)
+        setattr(one, grp, type("Group", (), {}))
+        assert paged_layer._plain_modules(one) is None
