@@ -1,14 +1,14 @@
 #!/usr/bin/env python
-"""Headline benchmark: greedy decode tokens/s of the layer-range path over paged KV (BASELINE.json).
+"""Headline benchmark: greedy decode tokens/s of the layer-range path over paged KV.
 
     python bench.py --gpus N --steps K --warmup W            # this repo's CUDA path
     python bench.py --impl reference --gpus N --steps K ...  # the reference's torch CPU path (oracle/_ref bytecode, else the oracle port)
 
-N = 1 : BASELINE configs[1] — Llama-3-8B shape, random-init bf16, block 16, batch 64, context 2k, decode; the line
-        also carries configs[4] (batch 8, context 32k, shared prefix) as `cfg5` and configs[0] (tiny model, in
-        full, GPU and host side by side) as `cpu_baseline_cfg1`, and configs[1] once more through the reference's own call
+N = 1 : Llama-3-8B shape, random-init bf16, block 16, batch 64, context 2k, decode; the line
+        also carries the long-context decode (batch 8, context 32k, shared prefix) as `cfg5` and the tiny model (in
+        full, GPU and host side by side) as `cpu_baseline_cfg1`, and the 8B shape once more through the reference's own call
         stack (DistributedInferenceSession.step -> servicer hop, host ids in / out) as `reference_api`.
-N > 1 : BASELINE configs[3] — Llama-3-70B shape layer-sharded over N ranks (torchrun, NCCL send/recv of
+N > 1 : Llama-3-70B shape layer-sharded over N ranks (torchrun, NCCL send/recv of
         activations, vocabulary-parallel head), batch 128, context 4k, strong scaling; the 8B shape weak-scaled over
         the same ranks rides along as `weak_scaled_8b`, the P/D hand-off as `pd_transfer`, and `parity` holds the
         token checks of the run (dgi_b200/bench_pipeline.py).
@@ -135,7 +135,7 @@ def cpu_reference_tokens_per_s(shape: str, batch: int, ctx: int, steps: int, war
 
     kind "reference": the reference's own ``ModelShard.forward`` / ``get_logits`` (oracle/_ref bytecode) run the step,
     over the legacy-convention HF layer of oracle/llama_ref.py with dense (k, v) tuples, fp32 (the installed
-    transformers no longer speaks the call convention of model_shard.py:209-215, SURVEY §8c).  kind "port": the same
+    transformers no longer speaks the call convention of model_shard.py:209-215).  kind "port": the same
     step spelled out here, when oracle/_ref was not built."""
     from oracle import llama_ref as L
 
@@ -395,7 +395,7 @@ def _single_leg(args, workload):
     synthetic_kv = args.synthetic_kv
     if workload["key"] == "cfg5":
         # config 5: one shared prefix of 24576 tokens (1536 blocks, reference-counted) + unique tails of
-        # 8192 - 512 i tokens (SURVEY.md §8d): ragged block tables, cascade attention, synthetic KV
+        # 8192 - 512 i tokens: ragged block tables, cascade attention, synthetic KV
         shared = (ctx * 3 // 4) // 16 * 16
         eng.allocate(B, ctx, shared_prefix_len=shared)
         ragged = [shared + (ctx - shared) - 512 * i * (ctx // 32768 or 1) - total_steps for i in range(B)]
@@ -542,7 +542,7 @@ def _single_leg(args, workload):
 
 
 def config1_side_by_side():
-    """BASELINE configs[0] IN FULL, un-extrapolated: tiny 4-layer model in 2 layer-range shards, batch 4, prompt 128,
+    """The CPU comparison in full, un-extrapolated: tiny 4-layer model in 2 layer-range shards, batch 4, prompt 128,
     64 greedy tokens, fp32 — the reference's torch CPU path (its own ModelShard from oracle/_ref, else the oracle port, + legacy
     HF layer with dense (k, v) tuples) on the host cores, and this repo's paged CUDA path on the GPU, both timed
     over the 63 decode steps after the prompt pass, tokens compared."""
@@ -617,7 +617,7 @@ def config1_side_by_side():
 
 
 def reference_api_leg(workload):
-    """configs[1] driven the way a user of the reference drives it (tools/session_bench.py): one hop over all layers,
+    """The 8B shape driven the way a user of the reference drives it (tools/session_bench.py): one hop over all layers,
     in-process transport, token ids from pinned host memory in and tokens back to the host every step."""
     import importlib.util
 
@@ -637,7 +637,7 @@ def run_single(args, workload):
     line = _single_leg(args, workload)
     dev = "cuda:0"
     if not args.workload and not args.batch and not args.context and not args.no_riders:
-        # configs[4] rides along on the N = 1 line: long-context decode over a shared prefix (cascade kernel)
+        # the long-context decode rides along on the N = 1 line: long-context decode over a shared prefix (cascade kernel)
         args5 = argparse.Namespace(**vars(args))
         args5.workload = "cfg5"
         five = _single_leg(args5, workload_for(args5))
