@@ -1,9 +1,7 @@
 // Attention of prompt portions over the paged cache on the fifth-generation tensor cores (16-bit storage types).
 //
-// A CTA serves 256 query rows of one sequence and one kv head (128 where the head sizes leave no room for more, and two such CTAs
-// per SM in small steps): up to 256 / rep
-// consecutive tokens x the rep = H / G query heads that read this kv head, so a key tile is fetched once for all of them.  Keys are
-// walked in tiles of 64.
+// A CTA serves 128 or 256 query rows of one sequence and one kv head: up to rows / rep consecutive tokens x the rep = H / G query heads that
+// read this kv head, so a key tile is fetched once for all of them.  Keys are walked in tiles of 64.
 //
 //   S = Q K^T   tcgen05.mma, 128 x 64 per half of the rows, both operands in shared memory (128-byte swizzled lines), S in tensor
 //               memory, two of them per half
@@ -13,19 +11,22 @@
 //               transposed descriptor; O stays in tensor memory in fp32 for the whole walk
 //
 // Four more warps copy pages a tile or two ahead - pages that divide 64 keys by the copy engine, one box of 64 columns per page and block of
-// columns, a sequence's last tile and other page sizes row by row with rows past the sequence zero-filled - and another one issues the
-// products; they meet at mbarriers only.  While the softmax works on tile i the tensor cores run S of tile i + 1 and P V of tile i - 1.
+// columns, a sequence's last tile and other page sizes row by row with rows past the sequence zero-filled - another one issues the products,
+// and four (where one CTA has the SM to itself) rescale O between the products of two tiles; they meet at mbarriers only.  While the softmax works
+// on tile i the tensor cores run S of tile i + 1 and P V of tile i - 1.  Of 256 rows, the two halves' warps take turns with the exponentials.
+// Queries of full tiles come by the copy engine; rows leave through shared memory in 16-byte pieces side by side.
 //
-// Measured on B200 (bf16, 8 x 2048 tokens, 16 heads over 4 kv heads of 128): 213 us plain, 257 us with distance biases (the mma.sync
-// kernel: 1419), 323 us with a soft cap, 156 us with a window of 512; latent 320 / 256, 4 portions of up to 1500 tokens of 16 heads behind
-// 700, window 512: 101 us (417).  Pages row by row by 64 threads per pool: 237, 274, 574 (with a soft cap by exponentials), 156, 104.  What a
-// tile of 64 keys x 256 rows takes: 1280 clocks of the tensor cores (S with 64 columns is bound by reading Q from shared memory), 1000 of
-// exponentials (two warps per scheduler at four per clock) beside as much of other work per score; about a third of the launch is the
-// CTAs' beginnings and ends.
+// What bounds it: the softmax's chain from S to P, 2000 to 2400 clocks per tile of 64 keys x 256 rows (bias and maximum 850, exponentials 950 beside the
+// other half's; the tensor cores need 1280, the exponentials alone 1024), and 9000 clocks of a CTA's beginning and end (of 22000: a row of the output
+// written by one thread took 5000, queries in 16-byte pieces 5000, code of modes that a launch does not use two to eight thousand in instruction
+// misses).  Rescaling by the softmax itself: 2900 clocks per tile.
+// Measured on B200 (bf16, us, before these / now): 8 x 2048 tokens, 16 heads over 4 kv heads of 128, plain 209 / 198, window of 512 138 / 123, with distance
+// biases, query temperature and gate 277 / 205, soft cap 319 / 242; 5 x 1024 with a cap under a window of 512 51 / 31; latent 320 / 256, 4 portions of up to
+// 1500 tokens of 16 heads behind 700, window 512: 91 / 68; 319 shapes of 4 .. 16 heads, 1.29 times on average, 64 x 96 tokens of 16 heads with keys of
+// their own 42 / 45.
 //
 // Weights are taken relative to the row's running maximum, so that the largest is 1 and loses nothing when P is rounded to the storage
-// type; O is scaled down whenever a row of the warp has a new maximum (with the tile's weights already written, so that P V of the tile
-// before runs under the exponentials).  (Scaling only once the maximum has grown by 2^8 leaves the largest weight anywhere in 1 .. 256, rounded
+// type; O is scaled down whenever a row of the warp has a new maximum.  (Scaling only once the maximum has grown by 2^8 leaves the largest weight anywhere in 1 .. 256, rounded
 // like any other while the sum is not: scores of standard deviation 4 and 10 over 2048 keys came out 0.0013 and 0.0011 from float64 before
 // the output's own rounding, 0.0005 and 0.0003 this way.)  A latent cache (values = the first DV columns of the key rows) is fetched once
 // and read through both descriptors.
@@ -156,6 +157,25 @@ __device__ __forceinline__ void tm_st16(uint32_t addr, const uint32_t (&u)[16]) 
       : "memory");
 }
 
+// a warp's 32 rows of N columns times the lanes' factors, W columns at a time
+template <int N, int W>
+__device__ __forceinline__ void scale_rows(uint32_t addr, float k) {
+#pragma unroll 1
+  for (int c = 0; c < N; c += W) {
+    float o[W];
+    if constexpr (W == 16) tm_ld16(o, addr + c);
+    else tm_ld32(o, addr + c);
+    tc_wait_ld();
+#pragma unroll
+    for (int x = 0; x < W; x += 16) {
+      uint32_t w[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) w[u] = __float_as_uint(o[x + u] * k);
+      tm_st16(addr + c + x, w);
+    }
+  }
+}
+
 __device__ __forceinline__ float exp2_fast(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -171,6 +191,32 @@ __device__ __forceinline__ f32x2 both(float x) {
 __device__ __forceinline__ void scale_shift(float& a, float& b, f32x2 k, f32x2 m) {
   asm("{\n.reg .b64 t;\nmov.b64 t, {%0, %1};\nfma.rn.f32x2 t, t, %2, %3;\nmov.b64 {%0, %1}, t;\n}\n" : "+f"(a), "+f"(b) : "l"(k), "l"(m));
 }
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void apart(float& a, float& b, f32x2 v) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 template <typename T>
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   if constexpr (std::is_same_v<T, __nv_bfloat16>) {
@@ -183,47 +229,59 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 // shared memory of one CTA, from a 1024-byte boundary
-template <int DK, int DV, bool ALIAS, int HALVES>
+template <int DK, int DV, bool ALIAS, int HALVES, int CTAS>
 struct Plan {
   static constexpr int kHalves = HALVES;                // sets of 128 rows
-  static constexpr int kCtas = HALVES == 1 && DK <= 128 ? 2 : 1;   // per SM
-  static constexpr int kSoft = kHalves * kRows, kNT = kSoft + kLoad + 32;
+  static constexpr int kCtas = CTAS;                    // per SM
+  // One CTA per SM: warps of their own rescale O.  (Two have no registers for them: their softmax does it.)
+  static constexpr int kScale = kCtas == 1 ? kRows : 0;
+  static constexpr int kSoft = kHalves * kRows, kNT = kSoft + kLoad + 32 + kScale;
+  // 17 warps: five on a scheduler leave 96 registers each; the softmax takes 32 more from the warps that copy and rescale (8 x 128 + 8 x 64 + 96 = 17 x 96)
+  static constexpr bool kSplitRegs = kNT == 17 * 32;
   static constexpr int kBufs = kCtas == 2 ? 2 : 3;      // of keys, and of values
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + kHalves * (DK / 64) * kRows * 128;
   static constexpr int kV = kK + kBufs * (DK / 64) * kBlk;
   static constexpr int kEnd = kV + (ALIAS ? 0 : kBufs * (DV / 64) * kBlk);
   static constexpr int kBar = kEnd;                    // barriers, the tensor memory's address, the failure flag
-  static constexpr int kPage = kBar + 256;             // int [2][2][64]: rows of the pools that a tile's keys / values are in (-1: none)
-  static constexpr int kLut = kPage + 2 * 2 * kKeys * 4;  // float [kLuts][rep][pitch]: biases of the tiles' distances
+  static constexpr int kFlags = kBar + 240, kPage = kBar + 256;   // int [2][2][64]: rows of the pools that a tile's keys / values are in (-1: none)
+  static constexpr int kCorr = kPage + 2 * 2 * kKeys * 4;     // float [2][rows]: what O is multiplied by before a tile
+  static constexpr int kLut = kCorr + (kScale ? 2 * kSoft * 4 : 0);  // float [kLuts][rep][pitch]: biases of the tiles' distances
   // A tile's biases are copied once S of the tile kBufs before it is done, hence P V of the one two before that, hence its softmax:
   // the last reader known to be through is tile i - kBufs - 2.
   static constexpr int kLuts = kBufs + 2;
   static constexpr int kO = 2 * kKeys;                 // columns of tensor memory per half: S0 | S1 | O
-  static constexpr int kHalfTm = kHalves == 2 || kCtas == 2 ? 256 : 512;
+  static constexpr int kHalfTm = DK <= 128 ? 256 : 512;
   static constexpr int kTm = kHalves * kHalfTm;
   static_assert(kO + DV <= kHalfTm, "tensor memory");
+  static_assert(kHalves * kRows * DV * 4 <= kEnd, "rows on their way out");
 };
 
-template <typename T, int DK, int DV, bool ALIAS, bool BIAS, int HALVES>
-__global__ void __launch_bounds__(Plan<DK, DV, ALIAS, HALVES>::kNT, Plan<DK, DV, ALIAS, HALVES>::kCtas)
-tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map) {
-  using P = Plan<DK, DV, ALIAS, HALVES>;
+enum Mode { kPlain, kBiased, kCapped };      // scores: as they are, with distance biases and query temperatures, with a soft cap
+
+template <typename T, int DK, int DV, bool ALIAS, int MODE, int HALVES, int CTAS>
+__global__ void __launch_bounds__(Plan<DK, DV, ALIAS, HALVES, CTAS>::kNT, CTAS)
+tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map,
+                 const __grid_constant__ CUtensorMap q_map) {
+  using P = Plan<DK, DV, ALIAS, HALVES, CTAS>;
   constexpr int NB = P::kBufs, kSoft = P::kSoft;
+  constexpr bool BIAS = MODE == kBiased, CAP = MODE == kCapped;      // a mode's code is all that its kernel has: first passes wait for instructions
   extern __shared__ unsigned char raw_smem[];
   unsigned char* sm = raw_smem + ((1024 - (smem_u32(raw_smem) & 1023)) & 1023);
   const uint32_t sm0 = smem_u32(sm);
   // barriers: queries in; keys of a buffer in, and read; values of a buffer in; P V of a value buffer done; per half: S of a buffer
-  // done, P of a buffer written.  All readers of one wait for a tile before the tile that completes it again can get that far.
+  // done, P of a buffer written, factors of O known, O rescaled.  All readers of one wait for a tile before the tile that completes it again can get that far.
   const uint32_t bar_q = sm0 + P::kBar, bar_k = bar_q + 8, bar_ke = bar_k + 24, bar_v = bar_ke + 24, bar_o = bar_v + 24,
-                 bar_s = bar_o + 24, bar_p = bar_s + 32;
-  volatile uint32_t* tm_slot = reinterpret_cast<volatile uint32_t*>(sm + P::kBar + 192);
-  volatile int* dead = reinterpret_cast<volatile int*>(sm + P::kBar + 196);
+                 bar_s = bar_o + 24, bar_p = bar_s + 32, bar_c = bar_p + 32, bar_r = bar_c + 32;
+  volatile uint32_t* tm_slot = reinterpret_cast<volatile uint32_t*>(sm + P::kFlags);
+  volatile int* dead = reinterpret_cast<volatile int*>(sm + P::kFlags + 4);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int g = blockIdx.y, rep = A.H / A.G, bs = A.block_size;
-  const int tok0 = A.tiles[3 * blockIdx.x], trow = A.tiles[3 * blockIdx.x + 2];
-  const int cnt = min(A.tiles[3 * blockIdx.x + 1], kSoft / rep), n_rows = cnt * rep;
+  // all kv heads of a tile, then the next tile's: with the tiles in order of their keys, the longest first, short ones fill the last round
+  const int place = blockIdx.x + gridDim.x * blockIdx.y, tile = place / A.G;
+  const int g = place - tile * A.G, rep = A.H / A.G, bs = A.block_size;
+  const int tok0 = A.tiles[3 * tile], trow = A.tiles[3 * tile + 2];
+  const int cnt = min(A.tiles[3 * tile + 1], kSoft / rep), n_rows = cnt * rep;
   const int halves = P::kHalves == 2 && n_rows > kRows ? 2 : 1;       // in use
   const int p0 = A.tok_pos[tok0], p_last = p0 + cnt - 1;
   auto first_seen = [&](int p) {
@@ -258,12 +316,14 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
     for (int b = 0; b < 4; ++b) {
       init(bar_s + 8 * b, 1);
       init(bar_p + 8 * b, kRows);
+      init(bar_c + 8 * b, kRows);
+      init(bar_r + 8 * b, kRows);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *dead = 0;
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sm0 + P::kBar + 192), "n"(P::kTm) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sm0 + P::kFlags), "n"(P::kTm) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
@@ -278,6 +338,7 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
   auto values_done = [&](int i) { return bar_wait(bar_o + 8 * (i % NB), (i / NB) & 1, dead); };
 
   if (warp >= kSoft / 32 && warp < (kSoft + kLoad) / 32) {
+    if constexpr (P::kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     // ---- the warps that copy pages: half of them keys, half values; a latent cache: all of them its rows ------------------------
     const bool values = !ALIAS && warp >= kSoft / 32 + kLoad / 64;
     constexpr int kTeam = ALIAS ? kLoad : kLoad / 2;
@@ -291,26 +352,28 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
     // `line` has them), the others (a sequence's last) row by row with zeros behind the last.
     const bool boxes = A.boxes != 0;
     const int n_pages = boxes ? kKeys / bs : 0;
+    constexpr int kLoadWarps = kTeam / 32;
+    const int my_page = (me & 31) * kLoadWarps + me / 32;        // the warps take turns with the pages: a copy costs its warp a hundred clocks
     auto whole = [&](int i) { return boxes && i < n_it && key0(i) + kKeys - 1 <= p_last; };
     // the page of one key of a tile (or the tile's page number `me`), looked up by the team's first threads a tile ahead of its copies
     auto look_up = [&](int i) {
-      if (whole(i)) return me < n_pages ? table[key0(i) / bs + me] : -1;
+      if (whole(i)) return my_page < n_pages ? table[key0(i) / bs + my_page] : -1;
       const int j = key0(i) + me;
       return me < kKeys && i < n_it && j <= p_last ? table[shift >= 0 ? j >> shift : j / bs] : -1;
     };
     auto biases = [&](int i) {      // entry [hh][x]: the bias of distance p0 - key0 - 63 + x
       const int d0 = p0 - key0(i) - (kKeys - 1), span = cnt + kKeys - 1;
       const uint32_t dst = smem_u32(lut_s + (i % P::kLuts) * rep * pitch);
-      for (int hh = 0; hh < rep; ++hh) {
-        const float* src = A.bias_lut + static_cast<int64_t>(g * rep + hh) * A.lut_len;
-        for (int x = me; x < span; x += kTeam) cp4(dst + 4 * (hh * pitch + x), src + min(max(d0 + x, 0), A.lut_len - 1));
+      for (int x = me; x < span; x += kTeam) {
+        const float* src = A.bias_lut + static_cast<int64_t>(g * rep) * A.lut_len + min(max(d0 + x, 0), A.lut_len - 1);
+        for (int hh = 0; hh < rep; ++hh, src += A.lut_len) cp4(dst + 4 * (hh * pitch + x), src);
       }
     };
     auto copy_pages = [&](int i, int page) {
-      if (me < n_pages) {
+      if (my_page < n_pages) {
         constexpr int kBox = 128;       // bytes of a box's row
         const int cols = values ? DV / 64 : DK / 64;
-        const uint32_t base = (values ? sm0 + P::kV + (i % NB) * (DV / 64) * kBlk : sm0 + P::kK + (i % NB) * (DK / 64) * kBlk) + me * bs * kBox;
+        const uint32_t base = (values ? sm0 + P::kV + (i % NB) * (DV / 64) * kBlk : sm0 + P::kK + (i % NB) * (DK / 64) * kBlk) + my_page * bs * kBox;
         if (page >= 0) {
           const uint32_t bar = (values ? bar_v : bar_k) + 8 * (i % NB);
           asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(cols * bs * kBox) : "memory");
@@ -360,7 +423,29 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((values ? bar_v : bar_k) + 8 * (i % NB)) : "memory");
     };
     int page = look_up(0);
-    const int ahead = min(n_it, NB);
+    auto free_again = [&](int i) {      // the buffer that tile i goes into has been read
+      if (values || ALIAS) values_done(i - NB);
+      else bar_wait(bar_ke + 8 * (i % NB), (i / NB - 1) & 1, dead);
+    };
+    // Pages by the copy engine arrive at the barrier by themselves, biases by their own arrival: nobody waits for a tile before the next
+    // is asked for.
+    const int by_boxes = boxes ? n_it : 0;
+    for (int i = 0; i < by_boxes; ++i) {
+      const int next = look_up(i + 1);
+      if (i >= NB) free_again(i);
+      copy(i, page);
+      page = next;
+      if (!whole(i)) {
+        cp_wait<0>();
+        arrived(i);
+      } else if (BIAS && !values) {
+        fence_smem_to_mma();
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_k + 8 * (i % NB)) : "memory");
+      } else {
+        arrived(i);
+      }
+    }
+    const int ahead = boxes ? 0 : min(n_it, NB);
     for (int i = 0; i < ahead; ++i) {      // a tile is handed over while the next one is under way
       const int next = look_up(i + 1);
       copy(i, page);
@@ -372,16 +457,15 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
     }
     cp_wait<0>();
     if (ahead > 0) arrived(ahead - 1);
-    for (int i = ahead; i < n_it; ++i) {
+    for (int i = max(ahead, by_boxes); i < n_it; ++i) {
       const int next = look_up(i + 1);
-      if (values || ALIAS) values_done(i - NB);
-      else bar_wait(bar_ke + 8 * (i % NB), (i / NB - 1) & 1, dead);
+      free_again(i);
       copy(i, page);
       page = next;
       cp_wait<0>();
       arrived(i);
     }
-  } else if (warp == (kSoft + kLoad) / 32) {
+  } else if (warp == (kSoft + kLoad + P::kScale) / 32) {
     // ---- products -----------------------------------------------------------------------------------------------------------------
     {
       auto scores = [&](int i) {
@@ -410,6 +494,7 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
         const uint32_t v = ALIAS ? sm0 + P::kK + (i % NB) * (DK / 64) * kBlk : sm0 + P::kV + (i % NB) * (DV / 64) * kBlk;
         for (int hf = 0; hf < halves; ++hf) {
           bar_wait(bar_p + 16 * hf + 8 * (i & 1), (i >> 1) & 1, dead);
+          if (P::kScale && i > 0) bar_wait(bar_r + 16 * hf + 8 * (i & 1), ((i - 1) >> 1) & 1, dead);
           tc_fence_after();
           const uint32_t t = tm + hf * P::kHalfTm;
 #pragma unroll
@@ -420,9 +505,39 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
       }
     }
     __syncwarp();
+  } else if (P::kScale && warp >= (kSoft + kLoad) / 32) {
+    if constexpr (P::kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    // ---- O to a tile's new maximum, between P V of the tile before and the tile's own: not on the softmax's way from tile to tile ----
+    const uint32_t quarter = static_cast<uint32_t>(32 * (warp & 3)) << 16;
+    const float* corr_s = reinterpret_cast<const float*>(sm + P::kCorr) + 32 * (warp & 3) + (tid & 31);
+    for (int i = 1; i < n_it; ++i) {
+      for (int hf = 0; hf < halves; ++hf) {
+        bar_wait(bar_c + 16 * hf + 8 * (i & 1), ((i - 1) >> 1) & 1, dead);
+        const float corr = corr_s[(i & 1) * kSoft + hf * kRows];
+        if (__any_sync(0xffffffffu, corr != 1.0f)) {
+          values_done(i - 1);
+          tc_fence_after();
+          scale_rows<DV, 32>(tm + hf * P::kHalfTm + quarter + P::kO, corr);
+          tc_wait_st();
+          tc_fence_before();
+        }
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_r + 16 * hf + 8 * (i & 1)) : "memory");
+      }
+    }
   } else {
     // ---- softmax: thread = row -------------------------------------------------------------------------------------------------------
-    {
+    if constexpr (P::kSplitRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
+    if (A.q_boxes && n_rows == kSoft) {
+      // a full tile: boxes of 64 columns x the group's heads x the tokens of 128 rows
+      if (tid == 0) {
+        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar_q), "n"(kSoft * DK * 2) : "memory");
+        for (int c = 0; c < P::kHalves * (DK / 64); ++c)
+          asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(sm0 + P::kQ + c * (kRows * 128)),
+                       "l"(&q_map), "r"(64 * (c % (DK / 64))), "r"(g * rep), "r"(tok0 + c / (DK / 64) * (kRows / rep)), "r"(bar_q) : "memory");
+      }
+      __syncwarp();
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_q) : "memory");
+    } else {
       constexpr int kCh = DK / 8;
       const T* qp = static_cast<const T*>(A.q);
 #pragma unroll 8
@@ -447,36 +562,31 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
     const int lo_p = live ? first_seen(p) : 0, lo_last = first_seen(p_last);
     float mult = A.scale;
     if (BIAS) mult *= 1.0f + A.temp_coef * logf(static_cast<float>((p + 1) / max(A.temp_every, 1)) + 1.0f);
-    const float two_over_cap = A.softcap > 0.f ? 2.0f / A.softcap : 0.f;
+    [[maybe_unused]] const float two_over_cap = CAP ? 2.0f / A.softcap : 0.f;
     // plain scores are compared before they are scaled: weight = 2^(s * k2 - m), in one multiply-add
-    const bool plain = !BIAS && A.softcap <= 0.f && mult > 0.f;
+    const bool plain = MODE == kPlain && mult > 0.f;
     const float k2 = plain ? mult * kLog2e : kLog2e;
     float m_ref = -INFINITY, l = 0.f;       // in powers of two; -inf until the row sees a key
     bool ok = true;
 
-    // O of the tiles before tile i to the new maximum where a row of the warp has one: after the tile's weights, with P V of the tile before
-    // under them, or (kEarly) before, where the registers do not hold the factor as well (96 with two CTAs per SM, biases: 378 -> 338 us
-    // of 8 x 2048 tokens; the other forms lose 3 .. 10% that way)
-    constexpr bool kEarly = BIAS && HALVES == 1;
-    auto rescale = [&](int i, bool grow, float corr) {
+    // O of the tiles before tile i to the new maximum where a row of the warp has one, with two CTAs per SM: before the tile's weights, as
+    // their 96 registers do not hold the factor as well (after them 3 .. 12% slower)
+    [[maybe_unused]] auto rescale = [&](int i, bool grow, float corr) {
       if (i == 0 || !__any_sync(0xffffffffu, grow)) return;
       ok = values_done(i - 1) && ok;
       tc_fence_after();
-      constexpr int kW = kEarly ? 16 : 32;
-#pragma unroll 1
-      for (int c = 0; c < DV; c += kW) {
-        float o[kW];
-        if constexpr (kEarly) tm_ld16(o, tm_row + P::kO + c);
-        else tm_ld32(o, tm_row + P::kO + c);
-        tc_wait_ld();
-#pragma unroll
-        for (int x = 0; x < kW; x += 16) {
-          uint32_t w[16];
-#pragma unroll
-          for (int u = 0; u < 16; ++u) w[u] = __float_as_uint(o[x + u] * corr);
-          tm_st16(tm_row + P::kO + c + x, w);
-        }
-      }
+      scale_rows<DV, 16>(tm_row + P::kO, corr);
+    };
+    [[maybe_unused]] float* corr_s = reinterpret_cast<float*>(sm + P::kCorr);
+    // Two warps share a scheduler, one of each half: they take turns with the exponentials, so that one's run under the other's maxima and
+    // rescaling (in step, each phase is waited for twice)
+    const bool turns = P::kHalves == 2 && halves == 2;
+    const int turn_bar = 3 + 2 * (warp & 3);
+    auto my_turn = [&](int i) {
+      if (turns && (hf > 0 || i > 0)) asm volatile("bar.sync %0, 64;" ::"r"(turn_bar + hf) : "memory");
+    };
+    auto their_turn = [&](int i) {
+      if (turns && (hf == 0 || i + 1 < mine)) asm volatile("bar.arrive %0, 64;" ::"r"(turn_bar + 1 - hf) : "memory");
     };
     for (int i = 0; i < mine; ++i) {
       const int j0 = key0(i);
@@ -491,28 +601,28 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
 #pragma unroll
         for (int c = 0; c < kKeys; ++c) s[c >> 5][c & 31] = fmaf(s[c >> 5][c & 31], mult, b[-c]);
       } else if (!plain) {
-        float far = A.softcap > 0.f ? 0.f : INFINITY;
+        [[maybe_unused]] float far = 0.f;
 #pragma unroll
         for (int c = 0; c < kKeys; ++c) {
           s[c >> 5][c & 31] *= mult;
-          far = fmaxf(far, fabsf(s[c >> 5][c & 31]));
+          if constexpr (CAP) far = fmaxf(far, fabsf(s[c >> 5][c & 31]));
         }
-        if (!__any_sync(0xffffffffu, far > 0.5f * A.softcap)) {
+        if constexpr (!CAP) {
+        } else if (!__any_sync(0xffffffffu, far > 0.5f * A.softcap)) {
           // all within half the cap: x tanh(u) / u, u = x / cap, by its series in u^2 (Chebyshev nodes on 0 .. 1/4, 3e-10): 1 / (1 + e^x) and
           // the difference from 1 took three times as long (5 x 1024 tokens of 16 heads, window 512: 99 us against 56) and lost the last
           // digits of small scores
-          const float per_cap = 0.5f * two_over_cap;
+          const f32x2 per_cap = both(0.5f * two_over_cap);
 #pragma unroll
-          for (int c = 0; c < kKeys; ++c) {
-            float& x = s[c >> 5][c & 31];
-            const float u = x * per_cap, t = u * u;
-            float q = fmaf(t, -0x1.b12a58p-8f, 0x1.5c8676p-6f);
-            q = fmaf(t, q, -0x1.b97d94p-5f);
-            q = fmaf(t, q, 0x1.110ec8p-3f);
-            q = fmaf(t, q, -0x1.555550p-2f);
-            x = fmaf(x * t, q, x);
+          for (int c = 0; c < kKeys; c += 2) {
+            const f32x2 x = pair(s[c >> 5][c & 31], s[c >> 5][(c & 31) + 1]), u = mul2(x, per_cap), t = mul2(u, u);
+            f32x2 q = fma2(t, both(-0x1.b12a58p-8f), both(0x1.5c8676p-6f));
+            q = fma2(t, q, both(-0x1.b97d94p-5f));
+            q = fma2(t, q, both(0x1.110ec8p-3f));
+            q = fma2(t, q, both(-0x1.555550p-2f));
+            apart(s[c >> 5][c & 31], s[c >> 5][(c & 31) + 1], fma2(mul2(x, t), q, x));
           }
-        } else if (A.softcap > 0.f) {
+        } else {
 #pragma unroll
           for (int c = 0; c < kKeys; ++c) {
             float& x = s[c >> 5][c & 31];
@@ -530,14 +640,29 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
       }
       float mx[4] = {s[0][0], s[0][1], s[0][2], s[0][3]};
 #pragma unroll
-      for (int c = 4; c < kKeys; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c >> 5][c & 31]);
-      const float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * k2;
+      for (int c = 4; c < kKeys - 4; c += 8) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mx[u] = max3(mx[u], s[c >> 5][(c & 31) + u], s[(c + 4) >> 5][((c + 4) & 31) + u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) mx[u] = fmaxf(mx[u], s[1][28 + u]);
+      const float m_new = max3(mx[0], mx[1], fmaxf(mx[2], mx[3])) * k2;
       const bool grow = m_new > m_ref;
       const float corr = grow ? exp2_fast(m_ref - m_new) : 1.0f;      // 0 where nothing was seen before
       if (grow) m_ref = m_new;
-      if constexpr (kEarly) rescale(i, grow, corr);
-      const f32x2 kk = both(k2), mm = both(m_ref == -INFINITY ? 0.f : -m_ref);     // a row that sees no key yet keeps weights 0
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      if constexpr (P::kScale > 0) {
+        if (i > 0) {
+          corr_s[(i & 1) * kSoft + tid] = corr;
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_c + 16 * hf + 8 * (i & 1)) : "memory");
+        }
+      } else {
+        rescale(i, grow, corr);
+      }
+      const f32x2 kk = both(k2);
+      f32x2 mm = both(m_ref == -INFINITY ? 0.f : -m_ref);     // a row that sees no key yet keeps weights 0
+      f32x2 sum[2] = {0ull, 0ull};
+      my_turn(i);
+      asm volatile("" : "+l"(mm));        // no exponential before it
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         uint32_t w[16];
@@ -547,14 +672,16 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
           scale_shift(a, b, kk, mm);
           a = exp2_fast(a);
           b = exp2_fast(b);
-          sum[c & 2] += a;
-          sum[(c & 2) + 1] += b;
+          sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], pair(a, b));
           w[c >> 1] = pack2<T>(a, b);
         }
         tm_st16(tm_row + (i & 1) * kKeys + x * 16, w);
       }
-      l = fmaf(l, corr, (sum[0] + sum[1]) + (sum[2] + sum[3]));
-      if constexpr (!kEarly) rescale(i, grow, corr);
+      their_turn(i);
+      float part[4];
+      apart(part[0], part[1], sum[0]);
+      apart(part[2], part[3], sum[1]);
+      l = fmaf(l, corr, (part[0] + part[1]) + (part[2] + part[3]));
       tc_wait_st();
       tc_fence_before();
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(my_p + 8 * (i & 1)) : "memory");
@@ -569,7 +696,7 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
     const float m_nat = m_ref * kLn2;
     const int64_t n = tok0 + t_row;
     if (gridDim.z > 1) {
-      const int64_t wr = (static_cast<int64_t>(blockIdx.z) * gridDim.x + blockIdx.x) * (kSoft / rep) + t_row;
+      const int64_t wr = (static_cast<int64_t>(blockIdx.z) * gridDim.x + tile) * (kSoft / rep) + t_row;
       float* dst = A.ws + (wr * A.H + h_row) * (DV + 2);
       if (live) {
         dst[0] = ok ? m_nat : NAN;
@@ -589,7 +716,7 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
             *reinterpret_cast<float2*>(dst + 2 + c + x) = n_it > 0 ? make_float2(o[x], o[x + 1]) : make_float2(0.f, 0.f);
         }
       }
-    } else {
+    } else if (hf < halves) {
       float f = 1.0f / l;
       if (A.sink && live) {
         const float sk = A.sink[h_row], M = fmaxf(m_nat, sk);
@@ -599,31 +726,71 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
       if (!ok) f = NAN;
       const T* gate = static_cast<const T*>(A.gate);
       if (gate && live && !A.gate_dim) f *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row])));
-#pragma unroll 1
-      for (int c = 0; c < DV; c += 32) {
-        float o[32];
-        __syncwarp();
+      // Rows go through shared memory (all products are done, queries and pages have been read), each warp its own, so that lanes side by side
+      // write pieces side by side; 16-byte pieces are swizzled by the row's number in its group of eight
+      auto scaled = [&](float (&o)[32], int c) {
         tm_ld32(o, tm_row + P::kO + c);
         tc_wait_ld();
-        if (!live) continue;       // reconverges at the loop's head
+        if (gate && A.gate_dim && live) {
 #pragma unroll
-        for (int x = 0; x < 32; ++x) {
-          o[x] *= f;
-          if (gate && A.gate_dim) o[x] *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row * A.gate_dim + c + x])));
+          for (int x = 0; x < 32; ++x) o[x] *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row * A.gate_dim + c + x])));
         }
-        const int64_t at = n * A.out_tok_stride + h_row * A.out_head_stride + c;
-        if (A.out_f32) {
-          float* dst = static_cast<float*>(A.out) + at;
 #pragma unroll
-          for (int x = 0; x < 32; x += 2) *reinterpret_cast<float2*>(dst + x) = make_float2(o[x], o[x + 1]);
-        } else {
-          T* dst = static_cast<T*>(A.out) + at;
-          if (A.out_vec) {
+        for (int x = 0; x < 32; ++x) o[x] *= f;
+      };
+      const int64_t at0 = n * A.out_tok_stride + h_row * A.out_head_stride;
+      auto rows_out = [&](auto* tag) {
+        using O = std::remove_pointer_t<decltype(tag)>;
+        constexpr int kPieces = DV * sizeof(O) / 16, kPer = 16 / sizeof(O);
+        const uint32_t own = sm0 + P::kQ + (hf * kRows + 32 * (warp & 3)) * (DV * static_cast<int>(sizeof(O)));
+        const int lane = tid & 31;
+#pragma unroll 1
+        for (int c = 0; c < DV; c += 32) {
+          float o[32];
+          __syncwarp();
+          scaled(o, c);
 #pragma unroll
-            for (int x = 0; x < 32; x += 8)
-              *reinterpret_cast<uint4*>(dst + x) = make_uint4(pack2<T>(o[x], o[x + 1]), pack2<T>(o[x + 2], o[x + 3]),
-                                                              pack2<T>(o[x + 4], o[x + 5]), pack2<T>(o[x + 6], o[x + 7]));
+          for (int x = 0; x < 32; x += kPer) {
+            uint32_t w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) w[u] = sizeof(O) == 4 ? __float_as_uint(o[x + u]) : pack2<T>(o[(x + 2 * u) % 32], o[(x + 2 * u + 1) % 32]);
+            const int piece = (c + x) / kPer;
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(own + lane * (kPieces * 16) + ((piece ^ (lane & 7)) << 4)), "r"(w[0]), "r"(w[1]),
+                         "r"(w[2]), "r"(w[3]) : "memory");
+          }
+        }
+        __syncwarp();
+        const unsigned seen = __ballot_sync(0xffffffffu, live);
+        constexpr int kRowsAtOnce = 32 / kPieces > 0 ? 32 / kPieces : 1;
+#pragma unroll 4
+        for (int u = 0; u < kPieces; ++u) {
+          const int r = kPieces >= 32 ? u * 32 / kPieces : u * kRowsAtOnce + lane / kPieces, piece = kPieces >= 32 ? (u * 32 + lane) % kPieces : lane % kPieces;
+          const int64_t to = __shfl_sync(0xffffffffu, at0, r);
+          if (seen >> r & 1) {
+            uint4 v;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(own + r * (kPieces * 16) + ((piece ^ (r & 7)) << 4)) : "memory");
+            *reinterpret_cast<uint4*>(static_cast<O*>(A.out) + to + piece * kPer) = v;
+          }
+        }
+      };
+      const bool whole_rows = A.out_vec && __all_sync(0xffffffffu, ok);     // after a failure copies may still be under way
+      if (whole_rows && A.out_f32) {
+        rows_out(static_cast<float*>(nullptr));
+      } else if (whole_rows) {
+        rows_out(static_cast<T*>(nullptr));
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < DV; c += 32) {
+          float o[32];
+          __syncwarp();
+          scaled(o, c);
+          if (!live) continue;       // reconverges at the loop's head
+          if (A.out_f32) {
+            float* dst = static_cast<float*>(A.out) + at0 + c;
+#pragma unroll
+            for (int x = 0; x < 32; x += 2) *reinterpret_cast<float2*>(dst + x) = make_float2(o[x], o[x + 1]);
           } else {
+            T* dst = static_cast<T*>(A.out) + at0 + c;
 #pragma unroll
             for (int x = 0; x < 32; x += 2) *reinterpret_cast<uint32_t*>(dst + x) = pack2<T>(o[x], o[x + 1]);
           }
@@ -637,18 +804,23 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tm), "n"(P::kTm));
 }
 
-// The pool as rows of `width` elements, fetched in boxes of 64 columns x one page; made for the launch (a microsecond) and not kept.
-// Its height is the largest a row's number allows: which rows are read is the block tables' business, as with plain loads.
-template <typename T>
-bool page_map(CUtensorMap* map, const void* pool, int width, int block_size) {
-  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                            const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+Encode tensor_map_encode() {
   static const Encode encode = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult qr;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess) p = nullptr;
     return reinterpret_cast<Encode>(p);
   }();
+  return encode;
+}
+
+// The pool as rows of `width` elements, fetched in boxes of 64 columns x one page; made for the launch (a microsecond) and not kept.
+// Its height is the largest a row's number allows: which rows are read is the block tables' business, as with plain loads.
+template <typename T>
+bool page_map(CUtensorMap* map, const void* pool, int width, int block_size) {
+  const Encode encode = tensor_map_encode();
   if (!encode || !aligned16(pool)) return false;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(width), 0x7fffffffu}, strides[1] = {2ull * width};
   const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(block_size)}, step[2] = {1, 1};
@@ -657,40 +829,68 @@ bool page_map(CUtensorMap* map, const void* pool, int width, int block_size) {
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename T, int DK, int DV, bool ALIAS, bool BIAS, int HALVES>
+// Queries as boxes of 64 columns x one kv head's heads x the tokens of 128 rows.  Only full tiles are fetched this way, so the number of
+// tokens does not matter.
+template <typename T>
+bool query_map(CUtensorMap* map, const TileAttn& A, int dk) {
+  const int rep = A.H / A.G;
+  const Encode encode = tensor_map_encode();
+  if (!encode || kRows % rep || A.q_head_stride <= 0 || A.q_tok_stride <= 0) return false;
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(dk), static_cast<cuuint64_t>(A.H), 0x7fffffffu};
+  const cuuint64_t strides[2] = {2ull * A.q_head_stride, 2ull * A.q_tok_stride};
+  const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(rep), static_cast<cuuint32_t>(kRows / rep)}, step[3] = {1, 1, 1};
+  return encode(map, std::is_same_v<T, __nv_bfloat16> ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(A.q), dims,
+                strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <typename T, int DK, int DV, bool ALIAS, int MODE, int HALVES, int CTAS>
 int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stream) {
-  using P = Plan<DK, DV, ALIAS, HALVES>;
+  using P = Plan<DK, DV, ALIAS, HALVES, CTAS>;
   const int rep = A.H / A.G;
   size_t smem = 1024 + P::kLut;
-  if (BIAS) smem += sizeof(float) * P::kLuts * rep * (((P::kSoft / rep + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep));
+  if (MODE == kBiased) smem += sizeof(float) * P::kLuts * rep * (((P::kSoft / rep + kKeys - 1 + 31) & ~31) + (rep >= 32 ? 1 : 32 / rep));
   smem = std::max<size_t>(smem, P::kCtas == 2 ? 80 * 1024 : 120 * 1024);   // no more CTAs per SM than tensor memory has room for
   if (smem > kMaxSmem) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
-  auto kern = tile_attn_kernel<T, DK, DV, ALIAS, BIAS, HALVES>;
+  auto kern = tile_attn_kernel<T, DK, DV, ALIAS, MODE, HALVES, CTAS>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   TileAttn B = A;
-  CUtensorMap k_map{}, v_map{};
+  CUtensorMap k_map{}, v_map{}, q_map{};
   // pages that divide a tile of keys, rows that start on 16 bytes
   B.boxes = A.block_size % 8 == 0 && kKeys % A.block_size == 0 && page_map<T>(&k_map, A.k_pool, DK, A.block_size) &&
             (ALIAS || (A.v_row % 8 == 0 && page_map<T>(&v_map, A.v_pool, A.v_row, A.block_size)));
-  kern<<<dim3(n_tiles, A.G, n_splits), P::kNT, smem, stream>>>(B, k_map, v_map);
+  B.q_boxes = query_map<T>(&q_map, A, DK);
+  kern<<<dim3(n_tiles, A.G, n_splits), P::kNT, smem, stream>>>(B, k_map, v_map, q_map);
   return check_launch("b200_tile_attn");
 }
 
+template <int DK, int DV, bool ALIAS>
+struct Shape {
+  static constexpr int dk = DK, dv = DV;
+  static constexpr bool alias = ALIAS;
+};
 template <typename T>
 int launch_shape(const TileAttn& A, int dk, int dv, bool alias, int rows, int n_tiles, int n_splits, cudaStream_t stream) {
-  auto grouped = [&](auto size) {
-    constexpr int D = decltype(size)::value;
-    if (rows == kRows) {
-      return A.bias_lut ? launch_tiles<T, D, D, false, true, 1>(A, n_tiles, n_splits, stream)
-                        : launch_tiles<T, D, D, false, false, 1>(A, n_tiles, n_splits, stream);
+  auto go = [&](auto shape, auto mode) {
+    constexpr int DK = decltype(shape)::dk, DV = decltype(shape)::dv, MODE = decltype(mode)::value;
+    if constexpr (!decltype(shape)::alias) {
+      if (rows != kRows) return launch_tiles<T, DK, DV, false, MODE, 2, 1>(A, n_tiles, n_splits, stream);
+      // one CTA per SM has registers for its scores and warps that rescale (4 heads over 1, plain, 5 x 1024: 25.4 us against 30.1 side by side; 8 over 2, 3 x
+      // 550: 17.8 / 20.4); more CTAs than SMs hide each other's beginnings (4 over 1, 64 x 96: 10.7 / 14.6)
+      if (static_cast<int64_t>(n_tiles) * A.G * n_splits > kNumSMs) return launch_tiles<T, DK, DV, false, MODE, 1, 2>(A, n_tiles, n_splits, stream);
     }
-    return A.bias_lut ? launch_tiles<T, D, D, false, true, 2>(A, n_tiles, n_splits, stream)
-                      : launch_tiles<T, D, D, false, false, 2>(A, n_tiles, n_splits, stream);
+    return launch_tiles<T, DK, DV, decltype(shape)::alias, MODE, 1, 1>(A, n_tiles, n_splits, stream);
   };
-  if (!alias && dk == 128 && dv == 128) return grouped(std::integral_constant<int, 128>{});
-  if (!alias && dk == 64 && dv == 64) return grouped(std::integral_constant<int, 64>{});
-  if (alias && dk == 256 && dv == 256) return launch_tiles<T, 256, 256, true, false, 1>(A, n_tiles, n_splits, stream);
-  if (alias && dk == 320 && dv == 256) return launch_tiles<T, 320, 256, true, false, 1>(A, n_tiles, n_splits, stream);
+  auto by_mode = [&](auto shape) {
+    if constexpr (!decltype(shape)::alias) {
+      if (A.bias_lut) return go(shape, std::integral_constant<int, kBiased>{});
+    }
+    return A.softcap > 0.f ? go(shape, std::integral_constant<int, kCapped>{}) : go(shape, std::integral_constant<int, kPlain>{});
+  };
+  if (!alias && dk == 128 && dv == 128) return by_mode(Shape<128, 128, false>{});
+  if (!alias && dk == 64 && dv == 64) return by_mode(Shape<64, 64, false>{});
+  if (alias && dk == 256 && dv == 256) return by_mode(Shape<256, 256, true>{});
+  if (alias && dk == 320 && dv == 256) return by_mode(Shape<320, 256, true>{});
   return fail(B200_ESHAPE, "b200_tile_attn: head sizes %d / %d are not built", dk, dv);
 }
 
@@ -703,14 +903,15 @@ bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, in
   return dk == dv && (dk == 64 || dk == 128);
 }
 
-// 256 rows share a fetched key tile and its biases, but only one such CTA runs per SM and nothing covers its beginning and end; with pages
-// by the copy engine two CTAs of 128 rows are ahead where the softmax does no more than scale (8 x 2048 tokens, 16 heads over 4: 213 us
-// against 225; 5 x 1024 under a window of 512: 44.6 / 46.0), 256 rows where it also adds biases or caps (257 against 285, 323 against 369;
-// 8 x 700 tokens of 8 heads, 1.2 rounds of CTAs, biases: 36.3 / 39.6) and the step fills the SMs once.  Pages that come row by row keep 256
-// rows from three rounds on (8 x 1000 tokens of 16 heads, pages of 24: 82 us against 94).
+// 256 rows share a fetched key tile and its biases and take turns with the exponentials; 128 rows have shorter beginnings and less of the causal
+// triangle to mask.  With biases or a cap 256 rows are ahead where heads share their keys and there is more than an SM's CTA and a half of 128 (16
+// over 4, 8 x 2048: 206 / 242 us against 241 / 285; 6 x 300 .. 640: 24 / 27 against 28 / 32; but 4 over 1, 8 x 700: 27 against 21 of plain
+// scores), 128 where they do not share (16 over 16, 8 x 700: 60 / 67 against 64 / 70; 64 x 96: 50 / 53 against 73 / 73).  Plain scores keep 128 rows.
+// Pages that come row by row keep 256 rows from one round of CTAs on with biases or a cap, from three without (8 x 1000 tokens of 16 heads, pages
+// of 24: 82 us against 94).
 int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy, bool boxes) {
-  const int64_t ctas = static_cast<int64_t>(n_tokens) * rep / (2 * kTileRows) * G;
-  const bool wide = heavy ? ctas >= kNumSMs : !boxes && ctas >= 3 * kNumSMs;
+  const int64_t ctas = static_cast<int64_t>(n_tokens) * rep / (2 * kTileRows) * G;      // of 256 rows
+  const bool wide = boxes ? heavy && rep > 1 && 4 * ctas > 3 * kNumSMs : ctas >= (heavy ? 1 : 3) * kNumSMs;
   return wide && dk <= 128 ? 2 * kTileRows : kTileRows;
 }
 

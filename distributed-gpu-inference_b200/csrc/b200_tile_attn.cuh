@@ -24,7 +24,7 @@ struct TileAttn {
   int gate_dim, out_f32, out_vec;            // gates per channel: the value size; 16-byte stores possible
   float scale, softcap, temp_coef;
   int temp_every;
-  int boxes;                                 // set by the launcher: pages come by the copy engine
+  int boxes, q_boxes;                        // set by the launcher: pages, and the queries of full tiles, come by the copy engine
 };
 
 bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, int dtype);

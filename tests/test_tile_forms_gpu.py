@@ -1,0 +1,43 @@
+"""The forms of the tile attention kernel that a launch's size and its operands' places choose: one CTA of 128 rows per SM or two, queries by
+the copy engine or in pieces (partial tiles, groups of heads that do not divide 128 rows), rows that leave through shared memory or not."""
+import pytest
+import torch
+
+from dgi_b200 import mixer_ops
+from test_tile_attention_gpu import F64, _case, _reference
+
+pytestmark = pytest.mark.gpu
+
+# H, G, key size, value size, value heads per key head
+LAYOUTS = {"4x128": (8, 2, 128, 128, 1), "4x64": (8, 2, 64, 64, 1), "6x128": (6, 1, 128, 128, 1), "1x64": (4, 4, 64, 64, 1)}
+
+
+@pytest.mark.parametrize("out", ["16", "32", "off"], ids=["half", "float", "off_16_bytes"])
+@pytest.mark.parametrize("mode", ["plain", "bias", "cap"])
+@pytest.mark.parametrize("many", [False, True], ids=["one_per_sm", "two_per_sm"])
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_forms(layout, many, mode, out):
+    H, G, dk, dv, div = LAYOUTS[layout]
+    cap = 128 // (H // G)
+    # portions of one, two and a half tiles; with `many`, more CTAs than SMs
+    portions = [(cap, 0), (2 * cap, 40), (cap + cap // 2, 100)] + ([(5, 70)] * (160 // G) if many else [])
+    q, k_pool, v_pool, st, rnd = _case(LAYOUTS[layout], portions, 16, torch.bfloat16)
+    n, scale = q.shape[0], dk ** -0.5
+    bias = rnd(H, 150) if mode == "bias" else None
+    kw = dict(softcap=4.0) if mode == "cap" else {}
+    gate = rnd(n, H * dv if mode == "cap" else H).to(torch.bfloat16)
+    wide = torch.full((n, H * dv + 4), 7.0, dtype=torch.float32 if out == "32" else torch.bfloat16, device="cuda")
+    o = wide[:, 2:2 + H * dv].unflatten(1, (H, dv)) if out == "off" else torch.empty(n, H, dv, dtype=wide.dtype, device="cuda")
+    tiles = st.prompt_tiles(1, cap)[0]
+    assert (tiles.shape[0] * G > 148) is many
+    mixer_ops.tile_attention(o, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, scale, rows=128, gate=gate, bias_lut=bias, **kw)
+    want = _reference(q, k_pool, v_pool, st, dv, div, scale, bias=bias, gate=gate, **kw)
+    # weights rounded to 8 bits and one rounding of the result, as in the tests of the options
+    tol = 1.5 * 2.0 ** -8
+    assert (o.to(F64) - want).norm() / want.norm() <= tol
+    assert ((o.to(F64) - want).norm(dim=2) / want.norm(dim=2)).max() <= 8 * tol
+    if out == "off":
+        assert (wide[:, :2] == 7).all() and (wide[:, 2 + H * dv:] == 7).all()
+    again = torch.empty_like(o)
+    mixer_ops.tile_attention(again, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, scale, rows=128, gate=gate, bias_lut=bias, **kw)
+    assert torch.equal(again, o)
