@@ -15,7 +15,7 @@
 // they come.  Weights are asked for before the launch in front has finished (they do not depend on it), inputs after.
 //
 // What bounds it: at the widths of small models (512: 6 MB of weights per layer) the launches and their latencies, not the bytes.  B200,
-// bf16, width 512, batch 4: 13 launches a layer from Python took 250 us of host time, this call with the checks before it 70 us.
+// bf16, width 512, batch 4: 13 launches a layer from Python took 250 us of host time, this call with the checks before it 58 us.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>

@@ -378,7 +378,7 @@ def one_call_batch(width: int, ff: int) -> int:
     graph, separate / one call: width 512, ff 1408 72 / 35 with one sequence, 79 / 46 with 16, 74 / 61 with 32; width 1024, ff 1408 95 / 59 and
     87 / 82, ff 2816 100 / 70 with 16, 93 / 92 with 17, 92 / 103 with 32, ff 8192 143 / 128 and 127 / 200; width 2048, ff 5632 149 / 124 with 8,
     137 / 138 with 9, ff 8192 167 / 141 and 147 / 158; 4 layers of width 4096, ff 14336, with one 563 / 712.  Launched from Python a layer takes
-    250 us of host time separately, 70 in one call, checks and allocations included."""
+    250 us of host time separately, 58 in one call, checks and allocations included (68 while both the layer and this call looked at the weights)."""
     if ff > 8192 or width > 2048:      # beyond 8192 not measured
         return 0
     return 8 if width > 1024 else 32 if ff + 2 * width <= 3584 else 16
@@ -394,11 +394,12 @@ def llama_decode_layer(x: torch.Tensor, norm1: torch.Tensor, eps1: float, weight
                        position_ids: Optional[torch.Tensor], inv_freq: Optional[torch.Tensor], rope_scaling: float,
                        cos: Optional[torch.Tensor], sin: Optional[torch.Tensor], k_pool: torch.Tensor, v_pool: torch.Tensor,
                        block_tables: torch.Tensor, context_lens: torch.Tensor, max_context_len: int, num_heads: int, num_splits: int = 0,
-                       flags: int = 0) -> torch.Tensor:
+                       flags: int = 0, pointers: Optional[Sequence[int]] = None) -> torch.Tensor:
     """One decoder layer over ``x [B, 1, W]`` (contiguous, f16 / bf16): norms, projections ``weights`` = q, k, v, o, gate, up, down
     (contiguous ``[out, in]``), RoPE, append and paged attention, SiLU feed-forward, residuals, in five launches.  RoPE from ``cos / sin
-    [B, D]``, or from ``position_ids`` (int64 ``[B, 1]``) and ``inv_freq`` (fp32 ``[D / 2]``).  Returns ``[B, 1, W]``."""
-    _need_cuda(x, norm1, norm2, k_pool, v_pool, block_tables, context_lens, *weights)
+    [B, D]``, or from ``position_ids`` (int64 ``[B, 1]``) and ``inv_freq`` (fp32 ``[D / 2]``).  Returns ``[B, 1, W]``.  ``pointers``: the
+    addresses of the weights, norm1 and norm2 of a caller that has looked at their types, layouts and places in this very call."""
+    _need_cuda(x, k_pool, v_pool, block_tables, context_lens)
     max_blocks, Hkv, bs, D = _pool_dims(k_pool)
     B, T, W = x.shape
     ff, dt = weights[4].shape[0], DTYPE_ID[x.dtype]
@@ -407,11 +408,16 @@ def llama_decode_layer(x: torch.Tensor, norm1: torch.Tensor, eps1: float, weight
     if x.dtype != k_pool.dtype:
         raise TypeError("q dtype must equal the pool dtype")
     shapes = ((num_heads * D, W), (Hkv * D, W), (Hkv * D, W), (W, num_heads * D), (ff, W), (ff, W), (W, ff))
-    if T != 1 or not x.is_contiguous() or tuple(tuple(w.shape) for w in weights) != shapes or norm1.numel() != W or norm2.numel() != W:
+    if T != 1 or not x.is_contiguous() or len(weights) != 7 or norm1.numel() != W or norm2.numel() != W:
         raise ValueError("inputs do not match the layer's sizes")
-    for t in (norm1, norm2, *weights):
-        if t.dtype != x.dtype or not t.is_contiguous():
-            raise ValueError("weights are contiguous in x's dtype")
+    if [w.shape for w in weights] != list(shapes):      # (sizes compare with tuples)
+        raise ValueError("inputs do not match the layer's sizes")
+    if pointers is None:
+        _need_cuda(norm1, norm2, *weights)
+        for t in (norm1, norm2, *weights):
+            if t.dtype != x.dtype or not t.is_contiguous():
+                raise ValueError("weights are contiguous in x's dtype")
+        pointers = [t.data_ptr() for t in (*weights, norm1, norm2)]
     if block_tables.dtype != torch.int32 or block_tables.dim() != 2 or block_tables.shape[0] != B:
         raise ValueError("block_tables must be int32 [B, n]")
     if block_tables.stride(1) != 1 and block_tables.shape[1] > 1:
@@ -430,9 +436,8 @@ def llama_decode_layer(x: torch.Tensor, norm1: torch.Tensor, eps1: float, weight
     out = torch.empty_like(x)
     with _timed():
         rc = lib.b200_llama_decode_layer(
-            out.data_ptr(), x.data_ptr(), W, norm1.data_ptr(), float(eps1), weights[0].data_ptr(), weights[1].data_ptr(),
-            weights[2].data_ptr(), weights[3].data_ptr(), norm2.data_ptr(), float(eps2), weights[4].data_ptr(), weights[5].data_ptr(),
-            weights[6].data_ptr(), 0 if cos is not None else position_ids.data_ptr(), 0 if cos is not None else inv_freq.data_ptr(),
+            out.data_ptr(), x.data_ptr(), W, pointers[7], float(eps1), pointers[0], pointers[1], pointers[2], pointers[3], pointers[8],
+            float(eps2), pointers[4], pointers[5], pointers[6], 0 if cos is not None else position_ids.data_ptr(), 0 if cos is not None else inv_freq.data_ptr(),
             float(rope_scaling), cos.data_ptr() if cos is not None else 0, sin.data_ptr() if cos is not None else 0, k_pool.data_ptr(),
             v_pool.data_ptr(), block_tables.data_ptr(), block_tables.stride(0) if B > 1 else block_tables.shape[1],
             context_lens.data_ptr(), B, W, ff, num_heads, Hkv, D, bs, max_blocks, int(max_context_len), int(num_splits), ws.data_ptr(),

@@ -328,8 +328,17 @@ class RaggedLayerCache:
     state: RaggedBatchState
 
 
-def _plain_weight(w: torch.Tensor, dtype: torch.dtype, device: int) -> bool:
-    return type(w) is nn.Parameter and w.dtype == dtype and w.get_device() == device and w.is_contiguous() and w.data_ptr() % 16 == 0
+def _plain_pointers(tensors, dtype: torch.dtype, device: int):
+    """The addresses of ``tensors`` where all are plain contiguous parameters of the dtype on the device that start on 16 bytes; else None."""
+    out = []
+    for w in tensors:
+        if type(w) is not nn.Parameter or w.dtype is not dtype or w.get_device() != device or not w.is_contiguous():
+            return None
+        at = w.data_ptr()
+        if at & 15:
+            return None
+        out.append(at)
+    return out
 
 
 def _plain_modules(layer: nn.Module):
@@ -339,15 +348,20 @@ def _plain_modules(layer: nn.Module):
     mod = nn.modules.module
     if mod._global_forward_hooks or mod._global_forward_pre_hooks:
         return None
-    groups = {grp: layer._modules.get(grp) for grp in ("self_attn", "mlp")}
-    if None in groups.values():
+    own = layer._modules
+    attn, mlp = own.get("self_attn"), own.get("mlp")
+    if attn is None or mlp is None:
         return None
-    linears = [groups[grp]._modules.get(name) for grp, name in layer._LINEARS]
-    norms = (layer._modules.get("input_layernorm"), layer._modules.get("post_attention_layernorm"))
-    if any(type(sub) is not nn.Linear or sub.bias is not None for sub in linears) or any(type(sub) is not RMSNorm for sub in norms):
-        return None
-    for sub in (*linears, *norms):
-        if sub._forward_hooks or sub._forward_pre_hooks or "forward" in sub.__dict__:
+    groups = {"self_attn": attn._modules, "mlp": mlp._modules}
+    linears = []
+    for grp, name in layer._LINEARS:
+        sub = groups[grp].get(name)
+        if type(sub) is not nn.Linear or sub._parameters.get("bias", sub) is not None or "bias" in sub.__dict__ or sub._forward_hooks or sub._forward_pre_hooks or "forward" in sub.__dict__:
+            return None
+        linears.append(sub)
+    norms = (own.get("input_layernorm"), own.get("post_attention_layernorm"))
+    for sub in norms:
+        if type(sub) is not RMSNorm or sub._forward_hooks or sub._forward_pre_hooks or "forward" in sub.__dict__:
             return None
     return linears, norms
 
@@ -452,14 +466,17 @@ class PagedLlamaDecoderLayer(nn.Module):
         if parts is None:
             return None
         linears, norms = parts
-        weights = [m.weight for m in linears]
+        # (a parametrized or pruned module has no such entry: its weight is made from others)
+        weights = [m._parameters.get("weight") for m in (*linears, *norms)]
+        if weights[4] is None:
+            return None
         ff = weights[4].shape[0]
         if B > ops.one_call_batch(self.hidden_size, ff) or not ops.llama_decode_layer_supported(
                 B, self.hidden_size, ff, self.num_heads, self.num_kv_heads, self.head_dim, kp.shape[2], x.dtype):
             return None
-        for w in (*weights, norms[0].weight, norms[1].weight):
-            if not _plain_weight(w, x.dtype, dev):
-                return None
+        pointers = _plain_pointers(weights, x.dtype, dev)
+        if pointers is None:
+            return None
         cos, sin = st.cos, st.sin
         if cos is None:
             f = self.inv_freq
@@ -469,9 +486,10 @@ class PagedLlamaDecoderLayer(nn.Module):
                 return None
         else:
             cos, sin = cos.reshape(B, self.head_dim), sin.reshape(B, self.head_dim)
-        return ops.llama_decode_layer(x, norms[0].weight, norms[0].variance_epsilon, weights, norms[1].weight, norms[1].variance_epsilon,
+        return ops.llama_decode_layer(x, weights[7], norms[0].variance_epsilon, weights[:7], weights[8], norms[1].variance_epsilon,
                                       position_ids, self.inv_freq, self.rope_attention_scaling, cos, sin, kp, handle.v_pool, st.block_tables,
-                                      st.context_lens, st.max_context_len, self.num_heads, num_splits=st.num_splits, flags=st.attn_flags)
+                                      st.context_lens, st.max_context_len, self.num_heads, num_splits=st.num_splits, flags=st.attn_flags,
+                                      pointers=pointers)
 
     # ---- forward -----------------------------------------------------------------------------------
     def forward(
