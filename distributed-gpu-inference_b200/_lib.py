@@ -318,6 +318,12 @@ MIXER_SIGNATURES = {
         c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p,
                 c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_size_t,
                 c_int, c_void_p]),
+    "b200_split_scan_ends": (
+        c_size_t, [c_int, c_int, c_int, c_int, c_int]),
+    "b200_split_scan_ext": (
+        c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p,
+                c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_size_t,
+                c_int, c_void_p, c_size_t, c_int, c_void_p]),
     "b200_delta_chunk_scan_supported": (
         c_int, [c_int, c_int, c_int]),
     "b200_delta_chunk_workspace": (

@@ -21,13 +21,17 @@
 // (relative 2-norm, bf16 inputs, portions of 1 .. 700 tokens; token by token / here): gated read-outs 6.50e-8 / 6.57e-8, state 9.3e-8 /
 // 7.0e-8; delta 1.31e-7 / 1.29e-7, 8.2e-8 / 8.1e-8; retention 3.8e-7 / 1.2e-7, 4.2e-7 / 1.1e-7.
 //
-// What bounds it.  The chain: latency - a chunk takes a lone warp per scheduler 1650 clocks (gated) and 2450 (delta) for 78 and 168
-// products of 8 clocks each, between which its conversions (two clocks each) stand; the CTAs of an SM overlap.  Two warps per 16 columns,
-// bulk copies and packed fp32 arithmetic were each slower.  The operands: issue slots, half of them, at seven CTAs per SM.
-// B200, bf16, 64 x 128 states, us token by token / here (operands + chain): gated, 6 portions of up to 1780 tokens of 16 heads 395 / 223
-// (68 + 155); delta, 8 x 2048 of 8 heads 467 / 304 (128 + 176); retention, 5 x 1024 of 16 heads 184 / 125 (36 + 89).
+// What bounds it.  The chain: latency - a chunk takes a lone warp per scheduler 1550 clocks (gated) and 2450 (delta) for 78 and 168
+// products of 8 clocks each, between which its conversions (two clocks each) stand; the CTAs of an SM overlap (three of them: 1250 clocks a
+// chunk, products 47 % of the time, issue slots as much).  Two warps per 16 columns, bulk copies and packed fp32 arithmetic were each slower.  Where
+// sequences and heads leave SMs idle the gated and the retention rule walk segments of a sequence at the same time (split_chain_kernel).  The
+// operands: accesses to shared memory (76 %) and issue slots (73 %), at eight CTAs per SM.
+// B200, bf16, 64 x 128 states, us token by token / here (operands + chain): gated, 6 portions of up to 1780 tokens of 16 heads 395 / 218
+// (67 + 151), 1 of 2048 of 4 heads 132 / 36 (in one piece 124); delta, 8 x 2048 of 8 heads 467 / 304 (128 + 176); retention, 5 x 1024 of 16 heads
+// 184 / 105 (27 + 78).
 #include <algorithm>
 #include <atomic>
+#include <cstddef>
 #include <type_traits>
 
 #include "../../include/b200_mixers.h"
@@ -79,6 +83,8 @@ struct SplitArgs {
   int* wild;              // the same order: the chunk holds a value that has no split
   int n_seqs, n_chunks;   // n_chunks: a bound of the step's
   int h0, heads;          // heads of this launch
+  int seg;                // chunks per segment (0: sequences in one piece), and where segments leave their ends: [slot][heads][64-column block]
+  float* ends;
   int H, G, dk, dv;
   int per_channel;        // delta: a decay logit and a bias per key channel (1) or one per head (0)
   int vec_qk, vec_a, vec_c;   // eight elements of q / k, a, the constants can be read at once
@@ -156,11 +162,12 @@ __device__ __forceinline__ int chunks_before(const SplitSeq* seqs, int seq) {
   for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
   return n;
 }
-// The sequence that chunk x of the step belongs to and its place in it (a warp's work); false: beyond the last.
-__device__ __forceinline__ bool find_chunk(const SplitSeq* seqs, int n_seqs, int x, int& seq, int& place) {
+// The sequence that piece x of the step belongs to and its place in it, a sequence having `pieces` of them (a warp's work); false: beyond the last.
+template <typename Pieces>
+__device__ __forceinline__ bool find_piece(const SplitSeq* seqs, int n_seqs, int x, int& seq, int& place, Pieces pieces) {
   const int lane = threadIdx.x & 31;
   for (int base = 0; base < n_seqs; base += 32) {
-    const int n = base + lane < n_seqs ? chunks_of(seqs[base + lane].count) : 0;
+    const int n = base + lane < n_seqs ? pieces(seqs[base + lane]) : 0;
     int sum = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -177,6 +184,17 @@ __device__ __forceinline__ bool find_chunk(const SplitSeq* seqs, int n_seqs, int
     x -= __shfl_sync(0xffffffffu, sum, 31);
   }
   return false;
+}
+
+// Segments that a sequence has beyond its first.
+__device__ __forceinline__ int extra_segments(const SplitSeq& s, int seg) { return (max(chunks_of(s.count), 1) - 1) / seg; }
+// The place that the first extra segment of `seq` has among all (a warp's work).
+__device__ __forceinline__ int extra_before(const SplitSeq* seqs, int seq, int seg) {
+  int n = 0;
+  for (int i = threadIdx.x & 31; i < seq; i += 32) n += extra_segments(seqs[i], seg);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+  return n;
 }
 
 // Eight elements of a row from channel e on, `left` of which exist.
@@ -249,7 +267,7 @@ split_prepare_kernel(const SplitArgs A) {
   extern __shared__ __align__(16) unsigned char prep_raw[];
   Prep<RULE>& sm = *reinterpret_cast<Prep<RULE>*>(prep_raw);
   int seq, place;
-  if (!find_chunk(A.seqs, A.n_seqs, blockIdx.x, seq, place)) return;
+  if (!find_piece(A.seqs, A.n_seqs, blockIdx.x, seq, place, [](const SplitSeq& s) { return chunks_of(s.count); })) return;
   const SplitSeq sq = A.seqs[seq];
   const int h = A.h0 + blockIdx.y, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_live = min(kTok, sq.count - place * kTok);
@@ -581,6 +599,7 @@ __device__ __forceinline__ void walk_tokens(const SplitArgs& A, const SplitSeq& 
 constexpr int kStages = 3;
 constexpr int kCols = 64;              // value columns of a CTA
 constexpr int kChainNT = 2 * kCols;
+constexpr int kEnd = kChainNT * 32 + 2 * kDK;     // floats of a segment's end: the state as its threads hold it, the product of its decays as two floats
 template <int RULE, typename T>
 struct Stage {
   Ops<RULE> ops;
@@ -639,21 +658,39 @@ __device__ __forceinline__ void mma6(Tiles& x, Tiles& s, Tiles& t, const Split& 
   mma_new(x[0], a.hi, b.hi.x, b.hi.y), mma_new(x[1], a.hi, b.hi.z, b.hi.w);
 }
 
-// Four warps of 16 value columns each
-template <int RULE, typename T>
-__global__ void __launch_bounds__(kChainNT)
-split_chain_kernel(const SplitArgs A) {
+// Four warps of 16 value columns each.
+//
+// Sequences in segments (A.seg; not the delta rule, whose decay is no diagonal): the first launch walks every sequence's first segment and, from a
+// zero state and without read-outs, those between the first and the last; the second launch (`later`) starts the others from
+// S <- F S + end over the segments before, F being a segment's product of decays.  The state pool is read by the first launch and
+// written by the one that walks a sequence's last segment.
+template <int RULE, typename T, int CTAS>
+__global__ void __launch_bounds__(kChainNT, CTAS)
+split_chain_kernel(const SplitArgs A, const bool later) {
   constexpr bool kHalfIn = std::is_same_v<T, __half>;
   using S_t = Stage<RULE, T>;
   extern __shared__ __align__(128) unsigned char chain_raw[];
   Chain<RULE, T>& sm = *reinterpret_cast<Chain<RULE, T>*>(chain_raw);
-  const SplitSeq sq = A.seqs[blockIdx.x];
+  int seq = blockIdx.x, seg = 0;
+  const bool cut = RULE != kDelta && A.seg > 0;
+  if (cut && (later || seq >= A.n_seqs)) {
+    const int x = later ? seq : seq - A.n_seqs, per = A.seg;
+    if (!find_piece(A.seqs, A.n_seqs, x, seq, seg, [per](const SplitSeq& s) { return extra_segments(s, per); })) return;
+    ++seg;
+  }
+  const SplitSeq sq = A.seqs[seq];
   const int h = A.h0 + blockIdx.y, H = A.H, dk = A.dk, dv = A.dv;
   const int col_cta = blockIdx.z * kCols;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_chunks = chunks_of(sq.count);
-  const int before = chunks_before(A.seqs, blockIdx.x);
-  const int64_t first = static_cast<int64_t>(before) * A.heads + blockIdx.y;
+  const int n_all = chunks_of(sq.count), last_seg = cut ? extra_segments(sq, A.seg) : 0;
+  const int c0 = cut ? seg * A.seg : 0, n_chunks = cut ? min(A.seg, n_all - c0) : n_all;
+  const int before = chunks_before(A.seqs, seq);
+  const bool made = before + n_all <= A.n_chunks;      // sequences that share tokens may have more chunks than the workspace: no operands
+  const int64_t first = static_cast<int64_t>(before + c0) * A.heads + blockIdx.y;
+  // a segment's end: threads' states in float4s, then the decays.  The first segment of a cut sequence has 1 / 0 in their place: walked by tokens / not
+  const int slot0_seg = last_seg > 0 ? extra_before(A.seqs, seq, A.seg) : 0;
+  auto end_of = [&](int s) { return A.ends + ((static_cast<int64_t>(slot0_seg + s) * A.heads + blockIdx.y) * gridDim.z + blockIdx.z) * kEnd; };
+  if (seg > 0 && (!made || (!later && seg == last_seg))) return;
 
   const int r = lane >> 2, c = lane & 3, m = lane >> 3, l8 = lane & 7;
   const int col = col_cta + 16 * warp + r;           // and col + 8
@@ -664,22 +701,57 @@ split_chain_kernel(const SplitArgs A) {
   const T* vp = static_cast<const T*>(A.v) + sq.tok0 * A.stride + static_cast<int64_t>(h) * dv + col_cta;
 
   float S[8][4];          // S^T: columns col, col + 8; channels 8 j + 2 c, + 1
-  const bool made = before + n_chunks <= A.n_chunks;      // sequences that share tokens may have more chunks than the workspace: no operands
-  bool odd = !made;
+  auto leave_end = [&](float* end) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < 8; ++j) reinterpret_cast<float4*>(end)[j * kChainNT + threadIdx.x] = make_float4(S[j][0], S[j][1], S[j][2], S[j][3]);
+  };
+  if (seg == 0) {
+    bool odd = !made;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int e = 8 * j + 2 * c + (i & 1);
-      S[j][i] = !sq.fresh && e < dk && (i >> 1 ? in1 : in0) ? sp[static_cast<int64_t>(e) * dv + 8 * (i >> 1)] : 0.f;
-      odd = odd || !tame(S[j][i]);
+    for (int j = 0; j < 8; ++j) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = 8 * j + 2 * c + (i & 1);
+        S[j][i] = !sq.fresh && e < dk && (i >> 1 ? in1 : in0) ? sp[static_cast<int64_t>(e) * dv + 8 * (i >> 1)] : 0.f;
+        odd = odd || !tame(S[j][i]);
+      }
     }
+    for (int i = threadIdx.x; made && i < n_all; i += kChainNT) odd = odd || A.wild[first + static_cast<int64_t>(i) * A.heads];
+    odd = __syncthreads_or(odd);
+    if (made && last_seg > 0 && threadIdx.x == 0) end_of(0)[kChainNT * 32] = odd ? 1.f : 0.f;
+    if (odd) {
+      walk_tokens<RULE, T>(A, sq, h, sp, op, vp, 16 * warp + r, in0, in1, reinterpret_cast<float*>(chain_raw));
+      return;
+    }
+  } else if (later) {
+    const float* end = end_of(0);
+    if (end[kChainNT * 32] != 0.f) return;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float4 x = reinterpret_cast<const float4*>(end)[j * kChainNT + threadIdx.x];
+      S[j][0] = x.x, S[j][1] = x.y, S[j][2] = x.z, S[j][3] = x.w;
+    }
+#pragma unroll 1
+    for (int s = 1; s < seg; ++s) {
+      end = end_of(s);
+      const float* f = end + kChainNT * 32;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 x = reinterpret_cast<const float4*>(end)[j * kChainNT + threadIdx.x];
+        const float2 hi = *reinterpret_cast<const float2*>(f + 8 * j + 2 * c), lo = *reinterpret_cast<const float2*>(f + kDK + 8 * j + 2 * c);
+        S[j][0] = fmaf(S[j][0], hi.x, fmaf(S[j][0], lo.x, x.x)), S[j][1] = fmaf(S[j][1], hi.y, fmaf(S[j][1], lo.y, x.y));
+        S[j][2] = fmaf(S[j][2], hi.x, fmaf(S[j][2], lo.x, x.z)), S[j][3] = fmaf(S[j][3], hi.y, fmaf(S[j][3], lo.y, x.w));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) S[j][0] = S[j][1] = S[j][2] = S[j][3] = 0.f;
   }
-  for (int i = threadIdx.x; made && i < n_chunks; i += kChainNT) odd = odd || A.wild[first + static_cast<int64_t>(i) * A.heads];
-  if (__syncthreads_or(odd)) {
-    walk_tokens<RULE, T>(A, sq, h, sp, op, vp, 16 * warp + r, in0, in1, reinterpret_cast<float*>(chain_raw));
-    return;
+  if (seg > 0) {
+    op += static_cast<int64_t>(c0) * kTok * o_tok;
+    vp += static_cast<int64_t>(c0) * kTok * A.stride;
   }
+  const int n_tok = sq.count - c0 * kTok;      // from the segment's first on
 
   // what a thread copies of every chunk: 16-byte pieces of the operands, eight values of one token
   constexpr int kPieces = sizeof(Ops<RULE>) / 16;
@@ -688,16 +760,17 @@ split_chain_kernel(const SplitArgs A) {
   const int v_tok = threadIdx.x >> 3, v_col = 8 * (threadIdx.x & 7), v_left = dv - col_cta - v_col;
   const bool v_wide = A.vec_v == 8 && dv - col_cta >= kCols;      // the same for all
   const T* v_src = vp + static_cast<int64_t>(v_tok) * A.stride + v_col;
-  auto fetch = [&](int q, int at) {        // called for q = 0, 1, 2 ..
+  auto fetch = [&](int q, int at, auto part) {        // called for q = 0, 1, 2 ..; `part`: what a state alone needs (k, and p behind it, to f_end)
     if (q < n_chunks) {
+      constexpr int kFrom = decltype(part)::value ? offsetof(OpsBase, k) / 16 : 0;
       S_t& st = sm.stages[at];
       const uint32_t dst = smem_addr(&st.ops) + 16 * threadIdx.x;
 #pragma unroll
-      for (int i = 0; i < kPieces; i += kChainNT) {
+      for (int i = kFrom; i < kPieces; i += kChainNT) {
         if (i + kChainNT <= kPieces || threadIdx.x < kPieces - i) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * i), "l"(src + i) : "memory");
       }
       src += src_step;
-      const bool live = q * kTok + v_tok < sq.count;              // zeros beyond the last token
+      const bool live = q * kTok + v_tok < n_tok;                 // zeros beyond the last token
       const T* from = live ? v_src : vp;
       T* to = &st.v[v_tok][v_col];
       if (v_wide) {
@@ -746,9 +819,8 @@ split_chain_kernel(const SplitArgs A) {
     mma(s[0], vh, b.mid.x, b.mid.y), mma(s[1], vh, b.mid.z, b.mid.w);
     if constexpr (kHalfIn) mma(s[0], vl, b.hi.x, b.hi.y), mma(s[1], vl, b.hi.z, b.hi.w);
   };
-  // the state's channels 16 kk .. + 15 at the chunk's end, and their parts for the next chunk
-  Split a[4];
-  auto step = [&](const Ops<RULE>& ops, int kk, const Tiles& z) {
+  // the state's channels 16 kk .. + 15 at the chunk's end
+  auto carry = [&](const Ops<RULE>& ops, int kk, const Tiles& z) {
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       const int j = 2 * kk + t;
@@ -756,12 +828,49 @@ split_chain_kernel(const SplitArgs A) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) S[j][i] = fmaf(S[j][i], i & 1 ? hi.y : hi.x, fmaf(S[j][i], i & 1 ? lo.y : lo.x, z[t][i]));
     }
+  };
+  if constexpr (RULE != kDelta) {
+    if (seg > 0 && !later) {                 // the state alone, from zero
+      float f = 1.f, f_lo = 0.f;             // threads 0 .. 63: the product of a channel's decays
+#pragma unroll
+      for (int q = 0; q < kStages - 1; ++q) fetch(q, q, std::true_type{});
+      int at = 0;
+#pragma unroll 1
+      for (int q = 0; q < n_chunks; ++q) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        __syncthreads();
+        const S_t& st = sm.stages[at];
+        at = at == kStages - 1 ? 0 : at + 1;
+        fetch(q + kStages - 1, at == kStages - 1 ? 0 : at + 1, std::true_type{});
+        values(st);
+        Tiles z0, z1, z2, z3;
+        mma_v2(z0, z1, frag(st.ops.k, 0), frag(st.ops.k, 1));
+        mma_v2(z2, z3, frag(st.ops.k, 2), frag(st.ops.k, 3));
+        if (threadIdx.x < kDK) {
+          const float g = st.ops.f_end[0][threadIdx.x], p = f * g;
+          f_lo = fmaf(f_lo, g, fmaf(f, st.ops.f_end[1][threadIdx.x], fmaf(f, g, -p)));
+          f = p;
+        }
+        carry(st.ops, 0, z0), carry(st.ops, 1, z1), carry(st.ops, 2, z2), carry(st.ops, 3, z3);
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      float* end = end_of(seg);
+      leave_end(end);
+      if (threadIdx.x < kDK) end[kChainNT * 32 + threadIdx.x] = f, end[kChainNT * 32 + kDK + threadIdx.x] = f_lo;
+      return;
+    }
+  }
+  Split a[4];          // the state's parts (delta rule)
+  auto step = [&](const Ops<RULE>& ops, int kk, const Tiles& z) {
+    carry(ops, kk, z);
     split_tiles(a[kk], S[2 * kk], S[2 * kk + 1]);
   };
+  if constexpr (RULE == kDelta) {
 #pragma unroll
-  for (int kk = 0; kk < 4; ++kk) split_tiles(a[kk], S[2 * kk], S[2 * kk + 1]);
+    for (int kk = 0; kk < 4; ++kk) split_tiles(a[kk], S[2 * kk], S[2 * kk + 1]);
+  }
 #pragma unroll
-  for (int q = 0; q < kStages - 1; ++q) fetch(q, q);
+  for (int q = 0; q < kStages - 1; ++q) fetch(q, q, std::false_type{});
   float* out = op + 2 * c * o_tok;
   int at = 0;
 #pragma unroll 1
@@ -785,7 +894,7 @@ split_chain_kernel(const SplitArgs A) {
       if constexpr (kHalfIn) mma(v[0], vl, one, 0u), mma(v[1], vl, 0u, one);
       add(w, y0), add(s0, t0);
       mma6x2(o, y, s, t, a[0], frag(ops.q, 0), a[1], frag(ops.q, 1));
-      fetch(q + kStages - 1, next);
+      fetch(q + kStages - 1, next, std::false_type{});
       add(x1, y1), add(s0, s1), add(s0, t1), add(w, x1), add(w, s0);
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
@@ -815,26 +924,32 @@ split_chain_kernel(const SplitArgs A) {
       step(ops, 3, s2);
       add(o, s);
     } else {
-      Tiles z0, z1, z2, z3, pv, ps, x2, y2, s2, t2;
-      mma_v2(z0, z1, frag(ops.k, 0), frag(ops.k, 1));
+      // channels in two halves: the state's parts live for their products only, so that their registers hold two halves of them and three CTAs fit an SM
+      Tiles z0, z1, pv, ps;
       mma_v(pv, ps, frag1(ops.p));
-      mma6x2(x, y, s, t, a[0], frag(ops.q, 0), a[1], frag(ops.q, 1));
-      fetch(q + kStages - 1, next);
-      mma_v2(z2, z3, frag(ops.k, 2), frag(ops.k, 3));
-      step(ops, 0, z0);
-      step(ops, 1, z1);
-      mma6x2(x2, y2, s2, t2, a[2], frag(ops.q, 2), a[3], frag(ops.q, 3));
-      add(x, y), add(ps, s), add(ps, t), add(x, pv);
-      step(ops, 2, z2);
-      step(ops, 3, z3);
-      add(x2, y2), add(ps, s2), add(ps, t2), add(x2, ps);
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
+      for (int kk = 0; kk < 4; kk += 2) {
+        Split a0, a1;
+        split_tiles(a0, S[2 * kk], S[2 * kk + 1]);
+        split_tiles(a1, S[2 * kk + 2], S[2 * kk + 3]);
+        mma_v2(z0, z1, frag(ops.k, kk), frag(ops.k, kk + 1));
+        mma6x2(x, y, s, t, a0, frag(ops.q, kk), a1, frag(ops.q, kk + 1));
+        if (kk == 0) fetch(q + kStages - 1, next, std::false_type{});
+        carry(ops, kk, z0), carry(ops, kk + 1, z1);
+        add(x, y), add(ps, s), add(ps, t);
+        if (kk == 0) {
+          add(x, pv);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) o[g][i] = x[g][i] + x2[g][i];
+          for (int g = 0; g < 2; ++g) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[g][i] = x[g][i];
+          }
+        } else {
+          add(x, ps), add(o, x);
+        }
       }
     }
-    const int n = sq.count - q * kTok;
+    const int n = n_tok - q * kTok;
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
 #pragma unroll
@@ -845,6 +960,10 @@ split_chain_kernel(const SplitArgs A) {
     out += kTok * o_tok;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (seg < last_seg) {
+    if (seg == 0) leave_end(end_of(0));
+    return;
+  }
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
 #pragma unroll
@@ -857,6 +976,8 @@ split_chain_kernel(const SplitArgs A) {
 
 // ---- host ---------------------------------------------------------------------------------------------------------------------------
 size_t ops_bytes(int rule) { return (rule == kDelta ? sizeof(Ops<kDelta>) : sizeof(Ops<kGated>)) + sizeof(int); }
+// Slots of segments' ends: a sequence of n chunks has (n - 1) / seg segments beyond its first.
+int64_t slots_bound(int n_chunks, int seg) { return n_chunks / seg; }
 int64_t chunk_bound(int n_tok, int n_seqs) { return static_cast<int64_t>(n_tok) / kTok + n_seqs; }
 
 template <int RULE, typename T>
@@ -871,12 +992,14 @@ int launch_split(SplitArgs& A, void* workspace, size_t bytes, cudaStream_t strea
   if (most <= 0) return fail(B200_EINVAL, "%s: workspace of %zu bytes, one head takes %zu", name, bytes, per_head);
   constexpr size_t smem = sizeof(Chain<RULE, T>);
   static_assert(kStages == 3 && sizeof(Prep<RULE>) <= 48 * 1024 && smem <= static_cast<size_t>(kMaxSmem));
-  auto chain = split_chain_kernel<RULE, T>;
+  // segments: three CTAs per SM (168 registers, a few words spilled); in one piece the walk is a lone warp's latency
+  auto chain = RULE != kDelta && A.seg > 0 ? split_chain_kernel<RULE, T, RULE == kDelta ? 2 : 3> : split_chain_kernel<RULE, T, 2>;
   static std::atomic<uint64_t> ready{0};      // a bit per device: the limit is always the same, a call need not set it again
   int device = 0;
   cudaGetDevice(&device);
   if (device >= 64 || !(ready.load(std::memory_order_acquire) >> device & 1)) {
-    cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaFuncSetAttribute(split_chain_kernel<RULE, T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (RULE != kDelta) cudaFuncSetAttribute(split_chain_kernel<RULE, T, RULE == kDelta ? 2 : 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (device < 64) ready.fetch_or(1ull << device, std::memory_order_release);
   }
   for (A.h0 = 0; A.h0 < A.H; A.h0 += most) {
@@ -885,8 +1008,13 @@ int launch_split(SplitArgs& A, void* workspace, size_t bytes, cudaStream_t strea
     A.wild = reinterpret_cast<int*>(A.ops + static_cast<size_t>(A.n_chunks) * A.heads * sizeof(Ops<RULE>));
     split_prepare_kernel<RULE, T><<<dim3(A.n_chunks, A.heads), 128, sizeof(Prep<RULE>), stream>>>(A);
     if (int rc = check_launch(name)) return rc;
-    chain<<<dim3(A.n_seqs, A.heads, (A.dv + kCols - 1) / kCols), kChainNT, smem, stream>>>(A);
+    const int extra = A.seg > 0 ? static_cast<int>(slots_bound(A.n_chunks, A.seg)) : 0, blocks = (A.dv + kCols - 1) / kCols;
+    chain<<<dim3(A.n_seqs + extra, A.heads, blocks), kChainNT, smem, stream>>>(A, false);
     if (int rc = check_launch(name)) return rc;
+    if (extra > 0) {
+      chain<<<dim3(extra, A.heads, blocks), kChainNT, smem, stream>>>(A, true);
+      if (int rc = check_launch(name)) return rc;
+    }
   }
   return 0;
 }
@@ -905,10 +1033,24 @@ size_t b200_split_scan_workspace(int rule, int n_tok, int n_seqs, int heads) {
   return static_cast<size_t>(chunk_bound(n_tok, n_seqs)) * heads * ops_bytes(rule == 1 ? kDelta : kGated);
 }
 
+size_t b200_split_scan_ends(int segment, int n_tok, int n_seqs, int heads, int dv) {
+  if (segment <= 0 || n_tok < 0 || n_seqs < 0 || heads < 0 || dv < 0) return 0;
+  return static_cast<size_t>(slots_bound(static_cast<int>(chunk_bound(n_tok, n_seqs)), segment)) * heads * ((dv + kCols - 1) / kCols) * kEnd * sizeof(float);
+}
+
 int b200_split_scan(int rule, float* o_raw, const void* q, const void* k, const void* v, int64_t in_stride, const void* beta_logit,
                     int64_t beta_stride, const void* a_logit, int64_t a_stride, const void* bias, const void* rate, const float* decay,
                     int per_channel, float* state, const int32_t* seqs, int n_seqs, int n_tok, int H, int G, int dk, int dv,
                     float unit_eps, float scale, void* workspace, size_t workspace_bytes, int dtype, void* stream) {
+  return b200_split_scan_ext(rule, o_raw, q, k, v, in_stride, beta_logit, beta_stride, a_logit, a_stride, bias, rate, decay, per_channel, state,
+                             seqs, n_seqs, n_tok, H, G, dk, dv, unit_eps, scale, workspace, workspace_bytes, 0, nullptr, 0, dtype, stream);
+}
+
+int b200_split_scan_ext(int rule, float* o_raw, const void* q, const void* k, const void* v, int64_t in_stride, const void* beta_logit,
+                        int64_t beta_stride, const void* a_logit, int64_t a_stride, const void* bias, const void* rate, const float* decay,
+                        int per_channel, float* state, const int32_t* seqs, int n_seqs, int n_tok, int H, int G, int dk, int dv,
+                        float unit_eps, float scale, void* workspace, size_t workspace_bytes, int segment, float* ends, size_t ends_bytes,
+                        int dtype, void* stream) {
   const char* name = "b200_split_scan";
   if (rule < 0 || rule > 2 || n_seqs < 0 || n_tok < 0 || H <= 0 || G <= 0 || H % G || dk <= 0 || dv <= 0) return fail(B200_EINVAL, "%s: bad sizes", name);
   if (!b200_split_scan_supported(dk, dtype)) return fail(B200_ESHAPE, "%s: key size %d or dtype %d not served", name, dk, dtype);
@@ -916,6 +1058,9 @@ int b200_split_scan(int rule, float* o_raw, const void* q, const void* k, const 
   const bool missing = rule == kRetention ? !decay : !bias || !rate || (rule == kDelta && (!beta_logit || !a_logit));
   if (!o_raw || !q || !k || !v || !state || !seqs || !workspace || missing) return fail(B200_EINVAL, "%s: null pointer", name);
   if (!aligned16(workspace)) return fail(B200_EINVAL, "%s: workspace is not 16-byte aligned", name);
+  if (segment < 0 || (segment > 0 && rule == kDelta)) return fail(B200_EINVAL, "%s: segments of %d chunks for rule %d", name, segment, rule);
+  if (segment > 0 && (!ends || !aligned16(ends) || ends_bytes < b200_split_scan_ends(segment, n_tok, n_seqs, H, dv)))
+    return fail(B200_EINVAL, "%s: no room for the ends of segments", name);
   SplitArgs A{};
   A.o = o_raw, A.q = q, A.k = k, A.v = v, A.stride = in_stride;
   A.beta = beta_logit, A.beta_stride = beta_stride, A.a = a_logit, A.a_stride = a_stride;
@@ -923,6 +1068,7 @@ int b200_split_scan(int rule, float* o_raw, const void* q, const void* k, const 
   A.state = state, A.seqs = reinterpret_cast<const SplitSeq*>(seqs);
   A.n_seqs = n_seqs, A.n_chunks = static_cast<int>(chunk_bound(n_tok, n_seqs));
   A.H = H, A.G = G, A.dk = dk, A.dv = dv, A.unit_eps = unit_eps, A.scale = scale;
+  A.seg = segment, A.ends = ends;
   auto st = static_cast<cudaStream_t>(stream);
   auto go = [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;

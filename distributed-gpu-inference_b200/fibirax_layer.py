@@ -189,12 +189,10 @@ class ParallelMixer(nn.Module):
             mixer_ops.mixed_paged_attention(attn, q.unflatten(1, (H, dk)), cache.k_pool, cache.v_pool, st.block_tables,
                                             st.tok_row, st.tok_pos, self.scale, sink=self.sink, window=self.window,
                                             softcap=self.softcap)
-        # right: retention over the state slots.  Few CTAs and long portions: parallel segments; B200, 64 x 128 states, us in chunks /
-        # in segments: 16 CTAs of 32 columns 1024 tokens 64 / 54, 2048 119 / 69; 32 CTAs 65 / 68, 120 / 90; 64 CTAs 68 / 90, 127 / 138.  The
-        # mixer from Python: 16 CTAs 768 tokens 149 / 154, 1152 146 / 146; 32 CTAs 1152 143 / 148, 1500 164 / 152; 64 CTAs 1500 189 / 210
+        # right: retention over the state slots: 16-bit types in chunks, which have segments of their own; others in the plan's segments
         ctas = Hr * ((dvr + 31) // 32)
         longest = st.max_count() if h.shape[0] >= mixer_ops.SPLIT_SCAN_FROM[2] else 0      # decode steps need not look
-        chunks = (ctas * len(st.spans) >= 64 or longest < 700 + 20 * ctas * len(st.spans)) and mixer_ops.split_scan_takes(2, longest, h.shape[0], len(st.spans), Hr, dkr, dvr, h.dtype)
+        chunks = mixer_ops.split_scan_takes(2, longest, h.shape[0], len(st.spans), Hr, dkr, dvr, h.dtype)
         o = mixer_ops.retention_scan(proj[:, c[3]:c[3] + Hr * dkr], proj[:, c[4]:c[4] + Hr * dkr],
                                      proj[:, c[5]:c[5] + Hr * dvr], self.decay, dkr ** -0.5, cache.rstate, st.scan_seqs,
                                      plan=None if chunks else st.scan_plan(ctas_per_seq=ctas), max_count=longest)

@@ -241,6 +241,12 @@ def _chunk_bytes(rule: int) -> int:
     return int(_lib_().b200_split_scan_workspace(rule, 0, 1, 1))
 
 
+@functools.lru_cache(maxsize=None)
+def _end_floats() -> int:
+    """What a segment leaves per head and 64 value columns."""
+    return int(_lib_().b200_split_scan_ends(1, 0, 1, 1, 64)) // 4
+
+
 def _chunk_workspace(one: int, H: int, device: torch.device) -> Optional[torch.Tensor]:
     """Room for the chunk operands (``one`` bytes a head) of as many of ``H`` heads as the device still holds; None: not for one."""
     heads = max(1, min(H, SPLIT_SCAN_WORKSPACE // one))
@@ -252,8 +258,23 @@ def _chunk_workspace(one: int, H: int, device: torch.device) -> Optional[torch.T
     return None
 
 
+def split_scan_segment(rule: int, longest: int, n: int, n_seqs: int, H: int, dv: int) -> int:
+    """Chunks per segment of a step in chunks; 0: its sequences in one piece.  Segments make the walk shorter and the work 1.4 times as much (the
+    state of the middle ones is walked twice), so they pay where the sequences leave SMs idle and the longest takes twice as long as an SM's share
+    of the work.  Not for the delta rule, whose decay is no diagonal.  B200, bf16, 64 x 128 states, us in one piece / in segments,
+    operands included: 4 heads, 1 of 2048 124 / 36, 8 of 2048 160 / 124, 8 of 512 45 / 44, 16 of 400 44 / (58), 1 of 512 38 / 24; 8 heads, 6 of 720 -
+    1780 139 / 105, 8 of 1024 102 / (118); 16 heads, 2 of 1000 79 / 67.  (More CTAs than SMs: 16 heads, 6 of 720 - 1780 225 / 181 in a graph by
+    themselves, but the gated mixer around them 361 / 362.)  Their length: short ones fill the chip from little work, long ones start seldom and add
+    fewer ends up (4 heads, 1 of 2048: 4 chunks 38, 8 35, 16 47; 16 heads, 1 of 8192: 8 chunks 321, 16 239, 32 239)."""
+    chunks, blocks = (longest + 15) // 16, H * -(-dv // 64)
+    share = (n // 16 + n_seqs) * blocks / 148
+    if rule == 1 or chunks < 32 or n_seqs * blocks > 148 or chunks < 2 * share:
+        return 0
+    return int(max(4 + share / 8, chunks / 32))
+
+
 def _split_scan(rule: int, o, q, k, v, stride: int, beta, a, bias, rate, decay, per_channel: bool, state, seqs, G: int, eps: float,
-                scale: float) -> bool:
+                scale: float, longest: int = 0) -> bool:
     """``b200_split_scan`` into ``o``; ``beta`` and ``a`` are (tensor or None, row stride).  False, with nothing done, where the device
     has no memory left for its workspace: the token-by-token scans need none."""
     _, H, dk, dv = state.shape
@@ -261,9 +282,16 @@ def _split_scan(rule: int, o, q, k, v, stride: int, beta, a, bias, rate, decay, 
     ws = _chunk_workspace((n // 16 + n_seqs) * _chunk_bytes(rule), H, q.device)
     if ws is None:
         return False
-    rc = lib.b200_split_scan(rule, o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), stride, _ptr(beta[0]), beta[1], _ptr(a[0]), a[1],
+    segment, ends = split_scan_segment(rule, longest, n, n_seqs, H, dv), None
+    if segment:
+        try:
+            ends = torch.empty((n // 16 + n_seqs) // segment * H * -(-dv // 64) * _end_floats(), dtype=torch.float32, device=q.device)
+        except torch.OutOfMemoryError:
+            segment = 0
+    rc = lib.b200_split_scan_ext(rule, o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), stride, _ptr(beta[0]), beta[1], _ptr(a[0]), a[1],
                              _ptr(bias), _ptr(rate), _ptr(decay), int(per_channel), state.data_ptr(), seqs.data_ptr(), n_seqs, n, H, G, dk,
-                             dv, float(eps), float(scale), ws.data_ptr(), ws.numel(), DTYPE_ID[q.dtype], _stream())
+                             dv, float(eps), float(scale), ws.data_ptr(), ws.numel(), segment, _ptr(ends),
+                                 4 * ends.numel() if segment else 0, DTYPE_ID[q.dtype], _stream())
     _lib.check_mixers(rc, "b200_split_scan")
     return True
 
@@ -290,7 +318,7 @@ def gated_scan(zq: torch.Tensor, zf: torch.Tensor, v: torch.Tensor, f_bias: torc
         raise ValueError("seqs must be contiguous int32 [n_seqs, 4]")
     o = torch.empty((n, H, dv), dtype=torch.float32, device=zq.device)
     if split_scan_takes(0, max_count, n, seqs.shape[0], H, dk, dv, zq.dtype) and _split_scan(
-            0, o, zq, zf, v, stride, (None, 0), (None, 0), f_bias, lower, None, False, state, seqs, H, 0.0, 0.0):
+            0, o, zq, zf, v, stride, (None, 0), (None, 0), f_bias, lower, None, False, state, seqs, H, 0.0, 0.0, max_count):
         return o
     rc = _lib_().b200_gated_scan(o.data_ptr(), zq.data_ptr(), zf.data_ptr(), v.data_ptr(), stride, f_bias.data_ptr(),
                                  lower.data_ptr(), state.data_ptr(), seqs.data_ptr(), seqs.shape[0], int(max_count), H, dk, dv,
@@ -906,7 +934,7 @@ def retention_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
     _check_seqs(seqs)
     o = torch.empty((n, H, dv), dtype=torch.float32, device=q.device)
     if plan is None and split_scan_takes(2, max_count, n, seqs.shape[0], H, dk, dv, q.dtype) and _split_scan(
-            2, o, q, k, v, stride, (None, 0), (None, 0), None, None, decay, False, state, seqs, H, 0.0, k_scale):
+            2, o, q, k, v, stride, (None, 0), (None, 0), None, None, decay, False, state, seqs, H, 0.0, k_scale, max_count):
         return o
     lib, dt, st = _lib_(), DTYPE_ID[q.dtype], _stream()
 

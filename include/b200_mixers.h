@@ -538,6 +538,14 @@ int b200_split_scan(int rule, float* o_raw, const void* q, const void* k, const 
                     int64_t beta_stride, const void* a_logit, int64_t a_stride, const void* bias, const void* rate, const float* decay,
                     int per_channel, float* state, const int32_t* seqs, int n_seqs, int n_tok, int H, int G, int dk, int dv,
                     float unit_eps, float scale, void* workspace, size_t workspace_bytes, int dtype, void* stream);
+/* The same with sequences in segments of `segment` chunks of 16 tokens that are walked at the same time (rules 0 and 2; 0: in one
+ * piece); ends: b200_split_scan_ends(segment, n_tok, n_seqs, H, dv) bytes, 16-byte aligned. */
+size_t b200_split_scan_ends(int segment, int n_tok, int n_seqs, int heads, int dv);
+int b200_split_scan_ext(int rule, float* o_raw, const void* q, const void* k, const void* v, int64_t in_stride, const void* beta_logit,
+                        int64_t beta_stride, const void* a_logit, int64_t a_stride, const void* bias, const void* rate, const float* decay,
+                        int per_channel, float* state, const int32_t* seqs, int n_seqs, int n_tok, int H, int G, int dk, int dv,
+                        float unit_eps, float scale, void* workspace, size_t workspace_bytes, int segment, float* ends, size_t ends_bytes,
+                        int dtype, void* stream);
 
 /* ---- the delta rule with one decay per head in chunks, and per-channel selective state spaces ---------------------- */
 
