@@ -25,10 +25,10 @@
 // products of 8 clocks each, between which its conversions (two clocks each) stand; the CTAs of an SM overlap (three of them: 1250 clocks a
 // chunk, products 47 % of the time, issue slots as much).  Two warps per 16 columns, bulk copies and packed fp32 arithmetic were each slower.  Where
 // sequences and heads leave SMs idle the gated and the retention rule walk segments of a sequence at the same time (split_chain_kernel).  The
-// operands: accesses to shared memory (76 %) and issue slots (73 %), at eight CTAs per SM.
-// B200, bf16, 64 x 128 states, us token by token / here (operands + chain): gated, 6 portions of up to 1780 tokens of 16 heads 395 / 218
-// (67 + 151), 1 of 2048 of 4 heads 132 / 36 (in one piece 124); delta, 8 x 2048 of 8 heads 467 / 304 (128 + 176); retention, 5 x 1024 of 16 heads
-// 184 / 105 (27 + 78).
+// operands: issue slots and accesses to shared memory, three quarters of both, at eight CTAs per SM.
+// B200, bf16, 64 x 128 states, us token by token / here (operands + chain): gated, 6 portions of up to 1780 tokens of 16 heads 395 / 212
+// (64 + 148), 1 of 2048 of 4 heads 132 / 36 (in one piece 124); delta, 8 x 2048 of 8 heads 467 / 290 (118 + 172; columns of P on eight lanes each, whose
+// reads of a row four columns repeat, and the operands copied out by the threads: 138); retention, 5 x 1024 of 16 heads 184 / 98 (25 + 73).
 #include <algorithm>
 #include <atomic>
 #include <cstddef>
@@ -326,65 +326,71 @@ split_prepare_kernel(const SplitArgs A) {
   const bool ok = big < kWild * kWild && most < 1.001f;      // false for NaN
   const int any = __syncthreads_or(!ok);
 
-  // column s of P (and of A): eight lanes share it, eight channels each; the decayed key walks down the tokens
+  // Columns of P (and of A), four to a warp: sixteen lanes share two, four channels each, so that a row of the tokens is read once for both; the
+  // decayed keys walk down the tokens
   {
-    const int s = 4 * w + (lane >> 3), c = lane & 7;
-    auto load8 = [&](f32x2 (&d)[4], const float* row) {
-      const ulonglong2 lo = *reinterpret_cast<const ulonglong2*>(row + 4 * c), hi = *reinterpret_cast<const ulonglong2*>(row + 32 + 4 * c);
-      d[0] = lo.x, d[1] = lo.y, d[2] = hi.x, d[3] = hi.y;
+    const int s0 = 4 * w + 2 * (lane >> 4), c = lane & 15;
+    auto load4 = [&](f32x2 (&d)[2], const float* row) {
+      const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(row + 4 * c);
+      d[0] = x.x, d[1] = x.y;
     };
-    auto dot8 = [](const f32x2 (&x)[4], const f32x2 (&y)[4]) {
-      const float2 a = halves(fma2(x[1], y[1], mul2(x[0], y[0]))), b = halves(fma2(x[3], y[3], mul2(x[2], y[2])));
-      return (a.x + a.y) + (b.x + b.y);
+    auto dot4 = [](const f32x2 (&x)[2], const f32x2 (&y)[2]) {
+      const float2 a = halves(fma2(x[1], y[1], mul2(x[0], y[0])));
+      return a.x + a.y;
     };
-    // four partial sums of every lane -> lanes 2 i and 2 i + 1 hold the sum of number i
-    auto sums = [&](const float (&v)[4]) {
-      const bool up4 = c & 4, up2 = c & 2;
-      float a[2];
+    // eight partial sums of every lane -> lanes 2 i and 2 i + 1 of the sixteen hold the sum of number i
+    auto sums = [&](const float (&v)[8]) {
+      const bool up8 = c & 8, up4 = c & 4, up2 = c & 2;
+      float a[4], b[2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float give = up8 ? v[i] : v[i + 4], keep = up8 ? v[i + 4] : v[i];
+        a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+      }
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const float give = up4 ? v[i] : v[i + 2], keep = up4 ? v[i + 2] : v[i];
-        a[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+        const float give = up4 ? a[i] : a[i + 2], keep = up4 ? a[i + 2] : a[i];
+        b[i] = keep + __shfl_xor_sync(0xffffffffu, give, 4);
       }
-      const float give = up2 ? a[0] : a[1], keep = up2 ? a[1] : a[0];
-      const float b = keep + __shfl_xor_sync(0xffffffffu, give, 2);
-      return b + __shfl_xor_sync(0xffffffffu, b, 1);
+      const float give = up2 ? b[0] : b[1], keep = up2 ? b[1] : b[0];
+      const float d = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+      return d + __shfl_xor_sync(0xffffffffu, d, 1);
     };
-    f32x2 kw[4];
-    load8(kw, sm.rows[1][s]);
-    auto block = [&](int t0, auto own) {          // four tokens; `own`: the block of s itself
+    f32x2 kw[2][2];
+    load4(kw[0], sm.rows[1][s0]);
+    load4(kw[1], sm.rows[1][s0 + 1]);
+    auto block = [&](int t0, auto own) {          // four tokens; `own`: the block of the columns themselves
       constexpr bool kOwn = decltype(own)::value;
-      float part[4];
-      [[maybe_unused]] float part_a[RULE == kDelta ? 4 : 1];
+      float part[8];
+      [[maybe_unused]] float part_a[RULE == kDelta ? 8 : 1];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int t = t0 + i;
-        f32x2 x[4];
+        f32x2 x[2];
         if (!kOwn || i > 0) {
-          const bool decays = !kOwn || t > s;
-          if constexpr (RULE == kRetention) {
-            const uint32_t f = __float_as_uint(decays && t < n_live ? ret : 1.0f);
+          if constexpr (RULE != kRetention) load4(x, sm.rows[RULE == kRetention ? 0 : 2][t]);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) kw[j] = mul2(kw[j], static_cast<f32x2>(f) << 32 | f);
-          } else {
-            load8(x, sm.rows[RULE == kRetention ? 0 : 2][t]);
+          for (int u = 0; u < 2; ++u) {
+            const bool decays = !kOwn || t > s0 + u;
+            [[maybe_unused]] const uint32_t f = __float_as_uint(decays && t < n_live ? ret : 1.0f);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if constexpr (RULE == kDelta) kw[j] = fma2(kw[j], decays ? x[j] : 0ull, kw[j]);
-              else kw[j] = mul2(kw[j], decays ? x[j] : 0x3f8000003f800000ull);
+            for (int j = 0; j < 2; ++j) {
+              if constexpr (RULE == kRetention) kw[u][j] = mul2(kw[u][j], static_cast<f32x2>(f) << 32 | f);
+              else if constexpr (RULE == kDelta) kw[u][j] = fma2(kw[u][j], decays ? x[j] : 0ull, kw[u][j]);
+              else kw[u][j] = mul2(kw[u][j], decays ? x[j] : 0x3f8000003f800000ull);
             }
           }
         }
-        load8(x, sm.rows[0][t]);
-        const float d = dot8(kw, x);
-        part[i] = !kOwn || t >= s ? d : 0.f;
+        load4(x, sm.rows[0][t]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) part[4 * u + i] = !kOwn || t >= s0 + u ? dot4(kw[u], x) : 0.f;
         if constexpr (RULE == kDelta) {
-          load8(x, sm.rows[1][t]);
-          const float e = dot8(kw, x);
-          part_a[i] = !kOwn || t > s ? e : 0.f;
+          load4(x, sm.rows[1][t]);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) part_a[4 * u + i] = !kOwn || t > s0 + u ? dot4(kw[u], x) : 0.f;
         }
       }
-      const int t = t0 + (c >> 1);
+      const int t = t0 + ((c >> 1) & 3), s = s0 + (c >> 3);
       const float p = sums(part);
       if ((c & 1) == 0) sm.p[t][s] = p;
       if constexpr (RULE == kDelta) {
@@ -392,7 +398,8 @@ split_prepare_kernel(const SplitArgs A) {
         if ((c & 1) == 0) sm.a[t][s] = sm.beta[t] * a;
       }
     };
-    for (int t = c; t < 4 * w; t += 8) {
+    for (int t = c >> 1; t < 4 * w; t += 8) {
+      const int s = s0 + (c & 1);
       sm.p[t][s] = 0.f;
       if constexpr (RULE == kDelta) sm.a[t][s] = 0.f;
     }
@@ -503,12 +510,17 @@ split_prepare_kernel(const SplitArgs A) {
     put(sm.ops.p[0], 32, to, reg, sm.p[t][s], sm.p[t][s + 1], 0.f, 0.f);
     if constexpr (RULE == kDelta) put(sm.ops.m[0], 32, to, reg, sm.a[t][s], sm.a[t][s + 1], 0.f, 0.f);
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
-  const int64_t place_of = static_cast<int64_t>(blockIdx.x) * A.heads + blockIdx.y;
-  uint4* dst = reinterpret_cast<uint4*>(A.ops + place_of * sizeof(Ops<RULE>));
-  const uint4* src = reinterpret_cast<const uint4*>(&sm.ops);
-  for (int i = threadIdx.x; i < static_cast<int>(sizeof(Ops<RULE>) / 16); i += 128) dst[i] = src[i];
-  if (threadIdx.x == 0) A.wild[place_of] = any;
+  if (threadIdx.x == 0) {      // out by the copy engine
+    const int64_t place_of = static_cast<int64_t>(blockIdx.x) * A.heads + blockIdx.y;
+    static_assert(sizeof(Ops<RULE>) % 16 == 0 && offsetof(Prep<RULE>, ops) == 0);
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(A.ops + place_of * static_cast<int64_t>(sizeof(Ops<RULE>))), "r"(smem_addr(&sm.ops)),
+                 "n"(sizeof(Ops<RULE>)) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    A.wild[place_of] = any;
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  }
 }
 
 // ---- token by token, for a (sequence, head) that holds a value without a split: a warp owns 16 columns, lane (r, c)
