@@ -241,12 +241,6 @@ def _chunk_bytes(rule: int) -> int:
     return int(_lib_().b200_split_scan_workspace(rule, 0, 1, 1))
 
 
-@functools.lru_cache(maxsize=None)
-def _end_floats() -> int:
-    """What a segment leaves per head and 64 value columns."""
-    return int(_lib_().b200_split_scan_ends(1, 0, 1, 1, 64)) // 4
-
-
 def _chunk_workspace(one: int, H: int, device: torch.device) -> Optional[torch.Tensor]:
     """Room for the chunk operands (``one`` bytes a head) of as many of ``H`` heads as the device still holds; None: not for one."""
     heads = max(1, min(H, SPLIT_SCAN_WORKSPACE // one))
@@ -264,13 +258,20 @@ def split_scan_segment(rule: int, longest: int, n: int, n_seqs: int, H: int, dv:
     of the work.  Not for the delta rule, whose decay is no diagonal.  B200, bf16, 64 x 128 states, us in one piece / in segments,
     operands included: 4 heads, 1 of 2048 124 / 36, 8 of 2048 160 / 124, 8 of 512 45 / 44, 16 of 400 44 / (58), 1 of 512 38 / 24; 8 heads, 6 of 720 -
     1780 139 / 105, 8 of 1024 102 / (118); 16 heads, 2 of 1000 79 / 67.  (More CTAs than SMs: 16 heads, 6 of 720 - 1780 225 / 181 in a graph by
-    themselves, but the gated mixer around them 361 / 362.)  Their length: short ones fill the chip from little work, long ones start seldom and add
+    themselves, but the gated mixer around them 361 / 362.)  Under 48 chunks they save less than the 7 us of host time that they take (8 heads, 6 of
+    210 - 690: 58 / 51).  Their length: short ones fill the chip from little work, long ones start seldom and add
     fewer ends up (4 heads, 1 of 2048: 4 chunks 38, 8 35, 16 47; 16 heads, 1 of 8192: 8 chunks 321, 16 239, 32 239)."""
     chunks, blocks = (longest + 15) // 16, H * -(-dv // 64)
-    share = (n // 16 + n_seqs) * blocks / 148
-    if rule == 1 or chunks < 32 or n_seqs * blocks > 148 or chunks < 2 * share:
+    if rule == 1 or chunks < 48 or n_seqs * blocks > 148:
         return 0
-    return int(max(4 + share / 8, chunks / 32))
+    share = (n // 16 + n_seqs) * blocks / 148
+    return int(max(4 + share / 8, chunks / 32)) if chunks >= 2 * share else 0
+
+
+@functools.lru_cache(maxsize=None)
+def _end_floats() -> int:
+    """What a segment leaves per head and 64 value columns."""
+    return int(_lib_().b200_split_scan_ends(1, 0, 1, 1, 64)) // 4
 
 
 def _split_scan(rule: int, o, q, k, v, stride: int, beta, a, bias, rate, decay, per_channel: bool, state, seqs, G: int, eps: float,
@@ -1243,6 +1244,25 @@ def router_logits(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
                                         x.shape[1], DTYPE_ID[x.dtype], _stream())
     _lib.check_mixers(rc, "b200_router_logits")
     return out
+
+
+@_timed
+def router_sigmoid_topk(x: torch.Tensor, w: torch.Tensor, top: int):
+    """``sigmoid_topk(router_logits(x, w), top)``; up to eight experts in one launch, the logits not written."""
+    E = w.shape[0]
+    if E > 8 or top > E:
+        return sigmoid_topk(router_logits(x, w), top)
+    _need_cuda(x, w)
+    if w.dtype != torch.float32 or x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1] \
+            or not x.is_contiguous() or not w.is_contiguous():
+        raise ValueError("x [n, width] is contiguous and w [E, width] contiguous fp32")
+    n = x.shape[0]
+    ids = torch.empty((n, top), dtype=torch.int32, device=x.device)
+    weights = torch.empty((n, top), dtype=torch.float32, device=x.device)
+    rc = _lib_().b200_router_sigmoid_topk(ids.data_ptr(), weights.data_ptr(), x.data_ptr(), w.data_ptr(), n, E, x.shape[1], int(top),
+                                          DTYPE_ID[x.dtype], _stream())
+    _lib.check_mixers(rc, "b200_router_sigmoid_topk")
+    return ids, weights
 
 
 # ---- recurrences decayed by one number per token and head, dynamic tanh norms (csrc/b200_recurrent_ops.cu) ------------
