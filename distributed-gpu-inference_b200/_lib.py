@@ -242,6 +242,8 @@ MIXER_SIGNATURES = {
                 c_int, c_int, c_void_p]),
     "b200_router_logits_ext": (
         c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
+    "b200_router_sigmoid_topk": (
+        c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_void_p]),
     "b200_group_topk": (
         c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int, c_int, c_float, c_float,
                 c_int, c_int, c_int, c_int, c_int, c_void_p]),

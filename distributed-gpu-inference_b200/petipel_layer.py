@@ -238,7 +238,7 @@ class SigmoidTopKMoE(nn.Module):
 
     def forward(self, h: torch.Tensor) -> torch.Tensor:
         n, top = h.shape[0], self.top
-        ids, w = mixer_ops.sigmoid_topk(mixer_ops.router_logits(h, self.w_router), top)
+        ids, w = mixer_ops.router_sigmoid_topk(h, self.w_router, top)
         order, where, offsets = mixer_ops.expert_order(ids, self.E)
         xs = mixer_ops.scaled_gather(h, w.reshape(-1), order, top)
         if self.grouped and n * top <= self.GROUPED_MAX_ROWS:

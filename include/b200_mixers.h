@@ -381,6 +381,10 @@ int b200_latent_rotary_append_ext(const void* q_rot, int64_t q_tok_stride, int64
 int b200_router_logits_ext(float* logits, const void* x, const float* w, const float* bias, int64_t n_tok, int E, int width,
                            int dtype, void* stream);
 
+/* b200_router_logits_ext and b200_sigmoid_topk in one launch, for up to eight experts (the logits stay in the kernel). */
+int b200_router_sigmoid_topk(int32_t* ids, float* weights, const void* x, const float* w, int64_t n_tok, int E, int width, int top, int dtype,
+                             void* stream);
+
 /* Routing over E outputs (the first E of every logits row; rows are logit_stride apart): scores s = softmax over the E logits
  * or, with sigmoid_scores, the logits' sigmoids; choice scores c = s + correction (NULL: c = s); a group's score is its largest
  * c or, with group_best = 2, the sum of its two largest; groups, keep and top as in b200_softmax_group_topk.  weights =
