@@ -103,6 +103,43 @@ __device__ __forceinline__ float row_logistic(float z) {
   return fmaf(fmaf(-q, lost, fmaf(-q, d, n)), r, q);
 }
 
+// The same of two numbers, the same bits: what is no exponential or reciprocal takes both at once.
+__device__ __forceinline__ float2 row_logistic2(float x, float y) {
+  using Pair = unsigned long long;
+  auto pair = [](float a, float b) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+  };
+  auto mul = [](Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+  };
+  auto add = [](Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+  };
+  auto fma = [](Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+  };
+  const float tx = expf(-fabsf(x)), ty = expf(-fabsf(y));
+  const Pair t = pair(tx, ty), d = add(pair(1.0f, 1.0f), t), n = pair(x < 0.f ? tx : 1.0f, y < 0.f ? ty : 1.0f);
+  float dx, dy, rx, ry;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(dx), "=f"(dy) : "l"(d));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rx) : "f"(dx));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ry) : "f"(dy));
+  const Pair r = pair(rx, ry), q = mul(n, r), minus_q = mul(n, pair(-rx, -ry));
+  const Pair lost = fma(add(d, pair(-1.0f, -1.0f)), pair(-1.0f, -1.0f), t);      // t - (d - 1): the product is exact
+  const Pair s = fma(fma(minus_q, lost, fma(minus_q, d, n)), r, q);
+  float2 out;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(out.x), "=f"(out.y) : "l"(s));
+  return out;
+}
+
 constexpr int kNumSMs = 148;  // B200
 constexpr int kMaxSmem = 227 * 1024;   // a CTA's shared memory: the limit to set where launches of one kernel differ in size (another
                                        // thread's smaller one between setting it and the launch would make that fail)
