@@ -19,9 +19,10 @@
 // What bounds it: the softmax's chain from S to P, 2000 to 2400 clocks per tile of 64 keys x 256 rows (bias and maximum 850, exponentials 950 beside the
 // other half's; the tensor cores need 1280, the exponentials alone 1024), and 9000 clocks of a CTA's beginning and end (of 22000: a row of the output
 // written by one thread took 5000, queries in 16-byte pieces 5000, code of modes that a launch does not use two to eight thousand in instruction
-// misses).  Rescaling by the softmax itself: 2900 clocks per tile.
+// misses).  Rescaling by the softmax itself: 2900 clocks per tile.  Issue slots are taken 45 % of the time: what is no maximum, exponential or load goes two at a time
+// (without: a tenth more instructions, 223 us against 217 in the mixer).
 // Measured on B200 (bf16, us, before these / now): 8 x 2048 tokens, 16 heads over 4 kv heads of 128, plain 209 / 198, window of 512 138 / 123, with distance
-// biases, query temperature and gate 277 / 205, soft cap 319 / 242; 5 x 1024 with a cap under a window of 512 51 / 31; latent 320 / 256, 4 portions of up to
+// biases, query temperature and gate 277 / 201, soft cap 319 / 242; 5 x 1024 with a cap under a window of 512 51 / 31; latent 320 / 256, 4 portions of up to
 // 1500 tokens of 16 heads behind 700, window 512: 91 / 68; 319 shapes of 4 .. 16 heads, 1.29 times on average, 64 x 96 tokens of 16 heads with keys of
 // their own 42 / 45.
 //
@@ -157,39 +158,11 @@ __device__ __forceinline__ void tm_st16(uint32_t addr, const uint32_t (&u)[16]) 
       : "memory");
 }
 
-// a warp's 32 rows of N columns times the lanes' factors, W columns at a time
-template <int N, int W>
-__device__ __forceinline__ void scale_rows(uint32_t addr, float k) {
-#pragma unroll 1
-  for (int c = 0; c < N; c += W) {
-    float o[W];
-    if constexpr (W == 16) tm_ld16(o, addr + c);
-    else tm_ld32(o, addr + c);
-    tc_wait_ld();
-#pragma unroll
-    for (int x = 0; x < W; x += 16) {
-      uint32_t w[16];
-#pragma unroll
-      for (int u = 0; u < 16; ++u) w[u] = __float_as_uint(o[x + u] * k);
-      tm_st16(addr + c + x, w);
-    }
-  }
-}
-
-__device__ __forceinline__ float exp2_fast(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 using f32x2 = unsigned long long;
 __device__ __forceinline__ f32x2 both(float x) {
   f32x2 r;
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
   return r;
-}
-// (a, b) <- (a, b) * k + m
-__device__ __forceinline__ void scale_shift(float& a, float& b, f32x2 k, f32x2 m) {
-  asm("{\n.reg .b64 t;\nmov.b64 t, {%0, %1};\nfma.rn.f32x2 t, t, %2, %3;\nmov.b64 {%0, %1}, t;\n}\n" : "+f"(a), "+f"(b) : "l"(k), "l"(m));
 }
 __device__ __forceinline__ f32x2 pair(float a, float b) {
   f32x2 r;
@@ -211,6 +184,39 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   f32x2 r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
+}
+// a warp's 32 rows of N columns times the lanes' factors, W columns at a time
+template <int N, int W>
+__device__ __forceinline__ void scale_rows(uint32_t addr, float k) {
+  const f32x2 kk = both(k);
+#pragma unroll 1
+  for (int c = 0; c < N; c += W) {
+    float o[W];
+    if constexpr (W == 16) tm_ld16(o, addr + c);
+    else tm_ld32(o, addr + c);
+    tc_wait_ld();
+#pragma unroll
+    for (int x = 0; x < W; x += 16) {
+      uint32_t w[16];
+#pragma unroll
+      for (int u = 0; u < 16; u += 2) {
+        float lo, hi;
+        apart(lo, hi, mul2(pair(o[x + u], o[x + u + 1]), kk));
+        w[u] = __float_as_uint(lo), w[u + 1] = __float_as_uint(hi);
+      }
+      tm_st16(addr + c + x, w);
+    }
+  }
+}
+
+__device__ __forceinline__ float exp2_fast(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// (a, b) <- (a, b) * k + m
+__device__ __forceinline__ void scale_shift(float& a, float& b, f32x2 k, f32x2 m) {
+  asm("{\n.reg .b64 t;\nmov.b64 t, {%0, %1};\nfma.rn.f32x2 t, t, %2, %3;\nmov.b64 {%0, %1}, t;\n}\n" : "+f"(a), "+f"(b) : "l"(k), "l"(m));
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
@@ -599,13 +605,19 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
       if constexpr (BIAS) {
         const float* b = lut_s + ((i % P::kLuts) * rep + (live ? hh : 0)) * pitch + (live ? t_row : 0) + kKeys - 1;
 #pragma unroll
-        for (int c = 0; c < kKeys; ++c) s[c >> 5][c & 31] = fmaf(s[c >> 5][c & 31], mult, b[-c]);
+        for (int c = 0; c < kKeys; c += 2) {
+          float& x = s[c >> 5][c & 31];
+          float& y = s[c >> 5][(c & 31) + 1];
+          apart(x, y, fma2(pair(x, y), both(mult), pair(b[-c], b[-c - 1])));
+        }
       } else if (!plain) {
         [[maybe_unused]] float far = 0.f;
 #pragma unroll
-        for (int c = 0; c < kKeys; ++c) {
-          s[c >> 5][c & 31] *= mult;
-          if constexpr (CAP) far = fmaxf(far, fabsf(s[c >> 5][c & 31]));
+        for (int c = 0; c < kKeys; c += 2) {
+          float& x = s[c >> 5][c & 31];
+          float& y = s[c >> 5][(c & 31) + 1];
+          apart(x, y, mul2(pair(x, y), both(mult)));
+          if constexpr (CAP) far = max3(far, fabsf(x), fabsf(y));
         }
         if constexpr (!CAP) {
         } else if (!__any_sync(0xffffffffu, far > 0.5f * A.softcap)) {
@@ -908,7 +920,7 @@ bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, in
 // over 4, 8 x 2048: 206 / 242 us against 241 / 285; 6 x 300 .. 640: 24 / 27 against 28 / 32; but 4 over 1, 8 x 700: 27 against 21 of plain
 // scores), 128 where they do not share (16 over 16, 8 x 700: 60 / 67 against 64 / 70; 64 x 96: 50 / 53 against 73 / 73).  Plain scores keep 128 rows.
 // Pages that come row by row keep 256 rows from one round of CTAs on with biases or a cap, from three without (8 x 1000 tokens of 16 heads, pages
-// of 24: 82 us against 94).
+// of 24: 82 us against 94 when the line was drawn; 79 now).
 int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy, bool boxes) {
   const int64_t ctas = static_cast<int64_t>(n_tokens) * rep / (2 * kTileRows) * G;      // of 256 rows
   const bool wide = boxes ? heavy && rep > 1 && 4 * ctas > 3 * kNumSMs : ctas >= (heavy ? 1 : 3) * kNumSMs;
