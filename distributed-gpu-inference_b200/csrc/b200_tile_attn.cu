@@ -865,6 +865,14 @@ int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stre
   smem = std::max<size_t>(smem, P::kCtas == 2 ? 80 * 1024 : 120 * 1024);   // no more CTAs per SM than tensor memory has room for
   if (smem > kMaxSmem) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
   auto kern = tile_attn_kernel<T, DK, DV, ALIAS, MODE, HALVES, CTAS>;
+  if constexpr (P::kSplitRegs) {
+    // the softmax waits for registers that the launch has to have: a build with fewer would wait for good
+    static const int regs = [](auto k) {
+      cudaFuncAttributes f{};
+      return cudaFuncGetAttributes(&f, k) == cudaSuccess ? f.numRegs : 0;
+    }(kern);
+    if (regs * P::kNT < (P::kSoft * 128 + (kLoad + P::kScale) * 64 + 32 * regs)) return fail(B200_EINVAL, "b200_tile_attn: built with %d registers per thread", regs);
+  }
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   TileAttn B = A;
   CUtensorMap k_map{}, v_map{}, q_map{};
