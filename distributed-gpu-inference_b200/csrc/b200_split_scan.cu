@@ -936,7 +936,7 @@ split_chain_kernel(const SplitArgs A, const bool later) {
       step(ops, 3, s2);
       add(o, s);
     } else {
-      // channels in two halves: the state's parts live for their products only, so that their registers hold two halves of them and three CTAs fit an SM
+      // channels in two halves: a half's parts of the state live for its products only, so that three CTAs fit an SM
       Tiles z0, z1, pv, ps;
       mma_v(pv, ps, frag1(ops.p));
 #pragma unroll

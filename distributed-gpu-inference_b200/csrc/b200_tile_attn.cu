@@ -22,7 +22,7 @@
 // misses).  Rescaling by the softmax itself: 2900 clocks per tile.  Issue slots are taken 45 % of the time: what is no maximum, exponential or load goes two at a time
 // (without: a tenth more instructions, 223 us against 217 in the mixer).
 // Measured on B200 (bf16, us, before these / now): 8 x 2048 tokens, 16 heads over 4 kv heads of 128, plain 209 / 198, window of 512 138 / 123, with distance
-// biases, query temperature and gate 277 / 201, soft cap 319 / 242; 5 x 1024 with a cap under a window of 512 51 / 31; latent 320 / 256, 4 portions of up to
+// biases, query temperature and gate 277 / 205 (before biases went two at a time), soft cap 319 / 242; 5 x 1024 with a cap under a window of 512 51 / 31; latent 320 / 256, 4 portions of up to
 // 1500 tokens of 16 heads behind 700, window 512: 91 / 68; 319 shapes of 4 .. 16 heads, 1.29 times on average, 64 x 96 tokens of 16 heads with keys of
 // their own 42 / 45.
 //
