@@ -743,12 +743,12 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
       auto scaled = [&](float (&o)[32], int c) {
         tm_ld32(o, tm_row + P::kO + c);
         tc_wait_ld();
-        if (gate && A.gate_dim && live) {
+#pragma unroll
+        for (int x = 0; x < 32; ++x) o[x] *= f;
+        if (gate && A.gate_dim && live) {      // after the row's factor: a gated row is the ungated one times its gates, to the bit
 #pragma unroll
           for (int x = 0; x < 32; ++x) o[x] *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row * A.gate_dim + c + x])));
         }
-#pragma unroll
-        for (int x = 0; x < 32; ++x) o[x] *= f;
       };
       const int64_t at0 = n * A.out_tok_stride + h_row * A.out_head_stride;
       auto rows_out = [&](auto* tag) {

@@ -41,3 +41,18 @@ def test_forms(layout, many, mode, out):
     again = torch.empty_like(o)
     mixer_ops.tile_attention(again, q, k_pool, v_pool, st.block_tables, tiles, st.tok_pos, scale, rows=128, gate=gate, bias_lut=bias, **kw)
     assert torch.equal(again, o)
+
+
+@pytest.mark.parametrize("layout,rows", [("4x128", 128), ("4x128", 256), ("4x64", 128), ("6x128", 128)])
+def test_gates_per_channel_come_last(layout, rows):
+    """A row with gates per channel is the row without them times the gates: the same products in the same order, fp32, to the bit."""
+    H, G, dk, dv, _div = LAYOUTS[layout]
+    cap = rows // (H // G)
+    q, k_pool, v_pool, st, rnd = _case(LAYOUTS[layout], [(cap, 0), (cap + cap // 3, 100)], 16, torch.bfloat16)
+    n = q.shape[0]
+    gate = rnd(n, H * dv).to(torch.bfloat16)
+    plain, gated = (torch.empty(n, H, dv, dtype=torch.float32, device="cuda") for _ in range(2))
+    args = q, k_pool, v_pool, st.block_tables, st.prompt_tiles(1, cap)[0], st.tok_pos, dk ** -0.5
+    mixer_ops.tile_attention(plain, *args, rows=rows)
+    mixer_ops.tile_attention(gated, *args, rows=rows, gate=gate)
+    assert torch.equal(gated, plain * (1.0 / (1.0 + torch.exp(-gate.float()))).view(n, H, dv))
