@@ -23,8 +23,10 @@
 // (without: a tenth more instructions, 223 us against 217 in the mixer).
 // Measured on B200 (bf16, us, before these / now): 8 x 2048 tokens, 16 heads over 4 kv heads of 128, plain 209 / 198, window of 512 138 / 123, with distance
 // biases, query temperature and gate 277 / 205 (before biases went two at a time), soft cap 319 / 242; 5 x 1024 with a cap under a window of 512 51 / 31; latent 320 / 256, 4 portions of up to
-// 1500 tokens of 16 heads behind 700, window 512: 91 / 68; 319 shapes of 4 .. 16 heads, 1.29 times on average, 64 x 96 tokens of 16 heads with keys of
-// their own 42 / 45.
+// 1500 tokens of 16 heads behind 700, window 512: 91 / 68; 319 shapes of 4 .. 16 heads, 1.29 times on average.
+// Portions smaller than a tile have walks of one or two key tiles, which wait for instructions: 16 heads with keys of their own, plain, 64 x 96 tokens
+// 41 / 41, 128 x 40 54 / 55, 256 x 20 102 / 102 (44, 61 and 116 with a loop for each way pages come and a loop for each form of the output in
+// the kernel, a division for a CTA's place, barriers of the rescaling warps where there are none, and rows of no token written to shared memory).
 //
 // Weights are taken relative to the row's running maximum, so that the largest is 1 and loses nothing when P is rounded to the storage
 // type; O is scaled down whenever a row of the warp has a new maximum.  (Scaling only once the maximum has grown by 2^8 leaves the largest weight anywhere in 1 .. 256, rounded
@@ -234,6 +236,75 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
+// Columns c .. c + 31 of a lane's row to its warp's rows in shared memory, as type O, 16-byte pieces swizzled by the row's number in its group
+// of eight
+template <typename T, int DV, typename O>
+__device__ __forceinline__ void stage_rows(const float (&o)[32], uint32_t rows, int c) {
+  constexpr int kPieces = DV * sizeof(O) / 16, kPer = 16 / sizeof(O);
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int x = 0; x < 32; x += kPer) {
+    uint32_t w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) w[u] = sizeof(O) == 4 ? __float_as_uint(o[x + u]) : pack2<T>(o[(x + 2 * u) % 32], o[(x + 2 * u + 1) % 32]);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(rows + lane * (kPieces * 16) + ((((c + x) / kPer) ^ (lane & 7)) << 4)), "r"(w[0]), "r"(w[1]),
+                 "r"(w[2]), "r"(w[3]) : "memory");
+  }
+}
+// ... and from there to memory, so that lanes side by side write pieces side by side; at0: where a lane's row begins
+template <typename O, int DV>
+__device__ __forceinline__ void staged_out(uint32_t rows, bool live, O* out, int64_t at0) {
+  constexpr int kPieces = DV * sizeof(O) / 16, kPer = 16 / sizeof(O), kRowsAtOnce = 32 / kPieces > 0 ? 32 / kPieces : 1;
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  const unsigned seen = __ballot_sync(0xffffffffu, live);
+#pragma unroll 4
+  for (int u = 0; u < kPieces; ++u) {
+    const int r = kPieces >= 32 ? u * 32 / kPieces : u * kRowsAtOnce + lane / kPieces, piece = kPieces >= 32 ? (u * 32 + lane) % kPieces : lane % kPieces;
+    const int64_t to = __shfl_sync(0xffffffffu, at0, r);
+    if (seen >> r & 1) {
+      uint4 v;
+      asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(rows + r * (kPieces * 16) + ((piece ^ (r & 7)) << 4)) : "memory");
+      *reinterpret_cast<uint4*>(out + to + piece * kPer) = v;
+    }
+  }
+}
+// A warp's rows of O out of tensor memory in the forms that most launches do not have: gates per channel, fp32, rows off 16 bytes (not staged).  A
+// function of its own keeps their code out of the kernel, whose short walks wait for instructions.
+template <typename T, int DV>
+__device__ __noinline__ void rows_out_other(uint32_t tm_o, uint32_t rows, float f, const T* gates, bool live, bool staged, bool out_f32, void* out, int64_t at0) {
+#pragma unroll 1
+  for (int c = 0; c < DV; c += 32) {
+    float o[32];
+    __syncwarp();
+    tm_ld32(o, tm_o + c);
+    tc_wait_ld();
+#pragma unroll
+    for (int x = 0; x < 32; ++x) o[x] *= f;
+    if (gates && live) {      // after the row's factor: a gated row is the ungated one times its gates, to the bit
+#pragma unroll
+      for (int x = 0; x < 32; ++x) o[x] *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gates[c + x])));
+    }
+    if (out_f32) {
+      if (staged) {
+        stage_rows<T, DV, float>(o, rows, c);
+      } else if (live) {
+        float* dst = static_cast<float*>(out) + at0 + c;
+#pragma unroll
+        for (int x = 0; x < 32; x += 2) *reinterpret_cast<float2*>(dst + x) = make_float2(o[x], o[x + 1]);
+      }
+    } else if (staged) {
+      stage_rows<T, DV, T>(o, rows, c);
+    } else if (live) {
+      T* dst = static_cast<T*>(out) + at0 + c;
+#pragma unroll
+      for (int x = 0; x < 32; x += 2) *reinterpret_cast<uint32_t*>(dst + x) = pack2<T>(o[x], o[x + 1]);
+    }
+  }
+  if (staged && out_f32) staged_out<float, DV>(rows, live, static_cast<float*>(out), at0);
+  else if (staged) staged_out<T, DV>(rows, live, static_cast<T*>(out), at0);
+}
+
 // shared memory of one CTA, from a 1024-byte boundary
 template <int DK, int DV, bool ALIAS, int HALVES, int CTAS>
 struct Plan {
@@ -284,8 +355,7 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   // all kv heads of a tile, then the next tile's: with the tiles in order of their keys, the longest first, short ones fill the last round
-  const int place = blockIdx.x + gridDim.x * blockIdx.y, tile = place / A.G;
-  const int g = place - tile * A.G, rep = A.H / A.G, bs = A.block_size;
+  const int tile = A.tile0 + blockIdx.y, g = blockIdx.x, rep = A.H / A.G, bs = A.block_size;
   const int tok0 = A.tiles[3 * tile], trow = A.tiles[3 * tile + 2];
   const int cnt = min(A.tiles[3 * tile + 1], kSoft / rep), n_rows = cnt * rep;
   const int halves = P::kHalves == 2 && n_rows > kRows ? 2 : 1;       // in use
@@ -322,8 +392,10 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
     for (int b = 0; b < 4; ++b) {
       init(bar_s + 8 * b, 1);
       init(bar_p + 8 * b, kRows);
-      init(bar_c + 8 * b, kRows);
-      init(bar_r + 8 * b, kRows);
+      if (P::kScale) {
+        init(bar_c + 8 * b, kRows);
+        init(bar_r + 8 * b, kRows);
+      }
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     *dead = 0;
@@ -434,42 +506,27 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
       else bar_wait(bar_ke + 8 * (i % NB), (i / NB - 1) & 1, dead);
     };
     // Pages by the copy engine arrive at the barrier by themselves, biases by their own arrival: nobody waits for a tile before the next
-    // is asked for.
-    const int by_boxes = boxes ? n_it : 0;
-    for (int i = 0; i < by_boxes; ++i) {
+    // is asked for.  Row by row a tile is handed over while the next one is under way, until the buffers are full.  One loop for both: the
+    // copies' code is there once.
+    for (int i = 0; i < n_it; ++i) {
       const int next = look_up(i + 1);
       if (i >= NB) free_again(i);
       copy(i, page);
       page = next;
-      if (!whole(i)) {
-        cp_wait<0>();
-        arrived(i);
-      } else if (BIAS && !values) {
+      if (!boxes && i < NB) {
+        if (i > 0) {
+          cp_wait<1>();
+          arrived(i - 1);
+        }
+        if (i + 1 < min(n_it, NB)) continue;
+      }
+      if (BIAS && !values && whole(i)) {
         fence_smem_to_mma();
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar_k + 8 * (i % NB)) : "memory");
       } else {
+        if (!whole(i)) cp_wait<0>();
         arrived(i);
       }
-    }
-    const int ahead = boxes ? 0 : min(n_it, NB);
-    for (int i = 0; i < ahead; ++i) {      // a tile is handed over while the next one is under way
-      const int next = look_up(i + 1);
-      copy(i, page);
-      page = next;
-      if (i > 0) {
-        cp_wait<1>();
-        arrived(i - 1);
-      }
-    }
-    cp_wait<0>();
-    if (ahead > 0) arrived(ahead - 1);
-    for (int i = max(ahead, by_boxes); i < n_it; ++i) {
-      const int next = look_up(i + 1);
-      free_again(i);
-      copy(i, page);
-      page = next;
-      cp_wait<0>();
-      arrived(i);
     }
   } else if (warp == (kSoft + kLoad + P::kScale) / 32) {
     // ---- products -----------------------------------------------------------------------------------------------------------------
@@ -708,7 +765,7 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
     const float m_nat = m_ref * kLn2;
     const int64_t n = tok0 + t_row;
     if (gridDim.z > 1) {
-      const int64_t wr = (static_cast<int64_t>(blockIdx.z) * gridDim.x + tile) * (kSoft / rep) + t_row;
+      const int64_t wr = (static_cast<int64_t>(blockIdx.z) * A.n_tiles + tile) * (kSoft / rep) + t_row;
       float* dst = A.ws + (wr * A.H + h_row) * (DV + 2);
       if (live) {
         dst[0] = ok ? m_nat : NAN;
@@ -728,85 +785,35 @@ tile_attn_kernel(const TileAttn A, const __grid_constant__ CUtensorMap k_map, co
             *reinterpret_cast<float2*>(dst + 2 + c + x) = n_it > 0 ? make_float2(o[x], o[x + 1]) : make_float2(0.f, 0.f);
         }
       }
-    } else if (hf < halves) {
+    } else if (__any_sync(0xffffffffu, p >= 0)) {      // (p >= 0: live; the rows' number need not be kept)
       float f = 1.0f / l;
-      if (A.sink && live) {
+      if (A.sink && p >= 0) {
         const float sk = A.sink[h_row], M = fmaxf(m_nat, sk);
         const float e = expf(m_nat - M);
         f = e / (l * e + expf(sk - M));
       }
       if (!ok) f = NAN;
       const T* gate = static_cast<const T*>(A.gate);
-      if (gate && live && !A.gate_dim) f *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row])));
-      // Rows go through shared memory (all products are done, queries and pages have been read), each warp its own, so that lanes side by side
-      // write pieces side by side; 16-byte pieces are swizzled by the row's number in its group of eight
-      auto scaled = [&](float (&o)[32], int c) {
-        tm_ld32(o, tm_row + P::kO + c);
-        tc_wait_ld();
-#pragma unroll
-        for (int x = 0; x < 32; ++x) o[x] *= f;
-        if (gate && A.gate_dim && live) {      // after the row's factor: a gated row is the ungated one times its gates, to the bit
-#pragma unroll
-          for (int x = 0; x < 32; ++x) o[x] *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row * A.gate_dim + c + x])));
-        }
-      };
+      if (gate && p >= 0 && !A.gate_dim) f *= 1.0f / (1.0f + expf(-Cvt<T>::to_f32(gate[n * A.gate_stride + h_row])));
+      const bool staged = A.out_vec && __all_sync(0xffffffffu, ok);     // after a failure copies may still be under way
       const int64_t at0 = n * A.out_tok_stride + h_row * A.out_head_stride;
-      auto rows_out = [&](auto* tag) {
-        using O = std::remove_pointer_t<decltype(tag)>;
-        constexpr int kPieces = DV * sizeof(O) / 16, kPer = 16 / sizeof(O);
-        const uint32_t own = sm0 + P::kQ + (hf * kRows + 32 * (warp & 3)) * (DV * static_cast<int>(sizeof(O)));
-        const int lane = tid & 31;
-#pragma unroll 1
-        for (int c = 0; c < DV; c += 32) {
-          float o[32];
-          __syncwarp();
-          scaled(o, c);
-#pragma unroll
-          for (int x = 0; x < 32; x += kPer) {
-            uint32_t w[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) w[u] = sizeof(O) == 4 ? __float_as_uint(o[x + u]) : pack2<T>(o[(x + 2 * u) % 32], o[(x + 2 * u + 1) % 32]);
-            const int piece = (c + x) / kPer;
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(own + lane * (kPieces * 16) + ((piece ^ (lane & 7)) << 4)), "r"(w[0]), "r"(w[1]),
-                         "r"(w[2]), "r"(w[3]) : "memory");
-          }
-        }
-        __syncwarp();
-        const unsigned seen = __ballot_sync(0xffffffffu, live);
-        constexpr int kRowsAtOnce = 32 / kPieces > 0 ? 32 / kPieces : 1;
-#pragma unroll 4
-        for (int u = 0; u < kPieces; ++u) {
-          const int r = kPieces >= 32 ? u * 32 / kPieces : u * kRowsAtOnce + lane / kPieces, piece = kPieces >= 32 ? (u * 32 + lane) % kPieces : lane % kPieces;
-          const int64_t to = __shfl_sync(0xffffffffu, at0, r);
-          if (seen >> r & 1) {
-            uint4 v;
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(own + r * (kPieces * 16) + ((piece ^ (r & 7)) << 4)) : "memory");
-            *reinterpret_cast<uint4*>(static_cast<O*>(A.out) + to + piece * kPer) = v;
-          }
-        }
-      };
-      const bool whole_rows = A.out_vec && __all_sync(0xffffffffu, ok);     // after a failure copies may still be under way
-      if (whole_rows && A.out_f32) {
-        rows_out(static_cast<float*>(nullptr));
-      } else if (whole_rows) {
-        rows_out(static_cast<T*>(nullptr));
+      // the warp's own rows (all products are done, queries and pages have been read)
+      const uint32_t own = sm0 + P::kQ + (hf * kRows + 32 * (warp & 3)) * (DV * 4);
+      if (!staged || A.out_f32 || (gate && A.gate_dim)) {
+        const T* gates = gate && A.gate_dim ? gate + n * A.gate_stride + h_row * A.gate_dim : nullptr;
+        rows_out_other<T, DV>(tm_row + P::kO, own, f, gates, p >= 0, staged, A.out_f32 != 0, A.out, at0);
       } else {
 #pragma unroll 1
         for (int c = 0; c < DV; c += 32) {
           float o[32];
           __syncwarp();
-          scaled(o, c);
-          if (!live) continue;       // reconverges at the loop's head
-          if (A.out_f32) {
-            float* dst = static_cast<float*>(A.out) + at0 + c;
+          tm_ld32(o, tm_row + P::kO + c);
+          tc_wait_ld();
 #pragma unroll
-            for (int x = 0; x < 32; x += 2) *reinterpret_cast<float2*>(dst + x) = make_float2(o[x], o[x + 1]);
-          } else {
-            T* dst = static_cast<T*>(A.out) + at0 + c;
-#pragma unroll
-            for (int x = 0; x < 32; x += 2) *reinterpret_cast<uint32_t*>(dst + x) = pack2<T>(o[x], o[x + 1]);
-          }
+          for (int x = 0; x < 32; ++x) o[x] *= f;
+          stage_rows<T, DV, T>(o, own, c);
         }
+        staged_out<T, DV>(own, p >= 0, static_cast<T*>(A.out), at0);
       }
     }
     __syncwarp();
@@ -880,8 +887,13 @@ int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stre
   B.boxes = A.block_size % 8 == 0 && kKeys % A.block_size == 0 && page_map<T>(&k_map, A.k_pool, DK, A.block_size) &&
             (ALIAS || (A.v_row % 8 == 0 && page_map<T>(&v_map, A.v_pool, A.v_row, A.block_size)));
   B.q_boxes = query_map<T>(&q_map, A, DK);
-  kern<<<dim3(n_tiles, A.G, n_splits), P::kNT, smem, stream>>>(B, k_map, v_map, q_map);
-  return check_launch("b200_tile_attn");
+  B.n_tiles = n_tiles;
+  constexpr int kMost = 65535;      // of a grid's second dimension
+  for (B.tile0 = 0; B.tile0 < n_tiles; B.tile0 += kMost) {
+    kern<<<dim3(A.G, std::min(kMost, n_tiles - B.tile0), n_splits), P::kNT, smem, stream>>>(B, k_map, v_map, q_map);
+    if (int rc = check_launch("b200_tile_attn")) return rc;
+  }
+  return 0;
 }
 
 template <int DK, int DV, bool ALIAS>

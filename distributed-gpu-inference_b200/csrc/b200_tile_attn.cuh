@@ -25,6 +25,7 @@ struct TileAttn {
   float scale, softcap, temp_coef;
   int temp_every;
   int boxes, q_boxes;                        // set by the launcher: pages, and the queries of full tiles, come by the copy engine
+  int tile0, n_tiles;                        // and the first tile of a launch, and how many the call has
 };
 
 bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, int dtype);

@@ -56,3 +56,21 @@ def test_gates_per_channel_come_last(layout, rows):
     mixer_ops.tile_attention(plain, *args, rows=rows)
     mixer_ops.tile_attention(gated, *args, rows=rows, gate=gate)
     assert torch.equal(gated, plain * (1.0 / (1.0 + torch.exp(-gate.float()))).view(n, H, dv))
+
+
+@pytest.mark.parametrize("n", [65535, 65536, 70001])
+def test_more_tiles_than_a_grid_has_rows(n):
+    """One token per tile: a grid's second dimension ends at 65535, the tiles behind it are another launch's."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    dk, page = 64, 16
+    q = torch.randn(n, 1, dk, generator=gen, device="cuda").to(torch.bfloat16)
+    pools = torch.randn(2, 3, 1, page, dk, generator=gen, device="cuda").to(torch.bfloat16)
+    pos = torch.randint(0, 3 * page, (n,), generator=gen, device="cuda", dtype=torch.int32)
+    tables = torch.tensor([[2, 0, 1]], dtype=torch.int32, device="cuda")
+    tiles = torch.stack([torch.arange(n, device="cuda"), torch.ones(n, device="cuda", dtype=torch.int64), torch.zeros(n, device="cuda", dtype=torch.int64)], 1).to(torch.int32)
+    out = torch.empty_like(q)
+    mixer_ops.tile_attention(out, q, pools[0], pools[1], tables, tiles.contiguous(), pos, dk ** -0.5, rows=128)
+    K, V = (p[tables[0].long(), 0].reshape(3 * page, dk).to(F64) for p in pools)
+    s = (q[:, 0].to(F64) @ K.T * dk ** -0.5).masked_fill(torch.arange(3 * page, device="cuda")[None] > pos[:, None], float("-inf"))
+    want = torch.softmax(s, 1) @ V
+    assert ((out[:, 0].to(F64) - want).norm(dim=1) / want.norm(dim=1)).max() <= 12 * 2.0 ** -8      # as the rows above
