@@ -948,12 +948,19 @@ int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy, bool boxes)
 }
 
 // Keys are divided while the chip has room for more CTAs, a share being worth its part of the merge: three tiles of 64 keys where
-// few rows are merged, eight otherwise.
+// few rows are merged, eight otherwise.  Room is one CTA per SM, whose form is ahead (4 heads with keys of their own, 8 x 64 tokens behind 1000: 4 shares
+// 20.8 us, 5, two per SM, 23.5; 4 over 1, 1000 behind 6000: 4 shares 47.6, 9 51.9; 16 over 4, 1 x 1024: undivided 51, in two 54), unless that
+// leaves a CTA more than 48 key tiles: then two CTAs per SM walk faster together (8 over 2 of 64, 1000 behind 6000, 64 CTAs: 2 shares of 55 tiles
+// 71 us, 4 59; at 36 tiles, 16 heads, 512 behind 4000, 2 shares 55, 4 64).
 int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int rows) {
-  const int64_t ctas = static_cast<int64_t>(n_tiles) * G, room = (rows == kTileRows && dk <= 128 ? 2 : 1) * kNumSMs;
-  if (ctas <= 0 || ctas * 2 > room) return 1;
-  const int share = ctas * rows <= 4096 ? 3 : 8;
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({16, room / ctas, key_tiles / share})));
+  const int64_t ctas = static_cast<int64_t>(n_tiles) * G;
+  auto divide = [&](int64_t room) {
+    if (ctas <= 0 || ctas * 2 > room) return 1;
+    const int share = ctas * rows <= 4096 ? 3 : 8;
+    return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({16, room / ctas, key_tiles / share})));
+  };
+  const int one_per_sm = divide(kNumSMs);
+  return rows == kTileRows && dk <= 128 && key_tiles > 48 * one_per_sm ? divide(2 * kNumSMs) : one_per_sm;
 }
 
 int tile_attn_launch(const TileAttn& A, int dk, int dv, bool alias, int rows, int n_tiles, int n_splits, int dtype, cudaStream_t stream) {

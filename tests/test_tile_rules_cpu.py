@@ -1,0 +1,17 @@
+"""How the tile attention divides a walk over the keys: host arithmetic only."""
+import pytest
+
+import dgi_b200  # noqa: F401
+from dgi_b200 import _lib
+
+
+@pytest.mark.parametrize("n_tiles,key_tiles,G,dk,rows,splits", [
+    # one CTA per SM, shares of 3 key tiles for few rows, of 8 otherwise
+    (1, 17, 4, 128, 128, 5), (8, 17, 4, 128, 128, 4), (8, 16, 4, 128, 128, 4), (32, 16, 4, 128, 128, 1), (37, 40, 2, 64, 128, 2), (38, 40, 2, 64, 128, 1),
+    # two per SM where one leaves more than 48 key tiles to a CTA
+    (16, 96, 4, 128, 128, 2), (16, 97, 4, 128, 128, 4), (32, 48, 4, 128, 128, 1), (32, 49, 4, 128, 128, 2), (38, 300, 4, 128, 128, 1),
+    # forms that have an SM to themselves
+    (16, 200, 4, 128, 256, 2), (32, 200, 4, 128, 256, 1), (63, 110, 1, 256, 128, 2), (74, 110, 1, 256, 128, 2), (75, 110, 1, 256, 128, 1),
+    (0, 10, 4, 128, 128, 1), (1, 1, 1, 64, 128, 1), (1, 1000, 1, 64, 128, 16)])
+def test_shares_of_a_walk(n_tiles, key_tiles, G, dk, rows, splits):
+    assert _lib.load_mixers().b200_tile_attn_splits(n_tiles, key_tiles, G, dk, rows) == splits
