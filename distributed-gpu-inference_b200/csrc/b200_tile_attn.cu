@@ -42,6 +42,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "../../include/b200_mixers.h"
@@ -315,6 +316,8 @@ struct Plan {
   static constexpr int kSoft = kHalves * kRows, kNT = kSoft + kLoad + 32 + kScale;
   // 17 warps: five on a scheduler leave 96 registers each; the softmax takes 32 more from the warps that copy and rescale (8 x 128 + 8 x 64 + 96 = 17 x 96)
   static constexpr bool kSplitRegs = kNT == 17 * 32;
+  // ... which a launch has to have: with fewer the softmax would wait for good
+  static constexpr bool enough(int regs) { return regs * kNT >= kSoft * 128 + (kLoad + kScale) * 64 + 32 * regs; }
   static constexpr int kBufs = kCtas == 2 ? 2 : 3;      // of keys, and of values
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + kHalves * (DK / 64) * kRows * 128;
@@ -863,6 +866,29 @@ bool query_map(CUtensorMap* map, const TileAttn& A, int dk) {
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Registers per thread that a kernel was built with, which every device runs; a query that fails is not kept.
+template <typename T, int DK, int DV, bool ALIAS, int MODE, int HALVES, int CTAS>
+cudaError_t built_registers(int* regs) {
+  static std::atomic<int> known{0};
+  *regs = known.load(std::memory_order_relaxed);
+  if (*regs > 0) return cudaSuccess;
+  cudaFuncAttributes f{};
+  const cudaError_t e = cudaFuncGetAttributes(&f, tile_attn_kernel<T, DK, DV, ALIAS, MODE, HALVES, CTAS>);
+  if (e == cudaSuccess) known.store(*regs = f.numRegs, std::memory_order_relaxed);
+  return e;
+}
+// Whether the kernels of 256 rows were built with the registers that they share out (unknown: yes, their launches ask again)
+template <typename T, int D>
+bool wide_built() {
+  auto fits = [](auto mode) {
+    int regs = 0;
+    if (built_registers<T, D, D, false, decltype(mode)::value, 2, 1>(&regs) == cudaSuccess) return Plan<D, D, false, 2, 1>::enough(regs);
+    cudaGetLastError();
+    return true;
+  };
+  return fits(std::integral_constant<int, kPlain>{}) && fits(std::integral_constant<int, kBiased>{}) && fits(std::integral_constant<int, kCapped>{});
+}
+
 template <typename T, int DK, int DV, bool ALIAS, int MODE, int HALVES, int CTAS>
 int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stream) {
   using P = Plan<DK, DV, ALIAS, HALVES, CTAS>;
@@ -873,12 +899,12 @@ int launch_tiles(const TileAttn& A, int n_tiles, int n_splits, cudaStream_t stre
   if (smem > kMaxSmem) return fail(B200_ESHAPE, "b200_tile_attn: %zu bytes of shared memory", smem);
   auto kern = tile_attn_kernel<T, DK, DV, ALIAS, MODE, HALVES, CTAS>;
   if constexpr (P::kSplitRegs) {
-    // the softmax waits for registers that the launch has to have: a build with fewer would wait for good
-    static const int regs = [](auto k) {
-      cudaFuncAttributes f{};
-      return cudaFuncGetAttributes(&f, k) == cudaSuccess ? f.numRegs : 0;
-    }(kern);
-    if (regs * P::kNT < (P::kSoft * 128 + (kLoad + P::kScale) * 64 + 32 * regs)) return fail(B200_EINVAL, "b200_tile_attn: built with %d registers per thread", regs);
+    int regs = 0;
+    if (const cudaError_t e = built_registers<T, DK, DV, ALIAS, MODE, HALVES, CTAS>(&regs); e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(static_cast<int>(e), "b200_tile_attn: %s", cudaGetErrorString(e));
+    }
+    if (!P::enough(regs)) return fail(B200_EINVAL, "b200_tile_attn: built with %d registers per thread", regs);
   }
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   TileAttn B = A;
@@ -944,7 +970,9 @@ bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, in
 int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy, bool boxes) {
   const int64_t ctas = static_cast<int64_t>(n_tokens) * rep / (2 * kTileRows) * G;      // of 256 rows
   const bool wide = boxes ? heavy && rep > 1 && 4 * ctas > 3 * kNumSMs : ctas >= (heavy ? 1 : 3) * kNumSMs;
-  return wide && dk <= 128 ? 2 * kTileRows : kTileRows;
+  if (!wide || dk > 128) return kTileRows;
+  const bool built = dk <= 64 ? wide_built<__nv_bfloat16, 64>() && wide_built<__half, 64>() : wide_built<__nv_bfloat16, 128>() && wide_built<__half, 128>();
+  return built ? 2 * kTileRows : kTileRows;
 }
 
 // Keys are divided while the chip has room for more CTAs, a share being worth its part of the merge: three tiles of 64 keys where

@@ -1,5 +1,6 @@
 """How the tile attention divides a walk over the keys: host arithmetic only."""
 import pytest
+import torch
 
 import dgi_b200  # noqa: F401
 from dgi_b200 import _lib
@@ -15,3 +16,16 @@ from dgi_b200 import _lib
     (0, 10, 4, 128, 128, 1), (1, 1, 1, 64, 128, 1), (1, 1000, 1, 64, 128, 16)])
 def test_shares_of_a_walk(n_tiles, key_tiles, G, dk, rows, splits):
     assert _lib.load_mixers().b200_tile_attn_splits(n_tiles, key_tiles, G, dk, rows) == splits
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the call must fail before anything is launched")
+@pytest.mark.parametrize("dk", [64, 128])
+def test_a_failed_register_query_is_reported_and_not_kept(dk):
+    """Tiles of 256 rows ask what their kernel was built with: without a device that fails, with the runtime's error and not as a build's fault, and the
+    row rule goes on without an answer."""
+    lib, at = _lib.load_mixers(), 1 << 20        # an aligned address that nothing reads
+    for _ in range(2):
+        rc = lib.b200_tile_attn(at, 8 * dk, dk, at, 8 * dk, dk, None, 0, 0, at, 2 * at, at, 4, at, 200, 256, at, None, None, 0, 0.1, 0.0, 0.0, 1, 0, 0, 0, 8, 2,
+                                dk, dk, dk, 1, 0, 16, 1, None, 2, None)
+        assert rc > 0 and b"registers" not in lib.b200_mixers_last_error()
+    assert lib.b200_tile_attn_rows_ext(4, 4, dk, 20000, 1) == 256
