@@ -258,14 +258,27 @@ def split_scan_segment(rule: int, longest: int, n: int, n_seqs: int, H: int, dv:
     of the work.  Not for the delta rule, whose decay is no diagonal.  B200, bf16, 64 x 128 states, us in one piece / in segments,
     operands included: 4 heads, 1 of 2048 124 / 36, 8 of 2048 160 / 124, 8 of 512 45 / 44, 16 of 400 44 / (58), 1 of 512 38 / 24; 8 heads, 6 of 720 -
     1780 139 / 105, 8 of 1024 102 / (118); 16 heads, 2 of 1000 79 / 67.  (More CTAs than SMs: 16 heads, 6 of 720 - 1780 225 / 181 in a graph by
-    themselves, but the gated mixer around them 361 / 362.)  Under 48 chunks they save less than the 7 us of host time that they take (8 heads, 6 of
-    210 - 690: 58 / 51).  Their length: short ones fill the chip from little work, long ones start seldom and add
-    fewer ends up (4 heads, 1 of 2048: 4 chunks 38, 8 35, 16 47; 16 heads, 1 of 8192: 8 chunks 321, 16 239, 32 239)."""
+    themselves, but the gated mixer around them 361 / 362; hardly fewer CTAs: 16 heads, 2 of 900 103 / 105 with the mixer, 2 of 1150 125 / 122.)
+    Under 48 chunks they save less than the 7 us of host time that they take (8 heads, 6 of 210 - 690: 58 / 51).  Their length: short ones fill the
+    chip from little work, long ones start seldom and add fewer ends up (4 heads, 1 of 2048: 4 chunks 38, 8 35, 16 47; 16 heads, 1 of 8192: 8
+    chunks 321, 16 239, 32 239)."""
     chunks, blocks = (longest + 15) // 16, H * -(-dv // 64)
     if rule == 1 or chunks < 48 or n_seqs * blocks > 148:
         return 0
     share = (n // 16 + n_seqs) * blocks / 148
-    return int(max(4 + share / 8, chunks / 32)) if chunks >= 2 * share else 0
+    return int(max(4 + share / 8, chunks / 32)) if chunks >= 2 * share + 8 else 0
+
+
+def split_segments_wait(rule: int, longest: int, n: int, H: int) -> bool:
+    """Whether a step of 48 chunks and more is better off without segments, which cost the host 6.5 us (a launch, a tensor): the mixer around
+    them takes the device less time in one piece than the host needs for it with segments, by the longest walk and, for what stands beside it,
+    the tokens and heads.  B200, bf16, 64 x 128 states, called from Python, us in one piece / in segments: gated, width 512, 1 of 760 77 / 84,
+    1000 78 / 85, 1300 93 / 85, 8 of up to 840 80 / 85, 940 90 / 85; width 1024, 1 of 1000 81 / 85, 1150 88 / 85, 2 of 900 84 / 85, 1000 90 / 86;
+    width 2048, 1 of 760 83 / 85, 900 93 / 86.  Attention beside retention, whose host side is longer: width 512, 1 of 1500 147 / 152, 2000 157 /
+    152, 4 of up to 1250 146 / 152, 1670 171 / 153; width 1024, 2 of 1150 147 / 154, 1300 162 / 153; width 2048, 1 of 1000 148 / 154, 1150 163 /
+    155."""
+    chunks = (longest + 15) // 16
+    return chunks >= 48 and (chunks + n * H * (37 + H) / 17000 < 128 if rule == 2 else chunks + n * H * (20 + H) / 20000 < 80)
 
 
 @functools.lru_cache(maxsize=None)
@@ -284,6 +297,8 @@ def _split_scan(rule: int, o, q, k, v, stride: int, beta, a, bias, rate, decay, 
     if ws is None:
         return False
     segment, ends = split_scan_segment(rule, longest, n, n_seqs, H, dv), None
+    if segment and split_segments_wait(rule, longest, n, H):
+        segment = 0
     if segment:
         try:
             ends = torch.empty((n // 16 + n_seqs) // segment * H * -(-dv // 64) * _end_floats(), dtype=torch.float32, device=q.device)
