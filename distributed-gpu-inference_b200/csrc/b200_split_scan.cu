@@ -514,7 +514,7 @@ split_prepare_kernel(const SplitArgs A) {
   __syncthreads();
   if (threadIdx.x == 0) {      // out by the copy engine
     const int64_t place_of = static_cast<int64_t>(blockIdx.x) * A.heads + blockIdx.y;
-    static_assert(sizeof(Ops<RULE>) % 16 == 0 && offsetof(Prep<RULE>, ops) == 0);
+    static_assert(sizeof(Ops<RULE>) % 16 == 0 && alignof(Ops<RULE>) % 16 == 0);      // what the copy asks of both ends
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(A.ops + place_of * static_cast<int64_t>(sizeof(Ops<RULE>))), "r"(smem_addr(&sm.ops)),
                  "n"(sizeof(Ops<RULE>)) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
