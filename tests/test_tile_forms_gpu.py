@@ -74,3 +74,40 @@ def test_more_tiles_than_a_grid_has_rows(n):
     s = (q[:, 0].to(F64) @ K.T * dk ** -0.5).masked_fill(torch.arange(3 * page, device="cuda")[None] > pos[:, None], float("-inf"))
     want = torch.softmax(s, 1) @ V
     assert ((out[:, 0].to(F64) - want).norm(dim=1) / want.norm(dim=1)).max() <= 12 * 2.0 ** -8      # as the rows above
+
+
+@pytest.mark.parametrize("out", ["16", "32", "off"], ids=["half", "float", "off_16_bytes"])
+@pytest.mark.parametrize("mode", ["plain", "bias", "cap"])
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_forms_of_256_rows(layout, mode, out):
+    """Full tiles, a second half with some rows, with one token and with none, one key tile and many."""
+    H, G, dk, dv, div = LAYOUTS[layout]
+    rep = H // G
+    cap, half = 256 // rep, 128 // rep
+    q, k_pool, v_pool, st, rnd = _case(LAYOUTS[layout], [(cap, 0), (2 * cap, 40), (half + half // 2, 100), (half + 1, 300), (half, 70), (half // 2, 0), (1, 9)], 16, torch.bfloat16)
+    n, scale = q.shape[0], dk ** -0.5
+    bias = rnd(H, 150) if mode == "bias" else None
+    kw = dict(softcap=4.0) if mode == "cap" else {}
+    gate = rnd(n, H * dv if mode == "cap" else H).to(torch.bfloat16)
+    wide = torch.full((n, H * dv + 4), 7.0, dtype=torch.float32 if out == "32" else torch.bfloat16, device="cuda")
+    o = wide[:, 2:2 + H * dv].unflatten(1, (H, dv)) if out == "off" else torch.empty(n, H, dv, dtype=wide.dtype, device="cuda")
+    mixer_ops.tile_attention(o, q, k_pool, v_pool, st.block_tables, st.prompt_tiles(1, cap)[0], st.tok_pos, scale, rows=256, gate=gate, bias_lut=bias, **kw)
+    want = _reference(q, k_pool, v_pool, st, dv, div, scale, bias=bias, gate=gate, **kw)
+    tol = 1.5 * 2.0 ** -8       # as above
+    assert (o.to(F64) - want).norm() / want.norm() <= tol
+    assert ((o.to(F64) - want).norm(dim=2) / want.norm(dim=2)).max() <= 8 * tol
+    if out == "off":
+        assert (wide[:, :2] == 7).all() and (wide[:, 2 + H * dv:] == 7).all()
+
+
+@pytest.mark.parametrize("rows", [128, 256])
+def test_queries_by_heads(rows):
+    """Queries whose heads lie further apart than their tokens: the same bits as side by side."""
+    H, G, dk, dv, _div = LAYOUTS["4x128"]
+    cap = rows // (H // G)
+    q, k_pool, v_pool, st, _rnd = _case(LAYOUTS["4x128"], [(2 * cap, 0), (cap + 3, 50)], 16, torch.bfloat16)
+    outs = []
+    for x in (q.contiguous(), q.transpose(0, 1).contiguous().transpose(0, 1)):
+        outs.append(torch.empty(q.shape[0], H, dv, dtype=torch.bfloat16, device="cuda"))
+        mixer_ops.tile_attention(outs[-1], x, k_pool, v_pool, st.block_tables, st.prompt_tiles(1, cap)[0], st.tok_pos, dk ** -0.5, rows=rows)
+    assert torch.equal(*outs)
