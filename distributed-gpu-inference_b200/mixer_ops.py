@@ -1261,12 +1261,16 @@ def router_logits(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
     return out
 
 
-@_timed
 def router_sigmoid_topk(x: torch.Tensor, w: torch.Tensor, top: int):
     """``sigmoid_topk(router_logits(x, w), top)``; up to eight experts in one launch, the logits not written."""
-    E = w.shape[0]
-    if E > 8 or top > E:
+    if w.shape[0] > 8 or top > w.shape[0]:
         return sigmoid_topk(router_logits(x, w), top)
+    return _router_sigmoid_topk(x, w, top)
+
+
+@_timed
+def _router_sigmoid_topk(x: torch.Tensor, w: torch.Tensor, top: int):
+    E = w.shape[0]
     _need_cuda(x, w)
     if w.dtype != torch.float32 or x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1] \
             or not x.is_contiguous() or not w.is_contiguous():

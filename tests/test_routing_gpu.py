@@ -36,3 +36,10 @@ def test_expert_order(n, E):
     want = torch.sort(key, stable=True).indices
     assert torch.equal(order, want) and torch.equal(where[order], torch.arange(n, device="cuda"))
     assert torch.equal(offsets.long(), torch.searchsorted(key[want], torch.arange(E + 1, device="cuda")))
+
+
+@pytest.mark.parametrize("E,launches", [(8, ["_router_sigmoid_topk"]), (12, ["router_logits", "sigmoid_topk"])])
+def test_every_launch_is_timed_once(E, launches, monkeypatch):
+    monkeypatch.setattr(mixer_ops, "EVENTS", [])
+    mixer_ops.router_sigmoid_topk(torch.randn(5, 64, device="cuda"), torch.randn(E, 64, device="cuda"), 2)
+    assert [name for name, _a, _b in mixer_ops.EVENTS] == launches
