@@ -300,6 +300,7 @@ MIXER_SIGNATURES = {
     "b200_tile_attn_rows": (c_int, [c_int] * 4),
     "b200_tile_attn_rows_ext": (c_int, [c_int] * 5),
     "b200_tile_attn_splits": (c_int, [c_int] * 5),
+    "b200_tile_attn_splits_ext": (c_int, [c_int] * 5 + [c_int64]),
     "b200_tile_attn": (
         c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p,
                 c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_float, c_float, c_float, c_int,

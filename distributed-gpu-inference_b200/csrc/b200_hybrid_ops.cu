@@ -1303,7 +1303,11 @@ int b200_tile_attn_rows_ext(int rep, int G, int dk, int n_tokens, int heavy) {
 }
 
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows) {
-  return tile_attn_splits(n_tiles, key_tiles, G, dk, tile_rows);
+  return tile_attn_splits(n_tiles, key_tiles, G, dk, tile_rows, static_cast<int64_t>(n_tiles) * tile_rows * G);
+}
+
+int b200_tile_attn_splits_ext(int n_tiles, int key_tiles, int G, int dk, int tile_rows, int64_t live_rows) {
+  return tile_attn_splits(n_tiles, key_tiles, G, dk, tile_rows, live_rows);
 }
 
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,

@@ -964,7 +964,9 @@ bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, in
 // 256 rows share a fetched key tile and its biases and take turns with the exponentials; 128 rows have shorter beginnings and less of the causal
 // triangle to mask.  With biases or a cap 256 rows are ahead where heads share their keys and there is more than an SM's CTA and a half of 128 (16
 // over 4, 8 x 2048: 206 / 242 us against 241 / 285; 6 x 300 .. 640: 24 / 27 against 28 / 32; but 4 over 1, 8 x 700: 27 against 21 of plain
-// scores), 128 where they do not share (16 over 16, 8 x 700: 60 / 67 against 64 / 70; 64 x 96: 50 / 53 against 73 / 73).  Plain scores keep 128 rows.
+// scores), 128 where they do not share (16 over 16, 8 x 700: 60 / 67 against 64 / 70; 64 x 96: 50 / 53 against 73 / 73).  Plain scores keep 128 rows:
+// ahead for short portions (16 over 4, 128 / 256 rows: 32 x 512 84 / 91, 8 x 700 38 / 39; 16 over 16 95 / 111, 48 / 55), behind for long ones
+// (16 over 4, 8 x 2048 188 / 184, 4 x 4000 314 / 297; 8 over 2 of 64, 8 x 2048 89 / 78), whose length the rule is not told.
 // Pages that come row by row keep 256 rows from one round of CTAs on with biases or a cap, from three without (8 x 1000 tokens of 16 heads, pages
 // of 24: 82 us against 94 when the line was drawn; 79 now).
 int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy, bool boxes) {
@@ -976,19 +978,26 @@ int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy, bool boxes)
 }
 
 // Keys are divided while the chip has room for more CTAs, a share being worth its part of the merge: three tiles of 64 keys where
-// few rows are merged, eight otherwise.  Room is one CTA per SM, whose form is ahead (4 heads with keys of their own, 8 x 64 tokens behind 1000: 4 shares
-// 20.8 us, 5, two per SM, 23.5; 4 over 1, 1000 behind 6000: 4 shares 47.6, 9 51.9; 16 over 4, 1 x 1024: undivided 51, in two 54), unless that
-// leaves a CTA more than 48 key tiles: then two CTAs per SM walk faster together (8 over 2 of 64, 1000 behind 6000, 64 CTAs: 2 shares of 55 tiles
-// 71 us, 4 59; at 36 tiles, 16 heads, 512 behind 4000, 2 shares 55, 4 64).
-int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int rows) {
+// few rows are merged, eight otherwise.  Room is one CTA per SM or two, whose walks are half as slow again each; which, by the sum of a walk and
+// its merge, in microseconds of a key tile: 0.7 ns for every share of a live row of 128 values, 2 for the launch.  Full tiles keep an SM each (16
+// heads over 4, 1 x 1024: undivided 18 us, in two 52; 8 x 64 tokens of 4 heads with keys of their own behind 1000: 4 shares 20.8, 5, two per SM,
+// 23.5) unless the walks are long (8 over 2 of 64, 1000 behind 6000: 2 shares 71, 4 59); few tokens are soon merged (4 heads with keys of their own, 20
+// x 4 tokens behind 3000: undivided 57, 3 shares 42; 8 x 2 behind 8000: 4 shares 45, 9 39).  Over 490 shapes and modes 0.4 % behind the better of the two.
+int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int rows, int64_t live_rows) {
   const int64_t ctas = static_cast<int64_t>(n_tiles) * G;
   auto divide = [&](int64_t room) {
     if (ctas <= 0 || ctas * 2 > room) return 1;
     const int share = ctas * rows <= 4096 ? 3 : 8;
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({16, room / ctas, key_tiles / share})));
   };
+  auto cost = [&](int splits) {
+    const double walk = static_cast<double>(key_tiles) / splits * (splits * ctas > kNumSMs ? 1.5 : 1.0);
+    return splits == 1 ? walk : walk + 2.0 + 0.0007 * static_cast<double>(live_rows) * splits * dk / 128;
+  };
   const int one_per_sm = divide(kNumSMs);
-  return rows == kTileRows && dk <= 128 && key_tiles > 48 * one_per_sm ? divide(2 * kNumSMs) : one_per_sm;
+  if (rows != kTileRows || dk > 128) return one_per_sm;
+  const int two_per_sm = divide(2 * kNumSMs);
+  return cost(two_per_sm) < cost(one_per_sm) ? two_per_sm : one_per_sm;
 }
 
 int tile_attn_launch(const TileAttn& A, int dk, int dv, bool alias, int rows, int n_tiles, int n_splits, int dtype, cudaStream_t stream) {

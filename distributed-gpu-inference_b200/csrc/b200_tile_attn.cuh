@@ -30,7 +30,7 @@ struct TileAttn {
 
 bool tile_attn_supported(int H, int G, int dk, int dv, bool alias, bool bias, int dtype);
 int tile_attn_rows(int rep, int G, int dk, int n_tokens, bool heavy, bool boxes);   // heavy: distance biases or a soft cap
-int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int rows);
+int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int rows, int64_t live_rows);   // live: tokens x heads of all tiles
 int tile_attn_launch(const TileAttn& A, int dk, int dv, bool alias, int rows, int n_tiles, int n_splits, int dtype, cudaStream_t stream);
 
 }  // namespace b200

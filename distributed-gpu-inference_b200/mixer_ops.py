@@ -779,7 +779,8 @@ def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_p
     seen = min(max_context, window + keep_first + 128) if window > 0 else max_context
     if chunk > 0:
         seen = min(seen, chunk + 128)
-    splits = lib.b200_tile_attn_splits(tiles.shape[0], (seen + 63) // 64, G, dk, int(rows)) if max_context > 0 else 1
+    # (tokens of the step's other portions among the live rows: at most what the tiles hold)
+    splits = lib.b200_tile_attn_splits_ext(tiles.shape[0], (seen + 63) // 64, G, dk, int(rows), min(n * H, tiles.shape[0] * int(rows) * G)) if max_context > 0 else 1
     if H * dv * 4 > 227 * 1024:     # more than the merge of splits holds
         splits = 1
     ws = torch.empty((splits, tiles.shape[0] * (rows // (H // G)), H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None

@@ -496,7 +496,7 @@ int b200_mixed_prompt_attn_ext3(void* out, int64_t out_tok_stride, int64_t out_h
 /* b200_mixed_prompt_attn_ext2 and b200_biased_prompt_attn for prompt portions on the fifth-generation tensor cores: tiles of up to
  * tile_rows / (H / G) tokens (int32 [n_tiles][3] = first packed row, tokens, row of the block table); tokens outside the tiles are not
  * touched.  tile_rows: 128 or (dk <= 128) 256; b200_tile_attn_rows_ext picks for n_tokens tokens, heavy = 1 with distance biases or a
- * soft cap, + 2 with pages other than 8, 16, 32 or 64 tokens (b200_tile_attn_rows: heavy = 0, for which 128 is ahead at every size).
+ * soft cap, + 2 with pages other than 8, 16, 32 or 64 tokens (b200_tile_attn_rows: heavy = 0, which always takes 128).
  * bias_lut fp32 [H][lut_len] with temp_coef / temp_every as in b200_biased_prompt_attn, or NULL.  The values are v_pool's
  * rows, or the first dv columns of the key rows when v_pool == k_pool.  n_splits > 1 divides the keys over as many CTAs and needs a
  * workspace fp32 [n_splits][n_tiles][tile_rows / (H / G)][H][dv + 2].  16-bit types, the sizes b200_tile_attn_supported names, 16-byte
@@ -505,6 +505,8 @@ int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bi
 int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens);
 int b200_tile_attn_rows_ext(int rep, int G, int dk, int n_tokens, int heavy);
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows);
+/* ... with tiles that are not full: live_rows = tokens x heads of all of them */
+int b200_tile_attn_splits_ext(int n_tiles, int key_tiles, int G, int dk, int tile_rows, int64_t live_rows);
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,
                    const int32_t* block_tables, int table_stride, const int32_t* tiles, int n_tiles, int tile_rows, const int32_t* tok_pos,
