@@ -11,7 +11,7 @@ worker/requirements.txt:3 — the Llama decoder layer that ``ModelShard.forward`
 algorithm is restated in ``oracle/llama_ref.py`` and anchored on the reference's call site
 (worker/distributed/model_shard.py:205-222).
 
-Pinning (oracle/make_golden.py, run in the build container where /root/reference is mounted):
+Pinning (oracle/make_golden.py, run where the reference's tree is mounted):
   * host logic — layer ranges, allocator schedules, prefix hashes, wire headers, serializer outputs — is pinned
     against outputs of the reference's own code (imported unmodified) and the reference's own test vectors;
   * the decoder-layer restatement is pinned by driving the reference's unmodified ``ModelShard.forward`` /
@@ -23,8 +23,8 @@ Pinning (oracle/make_golden.py, run in the build container where /root/reference
     ``index_select``-packed blocks.
 Fixtures live in tests/golden/.
 
-``oracle/_ref/`` (git-ignored, built by ``oracle/build_ref.py`` / ``__graft_entry__.build()`` where /root/reference is
-mounted, carried to the GPU box with the snapshot) holds the reference's own modules of the path as bytecode compiled
+``oracle/_ref/`` (git-ignored, built by ``oracle/build_ref.py`` / ``__graft_entry__.build()`` where the reference's
+tree is mounted, carried along with the built libraries) holds the reference's own modules of the path as bytecode compiled
 from the sources where they lie; ``oracle/ref_loader.py`` imports them.  With it the pinning above is re-checked
 against the reference itself wherever the suite runs (tests/test_reference_bytecode.py), and the timed CPU legs run
 the reference's own ``ModelShard.forward`` (``cpu_baseline.kind = "reference"``).

@@ -2,14 +2,13 @@
 """Recipe for ``oracle/_ref/``: the reference's own modules of this path, byte-compiled WHERE THEY LIE.
 
 The reference is pure Python, so "compiling it from its own source files" is ``py_compile``: each module below is
-compiled straight from ``/root/reference/<path>`` into ``oracle/_ref/<name>.bin`` (a .pyc under another suffix: the
-snapshot that carries the tree to the GPU box leaves ``*.pyc`` behind).  Only compiler output lands in
+compiled straight from ``/root/reference/<path>`` into ``oracle/_ref/<name>.bin`` (a .pyc under another suffix: copies
+of the tree leave ``*.pyc`` behind).  Only compiler output lands in
 the repository tree (no source is copied), ``oracle/_ref/`` is git-ignored, and — like the built ``.so`` — it travels
-to the GPU box with the snapshot, where ``/root/reference`` does not exist.  ``oracle/ref_loader.py`` imports the
+to machines where ``/root/reference`` does not exist.  ``oracle/ref_loader.py`` imports the
 bytecode; it is used by
 
-  * ``tests/test_reference_bytecode.py`` — the oracle restatements against the reference's own code, also on the GPU
-    box;
+  * ``tests/test_reference_bytecode.py`` — the oracle restatements against the reference's own code, also there;
   * ``bench.py``'s ``cpu_baseline`` / ``--impl reference`` legs — ``ModelShard.forward`` / ``get_logits`` of the
     reference itself drive the timed CPU path (``kind = "reference"``).
 

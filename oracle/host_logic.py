@@ -42,7 +42,7 @@ def blocks_for(seq_len: int, block_size: int) -> int:
 
 
 def slot_mapping(block_table: List[int], positions: List[int], block_size: int) -> List[int]:
-    """Device-side addressing derived in SURVEY.md §8(a): slot = table[t // bs] * bs + t % bs."""
+    """Device-side addressing: slot = table[t // bs] * bs + t % bs."""
     return [block_table[t // block_size] * block_size + t % block_size for t in positions]
 
 

@@ -19,7 +19,7 @@ Two pieces:
    needed at all; oracle/make_golden.py checks it token-exactly against transformers' ``generate()``.
 
 2. ``RefShard`` — restates ``ModelShard.forward`` / ``get_logits`` (worker/distributed/model_shard.py:173-246)
-   so the oracle also runs where /root/reference is not mounted (the GPU box).  make_golden.py drives the
+   so the oracle also runs where the reference's tree is not mounted.  make_golden.py drives the
    reference's unmodified class with the same layers and checks both agree bit for bit.
 """
 from __future__ import annotations

@@ -1,6 +1,6 @@
-"""Generate tests/golden/*.json from the REFERENCE ITSELF (run in the build container only).
+"""Generate tests/golden/*.json from the REFERENCE ITSELF (run where its tree is mounted).
 
-Usage:  python oracle/make_golden.py            (needs /root/reference mounted; the GPU box has no such path)
+Usage:  python oracle/make_golden.py            (needs /root/reference mounted)
 
 The reference is imported unmodified from /root/reference (read-only).  Two shims are needed to run it here and
 both are confined to this script:
@@ -219,7 +219,7 @@ def gen_serializer() -> None:
 
 # ---------------------------------------------------------------------------------------------------------
 def gen_tiny_decode(num_layers: int = 4, n_shards: int = 2, out_name: str = "tiny_decode.json") -> None:
-    """tiny 4-layer model, 2 reference ModelShards, batch 4, prompt 128, 64 greedy tokens.
+    """Tiny 4-layer model, 2 reference ModelShards, batch 4, prompt 128, 64 greedy tokens.
     (``num_layers=8, n_shards=8``: the same model twice as deep, one layer per reference ModelShard — the fixture
     an 8-rank pipeline is checked against.)"""
     torch.manual_seed(0)

@@ -1,6 +1,6 @@
 """Oracle (test infrastructure): torch restatement of the paged-KV device ops on whatever device the inputs are.
 
-The reference has no paged append / attention / pack (last paragraph); it only fixes the pool
+The reference has no paged append / attention / pack; it only fixes the pool
 layout ``[max_blocks, heads, block_size, head_dim]`` (worker/distributed/kv_cache.py:130-144) and copies whole
 blocks in ``_promote_to_gpu`` (:447-462).  These functions define the device ops in terms of torch indexing on
 that layout, which is what the CUDA kernels must reproduce:

@@ -1,6 +1,6 @@
 """GPU parity of the whole layer-range decode path: product ModelShards over paged KV (CUDA kernels through the
 C ABI) against (a) the golden tokens produced by the reference's own ModelShard.forward (tests/golden/
-tiny_decode.json, BASELINE config 1) and (b) the oracle's dense path run on the same device and dtype."""
+tiny_decode.json) and (b) the oracle's dense path run on the same device and dtype."""
 import pytest
 import torch
 
@@ -125,7 +125,7 @@ def test_batch_inference_protocol_of_the_reference_batcher(golden):
 
 
 def test_8b_shape_bf16_paged_path_vs_reference_dense_path():
-    """BASELINE config 2's shape (d 4096, 32 q / 8 kv heads, head_dim 128, ffn 14336, vocab 128256) cut to 4 layers,
+    """The 8B shape (d 4096, 32 q / 8 kv heads, head_dim 128, ffn 14336, vocab 128256) cut to 4 layers,
     bf16, batch 8, prompt 300, 24 greedy tokens: the paged CUDA path against the reference recipe (oracle dense
     path) on the same GPU, same weights.  Divergences are only accepted at near-ties of the reference's logits."""
     shape = dict(L.LLAMA3_8B)

@@ -1,6 +1,6 @@
 """GPU parity: the CUDA kernels, called through the C ABI, against the oracle (oracle/paged_ref.py) on the same
 seeded inputs.  Bit-exact for append / pack / unpack (byte movers); attention within 1e-2 of the fp32 formula
-(north_star tolerance for bf16), and much tighter for fp32 storage."""
+(the tolerance asked for bf16), and much tighter for fp32 storage."""
 import pytest
 import torch
 
@@ -169,7 +169,7 @@ def _attn_case(B, Hq, Hkv, D, bs, ctx_lens, dtype, seed, share_prefix_blocks=0, 
 
 
 def _rel_err(got, want):
-    # per (sequence, head): max |delta| / max |ref|  (SURVEY.md Appendix B parity definition)
+    # per (sequence, head): max |delta| / max |ref|
     num = (got.float() - want.float()).abs().amax(dim=-1)
     den = want.float().abs().amax(dim=-1).clamp_min(1e-6)
     return (num / den).max().item()
@@ -267,7 +267,7 @@ def test_attention_strided_q_and_prefix_sharing():
 
 
 def test_attention_split_invariance_and_linearity_large():
-    # size-independent properties at a BASELINE-size context (32k): the split count must not change the answer
+    # size-independent properties at a context of the benchmark's size (32k): the split count must not change the answer
     # beyond fp32 re-association, and attention is linear in V.
     B, Hq, Hkv, D, bs = 2, 32, 8, 128, 16
     q, k_pool, v_pool, tables, lens = _attn_case(B, Hq, Hkv, D, bs, [32768, 30000], torch.bfloat16, seed=17)

@@ -1,6 +1,6 @@
 """CPU: tiered KV manager and allocator behaviours the reference's tests describe
 (tests/test_worker_distributed_kv_cache.py:218-290, 329-343, 397-412, 459-496) — run here on CPU pools, which the
-reference itself cannot create (SURVEY.md §9 #1)."""
+reference itself cannot create."""
 import asyncio
 
 import pytest

@@ -44,7 +44,7 @@ def test_migrate_updates_index_dedups_and_reports_failure():
 
 def _reference_pd_scheduler():
     """The reference's own scheduler module: bytecode compiled from server/app/services/pd_scheduler.py by
-    oracle/build_ref.py (it travels to the GPU box; built here on first use when /root/reference is mounted)."""
+    oracle/build_ref.py (it travels with the tree; built on first use where the reference's is mounted)."""
     import os
 
     from oracle import build_ref, ref_loader

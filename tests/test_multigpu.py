@@ -421,7 +421,7 @@ def test_70b_shape_bf16_pipeline_of_two_processes_on_one_gpu_vs_reference_recipe
 
 
 def _pd_worker(rank, world, port, q):
-    """BASELINE config 3 in miniature: rank 0 runs the prompt pass, ships every sequence's KV blocks to rank 1,
+    """The prefill -> decode hand-off in miniature: rank 0 runs the prompt pass, ships every sequence's KV blocks to rank 1,
     rank 1 decodes.  Tokens must equal the reference's (golden) tokens for the same prompts."""
     import sys
     sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))

@@ -71,7 +71,7 @@ def test_prefix_hash(golden):
         assert H.prefix_hash(toks) == want
         assert ds.compute_prefix_hash(toks) == want
         assert kv.DistributedKVCacheManager.compute_prefix_hash(None, toks) == want
-    assert ds.compute_prefix_hash([1, 2, 3, 4, 5]) == "74f81fe167d99b4c"  # SURVEY.md §8 a8 probe
+    assert ds.compute_prefix_hash([1, 2, 3, 4, 5]) == "74f81fe167d99b4c"  # as the reference gives it
     assert g["prefix_hash_raises_for_256"]
     with pytest.raises(ValueError):
         ds.compute_prefix_hash([256])

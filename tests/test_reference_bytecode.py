@@ -1,5 +1,5 @@
-"""CPU: the reference's OWN code (oracle/_ref/*.bin, byte-compiled from /root/reference by oracle/build_ref.py and
-carried to the GPU box with the snapshot) against the committed fixtures, the oracle restatements and the product's
+"""CPU: the reference's OWN code (oracle/_ref/*.bin, byte-compiled from its tree by oracle/build_ref.py and
+carried along) against the committed fixtures, the oracle restatements and the product's
 host logic.  Where the fixtures pin the oracle to reference outputs recorded once, these tests re-run the reference
 itself, wherever the suite runs."""
 import os
@@ -106,7 +106,7 @@ def test_prefix_hash_and_stream_header_reference_vs_product(ref):
         assert prod_hash(None, ids) == want and H.prefix_hash(ids) == want
         assert ref["data_structures"].compute_prefix_hash(ids) == want  # the second definition, data_structures.py:293
     assert ref_hash(None, [1, 2, 3, 4, 5]) == "74f81fe167d99b4c"
-    with pytest.raises(ValueError):  # bytes() of an id >= 256: the reference's limit (SURVEY §9 #7)
+    with pytest.raises(ValueError):  # bytes() of an id >= 256: the reference's limit
         ref_hash(None, [256])
     for shape, dtype in (((2, 3), "bfloat16"), ((7,), "float16"), ((1, 2, 3, 4), "int64"), ((5, 5), "no_such_dtype")):
         want = ref["serialization"].StreamingTensorBuffer().write_header(shape, dtype)

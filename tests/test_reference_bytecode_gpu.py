@@ -109,11 +109,11 @@ def test_the_references_own_batcher_drives_the_paged_engine(ref, golden):
 
 @pytest.mark.parametrize("graphs", [False, True])
 def test_the_references_own_model_shard_forward_runs_the_paged_layers(ref, golden, graphs):
-    """SURVEY §8b seam 2, literally: the reference's unmodified ``ModelShard`` objects (bytecode of
+    """The reference's unmodified ``ModelShard`` objects (bytecode of
     worker/distributed/model_shard.py) hold this repository's paged decoder layers in their ``layers`` list; their own
     ``forward`` loop (:193-228) calls each layer with the legacy keyword signature and passes ``past_key_values[i]``
     through untouched — here the paged KV handle — and their own ``get_logits`` closes the step.  Two layer-range
-    shards: the golden tokens."""
+    shards of the tiny 4-layer model: the golden tokens."""
     from dgi_b200.engine import PagedDecodeEngine
 
     g = golden("tiny_decode.json")
@@ -143,10 +143,10 @@ def test_the_references_own_model_shard_forward_runs_the_paged_layers(ref, golde
 
 
 def test_the_references_own_session_steps_through_the_paged_servicers(ref, golden):
-    """SURVEY §8b seam 1 + 3, literally: the reference's own ``DistributedInferenceSession.step`` loop
+    """The reference's own ``DistributedInferenceSession.step`` loop
     (worker/distributed/session.py:271-337, bytecode) with ``WorkerSession`` swapped the way its tests swap it, two
     hops, each an ``InferenceServicer`` of this package over a layer-range shard and paged per-session KV: the golden
-    tokens of BASELINE config 1, positions and retries counted by the reference's code."""
+    tokens of the tiny 4-layer model, positions and retries counted by the reference's code."""
     from dgi_b200.worker.distributed import session as prod_session
     from dgi_b200.worker.distributed.kv_cache import DistributedKVCacheManager
     from dgi_b200.worker.distributed.servicer import InferenceServicer, ServicerTransport

@@ -1,6 +1,5 @@
 """The reference's OWN test files for the hot path, run against this package (tools/run_reference_tests.py aliases
-``worker.distributed.*`` / ``common.*`` to ``dgi_b200.*``).  Needs the reference checkout, so it runs in the build
-container and is skipped on the GPU box."""
+``worker.distributed.*`` / ``common.*`` to ``dgi_b200.*``).  Needs the reference checkout, and is skipped where there is none."""
 import os
 import subprocess
 import sys

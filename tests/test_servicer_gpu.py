@@ -1,7 +1,7 @@
 """GPU: the reference's own call stack for this path, end to end WITH a cache — DistributedInferenceSession.step →
 WorkerSession.forward → (transport) → InferenceServicer.Forward → _forward → ModelShard.forward over the session's
 paged KV (reference: worker/distributed/session.py:271-337, grpc_server.py:142-188,351-374) — must reproduce the
-golden tokens of the reference's ModelShard pair (BASELINE config 1)."""
+golden tokens of the reference's ModelShard pair."""
 import asyncio
 
 import pytest

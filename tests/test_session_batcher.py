@@ -89,7 +89,7 @@ def test_retry_counter_and_length_guard_and_failure():
 
 
 def test_session_manager_cleanup_does_not_deadlock():
-    # the reference hangs here forever (SURVEY.md §4): create_session holds the lock and re-enters close_session
+    # the reference hangs here forever: create_session holds the lock and re-enters close_session
     async def run():
         with patch(f"{MOD}.WorkerSession", _Fake):
             mgr = S.SessionManager(max_sessions=1)

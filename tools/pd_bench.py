@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""P/D KV hand-off benchmark (BASELINE config 3): 8B-shape, 4k-token prompts = 256 blocks x 32 layers x 64 KiB =
+"""P/D KV hand-off benchmark: 8B-shape, 4k-token prompts = 256 blocks x 32 layers x 64 KiB =
 512 MiB per sequence, prefill rank i -> decode rank i + N/2 over NVLink.  Run under torchrun with an even N.
 
 Reports, per pair (max over the pair's two ranks, CUDA-event timed between barriers) and aggregated over pairs:

@@ -1,6 +1,5 @@
 #!/usr/bin/env python
-"""Run the REFERENCE's own test files for the hot path against THIS package (drop-in check; build container only —
-/root/reference does not exist on the GPU box).
+"""Run the REFERENCE's own test files for the hot path against THIS package (drop-in check; needs the reference's tree).
 
 The reference's tests import ``worker.distributed.kv_cache``, ``common.serialization`` …; those names are aliased to
 ``dgi_b200.worker.distributed.kv_cache`` … before pytest collects, so every assertion the reference makes about its
