@@ -631,7 +631,7 @@ int attn_prefix(const AttnArgs& a, int dtype, int prefix_blocks, int prefix_spli
   // Who merges: a separate combine launch (attn_combine_kernel, a programmatic dependent of this grid, so its launch
   // latency hides behind the attention CTAs).  Merging inside the kernel by the last-arriving CTA of each row was
   // the better choice for short prefix runs before the combine became a dependent launch; measured again afterwards
-  // on B200 (tools/prefix_merge_probe.py, profiles/r02_prefix_merge_probe.jsonl, counters vouched for): the separate
+  // on B200 (profiles/r02_prefix_merge_probe.jsonl, counters vouched for): the separate
   // launch wins at every shape tried — 8 x (512 + 64): 17.5 vs 24.6 us, 64 x (2048 + 176): 41.0 vs 43.7 us,
   // config 5: 72.3 vs 80.4 us — because the rows of a CTA are merged by whichever CTA finishes last, at the very end
   // of the launch, with nothing left to overlap.  B200_PREFIX_SEPARATE_COMBINE=0 still selects the in-kernel merge.

@@ -22,8 +22,9 @@
 // 7.0e-8; delta 1.31e-7 / 1.29e-7, 8.2e-8 / 8.1e-8; retention 3.8e-7 / 1.2e-7, 4.2e-7 / 1.1e-7.
 //
 // What bounds it.  The chain: latency - a chunk takes a lone warp per scheduler 1550 clocks (gated) and 2450 (delta) for 78 and 168
-// products of 8 clocks each, between which its conversions (two clocks each) stand; the CTAs of an SM overlap (three of them: 1250 clocks a
-// chunk, products 47 % of the time, issue slots as much).  Two warps per 16 columns, bulk copies and packed fp32 arithmetic were each slower.  Where
+// products of 8 clocks each, between which its conversions (two clocks each) stand; the CTAs of an SM overlap (three of the segments' kernel, at 8 x
+// 2048 tokens of 16 heads, which run in one piece but for that measurement: 1250 clocks a chunk, products 47 % of the time, issue slots as
+// much).  Two warps per 16 columns, bulk copies and packed fp32 arithmetic were each slower.  Where
 // sequences and heads leave SMs idle the gated and the retention rule walk segments of a sequence at the same time (split_chain_kernel).  The
 // operands: issue slots and accesses to shared memory, three quarters of both, at eight CTAs per SM.
 // B200, bf16, 64 x 128 states, us token by token / here (operands + chain): gated, 6 portions of up to 1780 tokens of 16 heads 395 / 212

@@ -20,10 +20,10 @@
 // other half's; the tensor cores need 1280, the exponentials alone 1024), and 9000 clocks of a CTA's beginning and end (of 22000: a row of the output
 // written by one thread took 5000, queries in 16-byte pieces 5000, code of modes that a launch does not use two to eight thousand in instruction
 // misses).  Rescaling by the softmax itself: 2900 clocks per tile.  Issue slots are taken 45 % of the time: what is no maximum, exponential or load goes two at a time
-// (without: a tenth more instructions, 223 us against 217 in the mixer).
-// Measured on B200 (bf16, us, before these / now): 8 x 2048 tokens, 16 heads over 4 kv heads of 128, plain 209 / 198, window of 512 138 / 123, with distance
-// biases, query temperature and gate 277 / 205 (before biases went two at a time), soft cap 319 / 242; 5 x 1024 with a cap under a window of 512 51 / 31; latent 320 / 256, 4 portions of up to
-// 1500 tokens of 16 heads behind 700, window 512: 91 / 68; 319 shapes of 4 .. 16 heads, 1.29 times on average.
+// (without: a tenth more instructions, 3 % of the biased kernel's time).
+// Measured on B200 (bf16, us, before these / now, the kernel by itself): 8 x 2048 tokens, 16 heads over 4 kv heads of 128, plain 211 / 189, window of 512
+// 139 / 117, with distance biases, query temperature and gate 278 / 198, soft cap 319 / 238; 5 x 1024 with a cap under a window of 512 60 / 45; latent 320
+// / 256, 4 portions of 700 .. 1500 tokens of 16 heads behind 700, window 512: 98 / 76; 364 shapes and kinds of scores 0.87 times on average.
 // Portions smaller than a tile have walks of one or two key tiles, which wait for instructions: 16 heads with keys of their own, plain, 64 x 96 tokens
 // 41 / 41, 128 x 40 54 / 55, 256 x 20 102 / 102 (44, 61 and 116 with a loop for each way pages come and a loop for each form of the output in
 // the kernel, a division for a CTA's place, barriers of the rescaling warps where there are none, and rows of no token written to shared memory).
