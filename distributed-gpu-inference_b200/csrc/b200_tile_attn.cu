@@ -990,9 +990,10 @@ int tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int rows, int64_
     const int share = ctas * rows <= 4096 ? 3 : 8;
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>({16, room / ctas, key_tiles / share})));
   };
+  const int64_t live = std::min(live_rows, ctas * rows);      // (the call's tokens may have other portions among them)
   auto cost = [&](int splits) {
     const double walk = static_cast<double>(key_tiles) / splits * (splits * ctas > kNumSMs ? 1.5 : 1.0);
-    return splits == 1 ? walk : walk + 2.0 + 0.0007 * static_cast<double>(live_rows) * splits * dk / 128;
+    return splits == 1 ? walk : walk + 2.0 + 0.0007 * static_cast<double>(live) * splits * dk / 128;
   };
   const int one_per_sm = divide(kNumSMs);
   if (rows != kTileRows || dk > 128) return one_per_sm;

@@ -779,14 +779,14 @@ def tile_attention(out: torch.Tensor, q: torch.Tensor, k_pool: torch.Tensor, v_p
     seen = min(max_context, window + keep_first + 128) if window > 0 else max_context
     if chunk > 0:
         seen = min(seen, chunk + 128)
-    # (tokens of the step's other portions among the live rows: at most what the tiles hold)
-    splits = lib.b200_tile_attn_splits_ext(tiles.shape[0], (seen + 63) // 64, G, dk, int(rows), min(n * H, tiles.shape[0] * int(rows) * G)) if max_context > 0 else 1
+    n_tiles, rows = tiles.shape[0], int(rows)
+    splits = lib.b200_tile_attn_splits_ext(n_tiles, (seen + 63) // 64, G, dk, rows, n * H) if max_context > 0 else 1
     if H * dv * 4 > 227 * 1024:     # more than the merge of splits holds
         splits = 1
-    ws = torch.empty((splits, tiles.shape[0] * (rows // (H // G)), H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
+    ws = torch.empty((splits, n_tiles * (rows // (H // G)), H, dv + 2), dtype=torch.float32, device=q.device) if splits > 1 else None
     rc = lib.b200_tile_attn(out.data_ptr(), out.stride(0), out.stride(1), q.data_ptr(), q.stride(0), q.stride(1), _ptr(gate),
                             _rows2(gate) if gate is not None else 0, per_channel, k_pool.data_ptr(), v_pool.data_ptr(),
-                            block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), tiles.shape[0], int(rows), tok_pos.data_ptr(),
+                            block_tables.data_ptr(), block_tables.stride(0), tiles.data_ptr(), n_tiles, rows, tok_pos.data_ptr(),
                             _ptr(sink), _ptr(bias_lut), bias_lut.shape[1] if bias_lut is not None else 0, float(scale), float(softcap),
                             float(temp_coef), int(temp_every), int(window), int(keep_first), int(chunk), H, G, dk, dv, v_row,
                             int(value_div), int(out.dtype == torch.float32), bs, int(splits), _ptr(ws), DTYPE_ID[q.dtype], _stream())

@@ -505,7 +505,7 @@ int b200_tile_attn_supported(int H, int G, int dk, int dv, int same_pool, int bi
 int b200_tile_attn_rows(int rep, int G, int dk, int n_tokens);
 int b200_tile_attn_rows_ext(int rep, int G, int dk, int n_tokens, int heavy);
 int b200_tile_attn_splits(int n_tiles, int key_tiles, int G, int dk, int tile_rows);
-/* ... with tiles that are not full: live_rows = tokens x heads of all of them */
+/* ... with tiles that are not full: live_rows = tokens x heads of all of them, or more */
 int b200_tile_attn_splits_ext(int n_tiles, int key_tiles, int G, int dk, int tile_rows, int64_t live_rows);
 int b200_tile_attn(void* out, int64_t out_tok_stride, int64_t out_head_stride, const void* q, int64_t q_tok_stride, int64_t q_head_stride,
                    const void* gate, int64_t gate_stride, int gate_per_channel, const void* k_pool, const void* v_pool,

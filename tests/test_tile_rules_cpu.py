@@ -17,7 +17,7 @@ from dgi_b200 import _lib
 def test_shares_of_a_walk(n_tiles, key_tiles, G, dk, rows, splits):
     lib = _lib.load_mixers()
     assert lib.b200_tile_attn_splits(n_tiles, key_tiles, G, dk, rows) == splits
-    assert lib.b200_tile_attn_splits_ext(n_tiles, key_tiles, G, dk, rows, n_tiles * rows * G) == splits
+    assert lib.b200_tile_attn_splits_ext(n_tiles, key_tiles, G, dk, rows, n_tiles * rows * G + 100000) == splits
 
 
 @pytest.mark.parametrize("n_tiles,key_tiles,G,dk,live,splits", [
